@@ -169,6 +169,7 @@ def port_gerschgorin(rp, ci, v):
 
 def port_solve(rp, ci, v, B, X0, s, eps, bounds=None, maxit=100):
     """Returns (X, iterations, history of ||R(:,0)||)."""
+    rp, ci = np.ascontiguousarray(rp, np.int32), np.ascontiguousarray(ci, np.int32)
     B = np.ascontiguousarray(B, np.float64)
     X = np.array(X0, np.float64, order="C", copy=True)
     n, m = B.shape
