@@ -193,6 +193,13 @@ int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl
                 double *C1, int ldc1, double *C2, int ldc2, double *ws, size_t ws_bytes,
                 bool symmetric = false);
 size_t gram_workspace_bytes(int64_t n, int ka, int kb);
+// FP64 Gram from fp16 digit planes on tcgen05 (k_gram_x64.cu); launch_gram takes
+// it for CACG_GRAM_AUTO.  CACG_ERR_UNSUPPORTED: shape or workspace not for it.
+int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
+                    const double *R1, int64_t ldr1, int kb1, const double *R2, int64_t ldr2,
+                    int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
+                    size_t ws_bytes);
+size_t gram_x64_workspace_bytes(int64_t n, int ka, int kb);
 
 // dst = src for an n x w FP32 block (rows of lds / ldd values)
 int launch_copy_rows_f32(cudaStream_t st, int64_t n, int w, const float *src, int64_t lds,

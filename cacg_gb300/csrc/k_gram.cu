@@ -418,7 +418,7 @@ size_t gram_workspace_bytes(int64_t n, int ka, int kb) {
         size_t b2 = (size_t)q.nchunks * q.tilesA * q.tilesB * q.BA * q.BB * sizeof(double);
         best = std::max(best, std::max(b1, b2));
     }
-    return best;
+    return std::max(best, gram_x64_workspace_bytes(n, ka, kb));
 }
 
 template <typename T>
@@ -430,6 +430,13 @@ int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl
     if (ka <= 0 || kb <= 0 || n < 0 || !C1 || (kb2 > 0 && !C2)) return CACG_ERR_ARG;
     if (variant != CACG_GRAM_AUTO && variant != CACG_GRAM_FMA && variant != CACG_GRAM_DMMA)
         return CACG_ERR_UNSUPPORTED;
+    if constexpr (std::is_same<T, double>::value) {
+        if (variant == CACG_GRAM_AUTO) {
+            const int rc = launch_gram_x64(st, n, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1,
+                                           ldc1, C2, ldc2, ws, ws_bytes);
+            if (rc != CACG_ERR_UNSUPPORTED) return rc;
+        }
+    }
     if (variant == CACG_GRAM_AUTO) variant = CACG_GRAM_FMA;
     if (!std::is_same<T, double>::value) variant = CACG_GRAM_FMA;
     if (variant == CACG_GRAM_DMMA) {

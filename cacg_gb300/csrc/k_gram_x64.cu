@@ -1,0 +1,548 @@
+// k_gram_x64.cu -- FP64 Gram products C = L^T [R1 | R2] on the fp16 tensor
+// cores (tcgen05, sm_103a), from exact digit planes.
+//
+// Reference operations replaced (sclc/cacg): distributedMatLTransposeMatRMul
+// (src/BLAS3.c:699-726) and distributedMatLTransposeMatRMul_updated
+// (src/BLAS3.c:730-758) in FP64, with the allreduce that follows each.
+//
+// Why: this part's FP64 pipe gives 1.2 TFLOP/s, 1/1600 of its fp16 tensor
+// rate, and an FP64 FMA Gram keeps it 96 % busy; 28 fp16 digit-plane products
+// (x64_util.cuh) do the same sum 20 times faster, with less rounding.
+//
+// Four launches:
+//   colmax   the largest magnitude of every column over each row chunk (a
+//            column's digits share one scale per chunk);
+//   gram     split-K over row chunks, one CTA of 17 warps per SM: 16 converter
+//            warps copy 32-row steps to shared memory (cp.async into slots
+//            that only the copying thread reads: no barrier), split them into
+//            digit planes (MN-major core matrices, double-buffered) and one
+//            thread issues the MMAs.  The B planes are stacked side by side in
+//            the MMA's N dimension and the accumulators of p + q = 0 .. 6 lie
+//            side by side in tensor memory, so plane p of A is multiplied with
+//            planes 0 .. 6-p of B by one or two wide MMAs: A is read from
+//            shared memory 10 times a step instead of 28.  After 128 rows the
+//            integer sums (below 2^24, exact) are folded into integer
+//            registers (64 + 24 bits per output, exact), and scaled to FP64
+//            once per chunk;
+//   reduce   sums the chunks' FP64 partials in a fixed order.  Where a chunk
+//            raised its flag (Inf or NaN in a column, a column below 2^-959,
+//            a wait that ran out) it recomputes its outputs by FP64 FMAs.
+#include <algorithm>
+
+#include "cacg_internal.cuh"
+#include "tc5_util.cuh"
+#include "x64_util.cuh"
+
+namespace cacg {
+
+constexpr int kXgKT = 32;                          // rows per step
+constexpr int kXgM = 128;                          // MMA M (L columns, zero-padded)
+constexpr int kXgGroup = 4;                        // steps per accumulation group (128 rows)
+constexpr int kXgConvWarps = 16;
+constexpr int kXgThreads = 32 * kXgConvWarps + 32;  // + the MMA issuer's warp
+constexpr unsigned kXgABytes = kXPlanes * kXgM * kXgKT * 2;  // A planes of one step
+
+struct XgOperands {
+    const double *L, *R1, *R2;
+    int64_t ldl, ldr1, ldr2;
+    int ka, kb1, kb2;
+};
+
+// ------------------------------------------------------------ column maxima
+// emax[(chunk * sub + s) * (ka + kb) + column]: block (chunk, s) covers the
+// s-th part of the chunk's rows
+template <bool VEC>
+__global__ void __launch_bounds__(512)
+    gram_x64_colmax_kernel(int64_t n, int64_t rows_per_chunk, int64_t rows_per_sub, XgOperands o,
+                           uint32_t *__restrict__ emax) {
+    __shared__ uint32_t mx[3 * 256];
+    const int kc = o.ka + o.kb1 + o.kb2;
+    for (int i = threadIdx.x; i < kc; i += blockDim.x) mx[i] = 0u;
+    __syncthreads();
+    const int64_t c0 = (int64_t)blockIdx.x * rows_per_chunk;
+    const int64_t rb = c0 + (int64_t)blockIdx.y * rows_per_sub;
+    const int64_t re = min(min(n, c0 + rows_per_chunk), rb + rows_per_sub);
+    int base = 0;
+    for (int t = 0; t < 3; ++t) {
+        const double *p = t == 0 ? o.L : t == 1 ? o.R1 : o.R2;
+        const int64_t ld = t == 0 ? o.ldl : t == 1 ? o.ldr1 : o.ldr2;
+        const int w = t == 0 ? o.ka : t == 1 ? o.kb1 : o.kb2;
+        if (w > 0) {
+            const int tpr = VEC ? w / 2 : w;
+            const int rpb = blockDim.x / tpr;
+            const int r = threadIdx.x / tpr, c = (threadIdx.x % tpr) * (VEC ? 2 : 1);
+            if (r < rpb) {
+                uint32_t k0 = 0u, k1 = 0u;
+#pragma unroll 8
+                for (int64_t row = rb + r; row < re; row += rpb) {
+                    if constexpr (VEC) {
+                        const double2 v = __ldg(reinterpret_cast<const double2 *>(p + row * ld + c));
+                        k0 = max(k0, x64_key(v.x));
+                        k1 = max(k1, x64_key(v.y));
+                    } else {
+                        k0 = max(k0, x64_key(__ldg(p + row * ld + c)));
+                    }
+                }
+                atomicMax(&mx[base + c], k0);
+                if constexpr (VEC) atomicMax(&mx[base + c + 1], k1);
+            }
+        }
+        base += w;
+    }
+    __syncthreads();
+    uint32_t *out = emax + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * kc;
+    for (int i = threadIdx.x; i < kc; i += blockDim.x) out[i] = mx[i];
+}
+
+// -------------------------------------------------------------- the products
+__device__ __forceinline__ void xg_cp16(void *smem, const void *g, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(t5_smem_u32(smem)), "l"(g),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void xg_cp8(void *smem, const void *g, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(t5_smem_u32(smem)), "l"(g),
+                 "r"(bytes)
+                 : "memory");
+}
+
+// NB = 16 * NC columns of [R1 | R2] per output tile (7 NB <= 512 columns of
+// tensor memory); VEC: widths and row strides even and bases 16-byte aligned,
+// so a pair of columns is one 16-byte copy.
+template <int NC, bool VEC>
+__global__ void __launch_bounds__(kXgThreads, 1)
+    gram_x64_kernel(int64_t n, int64_t rows_per_chunk, XgOperands o, int BA, int tilesB, int sub,
+                    const uint32_t *__restrict__ emax, double *__restrict__ part,
+                    int *__restrict__ flags) {
+    constexpr int NB = 16 * NC;
+    constexpr int NQ = NB / 4;  // accumulator columns per converter thread
+    constexpr unsigned lbo_a = (kXgM / 8) * 128, lbo_b = (kXPlanes * NB / 8) * 128;
+    constexpr unsigned b_bytes = (kXgKT / 8) * lbo_b;
+    constexpr unsigned buf_bytes = kXgABytes + b_bytes;
+    constexpr int tmem_cols = NC == 1 ? 128 : NC == 2 ? 256 : 512;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    // [plane buffers x2][raw slots][scales][mbarriers][tmem slot][abort]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nunits = (BA / 8 + NB / 8) * (kXgKT / 8);
+    const int upw = (nunits + kXgConvWarps - 1) / kXgConvWarps;
+    double2 *raw = reinterpret_cast<double2 *>(smem_raw + 2 * buf_bytes);
+    int *esc = reinterpret_cast<int *>(smem_raw + 2 * buf_bytes +
+                                       (size_t)upw * kXgConvWarps * 32 * 16);
+    uint64_t *sfull = reinterpret_cast<uint64_t *>(esc + kXgM + NB);
+    uint64_t *sfree = sfull + 2;
+    uint64_t *gdone = sfree + 2;
+    uint64_t *gfree = gdone + 1;
+    unsigned *tmem_slot = reinterpret_cast<unsigned *>(gfree + 1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+    const int tile_a = blockIdx.y / tilesB, tile_b = blockIdx.y % tilesB;
+    const int a0 = tile_a * BA, b0 = tile_b * NB;
+    const int kb = o.kb1 + o.kb2, kc = o.ka + kb;
+    const int64_t rbeg = (int64_t)blockIdx.x * rows_per_chunk;
+    const int64_t rend = min(n, rbeg + rows_per_chunk);
+    const int64_t nsteps = rend > rbeg ? (rend - rbeg + kXgKT - 1) / kXgKT : 0;
+    int *flag = flags + (size_t)blockIdx.x * gridDim.y + blockIdx.y;
+
+    // scales of the tile's columns
+    bool bad = false;
+    if (tid < BA + NB) {
+        const int c = tid < BA ? (a0 + tid < o.ka ? a0 + tid : -1)
+                               : (b0 + tid - BA < kb ? o.ka + b0 + tid - BA : -1);
+        uint32_t key = 0u;
+        if (c >= 0)
+            for (int s = 0; s < sub; ++s)
+                key = max(key, emax[((size_t)blockIdx.x * sub + s) * kc + c]);
+        esc[tid] = x64_scale(key, &bad);
+    }
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) *flag = 1;
+        return;
+    }
+
+    // A columns past BA stay zero
+    for (unsigned i = tid; i < 2 * buf_bytes / 16; i += kXgThreads)
+        reinterpret_cast<uint4 *>(smem_raw)[i] = make_uint4(0, 0, 0, 0);
+    if (tid == 0) {
+        t5_mbar_init(&sfull[0], kXgConvWarps);
+        t5_mbar_init(&sfull[1], kXgConvWarps);
+        t5_mbar_init(&sfree[0], 1);
+        t5_mbar_init(&sfree[1], 1);
+        t5_mbar_init(gdone, 1);
+        t5_mbar_init(gfree, kXgConvWarps);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                         t5_smem_u32(tmem_slot)),
+                     "r"(tmem_cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    t5_fence_proxy_async();
+    t5_fence_before();
+    __syncthreads();
+    t5_fence_after();
+    const unsigned tmem = *tmem_slot;
+    auto group_end = [&](int64_t e) { return e % kXgGroup == kXgGroup - 1 || e == nsteps - 1; };
+
+    // outputs of this thread: L column 32 (warp % 4) + lane, tile columns
+    // [(warp / 4) NQ, + NQ): sum = ahi 2^24 + alo in units of 2^(Ea + Eb - 2106)
+    long long ahi[NQ];
+    unsigned alo[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        ahi[q] = 0;
+        alo[q] = 0u;
+    }
+    const int quad = warp & 3, quarter = warp >> 2;
+
+    if (warp < kXgConvWarps) {
+        // ------------------------------------------------------ converters
+        // unit id = warp + 16 u: column octet id / 4, row octet id % 4; lane:
+        // row lane / 4 of the octet, column pair lane % 4
+        const int lr = lane >> 2, lc = 2 * (lane & 3);
+        const int kg = warp & 3, oct0 = warp >> 2;  // id % 4; id / 4 = oct0 + 4 u
+        const int rowt = 8 * kg + lr;
+        const int c0 = 8 * oct0 + lc;
+        int rleft = (int)(rend - rbeg) - rowt;  // > 0: the next step has this thread's row
+        // this thread's row of the next step to copy, at tile column c0
+        const double *pL = o.L + (rbeg + rowt) * o.ldl + a0 + c0;
+        const double *p1 = o.R1 + (rbeg + rowt) * o.ldr1 + (b0 + c0 - BA);
+        const double *p2 = o.R2 + (rbeg + rowt) * o.ldr2 + (b0 + c0 - BA - o.kb1);
+        auto copy_unit = [&](int u) {
+            double2 *dst = raw + u * (kXgConvWarps * 32) + tid;
+            const int c = c0 + 32 * u;
+            const bool rv = rleft > 0;
+            auto src = [&](int e, bool &ok) -> const double * {
+                const int col = c + e - BA + b0;
+                const double *p = c < BA ? pL : col < o.kb1 ? p1 : p2;
+                ok = rv && (c < BA ? a0 + c + e < o.ka : col < kb);
+                return ok ? p + 32 * u + e : o.L;
+            };
+            bool ok;
+            const double *s0 = src(0, ok);
+            if constexpr (VEC) {
+                xg_cp16(dst, s0, ok ? 16 : 0);
+            } else {
+                xg_cp8(dst, s0, ok ? 8 : 0);
+                const double *s1 = src(1, ok);
+                xg_cp8(reinterpret_cast<double *>(dst) + 1, s1, ok ? 8 : 0);
+            }
+        };
+        auto next_rows = [&]() {
+            rleft -= kXgKT;
+            pL += kXgKT * o.ldl;
+            p1 += kXgKT * o.ldr1;
+            p2 += kXgKT * o.ldr2;
+        };
+        auto fold = [&](int64_t g) {
+            const bool okg = __all_sync(
+                0xffffffffu, t5_mbar_wait_or_abort(gdone, (unsigned)(g & 1), abort_flag));
+            if (!okg) return false;
+            t5_fence_after();
+            const unsigned ta = tmem + ((unsigned)(32 * quad) << 16) + (unsigned)(quarter * NQ);
+#pragma unroll
+            for (int c0 = 0; c0 < NQ; c0 += 4) {
+                unsigned r[kXPlanes][4];
+#pragma unroll
+                for (int d = 0; d < kXPlanes; ++d) t5_ld4_nowait(ta + d * NB + c0, r[d]);
+                t5_wait_ld();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    int D[kXPlanes];
+#pragma unroll
+                    for (int d = 0; d < kXPlanes; ++d) D[d] = __float2int_rn(__uint_as_float(r[d][q]));
+                    // |D[d]| <= (d + 1) 2^21: the int products fit
+                    const long long h =
+                        (long long)(D[0] * 256 + D[1]) * 65536 + (long long)(D[2] * 256 + D[3]);
+                    const long long l = (long long)D[4] * 65536 + (long long)D[5] * 256 +
+                                        (long long)D[6] + (long long)alo[c0 + q];
+                    ahi[c0 + q] += h + (l >> 24);
+                    alo[c0 + q] = (unsigned)l & 0xffffffu;
+                }
+            }
+            t5_fence_before();
+            __syncwarp();
+            if (lane == 0) t5_mbar_arrive(gfree);
+            return true;
+        };
+        for (int u = 0; u < upw; ++u)
+            if (warp + kXgConvWarps * u < nunits) copy_unit(u);
+        next_rows();
+        t5_cp_commit();
+        bool ok = true;
+        for (int64_t j = 0; j < nsteps && ok; ++j) {
+            const int b = (int)(j & 1);
+            if (j >= 2) {
+                const bool w =
+                    t5_mbar_wait_or_abort(&sfree[b], (unsigned)(((j >> 1) - 1) & 1), abort_flag);
+                if (!__all_sync(0xffffffffu, w)) {
+                    ok = false;
+                    break;
+                }
+            }
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            unsigned char *dbase = smem_raw + b * buf_bytes;
+            const bool more = j + 1 < nsteps;
+#pragma unroll 2
+            for (int u = 0; u < upw; ++u) {
+                const int oct = oct0 + 4 * u;
+                if (warp + kXgConvWarps * u >= nunits) break;
+                const double2 x = raw[u * (kXgConvWarps * 32) + tid];
+                if (more) copy_unit(u);  // into this thread's slot, just read
+                const int2 e = *reinterpret_cast<const int2 *>(esc + c0 + 32 * u);
+                uint32_t w[kXPlanes];
+                x64_planes2(x.x, x.y, e.x, e.y, w);
+                unsigned char *d;
+                unsigned pstride;
+                if (oct < BA / 8) {
+                    d = dbase + oct * 128 + kg * lbo_a;
+                    pstride = (kXgKT / 8) * lbo_a;
+                } else {
+                    d = dbase + kXgABytes + (oct - BA / 8) * 128 + kg * lbo_b;
+                    pstride = (NB / 8) * 128;
+                }
+                d += lr * 16 + lc * 2;
+#pragma unroll
+                for (int p = 0; p < kXPlanes; ++p)
+                    *reinterpret_cast<uint32_t *>(d + p * pstride) = w[p];
+            }
+            next_rows();
+            t5_cp_commit();
+            t5_fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) t5_mbar_arrive(&sfull[b]);
+            if (j >= 1 && group_end(j - 1)) ok = fold((j - 1) / kXgGroup);
+        }
+        if (ok && nsteps > 0) ok = fold((nsteps - 1) / kXgGroup);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (!ok && lane == 0) *abort_flag = 1;
+    } else if (tid == 32 * kXgConvWarps) {
+        // ---------------------------------------------------- MMA issuer
+        int64_t last = -1;
+        for (int64_t j = 0; j < nsteps; ++j) {
+            const int b = (int)(j & 1);
+            const int64_t g = j / kXgGroup;
+            if (!t5_mbar_wait_or_abort(&sfull[b], (unsigned)((j >> 1) & 1), abort_flag) ||
+                (j % kXgGroup == 0 && g >= 1 &&
+                 !t5_mbar_wait_or_abort(gfree, (unsigned)((g - 1) & 1), abort_flag))) {
+                *abort_flag = 1;
+                break;
+            }
+            t5_fence_after();
+            const unsigned abase = t5_smem_u32(smem_raw + b * buf_bytes);
+            const unsigned bbase = abase + kXgABytes;
+            const unsigned tr = (1u << 15) | (1u << 16);  // A, B MN-major
+#pragma unroll
+            for (int kk = 0; kk < kXgKT / 16; ++kk) {
+                const unsigned first = (j % kXgGroup == 0 && kk == 0) ? 0u : 1u;
+#pragma unroll
+                for (int p = 0; p < kXPlanes; ++p) {
+                    // plane p of A times planes 0 .. 6 - p of B: accumulators p .. 6
+                    const int N = (kXPlanes - p) * NB;
+                    const uint64_t ad = t5_desc_lbo(
+                        abase + p * (kXgKT / 8) * lbo_a + 2 * kk * lbo_a, lbo_a, 128);
+                    const uint64_t bd = t5_desc_lbo(bbase + 2 * kk * lbo_b, lbo_b, 128);
+                    const unsigned dt = tmem + p * NB;
+                    const unsigned acc = p == 0 ? first : 1u;
+                    if (N <= 256) {
+                        t5_mma(dt, ad, bd, x64_idesc(kXgM, N) | tr, acc);
+                    } else {
+                        t5_mma(dt, ad, bd, x64_idesc(kXgM, 256) | tr, acc);
+                        const uint64_t bd2 =
+                            t5_desc_lbo(bbase + 2 * kk * lbo_b + (256 / 8) * 128, lbo_b, 128);
+                        t5_mma(dt + 256, ad, bd2, x64_idesc(kXgM, N > 256 ? N - 256 : 16) | tr, acc);
+                    }
+                }
+            }
+            t5_commit(&sfree[b]);
+            if (group_end(j)) t5_commit(gdone);
+            last = j;
+        }
+        // every committed MMA finishes before tensor memory goes (bounded)
+        if (last >= 0) {
+            t5_mbar_wait(&sfree[last & 1], (unsigned)((last >> 1) & 1));
+            if (group_end(last)) t5_mbar_wait(gdone, (unsigned)((last / kXgGroup) & 1));
+        }
+    }
+    t5_fence_before();
+    const int gave_up = __syncthreads_or(*abort_flag);
+    if (warp == 0) {
+        t5_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem),
+                     "r"(tmem_cols));
+    }
+    if (tid == 0) *flag = gave_up;
+    if (gave_up || warp >= kXgConvWarps) return;
+    const int row_t = 32 * quad + lane;
+    if (row_t >= BA) return;
+    double *out = part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * (size_t)BA * NB +
+                  (size_t)row_t * NB + quarter * NQ;
+    const int ea = esc[row_t] - 2106;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const double v = fma((double)ahi[q], 16777216.0, (double)alo[q]);
+        out[q] = scalbn(v, ea + esc[BA + quarter * NQ + q]);
+    }
+}
+
+// Sum of the chunks' partials: four threads share an output, each sums a
+// contiguous quarter of the chunks in order, then the quarters are added in
+// order.  With a raised flag the same threads form the output from L, R1, R2.
+constexpr int kXrElems = 64;  // outputs per block
+
+__global__ void __launch_bounds__(4 * kXrElems)
+    gram_x64_reduce_kernel(const double *__restrict__ part, int nchunks, int ntiles, int BA, int NB,
+                           int tilesB, int64_t n, XgOperands o, double *__restrict__ C1, int ldc1,
+                           double *__restrict__ C2, int ldc2, const int *__restrict__ flags) {
+    __shared__ double qs[4][kXrElems];
+    const int el = threadIdx.x % kXrElems, q = threadIdx.x / kXrElems;
+    const int kb = o.kb1 + o.kb2;
+    const int idx = blockIdx.x * kXrElems + el;
+    const bool active = idx < o.ka * kb;
+    const int a = active ? idx / kb : 0, b = active ? idx % kb : 0;
+    int raised = 0;
+    for (int i = threadIdx.x; i < nchunks * ntiles; i += blockDim.x) raised |= flags[i];
+    raised = __syncthreads_or(raised);
+    double s = 0.0;
+    if (!raised) {
+        const int tile = (a / BA) * tilesB + (b / NB);
+        const size_t off = (size_t)tile * BA * NB + (size_t)(a % BA) * NB + (b % NB);
+        const size_t stride = (size_t)ntiles * BA * NB;
+        const int per = (nchunks + 3) / 4;
+        const int p1 = min(nchunks, q * per + per);
+        int p = q * per;
+        if (active) {
+            for (; p + 8 <= p1; p += 8) {
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = part[off + (size_t)(p + u) * stride];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) s += v[u];
+            }
+            for (; p < p1; ++p) s += part[off + (size_t)p * stride];
+        }
+    } else if (active) {
+        const double *R = b < o.kb1 ? o.R1 + b : o.R2 + (b - o.kb1);
+        const int64_t ldr = b < o.kb1 ? o.ldr1 : o.ldr2;
+        const int64_t per = (n + 3) / 4;
+        const int64_t r1 = min(n, q * per + per);
+#pragma unroll 8
+        for (int64_t r = q * per; r < r1; ++r) s = fma(o.L[r * o.ldl + a], R[r * ldr], s);
+    }
+    qs[q][el] = s;
+    __syncthreads();
+    if (q == 0 && active) {
+        const double t = ((qs[0][el] + qs[1][el]) + qs[2][el]) + qs[3][el];
+        if (b < o.kb1)
+            C1[(size_t)a * ldc1 + b] = t;
+        else
+            C2[(size_t)a * ldc2 + (b - o.kb1)] = t;
+    }
+}
+
+// ------------------------------------------------------------------- host
+struct XgPlan {
+    int BA, NB, tilesA, tilesB, nchunks, sub;
+    int64_t rows_per_chunk, rows_per_sub;
+    size_t smem, part_bytes, emax_bytes, total;
+};
+
+static XgPlan plan_x64(int64_t n, int ka, int kb) {
+    XgPlan p{};
+    auto up = [](int64_t x, int64_t q) { return (x + q - 1) / q * q; };
+    p.tilesA = (ka + kXgM - 1) / kXgM;
+    p.BA = (int)up((ka + p.tilesA - 1) / p.tilesA, 8);
+    p.tilesB = (kb + 63) / 64;
+    p.NB = (int)up((kb + p.tilesB - 1) / p.tilesB, 16);
+    const int tiles = p.tilesA * p.tilesB;
+    // one CTA per SM in all; chunks of at least two steps
+    int64_t nch = std::max<int64_t>(1, sm_count() / tiles);
+    p.rows_per_chunk = std::max<int64_t>(up((n + nch - 1) / nch, kXgKT), 2 * kXgKT);
+    p.nchunks = (int)std::max<int64_t>(1, (n + p.rows_per_chunk - 1) / p.rows_per_chunk);
+    const int64_t sub = std::max<int64_t>(
+        1, std::min<int64_t>(std::min<int64_t>(8, 1024 / p.nchunks), p.rows_per_chunk / 128));
+    p.rows_per_sub = up((p.rows_per_chunk + sub - 1) / sub, 8);
+    p.sub = (int)((p.rows_per_chunk + p.rows_per_sub - 1) / p.rows_per_sub);
+    const int nunits = (p.BA / 8 + p.NB / 8) * (kXgKT / 8);
+    const int upw = (nunits + kXgConvWarps - 1) / kXgConvWarps;
+    p.smem = 2 * ((size_t)kXgABytes + (size_t)(kXgKT / 8) * (kXPlanes * p.NB / 8) * 128) +
+             (size_t)upw * kXgConvWarps * 32 * 16 + (size_t)(kXgM + p.NB) * 4 + 6 * 8 + 16;
+    p.part_bytes = (size_t)p.nchunks * tiles * p.BA * p.NB * sizeof(double);
+    p.emax_bytes = (size_t)p.nchunks * p.sub * (ka + kb) * 4;
+    p.total = p.part_bytes + p.emax_bytes + (size_t)p.nchunks * tiles * sizeof(int) + 64;
+    return p;
+}
+
+size_t gram_x64_workspace_bytes(int64_t n, int ka, int kb) {
+    size_t b = 0;  // any narrower product with the same workspace fits as well
+    for (int w = 16; w < kb; w += 16) b = std::max(b, plan_x64(n, ka, w).total);
+    return std::max(b, plan_x64(n, ka, kb).total);
+}
+
+// n < 256: an FMA chain of so few rows rounds less than the planes drop.  Above,
+// this kernel is the faster one for every width: measured through cacg_k_gram at
+// n = 1369 / 16384 / 884736, k = 4 (+1): 45 / 51 / 217 us against 100 / 102 /
+// 1843 us of the FMA kernel; k = 96 (+16): 60 / 80 / 1207 against 240 / 428 / 15862.
+bool gram_x64_supported(int64_t n, int ka, int kb) {
+    return n >= 256 && ka > 0 && kb > 0 && ka <= 256 && kb <= 512;
+}
+
+template <int NC, bool VEC>
+static void xg_launch(dim3 grid, const XgPlan &p, cudaStream_t st, int64_t n, const XgOperands &o,
+                      const uint32_t *emax, double *part, int *flags) {
+    set_smem_attr(gram_x64_kernel<NC, VEC>, (int)max_smem_optin());
+    gram_x64_kernel<NC, VEC><<<grid, kXgThreads, p.smem, st>>>(n, p.rows_per_chunk, o, p.BA,
+                                                               p.tilesB, p.sub, emax, part, flags);
+}
+
+int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
+                    const double *R1, int64_t ldr1, int kb1, const double *R2, int64_t ldr2,
+                    int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
+                    size_t ws_bytes) {
+    const int kb = kb1 + kb2;
+    if (!gram_x64_supported(n, ka, kb)) return CACG_ERR_UNSUPPORTED;
+    const XgPlan p = plan_x64(n, ka, kb);
+    if (p.total > ws_bytes || !ws || p.smem > max_smem_optin()) return CACG_ERR_UNSUPPORTED;
+    double *part = ws;
+    uint32_t *emax = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(ws) + p.part_bytes);
+    int *flags = reinterpret_cast<int *>(reinterpret_cast<char *>(emax) + (p.emax_bytes + 15) / 16 * 16);
+    const XgOperands o{L, R1, R2, ldl, ldr1, ldr2, ka, kb1, kb2};
+    // 16-byte pairs: even widths, even strides, aligned bases
+    const bool vec = ka % 2 == 0 && kb1 % 2 == 0 && kb2 % 2 == 0 && ldl % 2 == 0 &&
+                     ldr1 % 2 == 0 && aligned16(L) && aligned16(R1) &&
+                     (kb2 == 0 || (ldr2 % 2 == 0 && aligned16(R2)));
+    const dim3 mgrid(p.nchunks, p.sub);
+    if (vec)
+        gram_x64_colmax_kernel<true><<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o,
+                                                            emax);
+    else
+        gram_x64_colmax_kernel<false><<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o,
+                                                             emax);
+    int rc = check_launch();
+    if (rc != CACG_OK) return rc;
+    const dim3 grid(p.nchunks, p.tilesA * p.tilesB);
+#define XG_CASE(NC)                                                       \
+    case NC:                                                              \
+        if (vec)                                                          \
+            xg_launch<NC, true>(grid, p, st, n, o, emax, part, flags);    \
+        else                                                              \
+            xg_launch<NC, false>(grid, p, st, n, o, emax, part, flags);   \
+        break;
+    switch (p.NB / 16) {
+        XG_CASE(1)
+        XG_CASE(2)
+        XG_CASE(3)
+        XG_CASE(4)
+        default:
+            return CACG_ERR_UNSUPPORTED;
+    }
+#undef XG_CASE
+    rc = check_launch();
+    if (rc != CACG_OK) return rc;
+    gram_x64_reduce_kernel<<<(ka * kb + kXrElems - 1) / kXrElems, 4 * kXrElems, 0, st>>>(
+        part, p.nchunks, p.tilesA * p.tilesB, p.BA, p.NB, p.tilesB, n, o, C1, ldc1, C2, ldc2, flags);
+    return check_launch();
+}
+
+}  // namespace cacg

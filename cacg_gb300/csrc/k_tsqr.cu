@@ -146,13 +146,13 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
     int rc = cudaMemsetAsync(bad, 0, sizeof(int), st) == cudaSuccess ? CACG_OK : CACG_ERR_CUDA;
     // pass 1: G = V^T V, R1, Q1 = V R1^{-1}
     if (rc == CACG_OK)
-        rc = launch_gram<double>(st, CACG_GRAM_FMA, n, V, ldv, k, V, ldv, k, nullptr, 0, 0, G, k,
+        rc = launch_gram<double>(st, CACG_GRAM_AUTO, n, V, ldv, k, V, ldv, k, nullptr, 0, 0, G, k,
                                  nullptr, 0, ws, gws, true);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R1, R1i, bad);
     if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, V, ldv, R1i, Q1, k);
     // pass 2: G2 = Q1^T Q1, R2, Q = Q1 R2^{-1}
     if (rc == CACG_OK)
-        rc = launch_gram<double>(st, CACG_GRAM_FMA, n, Q1, k, k, Q1, k, k, nullptr, 0, 0, G, k,
+        rc = launch_gram<double>(st, CACG_GRAM_AUTO, n, Q1, k, k, Q1, k, k, nullptr, 0, 0, G, k,
                                  nullptr, 0, ws, gws, true);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R2, R2i, bad);
     if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, R2i, Q, ldq);

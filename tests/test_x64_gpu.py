@@ -1,0 +1,84 @@
+"""FP64 products from fp16 digit planes (k_gram_x64.cu) against extended-precision sums.
+
+Bound of an output: with M_i the largest magnitude of column i, a digit value is within
+2^-55 M of its element, and the dropped plane products are below 2^-51 M_i M_j a row
+(6 products of two digits of at most 2^7, 2^16 below the lowest kept weight's 2^48 unit,
+against M_i M_j of at least 2^108); the chunk sums are FP64.  2^-50 M_i M_j a row covers
+all of it.
+"""
+import numpy as np
+import pytest
+
+import cacg_gb300 as cg
+from gpu_util import ptr
+
+pytestmark = pytest.mark.gpu
+
+
+def _block(torch, n, k, ld, off, kind, seed):
+    """An n x k view with row stride ld, off doubles into its allocation."""
+    base = torch.zeros(n * ld + off + 2, dtype=torch.float64, device="cuda")
+    v = torch.as_strided(base, (n, k), (ld, 1), off)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(n, k, dtype=torch.float64, device="cuda", generator=g)
+    if kind == "scaled":  # columns of very different magnitude, one of them zero
+        x *= 10.0 ** torch.linspace(-120, 90, k, device="cuda", dtype=torch.float64)
+        x[:, k // 2] = 0.0
+    elif kind == "spike":
+        x *= 1e-9
+        x[n // 3] = -3.0
+    elif kind == "edge":  # the largest significand at the top of every scale
+        x = torch.full_like(x, -(2.0 - 2.0 ** -52))
+    v.copy_(x)
+    return v
+
+
+def _gram(torch, L, R1, R2, variant=0):
+    ka, kb1, kb2 = L.shape[1], R1.shape[1], 0 if R2 is None else R2.shape[1]
+    C = torch.full((ka, kb1 + kb2), 7.0, dtype=torch.float64, device="cuda")
+    rc = cg.lib().cacg_k_gram(0, variant, L.shape[0], ptr(L), L.stride(0), ka, ptr(R1),
+                              R1.stride(0), kb1, ptr(R2), R2.stride(0) if kb2 else 0, kb2, ptr(C),
+                              kb1 + kb2, None)
+    assert rc == 0
+    return C.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,ka,kb1,kb2", [
+    (256, 8, 8, 1), (257, 9, 9, 3), (1000, 20, 20, 5), (2049, 64, 64, 8), (700, 96, 96, 16),
+    (300, 128, 129, 0), (333, 129, 64, 7), (260, 256, 48, 16), (152 * 64 + 1, 12, 17, 0),
+    (152 * 128 + 33, 8, 16, 0)])
+@pytest.mark.parametrize("kind", ["normal", "scaled", "spike", "edge"])
+@pytest.mark.parametrize("pad,off", [(0, 0), (3, 1)])
+def test_gram_fp64_planes(n, ka, kb1, kb2, kind, pad, off):
+    torch = pytest.importorskip("torch")
+    L = _block(torch, n, ka, ka + pad, off, kind, 1)
+    R1 = _block(torch, n, kb1, kb1 + pad, off, kind, 2)
+    R2 = _block(torch, n, kb2, kb2 + pad, off, kind, 3) if kb2 else None
+    C = _gram(torch, L, R1, R2)
+    l = L.cpu().numpy().astype(np.longdouble)
+    r = (R1 if R2 is None else torch.cat([R1, R2], 1)).cpu().numpy().astype(np.longdouble)
+    tol = n * 2.0 ** -50 * np.abs(l).max(0)[:, None] * np.abs(r).max(0)[None, :]
+    assert np.all(np.abs(C - l.T @ r) <= tol)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 4e-310])
+def test_gram_fp64_planes_outside_range(value):
+    """Values no scale holds: the reduction forms the product by FP64 FMAs."""
+    torch = pytest.importorskip("torch")
+    L = _block(torch, 1500, 24, 24, 0, "normal", 4)
+    R = _block(torch, 1500, 24, 24, 0, "normal", 5)
+    if np.isfinite(value):
+        L[:, 3] = value
+        R *= 1e200
+    else:
+        L[700, 3] = value
+        R[900, 5] = value
+    with np.errstate(all="ignore"):
+        got, ref = _gram(torch, L, R, None), _gram(torch, L, R, None, variant=1)
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    fin = np.isfinite(ref)
+    assert np.array_equal(got[~fin & ~np.isnan(ref)], ref[~fin & ~np.isnan(ref)])
+    # two FP64 sums of 1500 products in different orders
+    scale = np.abs(L.cpu().numpy()).T @ np.abs(R.cpu().numpy())
+    ok = fin & np.isfinite(scale)
+    assert np.all(np.abs(got - ref)[ok] <= 2 * 1500 * 2.0 ** -53 * scale[ok])
