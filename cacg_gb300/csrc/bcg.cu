@@ -64,7 +64,10 @@ struct BcgState {
                                    0, ca, cb, 0.0, A->avg_nnz);
     }
     int gram(const double *L, const double *Rm, double *C) {
-        return launch_gram<double>(st, p.gram_variant, n, L, m, m, Rm, m, m, nullptr, 0, 0, C,
+        // a matrix kept as CSR keeps the FMA sums, as in the s-step solver
+        const int v = p.gram_variant == CACG_GRAM_AUTO && A->dia_ndiag == 0 ? CACG_GRAM_FMA
+                                                                            : p.gram_variant;
+        return launch_gram<double>(st, v, n, L, m, m, Rm, m, m, nullptr, 0, 0, C,
                                    m, nullptr, 0, gram_ws, gram_ws_bytes);
     }
     // Y = M^{-1} RHS (m x m), M factored into F

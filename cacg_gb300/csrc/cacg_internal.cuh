@@ -200,6 +200,18 @@ int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, in
                     int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
                     size_t ws_bytes);
 size_t gram_x64_workspace_bytes(int64_t n, int ka, int kb);
+// FP64 tall x small products from digit planes (k_tsm_x64.cu), k <= 144:
+// Qout = S - Qin beta (Qout may be S); X += Q alpha, R -= AQ alpha, S0 = R,
+// norms; Y = A W.  *status gets kStatusTimeout if a bounded wait expires;
+// CACG_ERR_UNSUPPORTED for other shapes.
+int launch_qupdate_x64(cudaStream_t st, int64_t n, int k, double *Qout, int64_t ldo,
+                       const double *Qin, int64_t ldq, const double *S, int64_t lds,
+                       const double *beta, int *status);
+int launch_xrupdate_x64(cudaStream_t st, int64_t n, int k, int m, const double *Q,
+                        const double *AQ, int64_t ldq, const double *alpha, double *X, double *R,
+                        double *S0, int64_t lds, double *norms, double *ws, int *status);
+int launch_tallsmall_x64(cudaStream_t st, int64_t n, int K, int N, const double *A, int64_t lda,
+                         const double *W, int ldw, double *Y, int64_t ldy, int *status);
 
 // dst = src for an n x w FP32 block (rows of lds / ldd values)
 int launch_copy_rows_f32(cudaStream_t st, int64_t n, int w, const float *src, int64_t lds,

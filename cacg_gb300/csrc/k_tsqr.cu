@@ -111,8 +111,10 @@ static int chol_inv(cudaStream_t st, int k, const double *G, double *R, double *
 }
 
 static int tallsmall_triu(cudaStream_t st, int64_t n, int k, const double *X, int64_t ldx,
-                          const double *W, double *Y, int64_t ldy) {
+                          const double *W, double *Y, int64_t ldy, int *status) {
     if (n <= 0) return CACG_OK;
+    const int rc = launch_tallsmall_x64(st, n, k, k, X, ldx, W, k, Y, ldy, status);
+    if (rc != CACG_ERR_UNSUPPORTED) return rc;
     const int smem = (int)((size_t)k * k * sizeof(double));
     set_smem_attr(tallsmall_triu_kernel, kQrSmemMax);
     const int64_t blocks = std::min<int64_t>((n * k + kQrThreads - 1) / kQrThreads,
@@ -149,13 +151,13 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
         rc = launch_gram<double>(st, CACG_GRAM_AUTO, n, V, ldv, k, V, ldv, k, nullptr, 0, 0, G, k,
                                  nullptr, 0, ws, gws, true);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R1, R1i, bad);
-    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, V, ldv, R1i, Q1, k);
+    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, V, ldv, R1i, Q1, k, bad);
     // pass 2: G2 = Q1^T Q1, R2, Q = Q1 R2^{-1}
     if (rc == CACG_OK)
         rc = launch_gram<double>(st, CACG_GRAM_AUTO, n, Q1, k, k, Q1, k, k, nullptr, 0, 0, G, k,
                                  nullptr, 0, ws, gws, true);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R2, R2i, bad);
-    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, R2i, Q, ldq);
+    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, R2i, Q, ldq, bad);
     if (rc == CACG_OK) {
         triu_mul_kernel<<<1, kQrThreads, 0, st>>>(k, R2, R1, R);
         rc = check_launch();
@@ -168,6 +170,6 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
     }
     cudaFreeAsync(buf, st);
     if (rc != CACG_OK) cudaGetLastError();  // a refused launch leaves no error behind
-    if (rc == CACG_OK && hb) rc = CACG_ERR_BREAKDOWN;
+    if (rc == CACG_OK && hb) rc = hb & kStatusTimeout ? CACG_ERR_TIMEOUT : CACG_ERR_BREAKDOWN;
     return rc;
 }

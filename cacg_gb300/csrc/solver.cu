@@ -545,6 +545,12 @@ static void tridiag_extremes(const std::vector<double> &a, const std::vector<dou
     *hi = kth(k - 1);
 }
 
+// FP64 multiply-adds (n k k, n k m) from which the digit-plane updates are the
+// faster ones: below, the FMA kernels' work is less than the planes' set-up.
+// Q: n = 16384, k = 4 14.1 us FMA, 14.5 planes; n = 32768, k = 16 24 and 14.
+// X / R: n = 32768, k = 16, m = 4 31 and 33; n = 50653, k = 20, m = 5 51 and 49.
+constexpr double kPlanesQMin = 2e6, kPlanesXrMin = 4e6;
+
 struct Solver {
     const DevMatrix *A;
     int m, s, k, prec;
@@ -798,8 +804,13 @@ struct Solver {
                                                (const T *)b.S, k, b.beta);
                 }
             } else {
-                rc = launch_qupdate<T>(st, n, k, (T *)b.S, k, (const T *)b.Q, k, (const T *)b.S,
-                                       k, b.beta);
+                rc = CACG_ERR_UNSUPPORTED;
+                if (planes64() && (double)n * k * k >= kPlanesQMin)
+                    rc = launch_qupdate_x64(st, n, k, (T *)b.S, k, (const T *)b.Q, k,
+                                            (const T *)b.S, k, b.beta, b.status);
+                if (rc == CACG_ERR_UNSUPPORTED)
+                    rc = launch_qupdate<T>(st, n, k, (T *)b.S, k, (const T *)b.Q, k,
+                                           (const T *)b.S, k, b.beta);
             }
             prof.end();
             if (rc) return rc;
@@ -868,6 +879,16 @@ struct Solver {
         return p.gram_variant == CACG_GRAM_AUTO || p.gram_variant == CACG_GRAM_TC5;
     }
 
+    // FP64 products from digit planes (k_gram_x64.cu, k_tsm_x64.cu) where the
+    // variant is automatic and the matrix has a DIA view.  A matrix kept as CSR
+    // keeps the FMA sums: measured on random graphs (n = 50021, m = 6), the
+    // iteration turns any other rounding of its products into 1e-9 of X and more
+    // (the same FMA code on right-hand sides scaled by 1.1 moves X by up to
+    // 5e-9), against 1e-15 to 5e-10 on the stencil and diffusion matrices.
+    bool planes64() const {
+        return prec == CACG_FP64 && p.gram_variant == CACG_GRAM_AUTO && A->dia_ndiag > 0;
+    }
+
     // Gram with the variant for this precision: the mixed mode uses the
     // tensor-core kernel unless a CUDA-core variant is requested.
     template <typename T>
@@ -887,6 +908,7 @@ struct Solver {
                                       C2, ldc2, b.gram_ws, b.gram_ws_bytes);
         }
         int v = p.gram_variant == CACG_GRAM_TC ? CACG_GRAM_FMA : p.gram_variant;
+        if (v == CACG_GRAM_AUTO && std::is_same<T, double>::value && !planes64()) v = CACG_GRAM_FMA;
         return launch_gram<T>(st, v, n, Lm, k, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1, ldc1, C2,
                               ldc2, b.gram_ws, b.gram_ws_bytes,
                               symmetric && std::is_same<T, double>::value);
@@ -913,6 +935,13 @@ struct Solver {
                 int rc = launch_xrupdate_m16_tma(st, A->n, k, Q, AQ, k, b.alpha, X, b.R,
                                                  (float *)b.S, k, b.R32, b.norms, b.norm_ws,
                                                  b.status);
+                if (rc != CACG_ERR_UNSUPPORTED) return rc;
+            }
+        }
+        if constexpr (std::is_same<T, double>::value) {
+            if (planes64() && (double)A->n * k * m >= kPlanesXrMin) {
+                const int rc = launch_xrupdate_x64(st, A->n, k, m, Q, AQ, k, b.alpha, X, b.R, (T *)b.S,
+                                                   k, b.norms, b.norm_ws, b.status);
                 if (rc != CACG_ERR_UNSUPPORTED) return rc;
             }
         }

@@ -79,6 +79,16 @@ __device__ __forceinline__ void x64_planes2(double x0, double x1, int E0, int E1
         asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(w[p]) : "r"(u[p]), "r"(0x64806480u));
 }
 
+// (h 2^32 + l) 2^sc as FP64 (h and l exact in FP64): one rounding, the power of
+// two goes into the exponent field where it fits
+__device__ __forceinline__ double x64_make(long long h, long long l, int sc) {
+    const double t = fma((double)h, 4294967296.0, (double)l);
+    if (sc > -900 && sc < 900)
+        return (h | l) == 0 ? 0.0
+                            : __hiloint2double(__double2hiint(t) + (sc << 20), __double2loint(t));
+    return scalbn(t, sc);
+}
+
 // Instruction descriptor of kind::f16 with fp16 inputs and FP32 accumulation
 __host__ __device__ constexpr unsigned x64_idesc(int M, int N) {
     return (1u << 4) | ((unsigned)(N >> 3) << 17) | ((unsigned)(M >> 4) << 24);

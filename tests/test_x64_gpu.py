@@ -1,4 +1,4 @@
-"""FP64 products from fp16 digit planes (k_gram_x64.cu) against extended-precision sums.
+"""FP64 products from fp16 digit planes (k_gram_x64.cu, k_tsm_x64.cu) against extended-precision sums.
 
 Bound of an output: with M_i the largest magnitude of column i, a digit value is within
 2^-55 M of its element, and the dropped plane products are below 2^-51 M_i M_j a row
@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import cacg_gb300 as cg
+import oracle as O
 from gpu_util import ptr
 
 pytestmark = pytest.mark.gpu
@@ -82,3 +83,51 @@ def test_gram_fp64_planes_outside_range(value):
     scale = np.abs(L.cpu().numpy()).T @ np.abs(R.cpu().numpy())
     ok = fin & np.isfinite(scale)
     assert np.all(np.abs(got - ref)[ok] <= 2 * 1500 * 2.0 ** -53 * scale[ok])
+
+
+def _qr(torch, V):
+    n, k = V.shape
+    Q = torch.empty(n, k, dtype=torch.float64, device="cuda")
+    R = torch.empty(k, k, dtype=torch.float64, device="cuda")
+    assert cg.lib().cacg_k_tsqr(n, k, ptr(V), V.stride(0), ptr(Q), k, ptr(R), None) == 0
+    return Q.cpu().numpy(), R.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,k", [(256, 1), (300, 16), (129, 17), (1000, 31), (152 * 128 + 5, 33),
+                                 (400, 64), (513, 65), (2000, 96), (700, 113), (640, 128)])
+@pytest.mark.parametrize("pad,off", [(0, 0), (3, 1)])
+def test_tall_small_product_in_qr(n, k, pad, off):
+    """Y = A W at tile edges, through the QR: Q R = V and Q^T Q = I.  A product's error is
+    below 2^-50 of its row's and column's largest magnitudes a term; two passes, k terms."""
+    torch = pytest.importorskip("torch")
+    V = _block(torch, n, k, k + pad, off, "normal", 6)
+    V[:, :] *= 10.0 ** torch.linspace(-3, 3, n, device="cuda", dtype=torch.float64)[:, None]
+    Q, R = _qr(torch, V)
+    v = V.cpu().numpy()
+    assert np.max(np.abs(Q.T @ Q - np.eye(k))) <= 4 * k * 2.0 ** -50
+    assert np.linalg.norm(Q @ R - v) <= 4 * k * 2.0 ** -50 * np.linalg.norm(v)
+    # rows of small magnitude keep their own relative accuracy (a scale per row)
+    row = np.linalg.norm(Q @ R - v, axis=1) / np.linalg.norm(v, axis=1)
+    cond = np.linalg.cond(R)
+    assert np.max(row) <= 4 * k * 2.0 ** -50 * cond
+
+
+@pytest.mark.parametrize("kind,N,m,s", [("lap2d", 24, 1, 2), ("lap3d7", 9, 3, 5),
+                                        ("lap2d", 37, 5, 4), ("lap3d7", 17, 16, 4),
+                                        ("lap2d", 40, 17, 3), ("lap3d7", 15, 32, 4),
+                                        ("lap3d7", 16, 36, 4), ("lap2d", 45, 37, 2),
+                                        ("lap3d7", 15, 12, 8)])
+def test_solves_with_plane_products(kind, N, m, s):
+    """Gram, Q and X / R updates together at the widths and row counts where their tiles end,
+    against the oracle: the contract's +-1 iteration and 1e-6."""
+    rp, ci, v = cg.gen_matrix(kind, N, 0.1)
+    n = len(rp) - 1
+    B = cg.gen_rhs("normal", n, m, 7)
+    bounds = (0.1, 12.1 if kind == "lap3d7" else 8.1)
+    eps = 1e-7 * float(np.linalg.norm(B[:, 0]))
+    Xo, ito, _ = O.port_solve(rp, ci, v, B, np.zeros_like(B), s, eps, bounds, 200)
+    X, info = cg.solve(rp, ci, v, B, s=s, bounds=("given",) + bounds, tol=eps,
+                       tol_mode="abs_col0", maxit=200)
+    assert info["status"] == 0
+    assert abs(info["iterations"] - ito) <= 1
+    assert np.linalg.norm(X - Xo) <= 1e-6 * np.linalg.norm(Xo)
