@@ -36,10 +36,16 @@ struct DevMatrix {
     double *dia64 = nullptr;
     float *dia32 = nullptr;    // FP32 values (hi) ...
     float *dia32lo = nullptr;  // ... and val - hi, same allocation
+    // one-value view (k_dia_fix.cu): every off-diagonal nonzero equals fix_c; a
+    // presence bit per diagonal and row (NULL: the values differ)
+    uint32_t *fix_mask = nullptr;
+    double fix_c = 0;
+    int fix_dmain = -1;  // index of the main diagonal
     size_t owned_bytes = 0;
     cudaStream_t st = nullptr;  // stream of the stream-ordered allocations
     static int create(const cacg_csr *A, bool want_f32, DevMatrix *M, cudaStream_t st);
     int build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st);
+    int build_fix(const cacg_csr *A, cudaStream_t st);
     int ensure_f32(cudaStream_t st);
     void release();
 };
@@ -80,6 +86,28 @@ int launch_dia_ring(cudaStream_t st, const DevMatrix *A, int w, const float *X, 
 int launch_dia_wide(cudaStream_t st, const DevMatrix *A, int w, const float *X, int64_t ldx,
                     float *Y, int64_t ldy, const float *Z1, int64_t ldz1, const float *Z2,
                     int64_t ldz2, double ca, double cb, double cc);
+
+// The same product in FP64 for matrices with a one-value view, neighbour sums in
+// 64-bit fixed point (k_dia_fix.cu); xi: dia_fix_scratch_bytes(n, w), small:
+// dia_fix_small_bytes(w).  CACG_ERR_UNSUPPORTED without such a view or scratch,
+// and below kDiaFixMin products (nnz w): three launches then cost more than the
+// FMAs.  7-point n = 50653, w = 20 (7.0e6): 31.6 us against 28.4 us of the FMA
+// kernel; n = 262144, w = 8 (14.5e6): 42.8 against 46.4, w = 64: 210 against 316;
+// 27-point n = 884736, w = 16: 230 against 747, w = 96: 1471 against 4630.
+constexpr double kDiaFixMin = 1e7;
+// chain: calls of which each takes the Y of the one before as its X, with the
+// same scratch and nothing between that writes either: the column maxima of X
+// then come with it (of: the block they belong to; NULL at the first call)
+struct FixChain {
+    const double *of = nullptr;
+    int w = 0, set = 0, nparts = 0;
+};
+int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, int64_t ldx,
+                   double *Y, int64_t ldy, const double *Z1, int64_t ldz1, const double *Z2,
+                   int64_t ldz2, double ca, double cb, double cc, void *xi, void *small,
+                   FixChain *chain = nullptr);
+size_t dia_fix_scratch_bytes(int64_t n, int w);
+size_t dia_fix_small_bytes(int w);
 
 // Per-thread pinned host scratch of at least `bytes` (reused across calls).
 double *pinned_scratch(size_t bytes);

@@ -1,0 +1,485 @@
+// k_dia_fix.cu -- FP64 SpMM over the DIA view of matrices whose off-diagonal
+// nonzeros all have one value (finite-difference stencils with constant
+// coefficients; the main diagonal is arbitrary), with the neighbour sums in
+// 64-bit fixed point.
+//
+// Reference operations replaced (sclc/cacg): as k_dia.cu (spmm_csr_v1
+// src/BLAS3.c:20-155, spmm_csr_info_data_sep_BCBCG src/BLAS3.c:913-976 and the
+// basis axpbys src/BLAS3.c:828-847, 978-994), in FP64.
+//
+// Why: the FP64 pipe does 2 FMAs a clock per SM, so a 27-point row costs 13
+// clocks a column there, the integer pipe's additions 1.  With c the common
+// off-diagonal value, A x = D x + c sum_j x_j: x is written once as 57-bit
+// integers on a scale per column, the sum over the neighbours present in a row
+// (a bit per diagonal) is exact, and the FP64 pipe is left with one conversion
+// and two FMAs per output:
+//     Y = ca c S + (ca D [+ cb]) X + cb Z1 + cc Z2      (cb folded in if Z1 is X)
+// Each x is rounded at 2^-58 of its column's largest element, once; the FMA
+// chain rounds at 2^-53 of every partial sum.
+//
+// Measured at 27 points, n = 262144, w = 16 (75 us a step): FP64 pipe 62 % busy,
+// the rest the latency of the window reads; four rows a thread and three CTAs an
+// SM beat eight rows and two (91 us).  The sums are normalised to FP64 by integer
+// instructions, which leaves the FP64 pipe half as busy (35 -> 31 us a 7-point
+// step, n = 262144, w = 8).
+//
+// Three launches: column maxima (partials per block; left out in a chain of
+// basis steps, where the step that wrote X has left them), conversion (which
+// first reduces them), and the product.  A column that no scale holds (Inf, NaN, or a
+// largest magnitude beyond 2^+-400) sends the product to FP64 FMAs over the DIA values.
+#include <algorithm>
+#include <cmath>
+
+#include "cacg_internal.cuh"
+#include "cacg_solver.h"
+#include "x64_util.cuh"
+
+namespace cacg {
+
+namespace {
+
+constexpr int kFixThreads = 256;
+constexpr int kFixR = 4;                       // rows per thread
+constexpr int kFixW = kFixR + kDiaGroupMax - 1;  // window rows
+constexpr int kFixMaxBlocks = 608;             // partial maxima per column
+
+// mask[row]: bit d set where diagonal d of the row holds c; *bad when an
+// off-diagonal value is neither 0 nor c
+__global__ void fix_mask_kernel(int64_t n, int64_t npad, DiaDesc desc, int dmain,
+                                const double *__restrict__ v64, double c,
+                                uint32_t *__restrict__ mask, int *__restrict__ bad) {
+    for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < npad;
+         row += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t m = 0u;
+        bool ok = true;
+        for (int d = 0; d < desc.ndiag; ++d) {
+            if (d == dmain) continue;
+            const double v = v64[(size_t)d * npad + row];
+            if (v == c)
+                m |= 1u << d;
+            else if (v != 0.0)
+                ok = false;
+        }
+        mask[row] = m;
+        if (!ok) atomicOr(bad, 1);
+    }
+}
+
+// part[block * w + column]
+template <bool VEC>
+__global__ void __launch_bounds__(kFixThreads)
+    fix_colmax_kernel(int64_t n, int w, const double *__restrict__ X, int64_t ldx,
+                      uint32_t *__restrict__ part) {
+    extern __shared__ uint32_t fix_mx[];
+    for (int i = threadIdx.x; i < w; i += blockDim.x) fix_mx[i] = 0u;
+    __syncthreads();
+    const int tpr = VEC ? w / 2 : w;
+    const int rpb = blockDim.x / tpr;
+    const int r = threadIdx.x / tpr, c = (threadIdx.x % tpr) * (VEC ? 2 : 1);
+    if (r < rpb) {
+        uint32_t k0 = 0u, k1 = 0u;
+#pragma unroll 4
+        for (int64_t row = (int64_t)blockIdx.x * rpb + r; row < n; row += (int64_t)gridDim.x * rpb) {
+            if constexpr (VEC) {
+                const double2 v = __ldg(reinterpret_cast<const double2 *>(X + row * ldx + c));
+                k0 = max(k0, x64_key(v.x));
+                k1 = max(k1, x64_key(v.y));
+            } else {
+                k0 = max(k0, x64_key(__ldg(X + row * ldx + c)));
+            }
+        }
+        atomicMax(&fix_mx[c], k0);
+        if constexpr (VEC) atomicMax(&fix_mx[c + 1], k1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < w; i += blockDim.x) part[(size_t)blockIdx.x * w + i] = fix_mx[i];
+}
+
+// round(x 2^(1079 - E)), |x| < 2^(E - 1022): |result| <= 2^57
+__device__ __forceinline__ long long fix_from(double x, int E) {
+    const uint32_t xh = (uint32_t)__double2hiint(x), xl = (uint32_t)__double2loint(x);
+    const int s = E - (int)((xh >> 20) & 0x7ffu);
+    const uint32_t mh = (xh & 0xfffffu) | 0x100000u;
+    const uint64_t m5 = ((uint64_t)__funnelshift_l(xl, mh, 5) << 32) | (uint64_t)(xl << 5);
+    uint64_t m;  // twice the magnitude
+    asm("shr.u64 %0, %1, %2;" : "=l"(m) : "l"(m5), "r"(s));
+    const long long a = (long long)((m + 1) >> 1);
+    return (int32_t)xh < 0 ? -a : a;
+}
+
+// xi (n x wp, wp = w rounded up to even, the padding column zero); scale[0 .. w):
+// the columns' exponents, scale[w]: raised when a column has none
+template <bool VEC>
+__global__ void __launch_bounds__(kFixThreads)
+    fix_convert_kernel(int64_t n, int w, int wp, const double *__restrict__ X, int64_t ldx,
+                       const uint32_t *__restrict__ part, int nparts, long long *__restrict__ xi,
+                       int *__restrict__ scale) {
+    extern __shared__ uint32_t fix_mx[];
+    for (int i = threadIdx.x; i < wp; i += blockDim.x) fix_mx[i] = 0u;
+    __syncthreads();
+    // stripes of the partials: one atomic per thread and column group
+    const int ns = max(1, (int)blockDim.x / w);
+    if (threadIdx.x < ns * w || w > (int)blockDim.x) {
+        for (int c = threadIdx.x % w; c < w; c += blockDim.x) {
+            uint32_t k = 0u;
+#pragma unroll 8
+            for (int p = threadIdx.x / w; p < nparts; p += ns) k = max(k, part[(size_t)p * w + c]);
+            atomicMax(&fix_mx[c], k);
+        }
+    }
+    __syncthreads();
+    bool bad = false;
+    for (int i = threadIdx.x; i < wp; i += blockDim.x) {
+        const int e = x64_scale_mid(fix_mx[i], &bad);
+        fix_mx[i] = (uint32_t)e;
+        if (blockIdx.x == 0 && i < w) scale[i] = e;
+    }
+    const int any = __syncthreads_or(bad);
+    if (blockIdx.x == 0 && threadIdx.x == 0) scale[w] = any;
+    if (any) return;
+    const int tpr = wp / 2;
+    const int rpb = blockDim.x / tpr;
+    const int r = threadIdx.x / tpr, c = (threadIdx.x % tpr) * 2;
+    if (r >= rpb) return;
+    const int e0 = (int)fix_mx[c], e1 = (int)fix_mx[c + 1];
+#pragma unroll 4
+    for (int64_t row = (int64_t)blockIdx.x * rpb + r; row < n; row += (int64_t)gridDim.x * rpb) {
+        double2 v = make_double2(0.0, 0.0);
+        if constexpr (VEC) {
+            v = __ldg(reinterpret_cast<const double2 *>(X + row * ldx + c));
+        } else {
+            v.x = __ldg(X + row * ldx + c);
+            if (c + 1 < w) v.y = __ldg(X + row * ldx + c + 1);
+        }
+        *reinterpret_cast<longlong2 *>(xi + row * wp + c) =
+            make_longlong2(fix_from(v.x, e0), fix_from(v.y, e1));
+    }
+}
+
+struct FixArgs {
+    int64_t n, npad;
+    int w, wp, cpr, runs;  // columns; 2-column chunks a row; row runs per block
+    const uint32_t *mask;
+    const double *vals;  // DIA values (npad apart); the main diagonal is diagonal dmain
+    int dmain;           // -1: no main diagonal
+    double c, ca, cb, cc;
+    int c_pow2;  // ca c = +-2^c_pow2 (0 when it is no power of two)
+    int fold;    // Z1 is X: cb goes into the diagonal's factor
+    const double *X, *Z1, *Z2;
+    int64_t ldx, ldz1, ldz2, ldy;
+    double *Y;
+    const long long *xi;
+    const int *scale;
+    uint32_t *ymax;  // column maxima of Y, a partial per block (NULL: not wanted)
+};
+
+template <bool VEC>
+__device__ __forceinline__ double2 fix_ld(const double *p, int c, int w) {
+    if constexpr (VEC) {
+        return *reinterpret_cast<const double2 *>(p + c);
+    } else {
+        return make_double2(p[c], c + 1 < w ? p[c + 1] : 0.0);
+    }
+}
+
+// VEC: even w and strides, 16-byte aligned X, Y, Z1, Z2
+// MODE: the addends besides the diagonal's, by FP64 operations per output (half
+// of one for the diagonal's factor):
+//   kFixPow2  none, ca c = +-2^c_pow2 (one FMA)
+//   kFixNone  none (two);  kFixStep  Z2 with cc = -1 (two);  kFixAny  (up to four)
+enum { kFixPow2 = 0, kFixNone = 1, kFixStep = 2, kFixAny = 3 };
+
+template <bool VEC, int MODE>
+__global__ void __launch_bounds__(kFixThreads, 3)
+    fix_spmm_kernel(const __grid_constant__ FixArgs a, const __grid_constant__ DiaDesc desc) {
+    extern __shared__ uint32_t fix_mx[];
+    const int lr = threadIdx.x / a.cpr, c = 2 * (threadIdx.x % a.cpr);
+    const int BR = a.runs * kFixR;
+    const int64_t nblk = lr < a.runs ? (a.n + BR - 1) / BR : 0;
+    uint32_t k0 = 0u, k1 = 0u;
+    auto put_max = [&]() {
+        if (!a.ymax) return;
+        for (int i = threadIdx.x; i < a.wp; i += blockDim.x) fix_mx[i] = 0u;
+        __syncthreads();
+        if (lr < a.runs) {
+            atomicMax(&fix_mx[c], k0);
+            atomicMax(&fix_mx[c + 1], k1);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < a.w; i += blockDim.x)
+            a.ymax[(size_t)blockIdx.x * a.w + i] = fix_mx[i];
+    };
+    if (a.scale[a.w]) {
+        // a column without a scale: FP64 FMAs over the diagonals
+        for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+            for (int i = 0; i < kFixR; ++i) {
+                const int64_t row = blk * BR + (int64_t)lr * kFixR + i;
+                if (row >= a.n) break;
+                for (int q = 0; q < 2 && c + q < a.w; ++q) {
+                    double s = 0.0;
+                    for (int d = 0; d < desc.ndiag; ++d) {
+                        const int64_t xr = row + desc.off[d];
+                        if (xr < 0 || xr >= a.n) continue;
+                        s = fma(a.vals[(size_t)d * a.npad + row], a.X[xr * a.ldx + c + q], s);
+                    }
+                    double y = a.ca * s;
+                    if (a.Z1) y = fma(a.cb, a.Z1[row * a.ldz1 + c + q], y);
+                    if (a.Z2) y = fma(a.cc, a.Z2[row * a.ldz2 + c + q], y);
+                    a.Y[row * a.ldy + c + q] = y;
+                    (q ? k1 : k0) = max(q ? k1 : k0, x64_key(y));
+                }
+            }
+        }
+        put_max();
+        return;
+    }
+    const int e0 = c < a.w ? a.scale[c] : 1023, e1 = c + 1 < a.w ? a.scale[c + 1] : 1023;
+    const double cac = a.ca * a.c;
+    const int flip = cac < 0.0 ? (int)0x80000000 : 0;
+    // ca c on the columns' scales
+    const double c0 = scalbn(cac, e0 - 1079), c1 = scalbn(cac, e1 - 1079);
+    const double fca = a.ca, fcb = a.fold ? a.cb : 0.0;
+    for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        const int64_t r0 = blk * BR + (int64_t)lr * kFixR;
+        uint32_t m[kFixR];
+        {
+            const uint4 m0 = __ldg(reinterpret_cast<const uint4 *>(a.mask + r0));
+            m[0] = m0.x, m[1] = m0.y, m[2] = m0.z, m[3] = m0.w;
+        }
+        long long acc[kFixR][2];
+#pragma unroll
+        for (int i = 0; i < kFixR; ++i) acc[i][0] = acc[i][1] = 0;
+        for (int g = 0; g < desc.ngroups; ++g) {
+            const int d0 = desc.gstart[g], G = desc.gstart[g + 1] - d0;
+            const int64_t x0 = r0 + desc.off[d0];
+            longlong2 win[kFixW];
+            if (x0 >= 0 && x0 + kFixW <= a.n) {
+                const long long *xp = a.xi + x0 * a.wp + c;
+#pragma unroll
+                for (int t = 0; t < kFixW; ++t)
+                    if (t < kFixR + G - 1)
+                        win[t] = __ldg(reinterpret_cast<const longlong2 *>(xp + (int64_t)t * a.wp));
+            } else {
+#pragma unroll
+                for (int t = 0; t < kFixW; ++t) {
+                    if (t < kFixR + G - 1) {
+                        int64_t xr = x0 + t;
+                        xr = xr < 0 ? 0 : (xr >= a.n ? a.n - 1 : xr);  // its bit is clear
+                        win[t] = __ldg(reinterpret_cast<const longlong2 *>(a.xi + xr * a.wp + c));
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kDiaGroupMax; ++j) {
+                if (j < G) {
+                    const uint32_t bit = 1u << (d0 + j);
+#pragma unroll
+                    for (int i = 0; i < kFixR; ++i) {
+                        if (m[i] & bit) {
+                            acc[i][0] += win[i + j].x;
+                            acc[i][1] += win[i + j].y;
+                        }
+                    }
+                }
+            }
+        }
+        const double *dv = a.dmain >= 0 ? a.vals + (size_t)a.dmain * a.npad + r0 : nullptr;
+#pragma unroll
+        for (int i = 0; i < kFixR; ++i) {
+            const int64_t row = r0 + i;
+            if (row >= a.n) break;
+            const double f = fma(fca, dv ? __ldg(dv + i) : 0.0, fcb);
+            const double2 x = fix_ld<VEC>(a.X + row * a.ldx, c, a.w);
+            double t0 = x64_from_ll(acc[i][0]), t1 = x64_from_ll(acc[i][1]);
+            double2 y;
+            if constexpr (MODE == kFixPow2) {
+                // the scale, ca c and its sign go into the exponent field
+                t0 = x64_scaled(t0, acc[i][0] == 0, e0 - 1079 + a.c_pow2);
+                t1 = x64_scaled(t1, acc[i][1] == 0, e1 - 1079 + a.c_pow2);
+                t0 = __hiloint2double(__double2hiint(t0) ^ flip, __double2loint(t0));
+                t1 = __hiloint2double(__double2hiint(t1) ^ flip, __double2loint(t1));
+                y = make_double2(fma(f, x.x, t0), fma(f, x.y, t1));
+            } else {
+                if constexpr (MODE == kFixStep) {
+                    const double2 z = fix_ld<VEC>(a.Z2 + row * a.ldz2, c, a.w);
+                    y = make_double2(fma(f, x.x, -z.x), fma(f, x.y, -z.y));
+                } else {
+                    y = make_double2(f * x.x, f * x.y);
+                }
+                y.x = fma(t0, c0, y.x);
+                y.y = fma(t1, c1, y.y);
+                if constexpr (MODE == kFixAny) {
+                    if (a.Z1 && !a.fold) {
+                        const double2 z = fix_ld<VEC>(a.Z1 + row * a.ldz1, c, a.w);
+                        y.x = fma(a.cb, z.x, y.x);
+                        y.y = fma(a.cb, z.y, y.y);
+                    }
+                    if (a.Z2) {
+                        const double2 z = fix_ld<VEC>(a.Z2 + row * a.ldz2, c, a.w);
+                        y.x = fma(a.cc, z.x, y.x);
+                        y.y = fma(a.cc, z.y, y.y);
+                    }
+                }
+            }
+            k0 = max(k0, x64_key(y.x));
+            k1 = max(k1, x64_key(y.y));
+            double *yp = a.Y + row * a.ldy + c;
+            if constexpr (VEC) {
+                *reinterpret_cast<double2 *>(yp) = y;
+            } else {
+                yp[0] = y.x;
+                if (c + 1 < a.w) yp[1] = y.y;
+            }
+        }
+    }
+    put_max();
+}
+
+}  // namespace
+
+// one-value view of the matrix's off-diagonals (DevMatrix::build_dia): c from
+// the host arrays, presence bits on the device; leaves fix_mask NULL when the
+// off-diagonal values differ
+int DevMatrix::build_fix(const cacg_csr *A, cudaStream_t s) {
+    if (dia_ndiag <= 1 || !dia64) return CACG_OK;
+    double cv = 0.0;
+    bool found = false;
+    for (int64_t i = 0; i < A->n && !found; ++i)
+        for (int32_t e = A->row_ptr[i]; e < A->row_ptr[i + 1]; ++e)
+            if (A->col_idx[e] != i && A->val[e] != 0.0) {
+                cv = A->val[e];
+                found = true;
+                break;
+            }
+    if (!found || !std::isfinite(cv) || std::fabs(cv) < 1e-200 || std::fabs(cv) > 1e200)
+        return CACG_OK;
+    uint32_t *mk = nullptr;
+    int *bad = nullptr;
+    const size_t bytes = (size_t)(dia_npad + kFixThreads * kFixR) * 4;
+    if (cudaMallocAsync((void **)&mk, bytes, s) != cudaSuccess) {
+        cudaGetLastError();
+        return CACG_OK;
+    }
+    CACG_CUDA_TRY(cudaMallocAsync((void **)&bad, sizeof(int), s));
+    CACG_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int), s));
+    CACG_CUDA_TRY(cudaMemsetAsync(mk, 0, bytes, s));
+    int dm = -1;
+    for (int d = 0; d < dia_ndiag; ++d)
+        if (dia.off[d] == 0) dm = d;
+    const int blocks = (int)std::min<int64_t>((dia_npad + 255) / 256, (int64_t)sm_count() * 16);
+    fix_mask_kernel<<<blocks, 256, 0, s>>>(n, dia_npad, dia, dm, dia64, cv, mk, bad);
+    int rc = check_launch();
+    int hbad = 1;
+    if (rc == CACG_OK && (cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s) !=
+                              cudaSuccess ||
+                          cudaStreamSynchronize(s) != cudaSuccess))
+        rc = CACG_ERR_CUDA;
+    cudaFreeAsync(bad, s);
+    if (rc != CACG_OK || hbad) {
+        cudaFreeAsync(mk, s);
+        return rc;
+    }
+    fix_mask = mk;
+    fix_c = cv;
+    fix_dmain = dm;
+    owned_bytes += bytes;
+    return CACG_OK;
+}
+
+size_t dia_fix_scratch_bytes(int64_t n, int w) {
+    const size_t wp = (size_t)(w + 1) / 2 * 2;
+    return (size_t)n * wp * 8;
+}
+size_t dia_fix_small_bytes(int w) { return ((size_t)2 * kFixMaxBlocks * w + w + 1) * 4; }
+
+int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, int64_t ldx,
+                   double *Y, int64_t ldy, const double *Z1, int64_t ldz1, const double *Z2,
+                   int64_t ldz2, double ca, double cb, double cc, void *xi, void *small, FixChain *chain) {
+    if (!A->fix_mask || !xi || !small || w <= 0 || w > 2 * kFixThreads) return CACG_ERR_UNSUPPORTED;
+    if ((double)A->nnz * w < kDiaFixMin) return CACG_ERR_UNSUPPORTED;
+    const double cac = ca * A->fix_c;
+    if (!std::isfinite(cac)) return CACG_ERR_UNSUPPORTED;
+    FixArgs a{};
+    a.n = A->n;
+    a.npad = A->dia_npad;
+    a.w = w;
+    a.wp = (w + 1) / 2 * 2;
+    a.cpr = a.wp / 2;
+    a.runs = std::max(1, std::min(kFixThreads / a.cpr, 128));
+    a.mask = A->fix_mask;
+    a.vals = A->dia64;
+    a.dmain = A->fix_dmain;
+    a.c = A->fix_c;
+    a.ca = ca, a.cb = cb, a.cc = cc;
+    int ex = 0;
+    const double fr = std::frexp(std::fabs(cac), &ex);  // 0.5 for a power of two
+    const bool pow2 = fr == 0.5 && ex > -300 && ex < 300;
+    a.c_pow2 = pow2 ? ex - 1 : 0;
+    a.fold = Z1 && Z1 == X && ldz1 == ldx;
+    a.X = X, a.Z1 = Z1, a.Z2 = Z2, a.Y = Y;
+    a.ldx = ldx, a.ldz1 = ldz1, a.ldz2 = ldz2, a.ldy = ldy;
+    a.xi = (const long long *)xi;
+    uint32_t *parts = (uint32_t *)small;  // two sets: of X, and of Y for the next step
+    int *scale = (int *)(parts + (size_t)2 * kFixMaxBlocks * w);
+    const bool known = chain && chain->of == X && chain->w == w;
+    uint32_t *part = parts + (size_t)(known ? chain->set : 0) * kFixMaxBlocks * w;
+    a.scale = scale;
+    const bool xvec = w % 2 == 0 && ldx % 2 == 0 && aligned16(X);
+    const bool vec = xvec && ldy % 2 == 0 && aligned16(Y) &&
+                     (!Z1 || (ldz1 % 2 == 0 && aligned16(Z1))) &&
+                     (!Z2 || (ldz2 % 2 == 0 && aligned16(Z2)));
+    const int tpr = xvec ? w / 2 : w;
+    const int rpb = kFixThreads / tpr > 0 ? kFixThreads / tpr : 1;
+    if (tpr > kFixThreads) return CACG_ERR_UNSUPPORTED;
+    int g1 = (int)std::max<int64_t>(
+        1, std::min<int64_t>(std::min<int64_t>(kFixMaxBlocks, 4 * (int64_t)sm_count()),
+                             (A->n + 4 * rpb - 1) / (4 * rpb)));
+    const size_t sm = (size_t)(w + 2) * 4;
+    int rc = CACG_OK;
+    if (known)
+        g1 = chain->nparts;  // the step that wrote X left its maxima
+    else if (xvec)
+        fix_colmax_kernel<true><<<g1, kFixThreads, sm, st>>>(A->n, w, X, ldx, part);
+    else
+        fix_colmax_kernel<false><<<g1, kFixThreads, sm, st>>>(A->n, w, X, ldx, part);
+    if (!known) rc = check_launch();
+    if (rc != CACG_OK) return rc;
+    const int rpc = kFixThreads / a.cpr;
+    const int g2 = (int)std::max<int64_t>(
+        1, std::min<int64_t>((int64_t)sm_count() * 6, (A->n + 4 * rpc - 1) / (4 * rpc)));
+    if (xvec)
+        fix_convert_kernel<true><<<g2, kFixThreads, sm, st>>>(A->n, w, a.wp, X, ldx, part, g1,
+                                                              (long long *)xi, scale);
+    else
+        fix_convert_kernel<false><<<g2, kFixThreads, sm, st>>>(A->n, w, a.wp, X, ldx, part, g1,
+                                                               (long long *)xi, scale);
+    rc = check_launch();
+    if (rc != CACG_OK) return rc;
+    const int64_t nblk = (A->n + (int64_t)a.runs * kFixR - 1) / ((int64_t)a.runs * kFixR);
+    const unsigned blocks = (unsigned)std::min<int64_t>(nblk, std::min<int64_t>((int64_t)sm_count() * 3, kFixMaxBlocks));
+    if (chain) {
+        const int set = known ? chain->set ^ 1 : 1;
+        a.ymax = parts + (size_t)set * kFixMaxBlocks * w;
+        *chain = FixChain{Y, w, set, (int)blocks};
+    }
+    const int mode = !Z2 && (!Z1 || a.fold) ? (pow2 ? kFixPow2 : kFixNone)
+                     : Z2 && cc == -1.0 && (!Z1 || a.fold) ? kFixStep
+                                                           : kFixAny;
+#define FIX_CASE(M)                                                              \
+    case M:                                                                      \
+        if (vec)                                                                 \
+            fix_spmm_kernel<true, M><<<blocks, kFixThreads, sm, st>>>(a, A->dia);  \
+        else                                                                     \
+            fix_spmm_kernel<false, M><<<blocks, kFixThreads, sm, st>>>(a, A->dia); \
+        break;
+    switch (mode) {
+        FIX_CASE(kFixPow2)
+        FIX_CASE(kFixNone)
+        FIX_CASE(kFixStep)
+        FIX_CASE(kFixAny)
+    }
+#undef FIX_CASE
+    return check_launch();
+}
+
+}  // namespace cacg

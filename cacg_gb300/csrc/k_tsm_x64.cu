@@ -29,7 +29,7 @@
 // half of the time's issue slots); X/R update m = 16 4.5 -> 0.77 ms; n = 65536,
 // k = 128 1.89 -> 0.16 ms, m = 32 0.93 -> 0.13 ms; product error 1.3e-16 of the
 // result (FMA chain 0.8e-16 to 1.1e-16), QR factors' error unchanged.
-// A row that no scale holds (Inf, NaN, or magnitudes below 2^-959), or every
+// A row that no scale holds (Inf, NaN, or a largest magnitude beyond 2^+-400), or every
 // row when a column of the small matrix is such, is formed by FP64 FMAs in the
 // epilogue.  A wait that runs out sets kStatusTimeout.
 #include <algorithm>
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
     }
     __syncthreads();
     bool wbad = false;
-    if (tid < NB) colK[tid] = (uint32_t)x64_scale(colK[tid], &wbad);
+    if (tid < NB) colK[tid] = (uint32_t)x64_scale_mid(colK[tid], &wbad);
     const bool wide = __syncthreads_or(wbad) != 0;  // every row by FMAs
     for (int e = tid; e < Kp / 2 * NB; e += kXtThreads) {
         const int j = 2 * (e / NB), c = e % NB;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
 #pragma unroll
             for (int rg = 0; rg < kXtRG; ++rg) {
                 bool bad = wide;
-                E[rg] = x64_scale(key[rg], &bad);
+                E[rg] = x64_scale_mid(key[rg], &bad);
                 if (lc == 0) rowE[x * kXtM + 8 * (kXtRG * warp + rg) + lr] = bad ? -1 : E[rg];
                 if (more) pn[rg] = row_ptr(job + 1, rg, rvn[rg]);
                 key[rg] = 0u;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
                     const long long l = (long long)(D[4] * 16777216ll) +
                                         ((long long)D[5] * 65536 + (long long)D[6] * 256 + D[7]);
                     const int sc = E + (int)colK[cc + q] - (2154 - 40);
-                    v[q] = x64_make(h, l, sc);
+                    v[q] = x64_scaled(x64_join(h, l), (h | l) == 0, sc);
                 }
                 if (E < 0 && rv) {  // no scale for this row: FP64 FMAs
                     const double *a = (part ? g.A1 : g.A0) + row * g.lda;

@@ -119,7 +119,8 @@ int DevMatrix::create(const cacg_csr *A, bool want_f32, DevMatrix *M, cudaStream
         int rc = launch_cast_f64_f32(st, A->nnz, M->val, M->val32);
         if (rc) return rc;
     }
-    return M->build_dia(A, want_f32, st);
+    const int rc = M->build_dia(A, want_f32, st);
+    return rc != CACG_OK ? rc : M->build_fix(A, st);
 }
 
 int DevMatrix::ensure_f32(cudaStream_t st) {
@@ -146,6 +147,8 @@ void DevMatrix::release() {
     if (val32) cudaFreeAsync(val32, st);
     if (dia64) cudaFreeAsync(dia64, st);
     if (dia32) cudaFreeAsync(dia32, st);
+    if (fix_mask) cudaFreeAsync(fix_mask, st);
+    fix_mask = nullptr;
     rp = nullptr;
     ci = nullptr;
     val = nullptr;
@@ -163,6 +166,7 @@ static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 struct Layout {
     size_t S, Q, AQ, R, R32, R32p, Xff, Rff, Bnorm, small, gram, norm, lanczos, total;
     size_t o_S, o_Q, o_AQ, o_R, o_R32, o_R32p, o_Xff, o_Rff, o_small, o_gram, o_norm, o_lanczos;
+    size_t xi, fixs, o_xi, o_fixs;  // fixed-point copy of an n x m block, its scales
     size_t Ssl, R32sl, o_Ssl, o_Qsl, o_AQsl, o_R32sl;
     bool slices;
 };
@@ -181,7 +185,10 @@ static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slice
     const int k = s * m;
     const size_t es = prec == CACG_MIXED ? 4 : 8;
     L.slices = slices;
-    L.S = L.Q = L.AQ = align256((size_t)n * k * es + 64);
+    // FP64: the S buffer also holds the fixed-point copy of Q, an even number of
+    // columns wide
+    const int ks = prec == CACG_FP64 ? (k + 1) / 2 * 2 : k;
+    L.S = L.Q = L.AQ = align256((size_t)n * ks * es + 64);
     L.R = align256((size_t)n * m * 8);
     L.R32 = prec == CACG_MIXED ? align256((size_t)n * m * 4) : 0;
     // R32 again with its rows padded to 16 bytes, for the TMA-fed Gram when m
@@ -205,6 +212,8 @@ static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slice
                            : (size_t)0));
     L.norm = align256(norm_workspace_doubles(n, std::max(m, 2)) * sizeof(double) + 4096);
     L.lanczos = lanczos ? align256((size_t)3 * n * 8) : 0;
+    L.xi = prec == CACG_FP64 ? align256(dia_fix_scratch_bytes(n, m)) : 0;
+    L.fixs = prec == CACG_FP64 ? align256(dia_fix_small_bytes(k)) : 0;
     size_t o = 0;
     L.o_S = o; o += L.S;
     L.o_Q = o; o += L.Q;
@@ -218,6 +227,8 @@ static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slice
     L.o_gram = o; o += L.gram;
     L.o_norm = o; o += L.norm;
     L.o_lanczos = o; o += L.lanczos;
+    L.o_xi = o; o += L.xi;
+    L.o_fixs = o; o += L.fixs;
     L.o_Ssl = o; o += L.Ssl;
     L.o_Qsl = o; o += L.Ssl;
     L.o_AQsl = o; o += L.Ssl;
@@ -467,6 +478,7 @@ struct SolveBuffers {
     float *Xff;  // n x m hi, then n x m lo (mixed mode's float-float residual)
     float *Rff;  // the same for R (the float-float state of the mixed mode)
     double *lz;  // 3 x n (Lanczos)
+    void *xi, *fixs;  // FP64: fixed-point operand of the one-value SpMM, its scales
     Slices Ssl, Qsl, AQsl, R32sl;  // bf16 slice planes (mixed mode, when enabled)
 };
 
@@ -498,6 +510,8 @@ static void carve(char *base, const Layout &L, int m, int k, SolveBuffers *b) {
     b->norm_ws = (double *)(base + L.o_norm);
     b->norm_ws_doubles = (int64_t)((L.norm - 4096) / sizeof(double));
     b->lz = L.lanczos ? (double *)(base + L.o_lanczos) : nullptr;
+    b->xi = L.xi ? base + L.o_xi : nullptr;
+    b->fixs = L.fixs ? base + L.o_fixs : nullptr;
 }
 
 static void carve_slices(char *base, const Layout &L, int64_t n, int m, int k, SolveBuffers *b) {
@@ -579,8 +593,17 @@ struct Solver {
     // matrix has one (bit-identical to the CSR kernel), else over CSR.
     template <typename T>
     int spmm(const T *X, int64_t ldx, T *Y, int64_t ldy, int w, const T *Z1, int64_t ldz1,
-             const T *Z2, int64_t ldz2, double ca, double cb, double cc) {
+             const T *Z2, int64_t ldz2, double ca, double cb, double cc,
+             FixChain *chain = nullptr) {
         if (uses_dia()) {
+            if constexpr (std::is_same<T, double>::value) {
+                // the A Q product's operand is converted into the S buffer, free there
+                if (planes64() && p.spmm_format == CACG_SPMM_AUTO && w <= k) {
+                    int rc = launch_dia_fix(st, A, w, X, ldx, Y, ldy, Z1, ldz1, Z2, ldz2, ca, cb,
+                                            cc, w <= m ? b.xi : b.S, b.fixs, chain);
+                    if (rc != CACG_ERR_UNSUPPORTED) return rc;
+                }
+            }
             if constexpr (std::is_same<T, float>::value) {
                 if (p.spmm_format == CACG_SPMM_AUTO) {
                     int rc = launch_dia_ring(st, A, w, X, ldx, Y, ldy, Z1, ldz1, Z2, ldz2, ca, cb,
@@ -750,6 +773,7 @@ struct Solver {
         T *S = (T *)b.S;
         // basis T_1 .. T_{s-1} (T_0 = S[:, 0:m] already holds R)
         const double dn = (double)n, ees = (double)es();
+        FixChain chain;
         for (int j = 1; j < s; ++j) {
             const T *Tm1 = S + (size_t)(j - 1) * m;
             const T *Tm2 = j >= 2 ? S + (size_t)(j - 2) * m : nullptr;
@@ -765,7 +789,7 @@ struct Solver {
                 else
                     rc = spmm<T>(Tm1, k, S + (size_t)j * m, k, m, Tm1, k, Tm2, k, ca, cb, -1.0);
             } else {
-                rc = spmm<T>(Tm1, k, S + (size_t)j * m, k, m, Tm1, k, Tm2, k, ca, cb, -1.0);
+                rc = spmm<T>(Tm1, k, S + (size_t)j * m, k, m, Tm1, k, Tm2, k, ca, cb, -1.0, &chain);
             }
             prof.end();
             if (rc) return rc;

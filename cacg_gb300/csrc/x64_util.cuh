@@ -41,6 +41,14 @@ __device__ __forceinline__ int x64_scale(uint32_t key, bool *bad) {
     return e < kXMinExp ? kXMinExp : e;
 }
 
+// the same where results are scaled by exponent-field additions alone: scales
+// within 2^+-400 (x64_scaled's range for a product of two)
+__device__ __forceinline__ int x64_scale_mid(uint32_t key, bool *bad) {
+    const int e = (int)(key >> 20);
+    if (key != 0u && (e < 1023 - 400 || e > 1023 + 400)) *bad = true;
+    return key == 0u ? 1023 : e;
+}
+
 // the seven balanced digits of x at scale E, biased by 128: bytes 0 .. 5 of
 // (hi, lo) are d_0 + 128 .. d_5 + 128, the top 16 bits d_6 + 128 (0 .. 256)
 __device__ __forceinline__ void x64_digits(double x, int E, uint32_t &lo, uint32_t &hi) {
@@ -79,14 +87,32 @@ __device__ __forceinline__ void x64_planes2(double x0, double x1, int E0, int E1
         asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(w[p]) : "r"(u[p]), "r"(0x64806480u));
 }
 
-// (h 2^32 + l) 2^sc as FP64 (h and l exact in FP64): one rounding, the power of
-// two goes into the exponent field where it fits
-__device__ __forceinline__ double x64_make(long long h, long long l, int sc) {
-    const double t = fma((double)h, 4294967296.0, (double)l);
-    if (sc > -900 && sc < 900)
-        return (h | l) == 0 ? 0.0
-                            : __hiloint2double(__double2hiint(t) + (sc << 20), __double2loint(t));
-    return scalbn(t, sc);
+// h 2^32 + l as FP64, rounded once (|h|, |l| < 2^50): both are put into a
+// double's significand by integer additions, so the FP64 pipe does two additions
+// (a conversion from 64 bits holds it for several times as long)
+__device__ __forceinline__ double x64_join(long long h, long long l) {
+    const double a = __longlong_as_double(0x4538000000000000ll + h);  // 1.5 2^84 + h 2^32
+    const double b = __longlong_as_double(0x4338000000000000ll + l);  // 1.5 2^52 + l
+    return (a - (0x1.8p84 + 0x1.8p52)) + b;                           // the difference is exact
+}
+
+// v as FP64, rounded to nearest (ties away from zero), by integer instructions
+// alone: for kernels whose FP64 pipe is the busier one
+__device__ __forceinline__ double x64_from_ll(long long v) {
+    const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+    const int z = __clzll((long long)m);
+    const unsigned long long u = m << (z & 63);  // leading bit at 63 (0 for 0)
+    // the leading bit of u >> 11 adds one to the exponent field, and so does a rounding carry
+    const unsigned long long r = (u >> 11) + ((u >> 10) & 1ull);
+    const uint32_t e = u ? (uint32_t)(1023 + 62 - z) << 20 : 0u;
+    return __hiloint2double((int)(((uint32_t)(r >> 32) + e) | ((uint32_t)(v >> 32) & 0x80000000u)),
+                            (int)(uint32_t)r);
+}
+
+// t 2^sc, the power of two added to the exponent field (|sc| < 900, |t| between 1
+// and 2^79, or `zero`)
+__device__ __forceinline__ double x64_scaled(double t, bool zero, int sc) {
+    return zero ? 0.0 : __hiloint2double(__double2hiint(t) + (sc << 20), __double2loint(t));
 }
 
 // Instruction descriptor of kind::f16 with fp16 inputs and FP32 accumulation

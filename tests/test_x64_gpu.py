@@ -131,3 +131,66 @@ def test_solves_with_plane_products(kind, N, m, s):
     assert info["status"] == 0
     assert abs(info["iterations"] - ito) <= 1
     assert np.linalg.norm(X - Xo) <= 1e-6 * np.linalg.norm(Xo)
+
+
+def _residual_norms(rp, ci, v, B, X):
+    """Column norms of B - A X, rows summed in extended precision."""
+    AX = np.zeros(X.shape, np.longdouble)
+    rows = np.repeat(np.arange(len(rp) - 1), np.diff(rp))
+    for c in range(X.shape[1]):
+        t = v.astype(np.longdouble) * X[ci, c]
+        AX[:, c] = np.add.reduceat(t, rp[:-1])
+    assert np.all(np.diff(rp) > 0) and len(rows) == len(v)
+    return np.sqrt(((B - AX) ** 2).sum(0))
+
+
+@pytest.mark.parametrize("kind,N,m", [("lap2d", 1423, 1), ("lap2d", 827, 3), ("lap2d", 360, 16),
+                                      ("lap3d7", 67, 5), ("lap3d7", 40, 32), ("st3d27", 40, 7),
+                                      ("st3d27", 32, 16), ("st3d27", 61, 2)])
+@pytest.mark.parametrize("scale", [1.0, -0.3, 1e-30])
+def test_fixed_point_spmm_residual(kind, N, m, scale):
+    """B - A X of a one-value stencil matrix (no iterations: the residual alone).  An entry of
+    A X is within (27 2^-58 + 35 2^-53) 27 max|X| |c|, max|X| < 5.5 and the residual's RMS
+    above 4 |c|: 2e-13 of a column's norm."""
+    rp, ci, v = cg.gen_matrix(kind, N, 0.05)
+    v = v * scale  # another off-diagonal value, not a power of two
+    n = len(rp) - 1
+    assert len(v) * m >= 1e7  # the kernel's range
+    rng = np.random.default_rng(3)
+    X = np.clip(rng.standard_normal((n, m)), -5.5, 5.5)
+    X[:, 0] *= 1e-9  # a scale per column
+    B = rng.standard_normal((n, m)) * 2 * abs(scale)
+    B[:, 0] *= 1e-9
+    _, info = cg.solve(rp, ci, v, B, X0=X, s=4, bounds=("given", 0.05, 60.0), tol=1e-8, maxit=0)
+    ref = _residual_norms(rp, ci, v, B, X).astype(np.float64)
+    got = info["true_relres"] * np.linalg.norm(B, axis=0)
+    assert np.all(np.abs(got - ref) <= 2e-13 * ref)
+
+
+@pytest.mark.parametrize("kind,N,m,s", [("lap2d", 281, 9, 3), ("lap3d7", 33, 16, 4),
+                                        ("st3d27", 24, 16, 5), ("st3d27", 26, 13, 3)])
+def test_fixed_point_spmm_solves(kind, N, m, s):
+    """Basis steps and A Q with it, even and odd widths: the solution's residual, in numpy."""
+    rp, ci, v = cg.gen_matrix(kind, N, 0.1)
+    n = len(rp) - 1
+    B = cg.gen_rhs("normal", n, m, 11)
+    X, info = cg.solve(rp, ci, v, B, s=s, bounds="gerschgorin", tol=1e-9, maxit=400)
+    assert info["status"] == 0
+    r = _residual_norms(rp, ci, v, B, X).astype(np.float64) / np.linalg.norm(B, axis=0)
+    assert np.all(r <= 1.01e-9)
+    assert np.all(np.abs(r - info["true_relres"]) <= 1e-13)
+
+
+def test_fixed_point_spmm_outside_range():
+    """An infinite entry: the FMA path's pattern of Inf and NaN (the solve breaks down)."""
+    rp, ci, v = cg.gen_matrix("lap3d7", 73, 0.1)
+    n = len(rp) - 1
+    B = cg.gen_rhs("normal", n, 4, 5)
+    X0 = np.zeros_like(B)
+    X0[n // 2, 1] = np.inf
+    for fmt in ("auto", "dia_unstaged"):
+        _, info = cg.solve(rp, ci, v, B, X0=X0, s=4, bounds=("given", 0.1, 12.1), maxit=0,
+                           spmm_format=fmt)
+        assert np.array_equal(np.isfinite(info["true_relres"]), [True, False, True, True])
+        # X0's other columns are zero: their residual is B, summed in another order only
+        assert np.all(np.abs(info["true_relres"][[0, 2, 3]] - 1.0) <= n * 2.0 ** -53)
