@@ -29,7 +29,8 @@
 // higher fraction of HBM than the generic batched kernels) run on per-request
 // stream workers; CACG_SERVER_STREAMS sends every request there (the
 // previous design, kept for comparison).  max_active bounds the requests in
-// flight on both paths together.
+// flight on both paths together.  FP64 requests on few diagonals leave the
+// batched kernels from kFp64BatchRows rows on.
 //
 // Stream priorities: small requests (the engine's stream, or a stream worker
 // serving a request of at most batch_max_rows rows) run at the device's
@@ -124,6 +125,33 @@ static bool batch_eligible(const cacg_params &p, int m) {
            (p.bounds_mode == CACG_BOUNDS_GERSCHGORIN || p.bounds_mode == CACG_BOUNDS_GIVEN) &&
            (p.precision == CACG_FP64 || p.precision == CACG_MIXED) && p.maxit >= 0;
 }
+
+// Whether the nonzeros seem to lie on few diagonals (a DIA view): up to 256 rows
+// spread over the matrix hold at most kDiaMax distinct offsets.
+static bool looks_diagonal(const cacg_csr *A) {
+    int64_t offs[kDiaMax];
+    int cnt = 0;
+    const int64_t step = std::max<int64_t>(1, A->n / 256);
+    for (int64_t i = 0; i < A->n; i += step) {
+        for (int32_t e = A->row_ptr[i]; e < A->row_ptr[i + 1]; ++e) {
+            const int64_t o = (int64_t)A->col_idx[e] - i;
+            int j = 0;
+            while (j < cnt && offs[j] != o) ++j;
+            if (j < cnt) continue;
+            if (cnt == kDiaMax) return false;
+            offs[cnt++] = o;
+        }
+    }
+    return cnt > 0;
+}
+
+// FP64 requests of more rows than this leave the batched kernels (which do their
+// products on the FP64 pipe) for a stream worker, whose solver does them on the
+// tensor cores, if the caller has set no row limit and the matrix has diagonals
+// (others keep their FMA sums).  Bursts of 16 requests up to 35721 rows: 78 ms
+// all batched, 30 ms with 2048 or 4096 as the limit; of 20 up to 7921 rows: 33.6,
+// 16.4, 19.0; of 24 up to 59319 rows: 165, 55, 55.
+constexpr int64_t kFp64BatchRows = 2048;
 
 // ----------------------------------------------------------- autotuner
 // Per device and class: blocks per SM of each batched kernel kind, measured
@@ -1037,18 +1065,24 @@ int cacg_server_submit(cacg_server *srv, const cacg_csr *A, const double *B, int
     r->p = *p;
     r->X_out = X_out;
     r->batched = s->engine && batch_eligible(*p, m) && A->n <= s->small_rows();
-    if (r->batched) {
-        r->cost = blayout(A->n, A->nnz, m, p->s, p->precision == CACG_MIXED).total;
-    } else {
+    auto stream_cost = [&]() {
         // CSR (+ FP32 values) and, for diagonal-structured matrices, the DIA
         // view (at most 1.5 x nnz entries of FP64 + FP32 values)
         size_t mat = (size_t)(A->n + 1) * 4 + (size_t)A->nnz * (4 + 8 + 16) +
                      (p->precision == CACG_MIXED ? (size_t)A->nnz * 4 : 0) +
                      (size_t)A->nnz * 18 + (size_t)(A->n + 64) * 12 * 2;
-        r->cost = mat + 2 * (size_t)A->n * m * 8 +
-                  solve_workspace_bytes(A->n, m, p->s, p->precision,
-                                        p->bounds_mode == CACG_BOUNDS_LANCZOS);
-    }
+        return mat + 2 * (size_t)A->n * m * 8 +
+               solve_workspace_bytes(A->n, m, p->s, p->precision,
+                                     p->bounds_mode == CACG_BOUNDS_LANCZOS);
+    };
+    if (r->batched && s->cfg.batch_max_rows == 0 && p->precision == CACG_FP64 &&
+        p->gram_variant == CACG_GRAM_AUTO && p->spmm_format != CACG_SPMM_CSR &&
+        A->n > kFp64BatchRows && looks_diagonal(A) &&
+        (int64_t)stream_cost() <= s->cfg.mem_budget_bytes)
+        r->batched = false;
+    r->cost = r->batched
+                  ? blayout(A->n, A->nnz, m, p->s, p->precision == CACG_MIXED).total
+                  : stream_cost();
     if ((int64_t)r->cost > s->cfg.mem_budget_bytes) return CACG_ERR_BUSY;
     {
         std::lock_guard<std::mutex> lk(s->mu);

@@ -253,7 +253,8 @@ class Server:
                  graphs: bool = True, batch_max_rows: int = 0):
         """engine: "batched" (one launch per phase over all admitted requests,
         steps replayed from CUDA graphs; requests above batch_max_rows rows,
-        0 = 65536, -1 = no limit, take the per-request path) or "streams" (a
+        0 = 65536 and, for FP64 requests on few diagonals, 2048, -1 = no
+        limit, take the per-request path) or "streams" (a
         stream and the single-request solver per request)."""
         cfg = L.CacgServerConfig(mem_budget_bytes, max_active,
                                  {"batched": 0, "streams": 1}[engine], 0 if graphs else 1,

@@ -350,7 +350,9 @@ typedef struct cacg_server_config {
                                  instead of replaying its CUDA graph */
     int32_t batch_max_rows;   /* batched engine: requests with more rows take a
                                  stream worker and the single-request solver's
-                                 kernels (0: 65536; negative: no limit) */
+                                 kernels (0: 65536, and 2048 for FP64 requests
+                                 whose matrix has few diagonals; negative: no
+                                 limit) */
     int32_t reserved[4];
 } cacg_server_config;
 
