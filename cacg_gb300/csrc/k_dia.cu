@@ -861,20 +861,30 @@ int launch_dia_spmm(cudaStream_t st, const DevMatrix *A, int w, const T *X, int6
     const bool vec = w % VN == 0 && ldx % VN == 0 && ldy % VN == 0 && aligned16(X) &&
                      aligned16(Y) && (!Z1 || (ldz1 % VN == 0 && aligned16(Z1))) &&
                      (!Z2 || (ldz2 % VN == 0 && aligned16(Z2)));
-    // narrow blocks (<= 8 chunks a row): 4 rows a thread and more CTAs per SM
-    // hide the L2 latency of the X window; wide blocks: 8 rows a thread
-    // amortise the window over more FMAs
-    if (vec && w / VN <= 8)
-        return launch_dia_kernel<T, kDiaR / 2, VN>(st, A, vals, w, X, ldx, Y, ldy, Z1, ldz1, Z2,
+    // rows a thread: narrow blocks (<= 8 chunks a row) and unaligned ones (a
+    // column slice of width m % 4 != 0, scalar columns) take 4 and more CTAs per
+    // SM, which hides the L2 latency of the X window; wide blocks take 8, which
+    // amortises the window over more FMAs.  One row where that leaves too few
+    // threads for the SMs (the same FMAs in the same order): FP64, n = 16384, w = 1
+    // 7.3 us with 4 rows, 5.4 with one; n = 32768, w = 4 14.1 and 13.0; but n =
+    // 50653, w = 5 11.3 and 16.2, n = 32768, w = 16 16.4 and 28.9.
+    const int64_t cpr = vec ? w / VN : w;
+    int R = vec && cpr > 8 ? kDiaR : kDiaR / 2;
+    if (A->n * cpr / R < (int64_t)sm_count() * 128) R = 1;
+#define DIA_CASE(RR)                                                                            \
+    case RR:                                                                                    \
+        return vec ? launch_dia_kernel<T, RR, VN>(st, A, vals, w, X, ldx, Y, ldy, Z1, ldz1, Z2, \
+                                                  ldz2, ca, cb, cc)                             \
+                   : launch_dia_kernel<T, RR, 1>(st, A, vals, w, X, ldx, Y, ldy, Z1, ldz1, Z2,  \
+                                                 ldz2, ca, cb, cc);
+    switch (R) {
+        DIA_CASE(1)
+        DIA_CASE(4)
+        default:
+            return launch_dia_kernel<T, kDiaR, VN>(st, A, vals, w, X, ldx, Y, ldy, Z1, ldz1, Z2,
                                                    ldz2, ca, cb, cc);
-    if (vec)
-        return launch_dia_kernel<T, kDiaR, VN>(st, A, vals, w, X, ldx, Y, ldy, Z1, ldz1, Z2,
-                                               ldz2, ca, cb, cc);
-    // unaligned blocks (a column slice of width m % 4 != 0, e.g. a basis
-    // step T_j inside the n x k basis): scalar columns, still 4 rows a thread
-    // with the values staged (the same FMAs in the same order as R = 1)
-    return launch_dia_kernel<T, kDiaR / 2, 1>(st, A, vals, w, X, ldx, Y, ldy, Z1, ldz1, Z2, ldz2,
-                                              ca, cb, cc);
+    }
+#undef DIA_CASE
 }
 
 template int launch_dia_spmm<float>(cudaStream_t, const DevMatrix *, int, const float *, int64_t,

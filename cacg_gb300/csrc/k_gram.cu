@@ -212,6 +212,83 @@ __global__ void __launch_bounds__(kGramMaxThreads)
     (void)kb;
 }
 
+// The same sums for few outputs: a thread owns kE outputs wherever they lie
+// (the upper triangle of a symmetric leading block, then the columns past it)
+// instead of a 4 x 4 micro-tile, so every FP64 instruction carries 32 useful
+// lanes.  A row of an output is one FMA of 64 clocks on the quadrant's FP64 pipe
+// against two 8-byte shared loads, so the loads a micro-tile would share do not
+// matter.  Chunks, row order and partial tiles are gram_fma_kernel's: the same
+// bits.  FP64, n = 50021, symmetric k = 24 + 6: 14 FMA warp instructions a row
+// instead of 32.
+template <int kE>
+__global__ void __launch_bounds__(kGramMaxThreads)
+    gram_flat_kernel(int64_t n, int64_t rows_per_chunk, const double *__restrict__ L, int64_t ldl,
+                     int ka, const double *__restrict__ R1, int64_t ldr1, int kb1,
+                     const double *__restrict__ R2, int64_t ldr2, int kb2, int BA, int BB,
+                     double *__restrict__ part, int sym) {
+    constexpr int KT = GramKT<double>::value;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *Ls[2], *Rs[2];
+    Ls[0] = reinterpret_cast<double *>(smem_raw);
+    Rs[0] = Ls[0] + KT * BA;
+    Ls[1] = Rs[0] + KT * BB;
+    Rs[1] = Ls[1] + KT * BA;
+    const int kb = kb1 + kb2;
+    const int ntri = sym ? ka * (ka + 1) / 2 : 0;
+    const int rest0 = sym ? kb1 : 0, nrest = ka * (kb - rest0);
+    int ia[kE], ib[kE];
+    bool on[kE];
+    double acc[kE];
+#pragma unroll
+    for (int e = 0; e < kE; ++e) {
+        int t = threadIdx.x + e * blockDim.x;
+        on[e] = t < ntri + nrest;
+        ia[e] = ib[e] = 0;
+        acc[e] = 0.0;
+        if (on[e] && t < ntri) {
+            int a = 0;
+            while (t >= ka - a) {
+                t -= ka - a;
+                ++a;
+            }
+            ia[e] = a;
+            ib[e] = a + t;
+        } else if (on[e]) {
+            t -= ntri;
+            ia[e] = t / (kb - rest0);
+            ib[e] = rest0 + t % (kb - rest0);
+        }
+    }
+    const int64_t rbeg = (int64_t)blockIdx.x * rows_per_chunk;
+    const int64_t rend = min(n, rbeg + rows_per_chunk);
+    int64_t r0 = rbeg;
+    if (r0 < rend)
+        stage_slab<double, KT>(Ls[0], Rs[0], BA, BB, r0, rend, L, ldl, ka, 0, R1, ldr1, kb1, R2,
+                               ldr2, kb2, 0);
+    cp_async_commit();
+    int buf = 0;
+    for (; r0 < rend; r0 += KT, buf ^= 1) {
+        if (r0 + KT < rend)
+            stage_slab<double, KT>(Ls[buf ^ 1], Rs[buf ^ 1], BA, BB, r0 + KT, rend, L, ldl, ka, 0,
+                                   R1, ldr1, kb1, R2, ldr2, kb2, 0);
+        cp_async_commit();
+        cp_async_wait_1();
+        __syncthreads();
+        const double *ls = Ls[buf], *rs = Rs[buf];
+#pragma unroll
+        for (int r = 0; r < KT; ++r)
+#pragma unroll
+            for (int e = 0; e < kE; ++e)
+                acc[e] = fma(ls[r * BA + ia[e]], rs[r * BB + ib[e]], acc[e]);
+        __syncthreads();
+    }
+    cp_async_wait_all();
+    double *out = part + (size_t)blockIdx.x * (size_t)BA * BB;
+#pragma unroll
+    for (int e = 0; e < kE; ++e)
+        if (on[e]) out[ia[e] * BB + ib[e]] = acc[e];
+}
+
 // ------------------------------------------------------------ DMMA variant
 // FP64 tensor core: mma.sync.aligned.m8n8k4.row.col.f64.  A = L^T (8 x 4 per
 // step), B = R (4 x 8).  Each warp owns a list of 8x8 output tiles.
@@ -465,11 +542,34 @@ int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl
                                                                   ws);
             }
         } else {
-            set_smem_attr(gram_fma_kernel<T>, (int)max_smem_optin());
-            gram_fma_kernel<T><<<grid, p.threads, p.smem, st>>>(n, p.rows_per_chunk, L, ldl,
-                                                                ka, R1, ldr1, kb1, R2, ldr2,
-                                                                kb2, p.BA, p.BB, p.tilesB, ws,
-                                                                sym);
+            bool flat = false;
+            if constexpr (std::is_same<T, double>::value) {
+                // outputs a thread: one tile and at most two (the micro-tiles' warps
+                // fill up beyond)
+                const int outs = sym ? ka * (ka + 1) / 2 + ka * kb2 : ka * kb;
+                flat = p.tilesA == 1 && p.tilesB == 1 && outs <= 2 * kGramMaxThreads;
+                if (flat) {
+                    const int e = outs <= kGramMaxThreads ? 1 : 2;
+                    const int th = round_up((outs + e - 1) / e, 32);
+                    set_smem_attr(gram_flat_kernel<1>, (int)max_smem_optin());
+                    set_smem_attr(gram_flat_kernel<2>, (int)max_smem_optin());
+                    if (e == 1)
+                        gram_flat_kernel<1><<<p.nchunks, th, p.smem, st>>>(
+                            n, p.rows_per_chunk, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, p.BA,
+                            p.BB, ws, sym);
+                    else
+                        gram_flat_kernel<2><<<p.nchunks, th, p.smem, st>>>(
+                            n, p.rows_per_chunk, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, p.BA,
+                            p.BB, ws, sym);
+                }
+            }
+            if (!flat) {
+                set_smem_attr(gram_fma_kernel<T>, (int)max_smem_optin());
+                gram_fma_kernel<T><<<grid, p.threads, p.smem, st>>>(n, p.rows_per_chunk, L, ldl,
+                                                                    ka, R1, ldr1, kb1, R2, ldr2,
+                                                                    kb2, p.BA, p.BB, p.tilesB, ws,
+                                                                    sym);
+            }
         }
         int rc = check_launch();
         if (rc != CACG_OK) return rc;

@@ -40,6 +40,8 @@ constexpr int kXgM = 128;                          // MMA M (L columns, zero-pad
 constexpr int kXgGroup = 4;                        // steps per accumulation group (128 rows)
 constexpr int kXgConvWarps = 16;
 constexpr int kXgThreads = 32 * kXgConvWarps + 32;  // + the MMA issuer's warp
+constexpr int kXgMaxUnits = 6;  // (8 columns, 8 rows) units per warp and step
+constexpr int kXgMaxStages = 4;  // steps of raw rows in flight
 constexpr unsigned kXgABytes = kXPlanes * kXgM * kXgKT * 2;  // A planes of one step
 
 struct XgOperands {
@@ -112,7 +114,7 @@ __device__ __forceinline__ void xg_cp8(void *smem, const void *g, int bytes) {
 template <int NC, bool VEC>
 __global__ void __launch_bounds__(kXgThreads, 1)
     gram_x64_kernel(int64_t n, int64_t rows_per_chunk, XgOperands o, int BA, int tilesB, int sub,
-                    const uint32_t *__restrict__ emax, double *__restrict__ part,
+                    int stages, const uint32_t *__restrict__ emax, double *__restrict__ part,
                     int *__restrict__ flags) {
     constexpr int NB = 16 * NC;
     constexpr int NQ = NB / 4;  // accumulator columns per converter thread
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     const int upw = (nunits + kXgConvWarps - 1) / kXgConvWarps;
     double2 *raw = reinterpret_cast<double2 *>(smem_raw + 2 * buf_bytes);
     int *esc = reinterpret_cast<int *>(smem_raw + 2 * buf_bytes +
-                                       (size_t)upw * kXgConvWarps * 32 * 16);
+                                       (size_t)stages * upw * kXgConvWarps * 32 * 16);
     uint64_t *sfull = reinterpret_cast<uint64_t *>(esc + kXgM + NB);
     uint64_t *sfree = sfull + 2;
     uint64_t *gdone = sfree + 2;
@@ -143,25 +145,67 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     const int64_t nsteps = rend > rbeg ? (rend - rbeg + kXgKT - 1) / kXgKT : 0;
     int *flag = flags + (size_t)blockIdx.x * gridDim.y + blockIdx.y;
 
-    // scales of the tile's columns
+    // scales of the tile's columns: from the maxima kernel, or, where the
+    // operands stay in L2, from a pass over the chunk's rows
     bool bad = false;
-    if (tid < BA + NB) {
-        const int c = tid < BA ? (a0 + tid < o.ka ? a0 + tid : -1)
-                               : (b0 + tid - BA < kb ? o.ka + b0 + tid - BA : -1);
-        uint32_t key = 0u;
-        if (c >= 0)
-            for (int s = 0; s < sub; ++s)
-                key = max(key, emax[((size_t)blockIdx.x * sub + s) * kc + c]);
-        esc[tid] = x64_scale(key, &bad);
+    if (emax) {
+        if (tid < BA + NB) {
+            const int c = tid < BA ? (a0 + tid < o.ka ? a0 + tid : -1)
+                                   : (b0 + tid - BA < kb ? o.ka + b0 + tid - BA : -1);
+            uint32_t key = 0u;
+            if (c >= 0)
+                for (int s = 0; s < sub; ++s)
+                    key = max(key, emax[((size_t)blockIdx.x * sub + s) * kc + c]);
+            esc[tid] = x64_scale(key, &bad);
+        }
+    } else {
+        uint32_t *keys = reinterpret_cast<uint32_t *>(esc);
+        if (tid < BA + NB) keys[tid] = 0u;
+        __syncthreads();
+        const int tpr = (BA + NB) / 2, rpb = kXgThreads / tpr;
+        const int r = tid / tpr, c = 2 * (tid % tpr);
+        if (r < rpb) {
+            auto col_ptr = [&](int cc, int64_t &ld) -> const double * {
+                if (cc < BA) {
+                    ld = o.ldl;
+                    return a0 + cc < o.ka ? o.L + a0 + cc : nullptr;
+                }
+                const int g = b0 + cc - BA;
+                ld = g < o.kb1 ? o.ldr1 : o.ldr2;
+                return g < o.kb1 ? o.R1 + g : g < kb ? o.R2 + (g - o.kb1) : nullptr;
+            };
+            int64_t l0, l1;
+            const double *q0 = col_ptr(c, l0), *q1 = col_ptr(c + 1, l1);
+            uint32_t k0 = 0u, k1 = 0u;
+            if constexpr (VEC) {
+                if (q0) {
+#pragma unroll 8
+                    for (int64_t row = rbeg + r; row < rend; row += rpb) {
+                        const double2 v = __ldg(reinterpret_cast<const double2 *>(q0 + row * l0));
+                        k0 = max(k0, x64_key(v.x));
+                        k1 = max(k1, x64_key(v.y));
+                    }
+                }
+            } else {
+#pragma unroll 4
+                for (int64_t row = rbeg + r; row < rend; row += rpb) {
+                    if (q0) k0 = max(k0, x64_key(__ldg(q0 + row * l0)));
+                    if (q1) k1 = max(k1, x64_key(__ldg(q1 + row * l1)));
+                }
+            }
+            atomicMax(&keys[c], k0);
+            atomicMax(&keys[c + 1], k1);
+        }
+        __syncthreads();
+        if (tid < BA + NB) esc[tid] = x64_scale(keys[tid], &bad);
     }
     if (__syncthreads_or(bad)) {
         if (tid == 0) *flag = 1;
         return;
     }
 
-    // A columns past BA stay zero
-    for (unsigned i = tid; i < 2 * buf_bytes / 16; i += kXgThreads)
-        reinterpret_cast<uint4 *>(smem_raw)[i] = make_uint4(0, 0, 0, 0);
+    // (A columns past BA keep whatever shared memory holds: they reach only the
+    // accumulator lanes past BA, which nobody reads)
     if (tid == 0) {
         t5_mbar_init(&sfull[0], kXgConvWarps);
         t5_mbar_init(&sfull[1], kXgConvWarps);
@@ -209,8 +253,9 @@ __global__ void __launch_bounds__(kXgThreads, 1)
         const double *pL = o.L + (rbeg + rowt) * o.ldl + a0 + c0;
         const double *p1 = o.R1 + (rbeg + rowt) * o.ldr1 + (b0 + c0 - BA);
         const double *p2 = o.R2 + (rbeg + rowt) * o.ldr2 + (b0 + c0 - BA - o.kb1);
-        auto copy_unit = [&](int u) {
-            double2 *dst = raw + u * (kXgConvWarps * 32) + tid;
+        double2 *slot = raw + tid;  // this thread's slots: stage st, unit u at (st upw + u) 512
+        auto copy_unit = [&](int st, int u) {
+            double2 *dst = slot + (st * upw + u) * (kXgConvWarps * 32);
             const int c = c0 + 32 * u;
             const bool rv = rleft > 0;
             auto src = [&](int e, bool &ok) -> const double * {
@@ -266,11 +311,18 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             if (lane == 0) t5_mbar_arrive(gfree);
             return true;
         };
-        for (int u = 0; u < upw; ++u)
-            if (warp + kXgConvWarps * u < nunits) copy_unit(u);
-        next_rows();
-        t5_cp_commit();
+        for (int st = 0; st < stages; ++st) {
+            if (st < nsteps)
+                for (int u = 0; u < upw; ++u)
+                    if (warp + kXgConvWarps * u < nunits) copy_unit(st, u);
+            next_rows();
+            t5_cp_commit();
+        }
+        const int toff = kg * (int)lbo_a + lr * 16 + lc * 2 + oct0 * 128;
+        const int boff = (int)kXgABytes + kg * (int)lbo_b + lr * 16 + lc * 2 +
+                         (oct0 - BA / 8) * 128;
         bool ok = true;
+        int st = 0;
         for (int64_t j = 0; j < nsteps && ok; ++j) {
             const int b = (int)(j & 1);
             if (j >= 2) {
@@ -281,33 +333,37 @@ __global__ void __launch_bounds__(kXgThreads, 1)
                     break;
                 }
             }
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            // this step's rows have landed; up to stages - 1 later steps are in flight
+            switch (stages) {
+                case 1: asm volatile("cp.async.wait_group 0;\n" ::: "memory"); break;
+                case 2: asm volatile("cp.async.wait_group 1;\n" ::: "memory"); break;
+                case 3: asm volatile("cp.async.wait_group 2;\n" ::: "memory"); break;
+                default: asm volatile("cp.async.wait_group 3;\n" ::: "memory"); break;
+            }
             unsigned char *dbase = smem_raw + b * buf_bytes;
-            const bool more = j + 1 < nsteps;
-#pragma unroll 2
-            for (int u = 0; u < upw; ++u) {
-                const int oct = oct0 + 4 * u;
-                if (warp + kXgConvWarps * u >= nunits) break;
-                const double2 x = raw[u * (kXgConvWarps * 32) + tid];
-                if (more) copy_unit(u);  // into this thread's slot, just read
+            const bool more = j + stages < nsteps;
+#pragma unroll
+            for (int u = 0; u < kXgMaxUnits; ++u) {
+                if (u >= upw || warp + kXgConvWarps * u >= nunits) break;
+                const double2 x = slot[(st * upw + u) * (kXgConvWarps * 32)];
+                if (more) copy_unit(st, u);  // into this thread's slot, just read
                 const int2 e = *reinterpret_cast<const int2 *>(esc + c0 + 32 * u);
                 uint32_t w[kXPlanes];
                 x64_planes2(x.x, x.y, e.x, e.y, w);
-                unsigned char *d;
-                unsigned pstride;
-                if (oct < BA / 8) {
-                    d = dbase + oct * 128 + kg * lbo_a;
-                    pstride = (kXgKT / 8) * lbo_a;
-                } else {
-                    d = dbase + kXgABytes + (oct - BA / 8) * 128 + kg * lbo_b;
-                    pstride = (NB / 8) * 128;
-                }
-                d += lr * 16 + lc * 2;
+                if (oct0 + 4 * u < BA / 8) {
+                    unsigned char *d = dbase + toff + u * 512;
 #pragma unroll
-                for (int p = 0; p < kXPlanes; ++p)
-                    *reinterpret_cast<uint32_t *>(d + p * pstride) = w[p];
+                    for (int p = 0; p < kXPlanes; ++p)
+                        *reinterpret_cast<uint32_t *>(d + p * (kXgKT / 8) * (int)lbo_a) = w[p];
+                } else {
+                    unsigned char *d = dbase + boff + u * 512;
+#pragma unroll
+                    for (int p = 0; p < kXPlanes; ++p)
+                        *reinterpret_cast<uint32_t *>(d + p * (NB / 8) * 128) = w[p];
+                }
             }
             next_rows();
+            if (++st == stages) st = 0;
             t5_cp_commit();
             t5_fence_proxy_async();
             __syncwarp();
@@ -386,54 +442,51 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     }
 }
 
-// Sum of the chunks' partials: four threads share an output, each sums a
-// contiguous quarter of the chunks in order, then the quarters are added in
+// Sum of the chunks' partials: 16 threads share an output, each sums a
+// contiguous sixteenth of the chunks in order, then the sixteenths are added in
 // order.  With a raised flag the same threads form the output from L, R1, R2.
-constexpr int kXrElems = 64;  // outputs per block
+constexpr int kXrElems = 32, kXrSlices = 16;
 
-__global__ void __launch_bounds__(4 * kXrElems)
+__global__ void __launch_bounds__(kXrSlices *kXrElems)
     gram_x64_reduce_kernel(const double *__restrict__ part, int nchunks, int ntiles, int BA, int NB,
                            int tilesB, int64_t n, XgOperands o, double *__restrict__ C1, int ldc1,
                            double *__restrict__ C2, int ldc2, const int *__restrict__ flags) {
-    __shared__ double qs[4][kXrElems];
+    __shared__ double qs[kXrSlices][kXrElems];
     const int el = threadIdx.x % kXrElems, q = threadIdx.x / kXrElems;
     const int kb = o.kb1 + o.kb2;
     const int idx = blockIdx.x * kXrElems + el;
     const bool active = idx < o.ka * kb;
     const int a = active ? idx / kb : 0, b = active ? idx % kb : 0;
-    int raised = 0;
-    for (int i = threadIdx.x; i < nchunks * ntiles; i += blockDim.x) raised |= flags[i];
-    raised = __syncthreads_or(raised);
     double s = 0.0;
-    if (!raised) {
+    {
         const int tile = (a / BA) * tilesB + (b / NB);
         const size_t off = (size_t)tile * BA * NB + (size_t)(a % BA) * NB + (b % NB);
         const size_t stride = (size_t)ntiles * BA * NB;
-        const int per = (nchunks + 3) / 4;
+        const int per = (nchunks + kXrSlices - 1) / kXrSlices;
         const int p1 = min(nchunks, q * per + per);
-        int p = q * per;
+        if (active)
+#pragma unroll 10
+            for (int p = q * per; p < p1; ++p) s += part[off + (size_t)p * stride];
+    }
+    int raised = 0;
+    for (int i = threadIdx.x; i < nchunks * ntiles; i += blockDim.x) raised |= flags[i];
+    if (__syncthreads_or(raised)) {
+        s = 0.0;
         if (active) {
-            for (; p + 8 <= p1; p += 8) {
-                double v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = part[off + (size_t)(p + u) * stride];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) s += v[u];
-            }
-            for (; p < p1; ++p) s += part[off + (size_t)p * stride];
-        }
-    } else if (active) {
-        const double *R = b < o.kb1 ? o.R1 + b : o.R2 + (b - o.kb1);
-        const int64_t ldr = b < o.kb1 ? o.ldr1 : o.ldr2;
-        const int64_t per = (n + 3) / 4;
-        const int64_t r1 = min(n, q * per + per);
+            const double *R = b < o.kb1 ? o.R1 + b : o.R2 + (b - o.kb1);
+            const int64_t ldr = b < o.kb1 ? o.ldr1 : o.ldr2;
+            const int64_t per = (n + kXrSlices - 1) / kXrSlices;
+            const int64_t r1 = min(n, q * per + per);
 #pragma unroll 8
-        for (int64_t r = q * per; r < r1; ++r) s = fma(o.L[r * o.ldl + a], R[r * ldr], s);
+            for (int64_t r = q * per; r < r1; ++r) s = fma(o.L[r * o.ldl + a], R[r * ldr], s);
+        }
     }
     qs[q][el] = s;
     __syncthreads();
     if (q == 0 && active) {
-        const double t = ((qs[0][el] + qs[1][el]) + qs[2][el]) + qs[3][el];
+        double t = qs[0][el];
+#pragma unroll
+        for (int i = 1; i < kXrSlices; ++i) t += qs[i][el];
         if (b < o.kb1)
             C1[(size_t)a * ldc1 + b] = t;
         else
@@ -443,7 +496,8 @@ __global__ void __launch_bounds__(4 * kXrElems)
 
 // ------------------------------------------------------------------- host
 struct XgPlan {
-    int BA, NB, tilesA, tilesB, nchunks, sub;
+    int BA, NB, tilesA, tilesB, nchunks, sub, stages;
+    bool scan;  // column maxima inside the product kernel
     int64_t rows_per_chunk, rows_per_sub;
     size_t smem, part_bytes, emax_bytes, total;
 };
@@ -466,8 +520,18 @@ static XgPlan plan_x64(int64_t n, int ka, int kb) {
     p.sub = (int)((p.rows_per_chunk + p.rows_per_sub - 1) / p.rows_per_sub);
     const int nunits = (p.BA / 8 + p.NB / 8) * (kXgKT / 8);
     const int upw = (nunits + kXgConvWarps - 1) / kXgConvWarps;
-    p.smem = 2 * ((size_t)kXgABytes + (size_t)(kXgKT / 8) * (kXPlanes * p.NB / 8) * 128) +
-             (size_t)upw * kXgConvWarps * 32 * 16 + (size_t)(kXgM + p.NB) * 4 + 6 * 8 + 16;
+    const size_t planes = 2 * ((size_t)kXgABytes + (size_t)(kXgKT / 8) * (kXPlanes * p.NB / 8) * 128);
+    const size_t tables = (size_t)(kXgM + p.NB) * 4 + 6 * 8 + 16;
+    const size_t stage = (size_t)upw * kXgConvWarps * 32 * 16;
+    // raw steps in flight: with few columns a step's work is shorter than the
+    // latency of its copies
+    p.stages = kXgMaxStages;
+    while (p.stages > 1 && planes + tables + p.stages * stage > max_smem_optin()) --p.stages;
+    p.smem = planes + tables + p.stages * stage;
+    // small operands are read twice by the product kernel, which saves a launch
+    // (n = 16384, k = 4 (+1): 22.1 us with the maxima kernel, 20.4 without; n = 50653,
+    // k = 20 (+5): 41.7 either way); larger ones by a maxima kernel on more blocks
+    p.scan = (double)n * (ka * p.tilesB + (double)kb * p.tilesA) * 8.0 <= 4e6;
     p.part_bytes = (size_t)p.nchunks * tiles * p.BA * p.NB * sizeof(double);
     p.emax_bytes = (size_t)p.nchunks * p.sub * (ka + kb) * 4;
     p.total = p.part_bytes + p.emax_bytes + (size_t)p.nchunks * tiles * sizeof(int) + 64;
@@ -492,8 +556,8 @@ template <int NC, bool VEC>
 static void xg_launch(dim3 grid, const XgPlan &p, cudaStream_t st, int64_t n, const XgOperands &o,
                       const uint32_t *emax, double *part, int *flags) {
     set_smem_attr(gram_x64_kernel<NC, VEC>, (int)max_smem_optin());
-    gram_x64_kernel<NC, VEC><<<grid, kXgThreads, p.smem, st>>>(n, p.rows_per_chunk, o, p.BA,
-                                                               p.tilesB, p.sub, emax, part, flags);
+    gram_x64_kernel<NC, VEC><<<grid, kXgThreads, p.smem, st>>>(
+        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan ? nullptr : emax, part, flags);
 }
 
 int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
@@ -513,13 +577,15 @@ int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, in
                      ldr1 % 2 == 0 && aligned16(L) && aligned16(R1) &&
                      (kb2 == 0 || (ldr2 % 2 == 0 && aligned16(R2)));
     const dim3 mgrid(p.nchunks, p.sub);
-    if (vec)
+    int rc = CACG_OK;
+    if (p.scan) {
+    } else if (vec)
         gram_x64_colmax_kernel<true><<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o,
                                                             emax);
     else
         gram_x64_colmax_kernel<false><<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o,
                                                              emax);
-    int rc = check_launch();
+    if (!p.scan) rc = check_launch();
     if (rc != CACG_OK) return rc;
     const dim3 grid(p.nchunks, p.tilesA * p.tilesB);
 #define XG_CASE(NC)                                                       \
@@ -540,7 +606,7 @@ int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, in
 #undef XG_CASE
     rc = check_launch();
     if (rc != CACG_OK) return rc;
-    gram_x64_reduce_kernel<<<(ka * kb + kXrElems - 1) / kXrElems, 4 * kXrElems, 0, st>>>(
+    gram_x64_reduce_kernel<<<(ka * kb + kXrElems - 1) / kXrElems, kXrSlices * kXrElems, 0, st>>>(
         part, p.nchunks, p.tilesA * p.tilesB, p.BA, p.NB, p.tilesB, n, o, C1, ldc1, C2, ldc2, flags);
     return check_launch();
 }

@@ -509,8 +509,9 @@ __global__ void __launch_bounds__(256)
 }
 
 // X += Q alpha; R -= AQ alpha (products in T, additions in FP64); a thread
-// owns one row x 4 columns; norms partials per block.
-template <typename T>
+// owns one row x XC columns (4, or 2 or 1 for an m that 4 does not divide: no
+// FP64 work for columns past m); norms partials per block.
+template <typename T, int XC>
 __global__ void __launch_bounds__(256)
     xrupdate_direct_kernel(int64_t n, int k, int m, const T *__restrict__ Q,
                            const T *__restrict__ AQ, int64_t ldq,
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(256)
                            float *__restrict__ R32, double *__restrict__ part, Slices s0sl,
                            Slices r32sl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int G = (m + 3) / 4, mp = G * 4;
+    const int G = (m + XC - 1) / XC, mp = G * XC;
     T *As = reinterpret_cast<T *>(smem_raw);  // k x mp
     double *red = reinterpret_cast<double *>(As + (size_t)k * mp +
                                              ((size_t)k * mp * sizeof(T) % 16 ? 2 : 0));
@@ -531,10 +532,14 @@ __global__ void __launch_bounds__(256)
     const int rows_per_block = blockDim.x / G;
     const int lr = threadIdx.x / G, g = threadIdx.x % G;
     const bool active = lr < rows_per_block;
-    double sq[4] = {0.0, 0.0, 0.0, 0.0};
+    double sq[XC];
+#pragma unroll
+    for (int q = 0; q < XC; ++q) sq[q] = 0.0;
     for (int64_t row = (int64_t)blockIdx.x * rows_per_block + lr; active && row < n;
          row += (int64_t)gridDim.x * rows_per_block) {
-        T ax[4] = {T(0), T(0), T(0), T(0)}, ar[4] = {T(0), T(0), T(0), T(0)};
+        T ax[XC], ar[XC];
+#pragma unroll
+        for (int q = 0; q < XC; ++q) ax[q] = ar[q] = T(0);
         const T *qr = Q + row * ldq, *aqr = AQ + row * ldq;
         for (int j = 0; j < k; j += 4) {
             T q4[4], a4[4];
@@ -553,9 +558,9 @@ __global__ void __launch_bounds__(256)
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const T *al = As + (size_t)(j + u) * mp + g * 4;
+                const T *al = As + (size_t)(j + u) * mp + g * XC;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < XC; ++q) {
                     ax[q] = fma(q4[u], al[q], ax[q]);
                     ar[q] = fma(a4[u], al[q], ar[q]);
                 }
@@ -563,8 +568,8 @@ __global__ void __launch_bounds__(256)
         }
         float rf[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = g * 4 + q;
+        for (int q = 0; q < XC; ++q) {
+            const int c = g * XC + q;
             if (c < m) {
                 double x = X[row * m + c] + (double)ax[q];
                 double rv = R[row * m + c] - (double)ar[q];
@@ -584,13 +589,21 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     if (active)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) red[lr * mp + g * 4 + q] = sq[q];
+        for (int q = 0; q < XC; ++q) red[lr * mp + g * XC + q] = sq[q];
     __syncthreads();
-    for (int c = threadIdx.x; c < m; c += blockDim.x) {
-        double t = 0.0;
-        for (int rr = 0; rr < rows_per_block; ++rr) t += red[rr * mp + c];
-        part[(size_t)blockIdx.x * m + c] = t;
+    // rows in pairs (a fixed tree): one thread a column in row order took longer
+    // than the update itself for few columns (256 dependent FP64 additions; n =
+    // 16384, k = 4, m = 1: 16.8 us, 9.2 with the tree)
+    for (int h = rows_per_block; h > 1;) {
+        const int half = (h + 1) / 2;
+        if (active && lr < h - half)
+#pragma unroll
+            for (int q = 0; q < XC; ++q)
+                red[lr * mp + g * XC + q] += red[(lr + half) * mp + g * XC + q];
+        __syncthreads();
+        h = half;
     }
+    for (int c = threadIdx.x; c < m; c += blockDim.x) part[(size_t)blockIdx.x * m + c] = red[c];
 }
 
 template <typename T>
@@ -603,12 +616,16 @@ int launch_qupdate_direct(cudaStream_t st, int64_t n, int k, T *Qout, int64_t ld
                           const T *Qin, int64_t ldq, const T *S, int64_t lds,
                           const double *beta, Slices qsl) {
     const int G = k / 4;
-    int threads = std::max(G, (256 / G) * G);
+    int64_t ngroups = (n + kDqRows - 1) / kDqRows;
+    // few rows: smaller blocks, so that every SM gets some (n = 16384, k = 4: 12.1
+    // us on 16 SMs, 8.5 on 128)
+    const int64_t per_block = ngroups * G / (2 * (int64_t)sm_count());
+    const int want = per_block >= 128 ? 256 : (int)std::max<int64_t>(32, per_block);
+    int threads = std::max(G, (want / G) * G);
     if (threads > 256) threads = G;  // G <= 256 here
     const int groups_per_block = threads / G;
     size_t smem = (size_t)k * k * sizeof(T);
     set_smem_attr(qupdate_direct_kernel<T>, (int)max_smem_optin());
-    int64_t ngroups = (n + kDqRows - 1) / kDqRows;
     int64_t blocks = (ngroups + groups_per_block - 1) / groups_per_block;
     int64_t cap = (int64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
@@ -619,27 +636,44 @@ int launch_qupdate_direct(cudaStream_t st, int64_t n, int k, T *Qout, int64_t ld
 
 constexpr int kXrMaxBlocks = 2048;  // norm partials per xrupdate launch (upper bound)
 
-template <typename T>
-int launch_xrupdate_direct(cudaStream_t st, int64_t n, int k, int m, const T *Q, const T *AQ,
-                           int64_t ldq, const double *alpha, double *X, double *R, T *S0,
-                           int64_t lds, float *R32, double *norms, double *ws, Slices s0sl,
-                           Slices r32sl) {
-    const int G = (m + 3) / 4, mp = G * 4;
+template <typename T, int XC>
+static int launch_xrd(cudaStream_t st, int64_t n, int k, int m, const T *Q, const T *AQ,
+                      int64_t ldq, const double *alpha, double *X, double *R, T *S0, int64_t lds,
+                      float *R32, double *norms, double *ws, Slices s0sl, Slices r32sl) {
+    const int G = (m + XC - 1) / XC, mp = G * XC;
     if (G > 256) return CACG_ERR_ARG;
     const int threads = (256 / G) * G;
     const int rows_per_block = threads / G;
     size_t smem = (size_t)k * mp * sizeof(T) + 16 + (size_t)rows_per_block * mp * 8;
     if (smem > max_smem_optin()) return CACG_ERR_UNSUPPORTED;
-    set_smem_attr(xrupdate_direct_kernel<T>, (int)max_smem_optin());
+    set_smem_attr(xrupdate_direct_kernel<T, XC>, (int)max_smem_optin());
     int64_t blocks = (n + rows_per_block - 1) / rows_per_block;
     int64_t cap = std::min<int64_t>((int64_t)sm_count() * 8, kXrMaxBlocks);
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    xrupdate_direct_kernel<T><<<(unsigned)blocks, threads, smem, st>>>(
+    xrupdate_direct_kernel<T, XC><<<(unsigned)blocks, threads, smem, st>>>(
         n, k, m, Q, AQ, ldq, alpha, X, R, S0, lds, R32, norms ? ws : nullptr, s0sl, r32sl);
     int rc = check_launch();
     if (rc != CACG_OK || !norms) return rc;
     return launch_colsum(st, ws, (int)blocks, m, norms);
+}
+
+template <typename T>
+int launch_xrupdate_direct(cudaStream_t st, int64_t n, int k, int m, const T *Q, const T *AQ,
+                           int64_t ldq, const double *alpha, double *X, double *R, T *S0,
+                           int64_t lds, float *R32, double *norms, double *ws, Slices s0sl,
+                           Slices r32sl) {
+    // FP64: the pipe's time goes by columns, so none past m (m = 6, k = 24, n = 50021:
+    // 53 us with groups of 4, 41 with 2); FP32 keeps the fewer loads
+    if (std::is_same<T, double>::value && m % 4 != 0) {
+        if (m % 2 == 0)
+            return launch_xrd<T, 2>(st, n, k, m, Q, AQ, ldq, alpha, X, R, S0, lds, R32, norms, ws,
+                                    s0sl, r32sl);
+        return launch_xrd<T, 1>(st, n, k, m, Q, AQ, ldq, alpha, X, R, S0, lds, R32, norms, ws,
+                                s0sl, r32sl);
+    }
+    return launch_xrd<T, 4>(st, n, k, m, Q, AQ, ldq, alpha, X, R, S0, lds, R32, norms, ws, s0sl,
+                            r32sl);
 }
 
 // dst = src for an n x w FP32 block, rows of lds and ldd values

@@ -500,11 +500,11 @@ static void carve(char *base, const Layout &L, int m, int k, SolveBuffers *b) {
     b->QtR = sm; sm += (size_t)k * m;
     b->alpha = sm; sm += (size_t)k * m;
     b->norms = sm; sm += m;
+    b->status = (int *)sm; sm += 1;  // after the norms: both come back in one copy
     b->bnorm = sm; sm += m;
     b->tnorm = sm; sm += m;
     b->bounds = sm; sm += 2;
     b->scal = sm; sm += 16;
-    b->status = (int *)sm;
     b->gram_ws = (double *)(base + L.o_gram);
     b->gram_ws_bytes = L.gram;
     b->norm_ws = (double *)(base + L.o_norm);
@@ -974,10 +974,8 @@ struct Solver {
     }
 
     int fetch_norms(int *status_out) {
-        CACG_CUDA_TRY(cudaMemcpyAsync(h_pin, b.norms, m * sizeof(double),
+        CACG_CUDA_TRY(cudaMemcpyAsync(h_pin, b.norms, (m + 1) * sizeof(double),
                                       cudaMemcpyDeviceToHost, st));
-        CACG_CUDA_TRY(cudaMemcpyAsync(h_pin + m, b.status, sizeof(int), cudaMemcpyDeviceToHost,
-                                      st));
         CACG_CUDA_TRY(cudaStreamSynchronize(st));
         prof.harvest();
         int stv;

@@ -62,6 +62,22 @@ def test_gram_fp64_planes(n, ka, kb1, kb2, kind, pad, off):
     assert np.all(np.abs(C - l.T @ r) <= tol)
 
 
+@pytest.mark.parametrize("n,ka,kb1,kb2", [(7, 1, 1, 0), (1000, 4, 4, 1), (333, 24, 24, 6),
+                                          (5000, 24, 32, 0), (700, 25, 31, 0), (90, 48, 32, 0),
+                                          (2500, 49, 32, 0), (257, 96, 8, 8)])
+def test_gram_fp64_fma_few_outputs(n, ka, kb1, kb2):
+    """The FMA Gram around the output counts (768, 1536) where its thread layout changes: a
+    chain of at most n FMAs and the chunks' sum."""
+    torch = pytest.importorskip("torch")
+    L = _block(torch, n, ka, ka, 0, "normal", 1)
+    R1 = _block(torch, n, kb1, kb1 + 1, 1, "normal", 2)
+    R2 = _block(torch, n, kb2, kb2, 0, "normal", 3) if kb2 else None
+    C = _gram(torch, L, R1, R2, variant=1)
+    l = L.cpu().numpy().astype(np.longdouble)
+    r = (R1 if R2 is None else torch.cat([R1, R2], 1)).cpu().numpy().astype(np.longdouble)
+    assert np.all(np.abs(C - l.T @ r) <= (n + 4) * 2.0 ** -53 * (np.abs(l).T @ np.abs(r)))
+
+
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 4e-310])
 def test_gram_fp64_planes_outside_range(value):
     """Values no scale holds: the reduction forms the product by FP64 FMAs."""
