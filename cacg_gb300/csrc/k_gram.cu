@@ -391,6 +391,119 @@ __global__ void __launch_bounds__(512)
     }
 }
 
+// ------------------------------------------------------- few columns, FP64
+// At most 16 columns on each side: a thread owns one L column and all R columns
+// of the rows of its slot (threadIdx / ka), operands straight from L1, no
+// shared-memory slabs; slots are summed by lanes, then warps, then blocks, in a
+// fixed order.  Bound by launch latency for few rows, by the FP64 pipe for many.
+// n = 16384, 4 x 5: 23 us with the digit planes, 14.8 here.
+constexpr int kTinyMax = 16;
+constexpr int kTinyThreads = 256;
+constexpr int kTinyBlocks = 608;
+
+template <int KB>
+__global__ void __launch_bounds__(kTinyThreads)
+    gram_tiny_kernel(int64_t n, const double *__restrict__ L, int64_t ldl, int ka,
+                     const double *__restrict__ R1, int64_t ldr1, int kb1,
+                     const double *__restrict__ R2, int64_t ldr2, int kb2,
+                     double *__restrict__ part) {
+    __shared__ double ws[kTinyThreads / 32][kTinyMax][KB];
+    const int kb = kb1 + kb2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // slots of a warp: lanes a, a + ka, ... own L column a
+    const int spw = 32 / ka;  // slots per warp
+    const int a = lane % ka, slot = lane / ka;
+    const bool on = slot < spw;
+    const int64_t s0 = ((int64_t)blockIdx.x * (kTinyThreads / 32) + warp) * spw + slot;
+    const int64_t ns = (int64_t)gridDim.x * (kTinyThreads / 32) * spw;
+    double acc[KB];
+#pragma unroll
+    for (int j = 0; j < KB; ++j) acc[j] = 0.0;
+    if (on) {
+#pragma unroll 2
+        for (int64_t row = s0; row < n; row += ns) {
+            const double l = __ldg(L + row * ldl + a);
+            const double *p1 = R1 + row * ldr1, *p2 = R2 + row * ldr2 - kb1;
+            double r[KB];
+#pragma unroll
+            for (int j = 0; j < KB; ++j) r[j] = j < kb1 ? __ldg(p1 + j) : j < kb ? __ldg(p2 + j) : 0.0;
+#pragma unroll
+            for (int j = 0; j < KB; ++j) acc[j] = fma(l, r[j], acc[j]);
+        }
+    }
+    // slots of the warp, in slot order from the last to the first
+    for (int t = spw - 1; t > 0; --t) {
+#pragma unroll
+        for (int j = 0; j < KB; ++j) {
+            const double v = __shfl_down_sync(0xffffffffu, acc[j], ka);
+            if (on && slot + 1 == t) acc[j] += v;
+        }
+    }
+    if (on && slot == 0)
+#pragma unroll
+        for (int j = 0; j < KB; ++j) ws[warp][a][j] = acc[j];
+    __syncthreads();
+    for (int i = threadIdx.x; i < ka * kb; i += kTinyThreads) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kTinyThreads / 32; ++w) t += ws[w][i / kb][i % kb];
+        part[(size_t)blockIdx.x * ka * kb + i] = t;
+    }
+}
+
+// output i: 32 threads sum the blocks' partials (strided), then a fixed tree
+__global__ void __launch_bounds__(256)
+    gram_tiny_reduce_kernel(const double *__restrict__ part, int nblocks, int ka, int kb, int kb1,
+                            double *__restrict__ C1, int ldc1, double *__restrict__ C2, int ldc2) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= ka * kb) return;
+    double t = 0.0;
+#pragma unroll 4
+    for (int p = lane; p < nblocks; p += 32) t += part[(size_t)p * ka * kb + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) {
+        const int a = i / kb, b = i % kb;
+        if (b < kb1)
+            C1[(size_t)a * ldc1 + b] = t;
+        else
+            C2[(size_t)a * ldc2 + (b - kb1)] = t;
+    }
+}
+
+static size_t tiny_bytes(int ka, int kb) {
+    return ka <= kTinyMax && kb <= kTinyMax ? (size_t)kTinyBlocks * ka * kb * sizeof(double) : 0;
+}
+
+static int launch_gram_tiny(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
+                            const double *R1, int64_t ldr1, int kb1, const double *R2,
+                            int64_t ldr2, int kb2, double *C1, int ldc1, double *C2, int ldc2,
+                            double *ws, size_t ws_bytes) {
+    const int kb = kb1 + kb2;
+    if (n <= 0 || ka > kTinyMax || kb > kTinyMax || !ws || tiny_bytes(ka, kb) > ws_bytes)
+        return CACG_ERR_UNSUPPORTED;
+    // the digit planes' time hardly grows with the columns here, the FMAs' does.
+    // Through cacg_k_gram (about 38 us of it the call), planes and this: n = 884736,
+    // 8 x 10 222 and 162 us, 12 x 15 273 and 417; n = 50653, 12 x 15 52 and 60;
+    // n = 16384, 12 x 15 44 and 42
+    if (ka * kb > 80 && (double)n * ka * kb > 3e6) return CACG_ERR_UNSUPPORTED;
+    const int rows = (kTinyThreads / 32) * (32 / ka);  // rows a block takes at a time
+    const int blocks = (int)std::max<int64_t>(
+        1, std::min<int64_t>((n + 4 * rows - 1) / (4 * rows), std::min(4 * sm_count(), kTinyBlocks)));
+#define TINY_CASE(KB)                                                                             \
+    if (kb <= KB) {                                                                               \
+        gram_tiny_kernel<KB><<<blocks, kTinyThreads, 0, st>>>(n, L, ldl, ka, R1, ldr1, kb1, R2,   \
+                                                              ldr2, kb2, ws);                     \
+    } else
+    TINY_CASE(2) TINY_CASE(5) TINY_CASE(8) TINY_CASE(10) TINY_CASE(12) TINY_CASE(16) {}
+#undef TINY_CASE
+    int rc = check_launch();
+    if (rc != CACG_OK) return rc;
+    gram_tiny_reduce_kernel<<<(ka * kb + 7) / 8, 256, 0, st>>>(ws, blocks, ka, kb, kb1, C1, ldc1, C2,
+                                                               ldc2);
+    return check_launch();
+}
+
 // C[a][b] = sum over chunks p (in order) of part[p][tile(a,b)][a%BA][b%BB]
 // C = sum over chunks of the per-chunk partial tiles.  Four threads share one
 // output element: thread quarter q sums its contiguous quarter of the chunks
@@ -495,7 +608,7 @@ size_t gram_workspace_bytes(int64_t n, int ka, int kb) {
         size_t b2 = (size_t)q.nchunks * q.tilesA * q.tilesB * q.BA * q.BB * sizeof(double);
         best = std::max(best, std::max(b1, b2));
     }
-    return std::max(best, gram_x64_workspace_bytes(n, ka, kb));
+    return std::max(std::max(best, gram_x64_workspace_bytes(n, ka, kb)), tiny_bytes(ka, kb));
 }
 
 template <typename T>
@@ -509,7 +622,10 @@ int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl
         return CACG_ERR_UNSUPPORTED;
     if constexpr (std::is_same<T, double>::value) {
         if (variant == CACG_GRAM_AUTO) {
-            const int rc = launch_gram_x64(st, n, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1,
+            int rc = launch_gram_tiny(st, n, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1, ldc1, C2,
+                                      ldc2, ws, ws_bytes);
+            if (rc != CACG_ERR_UNSUPPORTED) return rc;
+            rc = launch_gram_x64(st, n, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1,
                                            ldc1, C2, ldc2, ws, ws_bytes);
             if (rc != CACG_ERR_UNSUPPORTED) return rc;
         }

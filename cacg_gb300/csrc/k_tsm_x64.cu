@@ -222,6 +222,19 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
             }
             const bool more = job + 1 < njobs;
             int E[kXtRG];
+            // the rows of two jobs on, into L2: the scan of the next job's rows below
+            // has only a few hundred instructions to hide its loads behind
+            if (job + 2 < njobs) {
+#pragma unroll
+                for (int rg = 0; rg < kXtRG; ++rg) {
+                    bool rp;
+                    const double *q = row_ptr(job + 2, rg, rp) - lc;
+                    if (rp)
+                        for (int b = 64 * lc; b < g.K * 8; b += 512)
+                            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(
+                                reinterpret_cast<const char *>(q) + b));
+                }
+            }
 #pragma unroll
             for (int rg = 0; rg < kXtRG; ++rg) {
                 bool bad = wide;

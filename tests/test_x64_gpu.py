@@ -62,20 +62,26 @@ def test_gram_fp64_planes(n, ka, kb1, kb2, kind, pad, off):
     assert np.all(np.abs(C - l.T @ r) <= tol)
 
 
-@pytest.mark.parametrize("n,ka,kb1,kb2", [(7, 1, 1, 0), (1000, 4, 4, 1), (333, 24, 24, 6),
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("n,ka,kb1,kb2", [(7, 1, 1, 0), (1000, 4, 4, 1), (31, 5, 5, 3),
+                                          (40000, 8, 8, 2), (700, 16, 16, 0), (1, 3, 9, 7),
+                                          (3000, 16, 1, 15), (100, 17, 8, 0), (333, 24, 24, 6),
                                           (5000, 24, 32, 0), (700, 25, 31, 0), (90, 48, 32, 0),
                                           (2500, 49, 32, 0), (257, 96, 8, 8)])
-def test_gram_fp64_fma_few_outputs(n, ka, kb1, kb2):
-    """The FMA Gram around the output counts (768, 1536) where its thread layout changes: a
-    chain of at most n FMAs and the chunks' sum."""
+def test_gram_fp64_few_outputs(n, ka, kb1, kb2, variant):
+    """The FMA Gram around the output counts (768, 1536) where its thread layout changes, and
+    the automatic variant's kernel for at most 16 columns a side: a chain of at most n FMAs
+    and the partial sums (the planes' bound, taken past 16 columns, is test_gram_fp64_planes')."""
     torch = pytest.importorskip("torch")
     L = _block(torch, n, ka, ka, 0, "normal", 1)
     R1 = _block(torch, n, kb1, kb1 + 1, 1, "normal", 2)
     R2 = _block(torch, n, kb2, kb2, 0, "normal", 3) if kb2 else None
-    C = _gram(torch, L, R1, R2, variant=1)
+    if variant == 0 and (max(ka, kb1 + kb2) > 16 or n * ka * (kb1 + kb2) > 3e6 and ka * kb1 > 80):
+        pytest.skip("not this kernel's shape")
+    C = _gram(torch, L, R1, R2, variant)
     l = L.cpu().numpy().astype(np.longdouble)
     r = (R1 if R2 is None else torch.cat([R1, R2], 1)).cpu().numpy().astype(np.longdouble)
-    assert np.all(np.abs(C - l.T @ r) <= (n + 4) * 2.0 ** -53 * (np.abs(l).T @ np.abs(r)))
+    assert np.all(np.abs(C - l.T @ r) <= (n + 40) * 2.0 ** -53 * (np.abs(l).T @ np.abs(r)))
 
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 4e-310])
