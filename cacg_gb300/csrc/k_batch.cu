@@ -35,6 +35,7 @@
 
 #include "batch.h"
 #include "cacg_internal.cuh"
+#include "lu_block.cuh"
 
 namespace cacg {
 
@@ -564,137 +565,56 @@ __global__ void __launch_bounds__(kBThreads) bk_gram_reduce(const BBatch *__rest
 // ------------------------------------------------------------ LU
 // Crout factor of QtAQ, unit-diagonal U, no pivoting (src/DLSsolvers.c:125-145):
 // F = the factors (k x k), the reciprocals of L's diagonal (k), the factors
-// transposed (k x k, for the solves' column sweeps).  Step dd: warp 0 updates
-// row dd + 1 and at once takes its pivot and scales it into U's row (the next
-// step's critical path), while warps 1-7 update rows dd + 2 .. k - 1 as one
-// flat range of (row, column) entries, so every FP64 instruction of the
-// trailing update carries 32 useful lanes; one barrier a step.
-__device__ __forceinline__ void blu_pivot_row(double *W, int k, int i, double *Dinv, int lane,
-                                              int &bad) {
-    double inv = 0.0;
-    if (lane == 0) {
-        const double piv = W[i * k + i];
-        if (piv == 0.0 || !isfinite(piv)) bad = 1;
-        inv = 1.0 / piv;
-        Dinv[i] = inv;
-    }
-    inv = __shfl_sync(0xffffffffu, inv, 0);
-    for (int c = i + 1 + lane; c < k; c += 32) W[i * k + c] *= inv;
-}
-
-__global__ void __launch_bounds__(kBThreads) bk_lu_factor(const BBatch *__restrict__ b) {
+// transposed (k x k, for the solves' column sweeps); one CTA per request
+// (lu_block.cuh).
+__global__ void __launch_bounds__(kLuBlockThreads) bk_lu_factor(const BBatch *__restrict__ b) {
     __shared__ double W[kBMaxK * kBMaxK];
+    __shared__ double s_inv;
+    __shared__ int s_bad;
     const int r = blockIdx.x;
     if (r >= b->nr) return;
     const BDesc &d = b->d[r];
     if (!(d.flags & kBActive)) return;
     const int k = d.k, kk = k * k;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x;
+    if (tid == 0) s_bad = 0;
     for (int i = tid; i < kk; i += blockDim.x) W[i] = d.QtAQ[i];
     __syncthreads();
     double *Dinv = d.F + kk, *FT = d.F + kk + k;
-    int bad = 0;
-    if (warp == 0) blu_pivot_row(W, k, 0, Dinv, lane, bad);
-    __syncthreads();
-    for (int dd = 0; dd + 1 < k; ++dd) {
-        const int x = k - dd - 1;  // trailing columns dd + 1 .. k - 1
-        const double *U = W + dd * k;
-        if (warp == 0) {
-            double *wr = W + (dd + 1) * k;
-            const double lid = wr[dd];
-            for (int c = dd + 1 + lane; c < k; c += 32) wr[c] = wr[c] - lid * U[c];
-            __syncwarp();
-            blu_pivot_row(W, k, dd + 1, Dinv, lane, bad);
-        } else {
-            const uint32_t mg = bdiv_magic(x);
-            for (int e = tid - 32; e < (x - 1) * x; e += kBThreads - 32) {
-                const int q = bdiv(e, x, mg);
-                double *wr = W + (dd + 2 + q) * k;
-                const int c = dd + 1 + (e - q * x);
-                wr[c] = wr[c] - wr[dd] * U[c];
-            }
-        }
-        __syncthreads();
-    }
+    lu_factor_block(W, k, Dinv, &s_inv, &s_bad);
     for (int e = tid; e < kk; e += blockDim.x) {
         const int i = e / k, jj = e - i * k;
         d.F[e] = W[e];
         FT[e] = W[jj * k + i];
     }
-    if (bad) atomicOr(d.status, kStatusBreakdown);
+    if (tid == 0 && s_bad) atomicOr(d.status, kStatusBreakdown);
 }
 
 // WHICH 0: beta = QtAQ_prev^{-1} QtAS (k columns); WHICH 1: alpha = QtAQ^{-1} QtR
-// (m columns).  A warp solves one column by column sweeps (lane l holds rows
-// l and l + 32): forward, y_i = z_i / L_ii through the reciprocal, then
-// z_j -= L_ji y_i for j > i; backward with U's unit diagonal, z_j -= U_ji x_i
-// for j < i (src/DLSsolvers.c:156-207).  The transposed factor in shared
-// memory makes each step's reads of L_ji / U_ji contiguous over the lanes;
-// the chain is 2k broadcasts and FMAs.
-constexpr int kBLuWarps = 8;
+// (m columns): column sweeps by one or two warps a column (lu_block.cuh), a warp
+// per quadrant of the SM.
+constexpr int kBLuWarps = 4;
 
 template <int WHICH>
 __global__ void __launch_bounds__(32 * kBLuWarps) bk_lu_solve(const BBatch *__restrict__ b) {
-    extern __shared__ __align__(16) double bl_smem[];
+    __shared__ double ys[kBLuWarps][kBMaxK];
     const int r = blockIdx.x;
     if (r >= b->nr) return;
     const BDesc &d = b->d[r];
     if (!(d.flags & kBActive) || (WHICH == 0 && d.it == 0)) return;
     const int k = d.k, kk = k * k;
     const int nrhs = WHICH == 0 ? k : d.m;
-    const int c0 = blockIdx.y * kBLuWarps;
-    if (c0 >= nrhs) return;
-    double *Dinv = bl_smem, *FT = bl_smem + k;
-    {
-        const double *src = d.F + kk;  // 1 / L_ii, then the transposed factors
-        for (int i = threadIdx.x; i < k + kk; i += blockDim.x) bl_smem[i] = src[i];
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, c = c0 + (threadIdx.x >> 5);
-    if (c >= nrhs) return;  // no block-wide barrier follows
+    const int nt = (k + 31) / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = warp / nt, w = warp - g * nt;
+    const int c = blockIdx.y * (kBLuWarps / nt) + g;
+    if (c >= nrhs) return;  // whole groups of warps; no block-wide barrier follows
     const double *RHS = WHICH == 0 ? d.QtAS : d.QtR;
     double *Y = WHICH == 0 ? d.beta : d.alpha;
-    constexpr int TT = kBMaxK / 32;
-    double z[TT];
-#pragma unroll
-    for (int t = 0; t < TT; ++t) {
-        const int jj = lane + 32 * t;
-        z[t] = jj < k ? RHS[(size_t)jj * nrhs + c] : 0.0;
-    }
-#pragma unroll
-    for (int t = 0; t < TT; ++t) {
-        for (int ii = 0; ii < 32; ++ii) {
-            const int i = 32 * t + ii;
-            if (i >= k) break;
-            const double yi = __shfl_sync(0xffffffffu, z[t], ii) * Dinv[i];
-            if (lane == ii) z[t] = yi;
-            const double *col = FT + (size_t)i * k;
-#pragma unroll
-            for (int tt = t; tt < TT; ++tt) {
-                const int jj = lane + 32 * tt;
-                if (jj > i && jj < k) z[tt] = fma(-col[jj], yi, z[tt]);
-            }
-        }
-    }
-#pragma unroll
-    for (int t = TT - 1; t >= 0; --t) {
-        for (int ii = 31; ii >= 0; --ii) {
-            const int i = 32 * t + ii;
-            if (i >= k) continue;
-            const double xi = __shfl_sync(0xffffffffu, z[t], ii);
-            const double *col = FT + (size_t)i * k;
-#pragma unroll
-            for (int tt = 0; tt <= t; ++tt) {
-                const int jj = lane + 32 * tt;
-                if (jj < i) z[tt] = fma(-col[jj], xi, z[tt]);
-            }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < TT; ++t) {
-        const int jj = lane + 32 * t;
-        if (jj < k) Y[(size_t)jj * nrhs + c] = z[t];
-    }
+    const int j = 32 * w + lane;
+    const double z = j < k ? RHS[(size_t)j * nrhs + c] : 0.0;
+    const double y = lu_sweep(k, nt, w, lane, 1 + g, z, d.F + kk, d.F + kk + k, ys[g]);
+    if (j < k) Y[(size_t)j * nrhs + c] = y;
 }
 
 // ------------------------------------------------------------ updates
@@ -947,20 +867,17 @@ int bl_gram(cudaStream_t st, const BBatch *b, int which, const BTune &tu) {
 }
 
 int bl_lu_factor(cudaStream_t st, const BBatch *b) {
-    bk_lu_factor<<<kBMax, kBThreads, 0, st>>>(b);
+    bk_lu_factor<<<kBMax, kLuBlockThreads, 0, st>>>(b);
     return check_launch();
 }
 
 int bl_lu_solve(cudaStream_t st, const BBatch *b, int which) {
-    const int smem = (int)(sizeof(double) * ((size_t)kBMaxK * kBMaxK + kBMaxK));
-    const dim3 grid(kBMax, (kBMaxK + kBLuWarps - 1) / kBLuWarps);
-    if (which == 0) {
-        set_smem_attr(bk_lu_solve<0>, smem);
-        bk_lu_solve<0><<<grid, 32 * kBLuWarps, smem, st>>>(b);
-    } else {
-        set_smem_attr(bk_lu_solve<1>, smem);
-        bk_lu_solve<1><<<grid, 32 * kBLuWarps, smem, st>>>(b);
-    }
+    // two columns a block at least (k <= 64)
+    const dim3 block(32 * kBLuWarps);
+    if (which == 0)
+        bk_lu_solve<0><<<dim3(kBMax, kBMaxK / 2), block, 0, st>>>(b);
+    else
+        bk_lu_solve<1><<<dim3(kBMax, kBMaxM / 2), block, 0, st>>>(b);
     return check_launch();
 }
 

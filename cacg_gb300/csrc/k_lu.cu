@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 
 #include "cacg_internal.cuh"
+#include "lu_block.cuh"
 
 namespace cacg {
 
@@ -141,72 +142,186 @@ __global__ void __cluster_dims__(kLucCtas, 1, 1) __launch_bounds__(kLucThreads)
     cluster.sync();  // no CTA leaves while another may still read its rows
 }
 
-// One CTA with one barrier per elimination step (k <= kLuLaMaxK): warp 0
-// updates row d + 1 at step d and at once takes its pivot and scales it into
-// U's row -- the next step's critical path -- while warps 1..7 update rows
-// d + 2 .. k - 1 as one flat range of (row, column) entries, so every FP64
-// instruction of the trailing update carries 32 useful lanes.  Every element
-// sees the same operations in the same order as lu_factor_kernel
-// (bit-identical factors); the two-barrier factor and the cluster factor pay
-// a barrier (a cluster barrier) and the serial pivot work at every step.
-constexpr int kLuLaThreads = 256;
-constexpr int kLuLaMaxK = 128;  // k x k doubles in shared memory (128 KB); taken for k <= 64
+// The cluster factor with the pivot rows pushed instead of pulled: CTA r owns
+// rows i = r (mod kLucCtas); the owner of row d + 1 updates it at step d ahead of
+// its other rows, takes the pivot and scales the row into U's, and writes it with
+// st.async into every CTA's copy of U, whose mbarrier of that row the bytes
+// complete.  No cluster barrier per step: the chain is one FMA, the division (340
+// clocks; an FMA is 64 on this part whatever the lanes), one product and the
+// transfer; the trailing update runs beside it.  Warp 0 holds the pivot alone on
+// its quadrant's FP64 pipe (warp 4 rests while this CTA takes a pivot).  Every
+// element sees the operations of lu_factor_kernel in the same order
+// (bit-identical factors).  k = 96: 69.5 us, k = 128: 117 (pulled: 135, 195).
+constexpr int kLupThreads = 256;
+constexpr int kLupMinK = 48;
+constexpr int kLupMaxK = 160;  // U (k x k) and the local rows in shared memory
+constexpr long long kLupPolls = 1ll << 22;
 
-__device__ __forceinline__ void lu_pivot_row(double *W, int k, int i, double *Dinv, int lane,
-                                             int &bad) {
-    double inv = 0.0;
-    if (lane == 0) {
-        const double piv = W[i * k + i];
-        if (piv == 0.0 || !isfinite(piv)) bad = 1;
-        inv = 1.0 / piv;
-        Dinv[i] = inv;
+__device__ __forceinline__ unsigned lup_u32(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ unsigned lup_map(unsigned a, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ bool lup_wait(uint64_t *bar) {
+    for (long long i = 0; i < kLupPolls; ++i) {
+        unsigned ok;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok)
+            : "r"(lup_u32(bar))
+            : "memory");
+        if (ok) return true;
     }
-    inv = __shfl_sync(0xffffffffu, inv, 0);
-    for (int c = i + 1 + lane; c < k; c += 32) W[i * k + c] *= inv;
+    return false;
 }
 
-__global__ void __launch_bounds__(kLuLaThreads)
+__global__ void __cluster_dims__(kLucCtas, 1, 1) __launch_bounds__(kLupThreads)
+    lu_factor_push_kernel(int k, const double *__restrict__ M, double *__restrict__ F,
+                          int *__restrict__ status) {
+    extern __shared__ __align__(16) double lup_sm[];
+    __shared__ double s_inv;
+    __shared__ int s_bad;
+    cgrp::cluster_group cluster = cgrp::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int nloc = (k - rank + kLucCtas - 1) / kLucCtas;
+    const int rows_max = (k + kLucCtas - 1) / kLucCtas;
+    double *U = lup_sm;                       // k x k: scaled pivot rows, columns past the pivot
+    double *Wl = U + (size_t)k * k;           // nloc x k: local rows
+    uint64_t *bar = reinterpret_cast<uint64_t *>(Wl + (size_t)rows_max * k);  // row d has arrived
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double *Dinv = F + (size_t)k * k;
+    for (int idx = tid; idx < nloc * k; idx += kLupThreads) {
+        const int li = idx / k, c = idx - li * k;
+        Wl[idx] = M[(size_t)(li * kLucCtas + rank) * k + c];
+    }
+    for (int d = tid; d < k; d += kLupThreads) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(lup_u32(&bar[d])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile(
+            "{\n"
+            ".reg .b64 st;\n"
+            "mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n"
+            "}\n" ::"r"(lup_u32(&bar[d])),
+            "r"(8 * (k - 1 - d))
+            : "memory");
+    }
+    if (tid == 0) s_bad = 0;
+    __syncthreads();
+    cluster.sync();  // every CTA's barriers expect their bytes
+
+    // warps 0 .. 3: row r updated with row d (d < 0: as it is), its pivot taken,
+    // scaled and pushed
+    auto pivot_row = [&](int r, int d) {
+        double *wr = Wl + (size_t)(r / kLucCtas) * k;
+        const double l = d >= 0 ? wr[d] : 0.0;
+        const double *ud = U + (size_t)(d >= 0 ? d : 0) * k;
+        double w[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = r + tid + 128 * e;
+            w[e] = c < k ? wr[c] : 0.0;
+            if (c < k && d >= 0) w[e] = fma(-l, ud[c], w[e]);
+        }
+        if (warp == 0) {
+            const double piv = __shfl_sync(0xffffffffu, w[0], 0);
+            const double inv = 1.0 / piv;
+            if (lane == 0) {
+                s_inv = inv;
+                Dinv[r] = inv;
+                if (lu_bad_pivot(piv)) s_bad = 1;
+            }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const double inv = s_inv;
+        const unsigned mb = lup_u32(&bar[r]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = r + tid + 128 * e;
+            if (c >= k) break;
+            if (c == r) {
+                wr[c] = w[e];
+                continue;
+            }
+            const double u = w[e] * inv;
+            wr[c] = u;
+            const unsigned dst = lup_u32(U + (size_t)r * k + c);
+#pragma unroll
+            for (unsigned q = 0; q < (unsigned)kLucCtas; ++q)
+                asm volatile(
+                    "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, "
+                    "[%2];" ::"r"(lup_map(dst, q)),
+                    "l"(__double_as_longlong(u)), "r"(lup_map(mb, q))
+                    : "memory");
+        }
+    };
+
+    bool ok = true;
+    if (rank == 0 && warp < 4) pivot_row(0, -1);
+    for (int d = 0; d + 1 < k; ++d) {
+        ok = lup_wait(&bar[d]);
+        if (__syncthreads_or(!ok)) {  // (also: the last step's rows are written)
+            ok = false;
+            break;
+        }
+        const bool mine = (d + 1) % kLucCtas == rank;
+        const double *ud = U + (size_t)d * k;
+        const int li0 = (d + 1 - rank + kLucCtas - 1) / kLucCtas + (mine ? 1 : 0);
+        if (mine && warp < 4) {
+            pivot_row(d + 1, d);
+        } else if (!mine || warp != 4) {
+            // local rows past the next pivot row: rows by warp, columns by lane
+            const int nw = mine ? 3 : kLupThreads / 32, w0 = mine ? warp - 5 : warp;
+            for (int li = li0 + w0; li < nloc; li += nw) {
+                double *wi = Wl + (size_t)li * k;
+                const double l = wi[d];
+                for (int c = d + 1 + lane; c < k; c += 32) wi[c] = fma(-l, ud[c], wi[c]);
+            }
+        }
+    }
+    __syncthreads();
+    double *FT = F + (size_t)k * k + k;
+    for (int idx = tid; idx < nloc * k; idx += kLupThreads) {
+        const int li = idx / k, c = idx - li * k;
+        const int i = li * kLucCtas + rank;
+        F[(size_t)i * k + c] = Wl[idx];
+        FT[(size_t)c * k + i] = Wl[idx];
+    }
+    if (tid == 0 && status) {
+        if (s_bad) atomicOr(status, kStatusBreakdown);
+        if (!ok) atomicOr(status, kStatusTimeout);
+    }
+    cluster.sync();  // no CTA leaves while another may still write into it
+}
+
+// One CTA (lu_block.cuh) for the small factors, where eight SMs' transfers cost
+// more than their FP64 pipes give.
+constexpr int kLuLaMaxK = 128;  // k x k doubles in shared memory (128 KB)
+
+__global__ void __launch_bounds__(kLuBlockThreads)
     lu_factor_la_kernel(int k, const double *__restrict__ M, double *__restrict__ F,
                         int *__restrict__ status) {
     extern __shared__ __align__(16) double lw[];
-    const int kk = k * k;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ double s_inv;
+    __shared__ int s_bad;
+    const int kk = k * k, tid = threadIdx.x;
+    if (tid == 0) s_bad = 0;
     for (int i = tid; i < kk; i += blockDim.x) lw[i] = M[i];
     __syncthreads();
-    double *Dinv = F + (size_t)kk;
-    int bad = 0;
-    if (warp == 0) lu_pivot_row(lw, k, 0, Dinv, lane, bad);
-    __syncthreads();
-    for (int d = 0; d + 1 < k; ++d) {
-        const int x = k - d - 1;  // trailing columns d + 1 .. k - 1
-        const double *U = lw + (size_t)d * k;
-        if (warp == 0) {
-            double *wr = lw + (size_t)(d + 1) * k;
-            const double lid = wr[d];
-            for (int c = d + 1 + lane; c < k; c += 32) wr[c] = wr[c] - lid * U[c];
-            __syncwarp();
-            lu_pivot_row(lw, k, d + 1, Dinv, lane, bad);
-        } else {
-            // entry e = q x + r of rows d + 2 .. k - 1: row d + 2 + q, column
-            // d + 1 + r; q = floor(e / x) as the high word of e * ceil(2^32 / x)
-            // (exact for e < 2^32 / x)
-            const uint32_t mg = x > 1 ? 0xFFFFFFFFu / (uint32_t)x + 1u : 0u;
-            for (int e = tid - 32; e < (x - 1) * x; e += kLuLaThreads - 32) {
-                const int q = x > 1 ? (int)__umulhi((uint32_t)e, mg) : e;
-                double *wr = lw + (size_t)(d + 2 + q) * k;
-                const int c = d + 1 + (e - q * x);
-                wr[c] = wr[c] - wr[d] * U[c];
-            }
-        }
-        __syncthreads();
-    }
+    lu_factor_block(lw, k, F + (size_t)kk, &s_inv, &s_bad);
     double *FT = F + (size_t)kk + k;
     for (int idx = tid; idx < kk; idx += blockDim.x) {
         const int i = idx / k, j = idx - i * k;
         F[idx] = lw[idx];
         FT[idx] = lw[(size_t)j * k + i];
     }
-    if (bad && status) atomicOr(status, kStatusBreakdown);
+    if (tid == 0 && s_bad && status) atomicOr(status, kStatusBreakdown);
 }
 
 // Y (k x r) from the factor F (k*k factors + k reciprocal diagonal) and RHS
@@ -257,105 +372,45 @@ __global__ void __launch_bounds__(kLuRC * kLuTPC)
     }
 }
 
-// Column-sweep ("axpy") triangular solves, one warp per right-hand side:
-// lane l owns rows l, l+32, ...; at forward step i the owner's value times
-// the stored reciprocal pivot is y_i, broadcast with one shuffle, and every
-// lane subtracts L[j][i] y_i from its rows j > i; the backward sweep does the
-// same with the unit upper factor.  The factor is staged transposed in shared
-// memory (FT[i][j] = F[j][i]), so step i reads row i of FT, conflict-free.
-// Same arithmetic as the substitution above, summed column by column
-// (agrees with the reference to rounding).  T = ceil(k / 32) rows per lane.
-constexpr int kLuWarpsPerCta = 2;
-
-template <int T>
-__global__ void __launch_bounds__(32 * kLuWarpsPerCta)
-    lu_solve_sweep_kernel(int k, const double *__restrict__ F, int r,
+// Column-sweep ("axpy") triangular solves, ceil(k / 32) warps per right-hand
+// side (lu_block.cuh), a warp per quadrant of the SM.  Same arithmetic as the
+// substitution above, summed column by column (agrees with the reference to
+// rounding).
+__global__ void __launch_bounds__(160)
+    lu_solve_sweep_kernel(int k, int nt, int cols, const double *__restrict__ F, int r,
                           const double *__restrict__ RHS, double *__restrict__ Y) {
-    extern __shared__ __align__(16) double FT[];  // k * k transposed, then k reciprocal pivots
-    double *Dinv = FT + (size_t)k * k;
-    {
-        // the factor kernel wrote FT after F and the pivots: contiguous copy,
-        // 16-byte loads issued 8 at a time (k (k + 1) is even: aligned)
-        const double2 *src = reinterpret_cast<const double2 *>(F + (size_t)k * k + k);
-        double2 *dst = reinterpret_cast<double2 *>(FT);
-        const int n2 = k * k / 2;
-        int q = threadIdx.x;
-        for (; q + 7 * (int)blockDim.x < n2; q += 8 * blockDim.x) {
-            double2 v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = src[q + u * blockDim.x];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) dst[q + u * blockDim.x] = v[u];
-        }
-        for (; q < n2; q += blockDim.x) dst[q] = src[q];
-        if ((k * k) & 1 && threadIdx.x == 0) FT[k * k - 1] = F[(size_t)k * k + k + k * k - 1];
-    }
-    for (int i = threadIdx.x; i < k; i += blockDim.x) Dinv[i] = F[(size_t)k * k + i];
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * kLuWarpsPerCta + (threadIdx.x >> 5);
-    if (c >= r) return;  // no block-wide barrier follows
-    double z[T];
-#pragma unroll
-    for (int t = 0; t < T; ++t) {
-        const int j = lane + 32 * t;
-        z[t] = j < k ? RHS[(size_t)j * r + c] : 0.0;
-    }
-    // forward: y_i = z_i / L_ii; z_j -= L_ji y_i (j > i)
-#pragma unroll
-    for (int t = 0; t < T; ++t) {
-        for (int ii = 0; ii < 32; ++ii) {
-            const int i = 32 * t + ii;
-            if (i >= k) break;
-            const double yi = __shfl_sync(0xffffffffu, z[t], ii) * Dinv[i];
-            if (lane == ii) z[t] = yi;
-            const double *col = FT + (size_t)i * k;
-#pragma unroll
-            for (int tt = t; tt < T; ++tt) {
-                const int j = lane + 32 * tt;
-                if (j > i && j < k) z[tt] = fma(-col[j], yi, z[tt]);
-            }
-        }
-    }
-    // backward (U unit diagonal): x_i = z_i; z_j -= U_ji x_i (j < i)
-#pragma unroll
-    for (int t = T - 1; t >= 0; --t) {
-        for (int ii = 31; ii >= 0; --ii) {
-            const int i = 32 * t + ii;
-            if (i >= k) continue;
-            const double xi = __shfl_sync(0xffffffffu, z[t], ii);
-            const double *col = FT + (size_t)i * k;
-#pragma unroll
-            for (int tt = 0; tt <= t; ++tt) {
-                const int j = lane + 32 * tt;
-                if (j < i) z[tt] = fma(-col[j], xi, z[tt]);
-            }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < T; ++t) {
-        const int j = lane + 32 * t;
-        if (j < k) Y[(size_t)j * r + c] = z[t];
-    }
-}
-
-template <int T>
-static int launch_sweep(cudaStream_t st, int k, const double *F, int r, const double *RHS,
-                        double *Y, size_t smem) {
-    set_smem_attr(lu_solve_sweep_kernel<T>, (int)max_smem_optin());
-    const int blocks = (r + kLuWarpsPerCta - 1) / kLuWarpsPerCta;
-    lu_solve_sweep_kernel<T><<<blocks, 32 * kLuWarpsPerCta, smem, st>>>(k, F, r, RHS, Y);
-    return check_launch();
+    __shared__ double ys[4][160];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = warp / nt, w = warp % nt;
+    const int c = blockIdx.x * cols + g;
+    if (c >= r) return;  // whole groups of warps; no block-wide barrier follows
+    const int j = 32 * w + lane;
+    const double z = j < k ? RHS[(size_t)j * r + c] : 0.0;
+    const double y = lu_sweep(k, nt, w, lane, 1 + g, z, F + (size_t)k * k, F + (size_t)k * k + k,
+                              ys[g]);
+    if (j < k) Y[(size_t)j * r + c] = y;
 }
 
 int launch_lu_factor(cudaStream_t st, int k, const double *M, double *F, int *status) {
     if (k <= 0) return CACG_ERR_ARG;
-    // k <= 64 (the serving stream's shapes): one CTA; larger k: the cluster
-    // (at k = 96 it measured 8 % less LU time per outer iteration)
+    // factor and one solve, one CTA / pulled rows before, pushed rows now: k = 44
+    // 46.8 and 51.5 us; k = 64 77 and 68; k = 96 169 and 107; k = 128 248 and 172;
+    // k = 160 321 and 241.  Above, U does not fit beside the local rows.
+    if (k >= kLupMinK && k <= kLupMaxK) {
+        const size_t psmem = ((size_t)k * k + (size_t)((k + kLucCtas - 1) / kLucCtas) * k + k) *
+                             sizeof(double);
+        const size_t room = max_smem_optin() - 64;  // beside the kernel's static variables
+        set_smem_attr(lu_factor_push_kernel, (int)room);
+        if (psmem <= room) {
+            lu_factor_push_kernel<<<kLucCtas, kLupThreads, psmem, st>>>(k, M, F, status);
+            if (cudaPeekAtLastError() == cudaSuccess) return check_launch();
+            cudaGetLastError();  // cluster launch refused: the pulling factors below
+        }
+    }
     if (k <= 64) {
         const size_t smem = (size_t)k * k * sizeof(double);
         set_smem_attr(lu_factor_la_kernel, kLuLaMaxK * kLuLaMaxK * (int)sizeof(double));
-        lu_factor_la_kernel<<<1, kLuLaThreads, smem, st>>>(k, M, F, status);
+        lu_factor_la_kernel<<<1, kLuBlockThreads, smem, st>>>(k, M, F, status);
         return check_launch();
     }
     if (k >= kLucCtas && k <= kLucMaxK) {
@@ -375,17 +430,11 @@ int launch_lu_factor(cudaStream_t st, int k, const double *M, double *F, int *st
 int launch_lu_solve(cudaStream_t st, int k, const double *F, int r, const double *RHS,
                     double *Y) {
     if (k <= 0 || r <= 0) return CACG_ERR_ARG;
-    {
-        const size_t sweep_smem = ((size_t)k * k + k) * sizeof(double);
-        if (k <= 160 && sweep_smem <= max_smem_optin()) {
-            switch ((k + 31) / 32) {
-                case 1: return launch_sweep<1>(st, k, F, r, RHS, Y, sweep_smem);
-                case 2: return launch_sweep<2>(st, k, F, r, RHS, Y, sweep_smem);
-                case 3: return launch_sweep<3>(st, k, F, r, RHS, Y, sweep_smem);
-                case 4: return launch_sweep<4>(st, k, F, r, RHS, Y, sweep_smem);
-                case 5: return launch_sweep<5>(st, k, F, r, RHS, Y, sweep_smem);
-            }
-        }
+    if (k <= 160) {
+        const int nt = (k + 31) / 32, cols = nt >= 3 ? 1 : 4 / nt;
+        lu_solve_sweep_kernel<<<(r + cols - 1) / cols, 32 * nt * cols, 0, st>>>(k, nt, cols, F, r,
+                                                                                RHS, Y);
+        return check_launch();
     }
     size_t zbytes = (size_t)k * kLuRC * sizeof(double);
     size_t fbytes = ((size_t)k * k + k) * sizeof(double);
