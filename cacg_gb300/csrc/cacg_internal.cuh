@@ -83,6 +83,16 @@ __device__ __forceinline__ void vload_plain(float (&d)[4], const float *p) {
     float4 v = *reinterpret_cast<const float4 *>(p);
     d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
 }
+// four values from an address with 16-byte alignment
+__device__ __forceinline__ void vload_plain4(double (&d)[4], const double *p) {
+    const double2 v = *reinterpret_cast<const double2 *>(p);
+    const double2 w = *reinterpret_cast<const double2 *>(p + 2);
+    d[0] = v.x; d[1] = v.y; d[2] = w.x; d[3] = w.y;
+}
+__device__ __forceinline__ void vload_plain4(float (&d)[4], const float *p) {
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+}
 __device__ __forceinline__ void vstore(double *p, const double (&d)[2]) {
     *reinterpret_cast<double2 *>(p) = make_double2(d[0], d[1]);
 }

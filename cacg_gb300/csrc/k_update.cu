@@ -18,6 +18,8 @@
 #include <cfloat>
 
 #include "cacg_internal.cuh"
+#include "ff_util.cuh"
+#include "tc5_util.cuh"
 
 namespace cacg {
 
@@ -429,10 +431,34 @@ template int launch_xrupdate_fast<float>(cudaStream_t, int64_t, int, int, const 
 // Used when k and the row strides are multiples of the vector width.
 
 // Qout[i][c..c+3] = S[i][c..c+3] - sum_j Qin[i][j] beta[j][c..c+3]; a thread
-// owns kDqRows rows x 4 columns.
+// owns kDqRows rows x 4 columns.  The next four columns of its Q rows are loaded
+// while it works on the current ones, and S's before the loop: the loop is a
+// chain of L2 latencies otherwise (n = 491401, k = 44, FP32: 117 us, 110 so).
+// VEC: S and Qout rows take 16-byte accesses.
 constexpr int kDqRows = 4;
 
-template <typename T>
+// floats between the rows of a staged tile: an odd count of 16-byte chunks, so
+// that 16-byte reads down the rows take all banks in turn
+__host__ __device__ constexpr int xr_tile_pitch(int k) { return (k / 4) % 2 ? k : k + 4; }
+
+__device__ __forceinline__ void dq_load4(float (&v)[4], const float *p) {
+    const float4 x = __ldg(reinterpret_cast<const float4 *>(p));
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void dq_load4(double (&v)[4], const double *p) {
+    const double2 x = __ldg(reinterpret_cast<const double2 *>(p));
+    const double2 y = __ldg(reinterpret_cast<const double2 *>(p + 2));
+    v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+}
+__device__ __forceinline__ void dq_store4(float *p, const float (&v)[4]) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void dq_store4(double *p, const double (&v)[4]) {
+    *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
+}
+
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
     qupdate_direct_kernel(int64_t n, int k, T *Qout, int64_t ldo, const T *__restrict__ Qin,
                           int64_t ldq, const T *S, int64_t lds, const double *__restrict__ beta,
@@ -450,57 +476,57 @@ __global__ void __launch_bounds__(256)
     for (int64_t rg = (int64_t)blockIdx.x * groups_per_block + lg; rg < ngroups;
          rg += (int64_t)gridDim.x * groups_per_block) {
         const int64_t r0 = rg * kDqRows;
-        T acc[kDqRows][4];
+        T acc[kDqRows][4], sv[kDqRows][4], nx[kDqRows][4];
+        const T *qp[kDqRows];
 #pragma unroll
-        for (int i = 0; i < kDqRows; ++i)
+        for (int i = 0; i < kDqRows; ++i) {
+            const int64_t row = r0 + i < n ? r0 + i : n - 1;
+            qp[i] = Qin + row * ldq;
+            dq_load4(nx[i], qp[i]);
+            const T *sp = S + row * lds + cg * 4;
+            if constexpr (VEC) {
+                vload_plain4(sv[i], sp);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sv[i][q] = sp[q];
+            }
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[i][q] = T(0);
+        }
         for (int j = 0; j < k; j += 4) {
             T qv[kDqRows][4];
 #pragma unroll
             for (int i = 0; i < kDqRows; ++i) {
-                const int64_t row = r0 + i < n ? r0 + i : n - 1;
-                if constexpr (sizeof(T) == 4) {
-                    float4 v = __ldg(reinterpret_cast<const float4 *>(Qin + row * ldq + j));
-                    qv[i][0] = v.x; qv[i][1] = v.y; qv[i][2] = v.z; qv[i][3] = v.w;
-                } else {
-                    double2 v0 = __ldg(reinterpret_cast<const double2 *>(Qin + row * ldq + j));
-                    double2 v1 = __ldg(reinterpret_cast<const double2 *>(Qin + row * ldq + j + 2));
-                    qv[i][0] = v0.x; qv[i][1] = v0.y; qv[i][2] = v1.x; qv[i][3] = v1.y;
-                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) qv[i][q] = nx[i][q];
+                if (j + 4 < k) dq_load4(nx[i], qp[i] + j + 4);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const T *w = Ws + (size_t)(j + u) * k + cg * 4;
-                T w0, w1, w2, w3;
-                if constexpr (sizeof(T) == 4) {
-                    float4 wv = *reinterpret_cast<const float4 *>(w);
-                    w0 = wv.x; w1 = wv.y; w2 = wv.z; w3 = wv.w;
-                } else {
-                    double2 wa = *reinterpret_cast<const double2 *>(w);
-                    double2 wb = *reinterpret_cast<const double2 *>(w + 2);
-                    w0 = wa.x; w1 = wa.y; w2 = wb.x; w3 = wb.y;
-                }
+                T wv[4];
+                vload_plain4(wv, w);
 #pragma unroll
-                for (int i = 0; i < kDqRows; ++i) {
-                    acc[i][0] = fma(qv[i][u], w0, acc[i][0]);
-                    acc[i][1] = fma(qv[i][u], w1, acc[i][1]);
-                    acc[i][2] = fma(qv[i][u], w2, acc[i][2]);
-                    acc[i][3] = fma(qv[i][u], w3, acc[i][3]);
-                }
+                for (int i = 0; i < kDqRows; ++i)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) acc[i][q] = fma(qv[i][u], wv[q], acc[i][q]);
             }
         }
 #pragma unroll
         for (int i = 0; i < kDqRows; ++i) {
             const int64_t row = r0 + i;
             if (row >= n) break;
-            const T *sp = S + row * lds + cg * 4;
             T *op = Qout + row * ldo + cg * 4;
-            T o[4] = {sp[0] - acc[i][0], sp[1] - acc[i][1], sp[2] - acc[i][2], sp[3] - acc[i][3]};
-            op[0] = o[0];
-            op[1] = o[1];
-            op[2] = o[2];
-            op[3] = o[3];
+            T o[4] = {sv[i][0] - acc[i][0], sv[i][1] - acc[i][1], sv[i][2] - acc[i][2],
+                      sv[i][3] - acc[i][3]};
+            if constexpr (VEC) {
+                dq_store4(op, o);
+            } else {
+                op[0] = o[0];
+                op[1] = o[1];
+                op[2] = o[2];
+                op[3] = o[3];
+            }
             if constexpr (sizeof(T) == 4) {
                 if (qsl.p) store_slices4(qsl, row * ldo + cg * 4, o);
             }
@@ -606,6 +632,146 @@ __global__ void __launch_bounds__(256)
     for (int c = threadIdx.x; c < m; c += blockDim.x) part[(size_t)blockIdx.x * m + c] = red[c];
 }
 
+// The same update for FP32 operands, with every access to device memory over
+// contiguous bytes: a tile of Q and AQ rows is copied to shared memory
+// (cp.async; the next tile's copy runs over this one's output), the products go
+// through shared memory too, and X, R, S0 and R32 are updated element by element
+// in memory order.  xrupdate_direct_kernel's stores leave 32 bytes between the
+// lanes of a warp and its loads touch a row per three lanes: the L1's line rate
+// bounds it (n = 491401, k = 44, m = 11: 136.9 us, 113.7 here, of which the FP64
+// pipe's three operations an element take 27; n = 300000, k = 8, m = 1: 37.7 and
+// 24.8).  Widening and rounding go by the bits: as conversions on the FP64 pipe they
+// cost 9 us of the first.  Three blocks an SM: 113.7 us, four with spills 123.3.
+// Row sums, their order and the rounding are those of that kernel.
+__global__ void __launch_bounds__(256, 3)
+    xrupdate_tile_kernel(int64_t n, int k, int m, const float *__restrict__ Q,
+                         const float *__restrict__ AQ, int64_t ldq,
+                         const double *__restrict__ alpha, double *__restrict__ X,
+                         double *__restrict__ R, float *__restrict__ S0, int64_t lds,
+                         float *__restrict__ R32, double *__restrict__ part) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int XC = 4;
+    const int G = (m + XC - 1) / XC, mp = G * XC;
+    const int rpb = blockDim.x / G, pitch = xr_tile_pitch(k);
+    float *As = reinterpret_cast<float *>(smem_raw);  // k x mp
+    float *Qs = As + (size_t)k * mp;                  // rpb x pitch, AQ's tile behind it
+    float *As2 = Qs + (size_t)rpb * pitch;
+    float *xs = As2 + (size_t)rpb * pitch;            // rpb x m products, R's behind X's
+    float *rs = xs + (size_t)rpb * mp;
+    double *red = reinterpret_cast<double *>(xs);     // after the last tile (rpb x mp)
+    const int tid = threadIdx.x, T = blockDim.x;
+    const int k4 = k / 4, dr = T / k4, dc = T % k4;
+    const int64_t step = (int64_t)gridDim.x * rpb;
+    int64_t row0 = (int64_t)blockIdx.x * rpb;
+    auto copy_tile = [&](int64_t r0) {
+        const int rows = (int)(n - r0 < rpb ? n - r0 : rpb);
+        int r = tid / k4, c = tid % k4;
+        while (r < rows) {
+            t5_cp16(Qs + (size_t)r * pitch + c * 4, Q + (r0 + r) * ldq + c * 4, 16);
+            t5_cp16(As2 + (size_t)r * pitch + c * 4, AQ + (r0 + r) * ldq + c * 4, 16);
+            r += dr;
+            c += dc;
+            if (c >= k4) {
+                c -= k4;
+                ++r;
+            }
+        }
+    };
+    if (row0 < n) copy_tile(row0);
+    t5_cp_commit();
+    for (int idx = tid; idx < k * mp; idx += T) {
+        const int j = idx / mp, c = idx % mp;
+        As[idx] = c < m ? float(alpha[(size_t)j * m + c]) : 0.f;
+    }
+    const int lr = tid / G, g = tid % G;
+    // this thread's elements of a tile in memory order: rpb * m <= T * XC of them
+    int er[XC], ec[XC];
+    double sq[XC];
+#pragma unroll
+    for (int i = 0; i < XC; ++i) {
+        er[i] = (tid + i * T) / m;
+        ec[i] = (tid + i * T) % m;
+        sq[i] = 0.0;
+    }
+    for (; row0 < n; row0 += step) {
+        const int rows = (int)(n - row0 < rpb ? n - row0 : rpb);
+        double xv[XC], rv0[XC];
+#pragma unroll
+        for (int i = 0; i < XC; ++i) {
+            const bool in = er[i] < rows;
+            const int64_t e = row0 * m + tid + i * T;
+            xv[i] = in ? X[e] : 0.0;
+            rv0[i] = in ? R[e] : 0.0;
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        if (lr < rows) {
+            float ax[XC], ar[XC];
+#pragma unroll
+            for (int q = 0; q < XC; ++q) ax[q] = ar[q] = 0.f;
+            const float *qr = Qs + (size_t)lr * pitch, *aqr = As2 + (size_t)lr * pitch;
+#pragma unroll 2
+            for (int j = 0; j < k; j += 4) {
+                float q4[4], a4[4];
+                vload_plain4(q4, qr + j);
+                vload_plain4(a4, aqr + j);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float al[4];
+                    vload_plain4(al, As + (size_t)(j + u) * mp + g * XC);
+#pragma unroll
+                    for (int q = 0; q < XC; ++q) {
+                        ax[q] = fma(q4[u], al[q], ax[q]);
+                        ar[q] = fma(a4[u], al[q], ar[q]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < XC; ++q) {
+                if (g * XC + q < m) {
+                    xs[lr * m + g * XC + q] = ax[q];
+                    rs[lr * m + g * XC + q] = ar[q];
+                }
+            }
+        }
+        __syncthreads();
+        if (row0 + step < n) copy_tile(row0 + step);
+        t5_cp_commit();
+#pragma unroll
+        for (int i = 0; i < XC; ++i) {
+            if (er[i] < rows) {
+                const int64_t e = row0 * m + tid + i * T;
+                const double x = xv[i] + ff_widen(xs[tid + i * T]);
+                const double rv = rv0[i] - ff_widen(rs[tid + i * T]);
+                X[e] = x;
+                R[e] = rv;
+                const float rf = ff_narrow(rv);
+                if (S0) S0[(row0 + er[i]) * lds + ec[i]] = rf;
+                if (R32) R32[e] = rf;
+                sq[i] = fma(rv, rv, sq[i]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (!part) return;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < XC; ++i)
+        if (er[i] < rpb) red[er[i] * mp + ec[i]] = sq[i];
+    __syncthreads();
+    for (int h = rpb; h > 1;) {
+        const int half = (h + 1) / 2;
+        if (lr < h - half)
+#pragma unroll
+            for (int q = 0; q < XC; ++q)
+                if (g * XC + q < m)
+                    red[lr * mp + g * XC + q] += red[(lr + half) * mp + g * XC + q];
+        __syncthreads();
+        h = half;
+    }
+    for (int c = tid; c < m; c += T) part[(size_t)blockIdx.x * m + c] = red[c];
+}
+
 template <typename T>
 static bool direct_ok(int k, int64_t ld, const void *a, const void *b) {
     return k % 4 == 0 && ld % 4 == 0 && aligned16(a) && (!b || aligned16(b));
@@ -625,16 +791,23 @@ int launch_qupdate_direct(cudaStream_t st, int64_t n, int k, T *Qout, int64_t ld
     if (threads > 256) threads = G;  // G <= 256 here
     const int groups_per_block = threads / G;
     size_t smem = (size_t)k * k * sizeof(T);
-    set_smem_attr(qupdate_direct_kernel<T>, (int)max_smem_optin());
+    const bool vec = lds % 4 == 0 && ldo % 4 == 0 && aligned16(S) && aligned16(Qout);
+    set_smem_attr(qupdate_direct_kernel<T, true>, (int)max_smem_optin());
+    set_smem_attr(qupdate_direct_kernel<T, false>, (int)max_smem_optin());
     int64_t blocks = (ngroups + groups_per_block - 1) / groups_per_block;
     int64_t cap = (int64_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    qupdate_direct_kernel<T><<<(unsigned)blocks, threads, smem, st>>>(n, k, Qout, ldo, Qin, ldq, S,
-                                                                      lds, beta, qsl);
+    if (vec)
+        qupdate_direct_kernel<T, true><<<(unsigned)blocks, threads, smem, st>>>(
+            n, k, Qout, ldo, Qin, ldq, S, lds, beta, qsl);
+    else
+        qupdate_direct_kernel<T, false><<<(unsigned)blocks, threads, smem, st>>>(
+            n, k, Qout, ldo, Qin, ldq, S, lds, beta, qsl);
     return check_launch();
 }
 
 constexpr int kXrMaxBlocks = 2048;  // norm partials per xrupdate launch (upper bound)
+constexpr size_t kXrTileSmem = 112 * 1024;  // at least two blocks of the tile kernel on an SM
 
 template <typename T, int XC>
 static int launch_xrd(cudaStream_t st, int64_t n, int k, int m, const T *Q, const T *AQ,
@@ -651,6 +824,19 @@ static int launch_xrd(cudaStream_t st, int64_t n, int k, int m, const T *Q, cons
     int64_t cap = std::min<int64_t>((int64_t)sm_count() * 8, kXrMaxBlocks);
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
+    if constexpr (std::is_same<T, float>::value && XC == 4) {
+        const size_t tsm = ((size_t)k * mp + (size_t)rows_per_block * 2 *
+                                                 (xr_tile_pitch(k) + mp)) * sizeof(float);
+        // (the direct kernel stores slice planes and takes the widest k)
+        if (!s0sl.p && !r32sl.p && tsm <= kXrTileSmem) {
+            set_smem_attr(xrupdate_tile_kernel, (int)kXrTileSmem);
+            xrupdate_tile_kernel<<<(unsigned)blocks, threads, tsm, st>>>(
+                n, k, m, Q, AQ, ldq, alpha, X, R, S0, lds, R32, norms ? ws : nullptr);
+            const int rc = check_launch();
+            if (rc != CACG_OK || !norms) return rc;
+            return launch_colsum(st, ws, (int)blocks, m, norms);
+        }
+    }
     xrupdate_direct_kernel<T, XC><<<(unsigned)blocks, threads, smem, st>>>(
         n, k, m, Q, AQ, ldq, alpha, X, R, S0, lds, R32, norms ? ws : nullptr, s0sl, r32sl);
     int rc = check_launch();
