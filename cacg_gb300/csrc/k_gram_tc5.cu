@@ -322,54 +322,77 @@ __global__ void __launch_bounds__(kT5Threads, 1)
 
 // ---------------------------------------------------------------------------
 // MN-major variant (the default where the operands allow TMA): raw FP32 rows
-// arrive as 32 x 32 boxes (128 bytes a row, 128-byte swizzle) by 2-D TMA
-// loads that one thread issues; the slices are stored MN-major (a core-matrix
-// row = 8 consecutive columns of one input row), so a thread converts a unit
-// (8 columns of one row) with two 16-byte shared loads, the split and three
-// 16-byte stores, without the column gather a K-major tile needs.  The 128-B
-// swizzle puts the 16-byte chunk c of row k at chunk c ^ (k & 7), so the 8
-// rows a quarter warp reads fall on distinct banks; the MN-major core matrix
-// rows (16 bytes at (k & 7) * 16) are conflict-free for the same 8 rows.
-// Descriptors (no swizzle, MN-major): SBO = 128 B between 8-column groups,
-// LBO = (MN / 8) * 128 B between 8-row (K) groups; instruction descriptor
-// with the A and B transpose bits.
-constexpr int kT5mBox = 32;                          // rows and FP32 columns of a box
-constexpr unsigned kT5mBoxBytes = kT5mBox * kT5mBox * 4;  // 4 KB
-
-constexpr int kT5wConvWarps = 16;                  // converter warps
-constexpr int kT5wConv = 32 * kT5wConvWarps;          // converter threads
-constexpr int kT5wThreads = kT5wConv + 64;            // + a loader warp and an MMA warp
-constexpr int kT5wUnits = 2;                          // conversion units per converter thread
-constexpr int kT5wNB = 2;                             // bf16 slice buffers
-
-// Warp-specialised pipeline, no CTA-wide barrier per step:
-//   loader (thread 512): waits empty[q], issues step j's TMA boxes into ring
-//     stage q = j % stages, completing on full[q];
-//   converters (warps 0-15): wait full[q] and sfree[b] (b = j % 2), split the
-//     stage into slice buffer b, fence the stores to the async proxy, arrive
-//     on sfull[b] and empty[q]; two steps after a group's last step they read
-//     its FP32 sum from TMEM (gdone[g & 1]) into the float-float registers and
-//     arrive on gfree[g & 1];
-//   MMA issuer (thread 544): waits sfull[b] (and gfree before a group reuses
-//     a TMEM buffer), issues the 12 MMAs, commits to sfree[b] and, at a
-//     group's end, to gdone[g & 1].
+// arrive as boxes of 32 rows x 16 columns (64 bytes a row, 64-byte swizzle) by
+// 2-D TMA loads that one thread issues; the slices are stored MN-major (a
+// core-matrix row = 8 consecutive columns of one input row), so a thread
+// converts a unit (8 columns of one row) with two 16-byte shared loads, the
+// split and three 16-byte stores, without the column gather a K-major tile
+// needs.  The swizzle puts the 16-byte chunk c of row k at chunk
+// c ^ (k / 2 & 3), so the 8 rows a quarter warp reads fall on distinct banks;
+// the MN-major core matrix rows (16 bytes at (k & 7) * 16) are conflict-free for
+// the same 8 rows.  Descriptors (no swizzle, MN-major): SBO = 128 B between
+// 8-column groups, LBO = (MN / 8) * 128 B between 8-row (K) groups; instruction
+// descriptor with the A and B transpose bits.  The A tile holds BA columns, not
+// 128: accumulator rows past BA take what lies behind it in shared memory and
+// are not read.
+//
+// Warp-specialised pipeline over steps of 32 rows, two steps a group:
+//   loader warp: waits empty[q], issues step j's TMA boxes into ring stage
+//     q = j % stages, completing on full[q];
+//   converter warps, in two halves, one for the first and one for the second
+//     step of every group: wait for full[q] and for a free slice buffer of
+//     their half (sfree, or gdone for the second half), split the step's units,
+//     fence the stores to the async proxy and arrive on sfull and empty[q];
+//   MMA warp: waits sfull (and gfree before a group reuses a TMEM buffer),
+//     issues the 12 MMAs, commits to sfree and, at a group's end, to gdone;
+//   16 sum warps: wait gdone, add the group's FP32 sum from TMEM to their
+//     float-float registers and arrive on gfree.
 // Every wait is bounded and also ends when another role has set the abort
 // flag; a role that times out sets kStatusTimeout and the flag, the loader
 // and the issuer then wait (bounded) for their own loads and MMAs in flight.
+//
+// What bounds it is the latency of these chains, not DRAM (74 % at 80 x 96) or
+// the tensor cores (half): one block an SM, and a barrier wait, a TMA or an MMA
+// issue cost a warp among 28 hundreds of cycles, 64 and 50.  Hence the sums on
+// warps of their own, the two halves, the loader and the issuer as whole warps
+// with one elected lane (their operands stay in uniform registers), paired
+// waits, and no test per row (rows past n and columns past an operand are zeros
+// that the loads fill in).  With 16 warps that converted and summed every step
+// and one-thread issuers: 450 us at n = 2M, 80 x 96 and 96.5 at n = 491401,
+// 44 x 55; now 300 and 69.  Boxes of 16 columns, not 32, carry at most 15 columns
+// past an operand, which leaves the wide tiles four stages.  The partition of
+// the rows, the MMAs' order in an accumulator and the sums' order do not depend
+// on any of this: the results are the same bits.
+constexpr int kT5mRows = 32, kT5mBox = 16;           // rows and FP32 columns of a box
+constexpr unsigned kT5mBoxBytes = kT5mRows * kT5mBox * 4;  // 2 KB
+
+constexpr int kT5wSumWarps = 16;  // warps that keep the float-float sums
+// converter warps (two halves): as many as their registers leave room for
+__host__ __device__ constexpr int t5w_conv_warps(int NC8) { return NC8 <= 4 ? 14 : 10; }
+// + a loader warp and an MMA warp
+__host__ __device__ constexpr int t5w_threads(int NC8) {
+    return 32 * (kT5wSumWarps + t5w_conv_warps(NC8) + 2);
+}
+
 template <int NC8>
-__global__ void __launch_bounds__(kT5wThreads, 1)
+__global__ void __launch_bounds__(t5w_threads(NC8), 1)
     gram_tc5m_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmR1,
                      const __grid_constant__ CUtensorMap tmR2, int64_t n, int64_t rows_per_chunk,
-                     int ka, int kb1, int kb2, int BA, int tilesB, int tmem_half, int stages,
+                     int ka, int kb1, int kb2, int BA, int tilesB, int tmem_half, int stages, int nbuf,
                      double *__restrict__ part, int *__restrict__ status, long long pipe_polls) {
     constexpr int BB = 16 * NC8;
-    constexpr int HC = BB / 4;  // accumulator columns per converter thread (a quarter row)
-    constexpr unsigned a_bytes = kT5M * kT5KT * 2, b_bytes = BB * kT5KT * 2;
-    constexpr unsigned buf_bytes = 3 * (a_bytes + b_bytes);
-    constexpr unsigned lbo_a = (kT5M / 8) * 128, lbo_b = (BB / 8) * 128;
+    constexpr int kConv = t5w_conv_warps(NC8), kTeam = kConv / 2, kThreads = t5w_threads(NC8);
+    constexpr int HC = BB / 4;  // accumulator columns per sum thread (a quarter row)
+    static_assert(kT5Flush == 2 && kT5mRows == kT5KT, "a group is two steps, one a half of the converters");
+    const unsigned a_bytes = (unsigned)BA * kT5KT * 2;
+    constexpr unsigned b_bytes = BB * kT5KT * 2;
+    const unsigned buf_bytes = 3 * (a_bytes + b_bytes);
+    const unsigned lbo_a = (unsigned)BA * 16;
+    constexpr unsigned lbo_b = BB * 16;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // [slice buffers][ring: stages x boxes x 4 KB, 1 KB aligned][mbarriers][tmem slot][abort]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // [slice buffers][ring: stages x boxes x 2 KB, 1 KB aligned][mbarriers][tmem slot][abort]
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, and known to be
     const int tile_a = blockIdx.y / tilesB, tile_b = blockIdx.y % tilesB;
     const int a0 = tile_a * BA, b0 = tile_b * BB;
     const int nbl = (BA + kT5mBox - 1) / kT5mBox;
@@ -379,36 +402,43 @@ __global__ void __launch_bounds__(kT5wThreads, 1)
     const int nbr2 = r2end > r2beg ? (r2end - r2beg + kT5mBox - 1) / kT5mBox : 0;
     const int c2 = r2beg - kb1;  // first R2 column of this tile's boxes
     const int nbox = nbl + nbr1 + nbr2;
-    const unsigned ring_off = (kT5wNB * buf_bytes + 1023) / 1024 * 1024;
+    const unsigned ring_off = (2 * nbuf * buf_bytes + 1023) / 1024 * 1024;
     unsigned char *ring = smem_raw + ring_off;
     const unsigned stage_bytes = (unsigned)nbox * kT5mBoxBytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + (size_t)stages * stage_bytes);
     uint64_t *empty = full + stages;
     uint64_t *sfull = empty + stages;
-    uint64_t *sfree = sfull + kT5wNB;
-    uint64_t *gdone = sfree + kT5wNB;
+    uint64_t *sfree = sfull + 4;  // sfull: [half][nbuf], sfree: [nbuf] of the first half
+    uint64_t *gdone = sfree + 2;
     uint64_t *gfree = gdone + 2;
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(gfree + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int64_t rbeg = (int64_t)blockIdx.x * rows_per_chunk;
     const int64_t rend = min(n, rbeg + rows_per_chunk);
-    const int64_t nsteps = rend > rbeg ? (rend - rbeg + kT5KT - 1) / kT5KT : 0;
+    const int nsteps = rend > rbeg ? (int)((rend - rbeg + kT5KT - 1) / kT5KT) : 0;
+    const int ngroups = (nsteps + 1) / 2;
+    const int nsh = nbuf - 1;  // 1 or 2 slice buffers a half
+    const bool even = (stages & 1) == 0;  // a stage always takes the same half's step
 
-    for (unsigned i = tid; i < kT5wNB * buf_bytes / 16; i += kT5wThreads)
-        reinterpret_cast<uint4 *>(smem_raw)[i] = make_uint4(0, 0, 0, 0);
+    // octets of the B tile past the operands' columns: zeros no conversion writes
+    const int na = BA / 8, n1 = b0 < kb1 ? (r1end - b0 + 7) / 8 : 0;
+    const int nb = n1 + min(2 * nbr2, BB / 8 - n1);
+    for (int i = tid; i < 2 * nbuf * 3 * 4 * (BB / 8 - nb) * 8; i += kThreads) {
+        const int c = i % 8, r = i / 8, o = nb + r % (BB / 8 - nb), t = r / (BB / 8 - nb);
+        *reinterpret_cast<uint4 *>(smem_raw + (t / 12) * buf_bytes + 3 * a_bytes + (t / 4 % 3) * b_bytes +
+                                   (t % 4) * lbo_b + o * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+    }
     if (tid == 0) {
         for (int q = 0; q < stages; ++q) {
             t5_mbar_init(&full[q], 1);
-            t5_mbar_init(&empty[q], kT5wConvWarps);
+            t5_mbar_init(&empty[q], even ? kTeam : kConv);
         }
-        for (int b = 0; b < kT5wNB; ++b) {
-            t5_mbar_init(&sfull[b], kT5wConvWarps);
+        for (int b = 0; b < 4; ++b) t5_mbar_init(&sfull[b], kTeam);
+        for (int b = 0; b < 2; ++b) {
             t5_mbar_init(&sfree[b], 1);
-        }
-        for (int x = 0; x < 2; ++x) {
-            t5_mbar_init(&gdone[x], 1);
-            t5_mbar_init(&gfree[x], kT5wConvWarps);
+            t5_mbar_init(&gdone[b], 1);
+            t5_mbar_init(&gfree[b], kT5wSumWarps);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -419,78 +449,47 @@ __global__ void __launch_bounds__(kT5wThreads, 1)
                      "r"(2 * tmem_half));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    t5_fence_proxy_async();
+    t5_fence_before();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    t5_fence_after();
     const unsigned tmem = *tmem_slot;
     auto fail = [&]() {
         *abort_flag = 1;
         atomicOr(status, kStatusTimeout);
     };
-    auto group_end = [&](int64_t e) { return e % kT5Flush == kT5Flush - 1 || e == nsteps - 1; };
 
-    float acc_hi[HC], acc_lo[HC];
-#pragma unroll
-    for (int q = 0; q < HC; ++q) acc_hi[q] = acc_lo[q] = 0.f;
-
-    int64_t issued = 0;  // loader: TMA fills issued
-    if (warp < kT5wConvWarps) {
-        // ------------------------------------------------------ converters
-        int usrc[kT5wUnits], uch[kT5wUnits], udst[kT5wUnits], uslice[kT5wUnits], urow[kT5wUnits];
-        const int noct = (BA + BB) / 8;
-#pragma unroll
-        for (int u = 0; u < kT5wUnits; ++u) {
-            const int id = tid + u * kT5wConv;
-            usrc[u] = -1;
-            uch[u] = 0;
-            udst[u] = 0;
-            uslice[u] = 0;
-            urow[u] = 0;
-            if (id < kT5KT * noct) {
-                const int k = id % kT5KT, o = id / kT5KT;
-                int box, col;
-                if (o < BA / 8) {
-                    box = (8 * o) / kT5mBox;
-                    col = (8 * o) % kT5mBox;
-                    udst[u] = o * 128 + (k / 8) * (int)lbo_a + (k % 8) * 16;
-                    uslice[u] = (int)a_bytes;
-                } else {
-                    const int cb = 8 * (o - BA / 8);
-                    if (b0 + cb < kb1) {
-                        box = nbl + cb / kT5mBox;
-                        col = cb % kT5mBox;
-                    } else {
-                        const int rel = b0 + cb - kb1 - c2;
-                        box = nbl + nbr1 + rel / kT5mBox;
-                        col = rel % kT5mBox;
-                    }
-                    udst[u] = 3 * (int)a_bytes + (o - BA / 8) * 128 + (k / 8) * (int)lbo_b +
-                              (k % 8) * 16;
-                    uslice[u] = (int)b_bytes;
-                }
-                // an octet past the operand's columns has no box: it converts zeros
-                usrc[u] = box < nbox ? box * (int)kT5mBoxBytes + k * 128 : -2;
-                uch[u] = col / 4;
-                urow[u] = k;
-            }
-        }
+    int issued = 0;  // loader: TMA fills issued
+    constexpr int kLoader = kT5wSumWarps + kConv;  // warp; the MMA warp follows
+    if (warp < kT5wSumWarps) {
+        // ------------------------------------------------------------ sums
         // warp w reads TMEM lanes 32 (w % 4) .. + 31 (its lane quadrant),
-        // columns [(w / 4) HC, + HC)
-        const int quad = warp & 3, quarter = warp >> 2;
-        // TMEM loads of up to 16 columns go out together, then one wait
-        auto flush = [&](int64_t step) {
-            const unsigned tb = (unsigned)(((step / kT5Flush) & 1) * tmem_half);
-            const unsigned ta = tmem + ((unsigned)(32 * quad) << 16) + tb + (unsigned)(quarter * HC);
+        // columns [(w / 4) HC, + HC); up to 16 columns' loads, then one wait
+        float acc_hi[HC], acc_lo[HC];
 #pragma unroll
-            for (int h0 = 0; h0 < NC8; h0 += 4) {
-                unsigned r[4][4];
+        for (int q = 0; q < HC; ++q) acc_hi[q] = acc_lo[q] = 0.f;
+        bool ok = true;
+        const unsigned tq = tmem + ((unsigned)(32 * (warp & 3)) << 16) + (unsigned)((warp >> 2) * HC);
+        for (int g = 0; g < ngroups; ++g) {
+            const bool w = t5_mbar_wait_or_abort(&gdone[g & 1], (unsigned)((g >> 1) & 1), abort_flag,
+                                                 pipe_polls);
+            if (!__all_sync(0xffffffffu, w)) {
+                if (lane == 0) fail();
+                ok = false;
+                break;
+            }
+            t5_fence_after();
+            const unsigned ta = tq + (unsigned)((g & 1) * tmem_half);
+            constexpr int kLd = NC8 <= 4 ? 4 : 2;  // registers
 #pragma unroll
-                for (int c4 = 0; c4 < 4; ++c4)
+            for (int h0 = 0; h0 < NC8; h0 += kLd) {
+                unsigned r[kLd][4];
+#pragma unroll
+                for (int c4 = 0; c4 < kLd; ++c4)
                     if (h0 + c4 < NC8) t5_ld4_nowait(ta + 4 * (h0 + c4), r[c4]);
                 t5_wait_ld();
 #pragma unroll
-                for (int c4 = 0; c4 < 4; ++c4) {
+                for (int c4 = 0; c4 < kLd; ++c4) {
                     if (h0 + c4 >= NC8) break;
 #pragma unroll
                     for (int q = 0; q < 4; q += 2) {
@@ -500,167 +499,207 @@ __global__ void __launch_bounds__(kT5wThreads, 1)
                     }
                 }
             }
-        };
-        // flush of the group ending at step e; false if its MMAs never completed
-        auto flush_group = [&](int64_t e) {
-            const int64_t g = e / kT5Flush;
-            const bool ok = __all_sync(0xffffffffu, t5_mbar_wait_or_abort(
-                                                        &gdone[g & 1], (unsigned)((g >> 1) & 1),
-                                                        abort_flag, pipe_polls));
-            if (!ok) return false;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            flush(e);
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            t5_fence_before();
             __syncwarp();
             if (lane == 0) t5_mbar_arrive(&gfree[g & 1]);
-            return true;
-        };
-        bool ok = true;
-        // ring stage and its phase, stepped (no division by the runtime depth)
-        int q = 0;
-        unsigned qph = 0;
-        for (int64_t j = 0; j < nsteps && ok; ++j) {
-            const int b = (int)(j % kT5wNB);
-            bool w = t5_mbar_wait_or_abort(&full[q], qph, abort_flag, pipe_polls);
-            if (w && j >= kT5wNB)
-                w = t5_mbar_wait_or_abort(&sfree[b], (unsigned)(((j / kT5wNB) - 1) & 1), abort_flag,
-                                          pipe_polls);
-            if (!__all_sync(0xffffffffu, w)) {
-                ok = false;
-                break;
-            }
-            const unsigned char *src = ring + (size_t)q * stage_bytes;
-            unsigned char *dbase = smem_raw + b * buf_bytes;
-            const int64_t r0 = rbeg + j * kT5KT;
+        }
+        // (a block that gave up elsewhere fails the whole product: its partial is not read)
+        const int row_t = 32 * (warp & 3) + lane;
+        if (ok && row_t < BA) {
+            double *out = part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * (size_t)BA * BB +
+                          (size_t)row_t * BB + (warp >> 2) * HC;
 #pragma unroll
-            for (int u = 0; u < kT5wUnits; ++u) {
-                if (usrc[u] == -1) continue;
-                const int sw = urow[u] & 7;
-                float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
-                if (usrc[u] >= 0 && r0 + urow[u] < rend) {
-                    v0 = *reinterpret_cast<const float4 *>(src + usrc[u] + ((uch[u] ^ sw) << 4));
-                    v1 = *reinterpret_cast<const float4 *>(src + usrc[u] +
-                                                           (((uch[u] + 1) ^ sw) << 4));
+            for (int q = 0; q < HC; ++q) out[q] = (double)acc_hi[q] + (double)acc_lo[q];
+        }
+    } else if (warp < kT5wSumWarps + kConv) {
+        // ------------------------------------------------------ converters
+        // half h converts step h of every group; a unit is 8 columns (octet o) of
+        // the step's 32 rows, a row a lane.  Octets past an operand's columns have
+        // no box (at the end of the B tile only): the buffers' zeros.
+        const int h = (warp - kT5wSumWarps) / kTeam, tw = (warp - kT5wSumWarps) % kTeam;
+        const int nocts = na + nb;
+        const int lsrc = lane * (kT5mBox * 4) + (((lane >> 1) & 3) << 4);
+        const int ldst_a = (lane / 8) * (int)lbo_a + (lane % 8) * 16;
+        const int ldst_b = (int)(3 * a_bytes) + (lane / 8) * (int)lbo_b + (lane % 8) * 16;
+        auto load_unit = [&](const unsigned char *src, int o, float4 (&v)[2]) {
+            int r = o, box = 0;
+            if (o >= na + n1)
+                r = o - na - n1, box = nbl + nbr1;
+            else if (o >= na)
+                r = o - na, box = nbl;
+            const int off = (box + (r >> 1)) * (int)kT5mBoxBytes + (lsrc ^ ((r & 1) << 5));
+            v[0] = *reinterpret_cast<const float4 *>(src + off);
+            v[1] = *reinterpret_cast<const float4 *>(src + (off ^ 16));
+        };
+        auto split_unit = [&](unsigned char *dbase, int o, const float4 (&v)[2]) {
+            unsigned hw[4], mw[4], lw[4];
+            t5_split2(v[0].x, v[0].y, hw[0], mw[0], lw[0]);
+            t5_split2(v[0].z, v[0].w, hw[1], mw[1], lw[1]);
+            t5_split2(v[1].x, v[1].y, hw[2], mw[2], lw[2]);
+            t5_split2(v[1].z, v[1].w, hw[3], mw[3], lw[3]);
+            unsigned char *d = dbase + (o < na ? ldst_a + o * 128 : ldst_b + (o - na) * 128);
+            const unsigned slice = o < na ? a_bytes : b_bytes;
+            *reinterpret_cast<uint4 *>(d) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            *reinterpret_cast<uint4 *>(d + slice) = make_uint4(mw[0], mw[1], mw[2], mw[3]);
+            *reinterpret_cast<uint4 *>(d + 2 * slice) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        };
+        const int mysteps = (nsteps + 1 - h) / 2;
+        bool ok = true;
+        int q = h % stages;  // this warp's next ring stage and its phase
+        unsigned qph = 0;
+        for (int g = 0; g < ngroups; ++g) {
+            const int x = h * nbuf + (g & nsh);  // this half's slice buffer of the group
+            if (g < mysteps) {
+                // the buffer's last MMAs: group gp's, whose second step gdone covers
+                const int gp = g - nbuf;
+                const bool w =
+                    gp < 0 ? t5_mbar_wait_or_abort(&full[q], qph, abort_flag, pipe_polls)
+                           : t5_mbar_wait2_or_abort(
+                                 &full[q], qph, h == 0 ? &sfree[g & nsh] : &gdone[gp & 1],
+                                 (unsigned)((h == 0 ? gp >> nsh : gp >> 1) & 1), abort_flag,
+                                 pipe_polls);
+                if (!__all_sync(0xffffffffu, w)) {
+                    ok = false;
+                    break;
                 }
-                unsigned hw[4], mw[4], lw[4];
-                t5_split2(v0.x, v0.y, hw[0], mw[0], lw[0]);
-                t5_split2(v0.z, v0.w, hw[1], mw[1], lw[1]);
-                t5_split2(v1.x, v1.y, hw[2], mw[2], lw[2]);
-                t5_split2(v1.z, v1.w, hw[3], mw[3], lw[3]);
-                unsigned char *d = dbase + udst[u];
-                *reinterpret_cast<uint4 *>(d) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                *reinterpret_cast<uint4 *>(d + uslice[u]) = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-                *reinterpret_cast<uint4 *>(d + 2 * uslice[u]) =
-                    make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                const unsigned char *src = ring + (size_t)q * stage_bytes;
+                unsigned char *dbase = smem_raw + x * buf_bytes;
+                int o = tw;
+                for (; o + kTeam < nocts; o += 2 * kTeam) {  // two units in flight
+                    float4 va[2], vb[2];
+                    load_unit(src, o, va);
+                    load_unit(src, o + kTeam, vb);
+                    split_unit(dbase, o, va);
+                    split_unit(dbase, o + kTeam, vb);
+                }
+                if (o < nocts) {
+                    float4 va[2];
+                    load_unit(src, o, va);
+                    split_unit(dbase, o, va);
+                }
+                // slices visible to the tensor cores; the stage may be refilled
+                t5_fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    t5_mbar_arrive(&sfull[x]);
+                    t5_mbar_arrive(&empty[q]);
+                }
             }
-            // slices visible to the tensor cores; the stage may be refilled
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-                t5_mbar_arrive(&sfull[b]);
-                t5_mbar_arrive(&empty[q]);
+            if (!even) {
+                // A wait's parity tells a fill from its neighbours only to a warp
+                // that sees each fill of the stage, and holds its refill back until
+                // it has.  With an odd count the halves take turns in a stage, so
+                // every warp sees, and releases, the other half's stage as well.
+                const int oj = 2 * g + 1 - h;  // its step
+                const int oq = h ? (q > 0 ? q - 1 : stages - 1) : (q + 1 < stages ? q + 1 : 0);
+                const unsigned oph = h ? (q > 0 ? qph : qph ^ 1u) : (q + 1 < stages ? qph : qph ^ 1u);
+                if (oj < nsteps) {
+                    const bool w = t5_mbar_wait_or_abort(&full[oq], oph, abort_flag, pipe_polls);
+                    if (!__all_sync(0xffffffffu, w)) {
+                        ok = false;
+                        break;
+                    }
+                    if (lane == 0) t5_mbar_arrive(&empty[oq]);
+                }
             }
-            if (++q == stages) {
-                q = 0;
+            q += 2;
+            if (q >= stages) {
+                q -= stages;
                 qph ^= 1u;
             }
-            if (j >= 2 && group_end(j - 2)) ok = flush_group(j - 2);
         }
-        // the last groups' sums
-        for (int64_t e = nsteps - 2; ok && e < nsteps; ++e)
-            if (e >= 0 && group_end(e)) ok = flush_group(e);
         if (!ok && lane == 0) fail();
-    } else if (tid == kT5wConv) {
+    } else if (warp == kLoader) {
         // ---------------------------------------------------------- loader
         int q = 0;
         unsigned qph = 0;  // phase of stage q's current fill
-        for (int64_t j = 0; j < nsteps; ++j) {
+        for (int j = 0; j < nsteps; ++j) {
             if (j > 0 && q == 0) qph ^= 1u;
-            if (j >= stages && !t5_mbar_wait_or_abort(&empty[q], qph ^ 1u, abort_flag, pipe_polls)) {
-                fail();
+            if (j >= stages &&
+                !__all_sync(0xffffffffu, t5_mbar_wait_or_abort(&empty[q], qph ^ 1u, abort_flag,
+                                                               pipe_polls))) {
+                if (lane == 0) fail();
                 break;
             }
             unsigned char *dst = ring + (size_t)q * stage_bytes;
-            const int row0 = (int)(rbeg + j * kT5KT);
-            tma_expect_tx(&full[q], stage_bytes);
-            for (int bx = 0; bx < nbl; ++bx)
-                tma_load_2d(dst + bx * kT5mBoxBytes, &tmL, a0 + kT5mBox * bx, row0, &full[q]);
-            for (int bx = 0; bx < nbr1; ++bx)
-                tma_load_2d(dst + (nbl + bx) * kT5mBoxBytes, &tmR1, b0 + kT5mBox * bx, row0,
-                            &full[q]);
-            for (int bx = 0; bx < nbr2; ++bx)
-                tma_load_2d(dst + (nbl + nbr1 + bx) * kT5mBoxBytes, &tmR2, c2 + kT5mBox * bx, row0,
-                            &full[q]);
+            const int row0 = (int)(rbeg + (int64_t)j * kT5KT);
+            if (t5_elect()) {
+                tma_expect_tx(&full[q], stage_bytes);
+                for (int bx = 0; bx < nbl; ++bx)
+                    tma_load_2d(dst + bx * kT5mBoxBytes, &tmL, a0 + kT5mBox * bx, row0, &full[q]);
+                for (int bx = 0; bx < nbr1; ++bx)
+                    tma_load_2d(dst + (nbl + bx) * kT5mBoxBytes, &tmR1, b0 + kT5mBox * bx, row0,
+                                &full[q]);
+                for (int bx = 0; bx < nbr2; ++bx)
+                    tma_load_2d(dst + (nbl + nbr1 + bx) * kT5mBoxBytes, &tmR2, c2 + kT5mBox * bx,
+                                row0, &full[q]);
+            }
+            __syncwarp();
             issued = j + 1;
             if (++q == stages) q = 0;
         }
-    } else if (tid == kT5wConv + 32) {
+    } else {
         // ---------------------------------------------------- MMA issuer
         const unsigned idesc = t5_idesc(kT5M, BB) | (1u << 15) | (1u << 16);  // A, B MN-major
-        int64_t last = -1;
-        for (int64_t j = 0; j < nsteps; ++j) {
-            const int b = (int)(j % kT5wNB);
-            const int64_t g = j / kT5Flush;
-            if (!t5_mbar_wait_or_abort(&sfull[b], (unsigned)((j / kT5wNB) & 1), abort_flag,
-                                       pipe_polls) ||
-                (j % kT5Flush == 0 && g >= 2 &&
-                 !t5_mbar_wait_or_abort(&gfree[g & 1], (unsigned)(((g >> 1) - 1) & 1),
-                                        abort_flag, pipe_polls))) {
-                fail();
+        const unsigned sbase = t5_smem_u32(smem_raw);
+        int last = -1;
+        for (int j = 0; j < nsteps; ++j) {
+            const int b = j & 1, g = j >> 1, x = b * nbuf + (g & nsh);
+            const unsigned sph = (unsigned)((g >> nsh) & 1);
+            const bool w =
+                b == 1 || g < 2
+                    ? t5_mbar_wait_or_abort(&sfull[x], sph, abort_flag, pipe_polls)
+                    : t5_mbar_wait2_or_abort(&sfull[x], sph, &gfree[g & 1],
+                                             (unsigned)(((g >> 1) - 1) & 1), abort_flag, pipe_polls);
+            if (!__all_sync(0xffffffffu, w)) {
+                if (lane == 0) fail();
                 break;
             }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const unsigned abase = t5_smem_u32(smem_raw + b * buf_bytes);
-            const unsigned bbase = abase + 3 * a_bytes;
+            t5_fence_after();
+            const unsigned abase = sbase + x * buf_bytes, bbase = abase + 3 * a_bytes;
             const unsigned dt = tmem + (unsigned)((g & 1) * tmem_half);
-            unsigned accumulate = (j % kT5Flush) != 0;
-            const int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};
+            // descriptors of the step's first 16 rows; offsets add to the address field
+            const uint64_t ad0 = t5_desc_lbo(abase, lbo_a, 128), bd0 = t5_desc_lbo(bbase, lbo_b, 128);
+            if (t5_elect()) {
+                const int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};
 #pragma unroll
-            for (int pr = 0; pr < 6; ++pr) {
+                for (int pr = 0; pr < 6; ++pr) {
 #pragma unroll
-                for (int kk = 0; kk < kT5KT / 16; ++kk) {
-                    const uint64_t ad =
-                        t5_desc_lbo(abase + pa[pr] * a_bytes + 2 * kk * lbo_a, lbo_a, 128);
-                    const uint64_t bd =
-                        t5_desc_lbo(bbase + pb[pr] * b_bytes + 2 * kk * lbo_b, lbo_b, 128);
-                    t5_mma(dt, ad, bd, idesc, accumulate);
-                    accumulate = 1;
+                    for (int kk = 0; kk < kT5KT / 16; ++kk)
+                        t5_mma(dt, ad0 + (uint64_t)((pa[pr] * a_bytes + 2 * kk * lbo_a) >> 4),
+                               bd0 + (uint64_t)((pb[pr] * b_bytes + 2 * kk * lbo_b) >> 4), idesc,
+                               pr + kk > 0 ? 1u : (unsigned)b);
                 }
+                if (b == 0) t5_commit(&sfree[x]);
+                if (b == 1 || j == nsteps - 1) t5_commit(&gdone[g & 1]);
             }
-            t5_commit(&sfree[b]);
-            if (group_end(j)) t5_commit(&gdone[g & 1]);
+            __syncwarp();
             last = j;
         }
         // every committed MMA finishes before TMEM goes (bounded), whether or
         // not another role gave up after this loop ended
         if (last >= 0) {
-            t5_mbar_wait(&sfree[last % kT5wNB], (unsigned)((last / kT5wNB) & 1));
-            const int64_t g = last / kT5Flush;
-            if (group_end(last)) t5_mbar_wait(&gdone[g & 1], (unsigned)((g >> 1) & 1));
+            const int g = last >> 1;
+            if ((last & 1) || last == nsteps - 1)
+                t5_mbar_wait(&gdone[g & 1], (unsigned)((g >> 1) & 1));
+            else
+                t5_mbar_wait(&sfree[g & nsh], (unsigned)((g >> nsh) & 1));
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    t5_fence_before();
     const int bad = __syncthreads_or(*abort_flag);
     // after a give-up some fills may never have been consumed: the loader lets
     // its last `stages` fills land (bounded) before its thread, and so the
     // CTA and its shared memory, can retire
-    if (bad && tid == kT5wConv)
-        for (int64_t j = issued - stages > 0 ? issued - stages : 0; j < issued; ++j)
+    if (bad && warp == kLoader)
+        for (int j = issued - stages > 0 ? issued - stages : 0; j < issued; ++j)
             t5_mbar_wait(&full[j % stages], (unsigned)((j / stages) & 1));
     if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        t5_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem),
                      "r"(2 * tmem_half));
     }
-    if (bad || warp >= kT5wConvWarps) return;
-    const int row_t = 32 * (warp & 3) + lane, quarter = warp >> 2;
-    if (row_t >= BA) return;
-    double *out = part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * (size_t)BA * BB +
-                  (size_t)row_t * BB + quarter * HC;
-#pragma unroll
-    for (int q = 0; q < HC; ++q) out[q] = (double)acc_hi[q] + (double)acc_lo[q];
 }
-
 
 // Poll limit of the warp-specialised Gram's pipeline waits (the drain waits
 // keep kT5SpinLimit): cacg_set_pipeline_wait_limit shortens it so a test can
@@ -738,39 +777,53 @@ static int launch_tc5m(cudaStream_t st, const T5Plan &p, int64_t n, const float 
     if (ldl % 4 || ldr1 % 4 || (kb2 > 0 && (ldr2 % 4 || kb1 % 8)) || !aligned16(L) ||
         !aligned16(R1) || (kb2 > 0 && !aligned16(R2)) || kb1map > kb1 || kb1map <= 0)
         return CACG_ERR_UNSUPPORTED;
-    const CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_128B;
+    const CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_64B;
     const CUtensorMapL2promotion pr = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
     CUtensorMap tmL, tmR1, tmR2;
-    if (!tma_encode_2d(&tmL, L, (uint64_t)ka, (uint64_t)n, (uint64_t)ldl * 4, kT5mBox, kT5mBox,
+    if (!tma_encode_2d(&tmL, L, (uint64_t)ka, (uint64_t)n, (uint64_t)ldl * 4, kT5mBox, kT5mRows,
                        sw, pr) ||
         !tma_encode_2d(&tmR1, R1, (uint64_t)kb1map, (uint64_t)n, (uint64_t)ldr1 * 4, kT5mBox,
-                       kT5mBox, sw, pr))
+                       kT5mRows, sw, pr))
         return CACG_ERR_UNSUPPORTED;
     if (kb2 > 0) {
         if (!tma_encode_2d(&tmR2, R2, (uint64_t)kb2, (uint64_t)n, (uint64_t)ldr2 * 4, kT5mBox,
-                           kT5mBox, sw, pr))
+                           kT5mRows, sw, pr))
             return CACG_ERR_UNSUPPORTED;
     } else {
         tmR2 = tmR1;  // never loaded
     }
-    const size_t buf = 3 * ((size_t)kT5M * kT5KT * 2 + (size_t)p.BB * kT5KT * 2);
-    const size_t ring_off = (kT5wNB * buf + 1023) / 1024 * 1024;
-    const int nbox_max = (p.BA + kT5mBox - 1) / kT5mBox + (p.BB + kT5mBox - 1) / kT5mBox + 1;
-    int stages = 4;
-    size_t smem = 0;
-    for (; stages >= 2; --stages) {
-        smem = ring_off + (size_t)stages * nbox_max * kT5mBoxBytes +
-               (2 * stages + 2 * kT5wNB + 4) * 8 + 16;
-        if (smem <= max_smem_optin()) break;
+    // the ring's stages and the slice buffers of a half of the converters: two
+    // buffers where four stages fit beside them (n = 2M, 80 x 96: 416 us with one
+    // buffer, 351 with two; three stages beside them took 447, one buffer and four
+    // 375, in an earlier form).  An odd count of stages costs a wait more a step:
+    // only where four do not fit.
+    const size_t buf = (size_t)3 * (p.BA + p.BB) * kT5KT * 2;
+    auto boxes = [](int cols) { return (std::max(cols, 0) + kT5mBox - 1) / kT5mBox; };
+    int nbox_max = 0;
+    for (int b0 = 0; b0 < kb1 + kb2; b0 += p.BB)
+        nbox_max = std::max(nbox_max, boxes(p.BA) + boxes(std::min(b0 + p.BB, kb1) - b0) +
+                                          boxes(std::min(b0 + p.BB, kb1 + kb2) - std::max(b0, kb1)));
+    auto smem_of = [&](int nb, int stg) {
+        return (2 * nb * buf + 1023) / 1024 * 1024 + (size_t)stg * nbox_max * kT5mBoxBytes +
+               (2 * stg + 10) * 8 + 16;
+    };
+    int nbuf = 2, stages = 8;
+    while (stages > 4 && smem_of(nbuf, stages) > max_smem_optin()) stages -= 2;
+    if (smem_of(nbuf, stages) > max_smem_optin()) {
+        nbuf = 1;
+        stages = 8;
+        while (stages > 4 && smem_of(nbuf, stages) > max_smem_optin()) stages -= 2;
+        while (stages >= 2 && smem_of(nbuf, stages) > max_smem_optin()) --stages;
+        if (stages < 2) return CACG_ERR_UNSUPPORTED;
     }
-    if (stages < 2) return CACG_ERR_UNSUPPORTED;
+    const size_t smem = smem_of(nbuf, stages);
     dim3 grid(p.nchunks, p.tilesA * p.tilesB);
 #define T5M_CASE(NC)                                                                               \
     case NC:                                                                                       \
         t5m_set_attr<NC>();                                                                        \
-        gram_tc5m_kernel<NC><<<grid, kT5wThreads, smem, st>>>(tmL, tmR1, tmR2, n, p.rows_per_chunk, \
+        gram_tc5m_kernel<NC><<<grid, t5w_threads(NC), smem, st>>>(tmL, tmR1, tmR2, n, p.rows_per_chunk, \
                                                              ka, kb1, kb2, p.BA, p.tilesB,         \
-                                                             p.tmem_half, stages, ws, status,      \
+                                                             p.tmem_half, stages, nbuf, ws, status,\
                                                              g_pipe_polls.load());                 \
         break;
     switch (p.BB / 16) {

@@ -96,6 +96,20 @@ __device__ __forceinline__ bool t5_mbar_try(uint64_t *bar, unsigned parity) {
     return ok != 0;
 }
 
+// one lane of a converged warp (the same one each time): code of a whole warp
+// with only the asynchronous issue under it keeps its operands in uniform registers
+__device__ __forceinline__ bool t5_elect() {
+    unsigned ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok));
+    return ok != 0;
+}
+
 // bounded wait; false on expiry
 __device__ __forceinline__ bool t5_mbar_wait(uint64_t *bar, unsigned parity) {
     for (long long i = 0; i < kT5SpinLimit; ++i)
@@ -114,6 +128,17 @@ __device__ __forceinline__ bool t5_mbar_wait_or_abort(uint64_t *bar, unsigned pa
         if ((i & 63) == 63 && *abort) return false;
     }
     return false;
+}
+
+// both barriers' phases; the two first tries are in flight together (a try costs a
+// warp among 28 some 250 cycles, even of a phase long complete)
+__device__ __forceinline__ bool t5_mbar_wait2_or_abort(uint64_t *a, unsigned pa, uint64_t *b,
+                                                       unsigned pb, const volatile int *abort,
+                                                       long long limit) {
+    bool wa = t5_mbar_try(a, pa), wb = t5_mbar_try(b, pb);
+    if (!wa) wa = t5_mbar_wait_or_abort(a, pa, abort, limit);
+    if (wa && !wb) wb = t5_mbar_wait_or_abort(b, pb, abort, limit);
+    return wa && wb;
 }
 
 __device__ __forceinline__ void t5_ld8(unsigned taddr, float (&v)[8]) {
