@@ -340,11 +340,11 @@ __global__ void __launch_bounds__(kT5Threads, 1)
 //   loader warp: waits empty[q], issues step j's TMA boxes into ring stage
 //     q = j % stages, completing on full[q];
 //   converter warps, in two halves, one for the first and one for the second
-//     step of every group: wait for full[q] and for a free slice buffer of
-//     their half (sfree, or gdone for the second half), split the step's units,
-//     fence the stores to the async proxy and arrive on sfull and empty[q];
+//     step of every group: wait for full[q] and for slice buffer j % nbuf (efree
+//     or gdone), split the step's units, fence the stores to the async proxy and
+//     arrive on sfull and empty[q];
 //   MMA warp: waits sfull (and gfree before a group reuses a TMEM buffer),
-//     issues the 12 MMAs, commits to sfree and, at a group's end, to gdone;
+//     issues the 12 MMAs, commits to efree or, at a group's end, to gdone;
 //   16 sum warps: wait gdone, add the group's FP32 sum from TMEM to their
 //     float-float registers and arrive on gfree.
 // Every wait is bounded and also ends when another role has set the abort
@@ -402,14 +402,14 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
     const int nbr2 = r2end > r2beg ? (r2end - r2beg + kT5mBox - 1) / kT5mBox : 0;
     const int c2 = r2beg - kb1;  // first R2 column of this tile's boxes
     const int nbox = nbl + nbr1 + nbr2;
-    const unsigned ring_off = (2 * nbuf * buf_bytes + 1023) / 1024 * 1024;
+    const unsigned ring_off = (nbuf * buf_bytes + 1023) / 1024 * 1024;
     unsigned char *ring = smem_raw + ring_off;
     const unsigned stage_bytes = (unsigned)nbox * kT5mBoxBytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + (size_t)stages * stage_bytes);
     uint64_t *empty = full + stages;
     uint64_t *sfull = empty + stages;
-    uint64_t *sfree = sfull + 4;  // sfull: [half][nbuf], sfree: [nbuf] of the first half
-    uint64_t *gdone = sfree + 2;
+    uint64_t *efree = sfull + 4;
+    uint64_t *gdone = efree + 2;
     uint64_t *gfree = gdone + 2;
     unsigned *tmem_slot = reinterpret_cast<unsigned *>(gfree + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -418,13 +418,12 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
     const int64_t rend = min(n, rbeg + rows_per_chunk);
     const int nsteps = rend > rbeg ? (int)((rend - rbeg + kT5KT - 1) / kT5KT) : 0;
     const int ngroups = (nsteps + 1) / 2;
-    const int nsh = nbuf - 1;  // 1 or 2 slice buffers a half
     const bool even = (stages & 1) == 0;  // a stage always takes the same half's step
 
     // octets of the B tile past the operands' columns: zeros no conversion writes
     const int na = BA / 8, n1 = b0 < kb1 ? (r1end - b0 + 7) / 8 : 0;
     const int nb = n1 + min(2 * nbr2, BB / 8 - n1);
-    for (int i = tid; i < 2 * nbuf * 3 * 4 * (BB / 8 - nb) * 8; i += kThreads) {
+    for (int i = tid; i < nbuf * 3 * 4 * (BB / 8 - nb) * 8; i += kThreads) {
         const int c = i % 8, r = i / 8, o = nb + r % (BB / 8 - nb), t = r / (BB / 8 - nb);
         *reinterpret_cast<uint4 *>(smem_raw + (t / 12) * buf_bytes + 3 * a_bytes + (t / 4 % 3) * b_bytes +
                                    (t % 4) * lbo_b + o * 128 + c * 16) = make_uint4(0, 0, 0, 0);
@@ -436,7 +435,7 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
         }
         for (int b = 0; b < 4; ++b) t5_mbar_init(&sfull[b], kTeam);
         for (int b = 0; b < 2; ++b) {
-            t5_mbar_init(&sfree[b], 1);
+            t5_mbar_init(&efree[b], 1);
             t5_mbar_init(&gdone[b], 1);
             t5_mbar_init(&gfree[b], kT5wSumWarps);
         }
@@ -545,19 +544,19 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
         };
         const int mysteps = (nsteps + 1 - h) / 2;
         bool ok = true;
-        int q = h % stages;  // this warp's next ring stage and its phase
+        int x = h % nbuf;    // this warp's next slice buffer
+        int q = h % stages;  // its next ring stage and the stage's phase
         unsigned qph = 0;
         for (int g = 0; g < ngroups; ++g) {
-            const int x = h * nbuf + (g & nsh);  // this half's slice buffer of the group
             if (g < mysteps) {
-                // the buffer's last MMAs: group gp's, whose second step gdone covers
-                const int gp = g - nbuf;
+                // step t's MMAs read the buffer last; a first step's completion is
+                // efree of its group, a second step's gdone
+                const int t = 2 * g + h - nbuf;
                 const bool w =
-                    gp < 0 ? t5_mbar_wait_or_abort(&full[q], qph, abort_flag, pipe_polls)
-                           : t5_mbar_wait2_or_abort(
-                                 &full[q], qph, h == 0 ? &sfree[g & nsh] : &gdone[gp & 1],
-                                 (unsigned)((h == 0 ? gp >> nsh : gp >> 1) & 1), abort_flag,
-                                 pipe_polls);
+                    t < 0 ? t5_mbar_wait_or_abort(&full[q], qph, abort_flag, pipe_polls)
+                          : t5_mbar_wait2_or_abort(&full[q], qph,
+                                                   (t & 1 ? gdone : efree) + ((t >> 1) & 1),
+                                                   (unsigned)((t >> 2) & 1), abort_flag, pipe_polls);
                 if (!__all_sync(0xffffffffu, w)) {
                     ok = false;
                     break;
@@ -602,6 +601,8 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
                     if (lane == 0) t5_mbar_arrive(&empty[oq]);
                 }
             }
+            x += 2;
+            if (x >= nbuf) x -= nbuf;
             q += 2;
             if (q >= stages) {
                 q -= stages;
@@ -642,14 +643,14 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
         // ---------------------------------------------------- MMA issuer
         const unsigned idesc = t5_idesc(kT5M, BB) | (1u << 15) | (1u << 16);  // A, B MN-major
         const unsigned sbase = t5_smem_u32(smem_raw);
-        int last = -1;
+        int last = -1, x = 0;  // x, xph: the step's slice buffer and its use's phase
+        unsigned xph = 0;
         for (int j = 0; j < nsteps; ++j) {
-            const int b = j & 1, g = j >> 1, x = b * nbuf + (g & nsh);
-            const unsigned sph = (unsigned)((g >> nsh) & 1);
+            const int b = j & 1, g = j >> 1;
             const bool w =
                 b == 1 || g < 2
-                    ? t5_mbar_wait_or_abort(&sfull[x], sph, abort_flag, pipe_polls)
-                    : t5_mbar_wait2_or_abort(&sfull[x], sph, &gfree[g & 1],
+                    ? t5_mbar_wait_or_abort(&sfull[x], xph, abort_flag, pipe_polls)
+                    : t5_mbar_wait2_or_abort(&sfull[x], xph, &gfree[g & 1],
                                              (unsigned)(((g >> 1) - 1) & 1), abort_flag, pipe_polls);
             if (!__all_sync(0xffffffffu, w)) {
                 if (lane == 0) fail();
@@ -670,20 +671,22 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
                                bd0 + (uint64_t)((pb[pr] * b_bytes + 2 * kk * lbo_b) >> 4), idesc,
                                pr + kk > 0 ? 1u : (unsigned)b);
                 }
-                if (b == 0) t5_commit(&sfree[x]);
+                if (b == 0) t5_commit(&efree[g & 1]);
                 if (b == 1 || j == nsteps - 1) t5_commit(&gdone[g & 1]);
             }
             __syncwarp();
             last = j;
+            if (++x == nbuf) {
+                x = 0;
+                xph ^= 1u;
+            }
         }
         // every committed MMA finishes before TMEM goes (bounded), whether or
         // not another role gave up after this loop ended
         if (last >= 0) {
             const int g = last >> 1;
-            if ((last & 1) || last == nsteps - 1)
-                t5_mbar_wait(&gdone[g & 1], (unsigned)((g >> 1) & 1));
-            else
-                t5_mbar_wait(&sfree[g & nsh], (unsigned)((g >> nsh) & 1));
+            t5_mbar_wait((last & 1) || last == nsteps - 1 ? &gdone[g & 1] : &efree[g & 1],
+                         (unsigned)((g >> 1) & 1));
         }
     }
     t5_fence_before();
@@ -792,11 +795,9 @@ static int launch_tc5m(cudaStream_t st, const T5Plan &p, int64_t n, const float 
     } else {
         tmR2 = tmR1;  // never loaded
     }
-    // the ring's stages and the slice buffers of a half of the converters: two
-    // buffers where four stages fit beside them (n = 2M, 80 x 96: 416 us with one
-    // buffer, 351 with two; three stages beside them took 447, one buffer and four
-    // 375, in an earlier form).  An odd count of stages costs a wait more a step:
-    // only where four do not fit.
+    // as many slice buffers (2 to 4) as leave room for a ring of four stages
+    // (n = 2M, 96 x 96 and 96 x 112: 426 us a product with two, 360 with three).
+    // An odd count of stages costs a wait more a step: only where four do not fit.
     const size_t buf = (size_t)3 * (p.BA + p.BB) * kT5KT * 2;
     auto boxes = [](int cols) { return (std::max(cols, 0) + kT5mBox - 1) / kT5mBox; };
     int nbox_max = 0;
@@ -804,18 +805,14 @@ static int launch_tc5m(cudaStream_t st, const T5Plan &p, int64_t n, const float 
         nbox_max = std::max(nbox_max, boxes(p.BA) + boxes(std::min(b0 + p.BB, kb1) - b0) +
                                           boxes(std::min(b0 + p.BB, kb1 + kb2) - std::max(b0, kb1)));
     auto smem_of = [&](int nb, int stg) {
-        return (2 * nb * buf + 1023) / 1024 * 1024 + (size_t)stg * nbox_max * kT5mBoxBytes +
+        return (nb * buf + 1023) / 1024 * 1024 + (size_t)stg * nbox_max * kT5mBoxBytes +
                (2 * stg + 10) * 8 + 16;
     };
-    int nbuf = 2, stages = 8;
+    int nbuf = 4, stages = 8;
+    while (nbuf > 2 && smem_of(nbuf, 4) > max_smem_optin()) --nbuf;
     while (stages > 4 && smem_of(nbuf, stages) > max_smem_optin()) stages -= 2;
-    if (smem_of(nbuf, stages) > max_smem_optin()) {
-        nbuf = 1;
-        stages = 8;
-        while (stages > 4 && smem_of(nbuf, stages) > max_smem_optin()) stages -= 2;
-        while (stages >= 2 && smem_of(nbuf, stages) > max_smem_optin()) --stages;
-        if (stages < 2) return CACG_ERR_UNSUPPORTED;
-    }
+    while (stages >= 2 && smem_of(nbuf, stages) > max_smem_optin()) --stages;
+    if (stages < 2) return CACG_ERR_UNSUPPORTED;
     const size_t smem = smem_of(nbuf, stages);
     dim3 grid(p.nchunks, p.tilesA * p.tilesB);
 #define T5M_CASE(NC)                                                                               \
