@@ -27,12 +27,22 @@
 // other DIA kernels and the CSR kernels do, so the results are bit-identical
 // to theirs.
 //
+// Values.  Large matrices whose off-diagonal nonzeros have one value (the view of
+// k_dia_fix.cu) read a presence word and the main diagonal per row, a block ahead
+// like Z2, instead of the DIA values: 8 bytes a row for 108 at 27 points, and no
+// value reads from shared memory, which were a third of its accesses.  A warp whose
+// rows all have every neighbour multiplies by the constant; the others pick c or 0 by
+// bit.  The products and their order are the same.  At 27 points, n = 2M: 174 us a
+// step, 157 with the view, 150 with the FMAs packed in pairs; the bound left is the
+// latency of two blocks of five warps an SM (DRAM 40 %).
+//
 // Items (sb consecutive blocks of one 16-column tile) go round-robin to the
 // CTAs, so at any time the CTAs work on neighbouring rows, and an X row that
 // the three bands read (N^2 rows apart) is an L2 hit after its first read.
 // The waits on the TMA barriers are bounded: on expiry the CTA sets
 // kStatusTimeout, waits (bounded) for the loads it has in flight and returns.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "cacg_internal.cuh"
@@ -54,6 +64,11 @@ constexpr int kRingBandMax = 4;
 constexpr int kRingMirror = 8;  // rows of slot 0 repeated after a ring's end
 constexpr int kRingItemsPerCta = 8;
 constexpr int kRingSmemMax = 227 * 1024;
+// DIA values (diagonals x n) from which the one-value view is read instead: at 27
+// points n = 2M a step takes 150 us instead of 174, n = 262144 29.9 instead of 31.5;
+// n = 50653 14.9 instead of 13.6, and 5 points n = 9409 16.0 instead of 14.7 (six
+// more loads before an item's first block)
+constexpr double kRingOneValMin = 5e6;
 
 struct RingDesc {
     int nb;                        // bands
@@ -99,16 +114,41 @@ __device__ __forceinline__ void ring_issue(unsigned char *sm, const RingDesc &rd
                 tma_load_2d(sm + rd.soff[b] + rd.cap[b] * kRingRowBytes, tmm, col0, y, bar);
         }
     }
-    tma_load_2d(vdst, tmv, (int)(R0 + (int64_t)t * kRingBR), 0, bar);
+    if (rd.vtx) tma_load_2d(vdst, tmv, (int)(R0 + (int64_t)t * kRingBR), 0, bar);
+}
+
+// Where the values of a row come from: the staged DIA values, or the one-value
+// view (c wherever the row has an off-diagonal, its presence bits, and the main
+// diagonal): kRingFull when no row of the warp misses one.
+enum { kRingVals, kRingFull, kRingBits };
+struct RingRow {
+    float c;                // the off-diagonal value
+    int dmain;              // index of the main diagonal
+    uint32_t bits[kRingR];  // per row: bit d set where diagonal d holds c
+    float diag[kRingR];
+};
+
+// (a0, a1) += v (x0, x1): two FMAs as one packed instruction
+__device__ __forceinline__ void ring_fma2(float v, float x0, float x1, float &a0, float &a1) {
+    asm("{\n"
+        ".reg .b64 v, x, a;\n"
+        "mov.b64 v, {%2, %2};\n"
+        "mov.b64 x, {%3, %4};\n"
+        "mov.b64 a, {%0, %1};\n"
+        "fma.rn.f32x2 a, v, x, a;\n"
+        "mov.b64 {%0, %1}, a;\n"
+        "}\n"
+        : "+f"(a0), "+f"(a1)
+        : "f"(v), "f"(x0), "f"(x1));
 }
 
 // One group of G adjacent diagonals: the window of R + G - 1 staged rows
 // starting at ring row q < cap (the mirror rows continue the ring past cap),
-// G x R values from vp (stride BR per diagonal), FMAs into acc in diagonal
-// order.
-template <int G>
-__device__ __forceinline__ void ring_group(const unsigned char *ring, int q, const float *vp,
-                                           float4 (&acc)[kRingR]) {
+// G x R values (kRingVals: from vp, stride BR per diagonal; else of diagonals
+// d0 .. of rr), FMAs into acc in diagonal order.
+template <int G, int MODE>
+__device__ __forceinline__ void ring_group(const unsigned char *ring, int q, const float *vp, int d0,
+                                           const RingRow &rr, float4 (&acc)[kRingR]) {
     constexpr int W = kRingR + G - 1;
     static_assert(W - 1 <= kRingMirror, "window longer than the mirror");
     float4 win[W];
@@ -119,13 +159,20 @@ __device__ __forceinline__ void ring_group(const unsigned char *ring, int q, con
     for (int j = 0; j < G; ++j) {
         float v[kRingR];
 #pragma unroll
-        for (int i = 0; i < kRingR; ++i) v[i] = vp[j * kRingBR + i];
+        for (int i = 0; i < kRingR; ++i) {
+            if constexpr (MODE == kRingVals)
+                v[i] = vp[j * kRingBR + i];
+            else if (d0 + j == rr.dmain)
+                v[i] = rr.diag[i];
+            else if constexpr (MODE == kRingFull)
+                v[i] = rr.c;
+            else
+                v[i] = (rr.bits[i] >> (d0 + j)) & 1u ? rr.c : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < kRingR; ++i) {
-            acc[i].x = fmaf(v[i], win[i + j].x, acc[i].x);
-            acc[i].y = fmaf(v[i], win[i + j].y, acc[i].y);
-            acc[i].z = fmaf(v[i], win[i + j].z, acc[i].z);
-            acc[i].w = fmaf(v[i], win[i + j].w, acc[i].w);
+            ring_fma2(v[i], win[i + j].x, win[i + j].y, acc[i].x, acc[i].y);
+            ring_fma2(v[i], win[i + j].z, win[i + j].w, acc[i].z, acc[i].w);
         }
     }
 }
@@ -133,14 +180,15 @@ __device__ __forceinline__ void ring_group(const unsigned char *ring, int q, con
 // NB > 0: NB bands of GPB groups of G diagonals each (the 27-point stencil's
 // 3 x 3 x 3), loops unrolled so the window loads of later groups can be
 // issued ahead of earlier groups' FMAs; NB = 0: any layout, read from rd.
-template <int NB, int GPB, int G>
+template <int NB, int GPB, int G, bool ONEVAL>
 __global__ void __launch_bounds__(kRingThreads + 32, 2)
     dia_ring_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmm,
                     const __grid_constant__ CUtensorMap tmv,
                     int64_t n, int64_t nitems, const DiaDesc desc, const __grid_constant__ RingDesc rd,
                     float *__restrict__ Y, int64_t ldy, const float *__restrict__ Z1, int64_t ldz1,
                     const float *__restrict__ Z2, int64_t ldz2, float ca, float cb, float cc,
-                    int *__restrict__ status) {
+                    const uint32_t *__restrict__ bits, const float *__restrict__ diag, float cval,
+                    int dmain, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char ring_smem[];
     // full[2]: block u's loads landed (TMA); done[2]: all 128 compute threads
     // finished block u (its ring slots and value buffer may be refilled)
@@ -231,9 +279,24 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2)
                              : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         load_z2(0, z2v);
+        // the one-value view's rows too
+        RingRow rr, rn;
+        rr.c = rn.c = cval;
+        rr.dmain = rn.dmain = NB > 0 ? NB * GPB * G / 2 : dmain;
+        auto load_row = [&](int tt, RingRow &dst) {
+            const int64_t rb = R0 + (int64_t)tt * kRingBR + rowoff;
+#pragma unroll
+            for (int i = 0; i < kRingR; ++i) {
+                const bool in = tt < nbk && rb + i < n;
+                dst.bits[i] = in ? bits[rb + i] : 0u;
+                dst.diag[i] = in ? diag[rb + i] : 0.f;
+            }
+        };
+        if constexpr (ONEVAL) load_row(0, rr);
         for (int t = 0; t < nbk; ++t, ++u) {
             const int64_t rbase = R0 + (int64_t)t * kRingBR + rowoff;
             load_z2(t + 1, z2n);
+            if constexpr (ONEVAL) load_row(t + 1, rn);
             // Z1 from global memory (when the ring does not hold it) goes out
             // before the barrier wait
             const bool z1g = Z1 && rd.z1band < 0;
@@ -260,39 +323,57 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2)
 #pragma unroll
             for (int i = 0; i < kRingR; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             int zq = -1;  // ring row of the thread's first row in the Z1 band
+            auto sums = [&](auto mode) {
+                constexpr int MODE = decltype(mode)::value;
 #pragma unroll
-            for (int b = 0; b < (NB > 0 ? NB : kRingBandMax); ++b) {
-                if (NB > 0 || b < rd.nb) {
-                    const unsigned char *ring = ring_smem + rd.soff[b] + c * 16;
-                    const int cap = rd.cap[b];
-                    const int qb = base[b] + rowoff;
-                    if (b == rd.z1band) {
-                        zq = qb + rd.z1rel;
-                        if (zq >= cap) zq -= cap;
-                    }
-                    if constexpr (NB > 0) {
-#pragma unroll
-                        for (int gg = 0; gg < GPB; ++gg) {
-                            const int g = b * GPB + gg;
-                            int q = qb + rd.grel[g];
-                            if (q >= cap) q -= cap;
-                            ring_group<G>(ring, q, vb + (rd.gdg[g] & 0xFF) * kRingBR, acc);
+                for (int b = 0; b < (NB > 0 ? NB : kRingBandMax); ++b) {
+                    if (NB > 0 || b < rd.nb) {
+                        const unsigned char *ring = ring_smem + rd.soff[b] + c * 16;
+                        const int cap = rd.cap[b];
+                        const int qb = base[b] + rowoff;
+                        if (b == rd.z1band) {
+                            zq = qb + rd.z1rel;
+                            if (zq >= cap) zq -= cap;
                         }
-                    } else {
-                        for (int g = rd.gfirst[b]; g < rd.gfirst[b + 1]; ++g) {
-                            int q = qb + rd.grel[g];
-                            if (q >= cap) q -= cap;
-                            const int dg = rd.gdg[g];
-                            const float *vp = vb + (dg & 0xFF) * kRingBR;
-                            switch (dg >> 8) {
-                                case 1: ring_group<1>(ring, q, vp, acc); break;
-                                case 2: ring_group<2>(ring, q, vp, acc); break;
-                                case 3: ring_group<3>(ring, q, vp, acc); break;
-                                default: ring_group<4>(ring, q, vp, acc); break;
+                        if constexpr (NB > 0) {
+#pragma unroll
+                            for (int gg = 0; gg < GPB; ++gg) {
+                                const int g = b * GPB + gg;
+                                int q = qb + rd.grel[g];
+                                if (q >= cap) q -= cap;
+                                ring_group<G, MODE>(ring, q, vb + (rd.gdg[g] & 0xFF) * kRingBR, g * G,
+                                                    rr, acc);
+                            }
+                        } else {
+                            for (int g = rd.gfirst[b]; g < rd.gfirst[b + 1]; ++g) {
+                                int q = qb + rd.grel[g];
+                                if (q >= cap) q -= cap;
+                                const int dg = rd.gdg[g];
+                                const float *vp = vb + (dg & 0xFF) * kRingBR;
+                                switch (dg >> 8) {
+                                    case 1: ring_group<1, MODE>(ring, q, vp, dg & 0xFF, rr, acc); break;
+                                    case 2: ring_group<2, MODE>(ring, q, vp, dg & 0xFF, rr, acc); break;
+                                    case 3: ring_group<3, MODE>(ring, q, vp, dg & 0xFF, rr, acc); break;
+                                    default: ring_group<4, MODE>(ring, q, vp, dg & 0xFF, rr, acc); break;
+                                }
                             }
                         }
                     }
                 }
+            };
+            if constexpr (ONEVAL) {
+                constexpr uint32_t dbit = NB > 0 ? 1u << (NB * GPB * G / 2) : 0u;
+                const uint32_t all = (desc.ndiag < 32 ? (1u << desc.ndiag) - 1u : ~0u) &
+                                     ~(NB > 0 ? dbit : 1u << dmain);
+                bool full = true;
+#pragma unroll
+                for (int i = 0; i < kRingR; ++i) full = full && rr.bits[i] == all;
+                if (__all_sync(0xffffffffu, full))
+                    sums(std::integral_constant<int, kRingFull>());
+                else
+                    sums(std::integral_constant<int, kRingBits>());
+            } else {
+                sums(std::integral_constant<int, kRingVals>());
             }
             float *yp = Y + rbase * ldy + col;
 #pragma unroll
@@ -335,13 +416,14 @@ __global__ void __launch_bounds__(kRingThreads + 32, 2)
             t5_mbar_arrive(&done[u & 1]);
 #pragma unroll
             for (int i = 0; i < kRingR; ++i) z2v[i] = z2n[i];
+            if constexpr (ONEVAL) rr = rn;
         }
     }
 }
 
 // Bands, rings and shared-memory layout for the matrix's diagonals; false
 // when they do not fit.
-bool ring_plan(const DiaDesc &D, RingDesc *rd, size_t *smem) {
+bool ring_plan(const DiaDesc &D, bool oneval, RingDesc *rd, size_t *smem) {
     std::vector<int> gfirst;
     std::vector<int64_t> lo, hi;
     for (int g = 0; g < D.ngroups; ++g) {
@@ -380,7 +462,7 @@ bool ring_plan(const DiaDesc &D, RingDesc *rd, size_t *smem) {
             rd->gdg[g] = D.gstart[g] | ((D.gstart[g + 1] - D.gstart[g]) << 8);
         }
     rd->voff = (int)off;
-    rd->vtx = D.ndiag * kRingBR * 4;
+    rd->vtx = oneval ? 0 : D.ndiag * kRingBR * 4;
     rd->vbytes = (rd->vtx + 127) / 128 * 128;
     off += 2 * (size_t)rd->vbytes;
     rd->boff = (int)off;
@@ -389,14 +471,14 @@ bool ring_plan(const DiaDesc &D, RingDesc *rd, size_t *smem) {
     return off <= (size_t)kRingSmemMax;
 }
 
-template <int NB, int GPB, int G>
-int ring_launch(cudaStream_t st, const CUtensorMap &tmx, const CUtensorMap &tmm,
+template <int NB, int GPB, int G, bool ONEVAL>
+int ring_launch(cudaStream_t st, const DevMatrix *A, const CUtensorMap &tmx, const CUtensorMap &tmm,
                 const CUtensorMap &tmv, int64_t n, const DiaDesc &desc, RingDesc &rd, size_t smem,
                 float *Y, int64_t ldy, const float *Z1, int64_t ldz1, const float *Z2, int64_t ldz2,
                 float ca, float cb, float cc, int *status) {
-    set_smem_attr(dia_ring_kernel<NB, GPB, G>, kRingSmemMax);
+    set_smem_attr(dia_ring_kernel<NB, GPB, G, ONEVAL>, kRingSmemMax);
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dia_ring_kernel<NB, GPB, G>,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dia_ring_kernel<NB, GPB, G, ONEVAL>,
                                                       kRingThreads + 32, smem) != cudaSuccess ||
         occ < 1) {
         cudaGetLastError();
@@ -411,8 +493,10 @@ int ring_launch(cudaStream_t st, const CUtensorMap &tmx, const CUtensorMap &tmm,
     rd.sb = (int)std::max<int64_t>(2 * kmax, (nblk + want - 1) / want);
     const int64_t nitems = (nblk + rd.sb - 1) / rd.sb * rd.tiles;
     const int64_t grid = std::min<int64_t>(grid0, nitems);
-    dia_ring_kernel<NB, GPB, G><<<(unsigned)grid, kRingThreads + 32, smem, st>>>(
-        tmx, tmm, tmv, n, nitems, desc, rd, Y, ldy, Z1, ldz1, Z2, ldz2, ca, cb, cc, status);
+    dia_ring_kernel<NB, GPB, G, ONEVAL><<<(unsigned)grid, kRingThreads + 32, smem, st>>>(
+        tmx, tmm, tmv, n, nitems, desc, rd, Y, ldy, Z1, ldz1, Z2, ldz2, ca, cb, cc, A->fix_mask,
+        ONEVAL ? A->dia32 + (size_t)A->fix_dmain * A->dia_npad : nullptr, (float)A->fix_c,
+        A->fix_dmain, status);
     return check_launch();
 }
 
@@ -434,7 +518,10 @@ int launch_dia_ring(cudaStream_t st, const DevMatrix *A, int w, const float *X, 
     if (A->dia_npad % 4 || !aligned16(A->dia32)) return CACG_ERR_UNSUPPORTED;
     RingDesc rd;
     size_t smem = 0;
-    if (!ring_plan(A->dia, &rd, &smem)) return CACG_ERR_UNSUPPORTED;
+    // constant off-diagonals: a presence word and the main diagonal per row
+    const bool oneval = A->fix_mask && A->fix_dmain >= 0 && A->dia_ndiag <= 32 &&
+                        (double)A->dia_ndiag * n >= kRingOneValMin;
+    if (!ring_plan(A->dia, oneval, &rd, &smem)) return CACG_ERR_UNSUPPORTED;
     if (!(Z1 == X && ldz1 == ldx)) rd.z1band = -1;  // Z1 read from global memory
     rd.tiles = w / kRingCols;
     CUtensorMap tmx, tmm, tmv;
@@ -450,11 +537,14 @@ int launch_dia_ring(cudaStream_t st, const DevMatrix *A, int w, const float *X, 
     bool box333 = rd.nb == 3 && A->dia.ngroups == 9;
     for (int b = 0; box333 && b < 3; ++b) box333 = rd.gfirst[b] == 3 * b;
     for (int g = 0; box333 && g < 9; ++g) box333 = (rd.gdg[g] >> 8) == 3;
-    if (box333)
-        return ring_launch<3, 3, 3>(st, tmx, tmm, tmv, n, A->dia, rd, smem, Y, ldy, Z1, ldz1, Z2,
-                                    ldz2, (float)ca, (float)cb, (float)cc, status);
-    return ring_launch<0, 0, 0>(st, tmx, tmm, tmv, n, A->dia, rd, smem, Y, ldy, Z1, ldz1, Z2,
-                                ldz2, (float)ca, (float)cb, (float)cc, status);
+#define RING_LAUNCH(NB, GPB, G, ONE)                                                              \
+    ring_launch<NB, GPB, G, ONE>(st, A, tmx, tmm, tmv, n, A->dia, rd, smem, Y, ldy, Z1, ldz1, Z2, \
+                                 ldz2, (float)ca, (float)cb, (float)cc, status)
+    if (oneval)
+        return box333 && A->fix_dmain == 13 ? RING_LAUNCH(3, 3, 3, true)
+                                            : RING_LAUNCH(0, 0, 0, true);
+    return box333 ? RING_LAUNCH(3, 3, 3, false) : RING_LAUNCH(0, 0, 0, false);
+#undef RING_LAUNCH
 }
 
 }  // namespace cacg

@@ -66,3 +66,17 @@ def test_gram_tc5_tiles(torch_cuda, n, ka, kb1, kb2):
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
     ref, bound = L.double().T @ R, L.double().abs().T @ R.abs()
     assert bool(((out[0] - ref).abs() <= 2.0 ** -14 * bound).all())
+
+
+@pytest.mark.parametrize("kind,N,shift", [("st3d27", 58, 0.1), ("st3d27", 61, 0.0),
+                                          ("lap2d", 1003, 0.05)])
+def test_staged_spmm_one_value(torch_cuda, kind, N, shift):
+    """Constant-coefficient stencils at sizes that read presence bits instead of the DIA values:
+    the unstaged kernel reads the values, with the same FMAs in the same order."""
+    rp, ci, v = cg.gen_matrix(kind, N, shift)
+    n = len(rp) - 1
+    assert {"st3d27": 27, "lap2d": 5}[kind] * n >= 5e6  # the branch's range
+    B = cg.gen_rhs("normal", n, 16, 5)
+    X = [cg.solve(rp, ci, v, B, s=3, bounds="gerschgorin", tol=1e-8, maxit=4, precision="mixed",
+                  spmm_format=f)[0] for f in ("auto", "dia_unstaged")]
+    assert np.all(np.isfinite(X[0])) and np.array_equal(X[0], X[1])
