@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     constexpr int tmem_cols = NC == 1 ? 128 : NC == 2 ? 256 : 512;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // [plane buffers x2][raw slots][scales][mbarriers][tmem slot][abort]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, and known to be
     const int nunits = (BA / 8 + NB / 8) * (kXgKT / 8);
     const int upw = (nunits + kXgConvWarps - 1) / kXgConvWarps;
     double2 *raw = reinterpret_cast<double2 *>(smem_raw + 2 * buf_bytes);
@@ -373,46 +374,51 @@ __global__ void __launch_bounds__(kXgThreads, 1)
         if (ok && nsteps > 0) ok = fold((nsteps - 1) / kXgGroup);
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         if (!ok && lane == 0) *abort_flag = 1;
-    } else if (tid == 32 * kXgConvWarps) {
-        // ---------------------------------------------------- MMA issuer
+    } else {
+        // ------------- MMA issuer: a whole warp, one elected lane at the MMAs
         int64_t last = -1;
         for (int64_t j = 0; j < nsteps; ++j) {
             const int b = (int)(j & 1);
             const int64_t g = j / kXgGroup;
-            if (!t5_mbar_wait_or_abort(&sfull[b], (unsigned)((j >> 1) & 1), abort_flag) ||
-                (j % kXgGroup == 0 && g >= 1 &&
-                 !t5_mbar_wait_or_abort(gfree, (unsigned)((g - 1) & 1), abort_flag))) {
-                *abort_flag = 1;
+            const bool w =
+                t5_mbar_wait_or_abort(&sfull[b], (unsigned)((j >> 1) & 1), abort_flag) &&
+                (j % kXgGroup != 0 || g < 1 ||
+                 t5_mbar_wait_or_abort(gfree, (unsigned)((g - 1) & 1), abort_flag));
+            if (!__all_sync(0xffffffffu, w)) {
+                if (lane == 0) *abort_flag = 1;
                 break;
             }
             t5_fence_after();
             const unsigned abase = t5_smem_u32(smem_raw + b * buf_bytes);
             const unsigned bbase = abase + kXgABytes;
             const unsigned tr = (1u << 15) | (1u << 16);  // A, B MN-major
+            if (t5_elect()) {
 #pragma unroll
-            for (int kk = 0; kk < kXgKT / 16; ++kk) {
-                const unsigned first = (j % kXgGroup == 0 && kk == 0) ? 0u : 1u;
+                for (int kk = 0; kk < kXgKT / 16; ++kk) {
+                    const unsigned first = (j % kXgGroup == 0 && kk == 0) ? 0u : 1u;
 #pragma unroll
-                for (int p = 0; p < kXPlanes; ++p) {
-                    // plane p of A times planes 0 .. 6 - p of B: accumulators p .. 6
-                    const int N = (kXPlanes - p) * NB;
-                    const uint64_t ad = t5_desc_lbo(
-                        abase + p * (kXgKT / 8) * lbo_a + 2 * kk * lbo_a, lbo_a, 128);
-                    const uint64_t bd = t5_desc_lbo(bbase + 2 * kk * lbo_b, lbo_b, 128);
-                    const unsigned dt = tmem + p * NB;
-                    const unsigned acc = p == 0 ? first : 1u;
-                    if (N <= 256) {
-                        t5_mma(dt, ad, bd, x64_idesc(kXgM, N) | tr, acc);
-                    } else {
-                        t5_mma(dt, ad, bd, x64_idesc(kXgM, 256) | tr, acc);
-                        const uint64_t bd2 =
-                            t5_desc_lbo(bbase + 2 * kk * lbo_b + (256 / 8) * 128, lbo_b, 128);
-                        t5_mma(dt + 256, ad, bd2, x64_idesc(kXgM, N > 256 ? N - 256 : 16) | tr, acc);
+                    for (int p = 0; p < kXPlanes; ++p) {
+                        // plane p of A times planes 0 .. 6 - p of B: accumulators p .. 6
+                        const int N = (kXPlanes - p) * NB;
+                        const uint64_t ad = t5_desc_lbo(
+                            abase + p * (kXgKT / 8) * lbo_a + 2 * kk * lbo_a, lbo_a, 128);
+                        const uint64_t bd = t5_desc_lbo(bbase + 2 * kk * lbo_b, lbo_b, 128);
+                        const unsigned dt = tmem + p * NB;
+                        const unsigned acc = p == 0 ? first : 1u;
+                        if (N <= 256) {
+                            t5_mma(dt, ad, bd, x64_idesc(kXgM, N) | tr, acc);
+                        } else {
+                            t5_mma(dt, ad, bd, x64_idesc(kXgM, 256) | tr, acc);
+                            const uint64_t bd2 =
+                                t5_desc_lbo(bbase + 2 * kk * lbo_b + (256 / 8) * 128, lbo_b, 128);
+                            t5_mma(dt + 256, ad, bd2, x64_idesc(kXgM, N > 256 ? N - 256 : 16) | tr, acc);
+                        }
                     }
                 }
+                t5_commit(&sfree[b]);
+                if (group_end(j)) t5_commit(gdone);
             }
-            t5_commit(&sfree[b]);
-            if (group_end(j)) t5_commit(gdone);
+            __syncwarp();
             last = j;
         }
         // every committed MMA finishes before tensor memory goes (bounded)

@@ -94,7 +94,8 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
     constexpr int kTmem = kBufs * kAcc <= 256 ? 256 : 512;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // [A planes x2][W planes][row scales x2][column keys / scales][mbarriers][tmem slot][abort]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, and known to be
     const int Kp = (g.K + 15) / 16 * 16;
     const int nchunk = (Kp + kXtKC - 1) / kXtKC;
     const unsigned sbo_b = (unsigned)(Kp / 8) * 128;
@@ -426,8 +427,8 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
             if (lane == 0) t5_mbar_arrive(&tfree[x]);
         }
         if (!ok && lane == 0) *abort_flag = 1;
-    } else if (lane == 0) {
-        // ---------------------------------------------------- MMA issuer
+    } else {
+        // ------------- MMA issuer: a whole warp, one elected lane at the MMAs
         int64_t step = 0, last = -1;
         bool ok = true;
         for (int64_t job = 0; job < njobs && ok; ++job) {
@@ -438,43 +439,48 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
             if (kBufs == 1 && job >= 1)
                 ok = t5_mbar_wait_or_abort(&tfree[x ^ 1], (unsigned)(((job - 1) >> 1) & 1),
                                            abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             for (int ch = 0; ch < nchunk; ++ch, ++step) {
                 const int b = (int)(step & 1);
-                ok = t5_mbar_wait_or_abort(&sfull[b], (unsigned)((step >> 1) & 1), abort_flag);
+                ok = __all_sync(0xffffffffu, t5_mbar_wait_or_abort(
+                                                 &sfull[b], (unsigned)((step >> 1) & 1), abort_flag));
                 if (!ok) break;
                 t5_fence_after();
                 const unsigned abase = t5_smem_u32(smem_raw + b * kXtABytes);
                 const unsigned bbase = t5_smem_u32(wpl);
                 const unsigned dset = tmem + (kBufs == 2 ? x : 0) * kAcc;
                 const int nk = min(2, Kp / 16 - 2 * ch);
-                for (int kk = 0; kk < nk; ++kk) {
-                    const unsigned first = (ch == 0 && kk == 0) ? 0u : 1u;
-                    const unsigned bk = bbase + (4 * ch + 2 * kk) * 128;
-                    // accumulators [d0, d0 + nd) of plane p with planes d0 - p ..: at
-                    // most 256 columns an MMA
-                    auto run = [&](int p, int d0, int nd, unsigned acc) {
-                        const uint64_t ad = t5_desc(abase + p * kXtPlane + kk * 256, 512);
-                        const unsigned bp = bk + (unsigned)((d0 - p) * (NB / 8)) * sbo_b;
-                        const int N = nd * NB;
-                        t5_mma(dset + d0 * NB, ad, t5_desc(bp, sbo_b),
-                               x64_idesc(kXtM, N < 256 ? N : 256), acc);
-                        if (N > 256)
-                            t5_mma(dset + d0 * NB + 256, ad, t5_desc(bp + 32 * sbo_b, sbo_b),
-                                   x64_idesc(kXtM, N - 256), acc);
-                    };
-                    run(0, 0, 7, first);
-                    run(1, 1, 6, 1u);
-                    run(1, 7, 1, first);
+                if (t5_elect()) {
+                    for (int kk = 0; kk < nk; ++kk) {
+                        const unsigned first = (ch == 0 && kk == 0) ? 0u : 1u;
+                        const unsigned bk = bbase + (4 * ch + 2 * kk) * 128;
+                        // accumulators [d0, d0 + nd) of plane p with planes d0 - p ..: at
+                        // most 256 columns an MMA
+                        auto run = [&](int p, int d0, int nd, unsigned acc) {
+                            const uint64_t ad = t5_desc(abase + p * kXtPlane + kk * 256, 512);
+                            const unsigned bp = bk + (unsigned)((d0 - p) * (NB / 8)) * sbo_b;
+                            const int N = nd * NB;
+                            t5_mma(dset + d0 * NB, ad, t5_desc(bp, sbo_b),
+                                   x64_idesc(kXtM, N < 256 ? N : 256), acc);
+                            if (N > 256)
+                                t5_mma(dset + d0 * NB + 256, ad, t5_desc(bp + 32 * sbo_b, sbo_b),
+                                       x64_idesc(kXtM, N - 256), acc);
+                        };
+                        run(0, 0, 7, first);
+                        run(1, 1, 6, 1u);
+                        run(1, 7, 1, first);
 #pragma unroll
-                    for (int p = 2; p < kXPlanes; ++p) run(p, p, kXtDiag - p, 1u);
+                        for (int p = 2; p < kXPlanes; ++p) run(p, p, kXtDiag - p, 1u);
+                    }
+                    t5_commit(&sfree[b]);
+                    if (ch + 1 == nchunk) t5_commit(&tdone[x]);
                 }
-                t5_commit(&sfree[b]);
-                if (ch + 1 == nchunk) t5_commit(&tdone[x]);
+                __syncwarp();
                 last = step;
             }
         }
-        if (!ok) *abort_flag = 1;
+        if (!ok && lane == 0) *abort_flag = 1;
         // every committed MMA finishes before tensor memory goes (bounded)
         if (last >= 0) t5_mbar_wait(&sfree[last & 1], (unsigned)((last >> 1) & 1));
     }
