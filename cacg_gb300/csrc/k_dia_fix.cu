@@ -43,16 +43,16 @@ constexpr int kFixR = 4;                       // rows per thread
 constexpr int kFixW = kFixR + kDiaGroupMax - 1;  // window rows
 constexpr int kFixMaxBlocks = 608;             // partial maxima per column
 
-// mask[row]: bit d set where diagonal d of the row holds c; *bad when an
-// off-diagonal value is neither 0 nor c
-__global__ void fix_mask_kernel(int64_t n, int64_t npad, DiaDesc desc, int dmain,
+// mask[row]: bit d set where diagonal d of the row holds c, 0 in rows [npad, nall);
+// *bad when an off-diagonal value is neither 0 nor c
+__global__ void fix_mask_kernel(int64_t npad, int64_t nall, DiaDesc desc, int dmain,
                                 const double *__restrict__ v64, double c,
                                 uint32_t *__restrict__ mask, int *__restrict__ bad) {
-    for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < npad;
+    for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < nall;
          row += (int64_t)gridDim.x * blockDim.x) {
         uint32_t m = 0u;
         bool ok = true;
-        for (int d = 0; d < desc.ndiag; ++d) {
+        for (int d = 0; row < npad && d < desc.ndiag; ++d) {
             if (d == dmain) continue;
             const double v = v64[(size_t)d * npad + row];
             if (v == c)
@@ -353,28 +353,35 @@ int DevMatrix::build_fix(const cacg_csr *A, cudaStream_t s) {
             }
     if (!found || !std::isfinite(cv) || std::fabs(cv) < 1e-200 || std::fabs(cv) > 1e200)
         return CACG_OK;
+    // a few rows on the host first: most matrices of several values end here
+    for (int t = 0; t < 64; ++t) {
+        const int64_t i = A->n / 64 * t + A->n % 64 * t / 64;
+        for (int32_t e = A->row_ptr[i]; e < A->row_ptr[i + 1]; ++e)
+            if (A->col_idx[e] != i && A->val[e] != 0.0 && A->val[e] != cv) return CACG_OK;
+    }
+    // presence words, the padding that the kernels read past npad, the flag
+    const int64_t nall = dia_npad + kFixThreads * kFixR;
     uint32_t *mk = nullptr;
-    int *bad = nullptr;
-    const size_t bytes = (size_t)(dia_npad + kFixThreads * kFixR) * 4;
+    const size_t bytes = (size_t)nall * 4 + 16;
     if (cudaMallocAsync((void **)&mk, bytes, s) != cudaSuccess) {
         cudaGetLastError();
         return CACG_OK;
     }
-    CACG_CUDA_TRY(cudaMallocAsync((void **)&bad, sizeof(int), s));
-    CACG_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int), s));
-    CACG_CUDA_TRY(cudaMemsetAsync(mk, 0, bytes, s));
+    int *bad = (int *)(mk + nall);
+    int rc = cudaMemsetAsync(bad, 0, sizeof(int), s) == cudaSuccess ? CACG_OK : CACG_ERR_CUDA;
     int dm = -1;
     for (int d = 0; d < dia_ndiag; ++d)
         if (dia.off[d] == 0) dm = d;
-    const int blocks = (int)std::min<int64_t>((dia_npad + 255) / 256, (int64_t)sm_count() * 16);
-    fix_mask_kernel<<<blocks, 256, 0, s>>>(n, dia_npad, dia, dm, dia64, cv, mk, bad);
-    int rc = check_launch();
+    const int blocks = (int)std::min<int64_t>((nall + 255) / 256, (int64_t)sm_count() * 16);
+    if (rc == CACG_OK) {
+        fix_mask_kernel<<<blocks, 256, 0, s>>>(dia_npad, nall, dia, dm, dia64, cv, mk, bad);
+        rc = check_launch();
+    }
     int hbad = 1;
     if (rc == CACG_OK && (cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s) !=
                               cudaSuccess ||
                           cudaStreamSynchronize(s) != cudaSuccess))
         rc = CACG_ERR_CUDA;
-    cudaFreeAsync(bad, s);
     if (rc != CACG_OK || hbad) {
         cudaFreeAsync(mk, s);
         return rc;
