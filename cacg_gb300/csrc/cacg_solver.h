@@ -37,7 +37,7 @@ struct DevMatrix {
     float *dia32 = nullptr;    // FP32 values (hi) ...
     float *dia32lo = nullptr;  // ... and val - hi, same allocation
     // one-value view (k_dia_fix.cu): every off-diagonal nonzero equals fix_c; a
-    // presence bit per diagonal and row (NULL: the values differ)
+    // presence bit per diagonal and row, behind dia64's values (NULL: the values differ)
     uint32_t *fix_mask = nullptr;
     double fix_c = 0;
     int fix_dmain = -1;  // index of the main diagonal
@@ -107,6 +107,7 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
                    int64_t ldz2, double ca, double cb, double cc, void *xi, void *small,
                    FixChain *chain = nullptr);
 size_t dia_fix_scratch_bytes(int64_t n, int w);
+size_t dia_fix_mask_bytes(int64_t npad);
 size_t dia_fix_small_bytes(int w);
 
 // Per-thread pinned host scratch of at least `bytes` (reused across calls).

@@ -163,11 +163,12 @@ int DevMatrix::build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st) {
     }
     desc.gstart[desc.ngroups] = nd;
     const int64_t npad = (n + kDiaR - 1) / kDiaR * kDiaR + kDiaR;
-    const size_t b64 = (size_t)nd * npad * 8, b32 = want_f32 ? (size_t)2 * nd * npad * 4 : 0;
+    // the one-value view's words lie behind the FP64 values
+    const size_t b64 = (size_t)nd * npad * 8, bfix = dia_fix_mask_bytes(npad), b32 = want_f32 ? (size_t)2 * nd * npad * 4 : 0;
     double *v64 = nullptr;
     float *v32 = nullptr;
     int *bad = nullptr;
-    if (cudaMallocAsync((void **)&v64, b64, st) != cudaSuccess) {
+    if (cudaMallocAsync((void **)&v64, b64 + bfix, st) != cudaSuccess) {
         cudaGetLastError();
         return CACG_OK;  // no room for the view: CSR only
     }
@@ -201,7 +202,7 @@ int DevMatrix::build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st) {
     dia32 = v32;
     dia32lo = v32 ? v32 + (size_t)nd * npad : nullptr;
     dia_ndiag = nd;
-    owned_bytes += b64 + b32;
+    owned_bytes += b64 + bfix + b32;
     return CACG_OK;
 }
 

@@ -361,12 +361,7 @@ int DevMatrix::build_fix(const cacg_csr *A, cudaStream_t s) {
     }
     // presence words, the padding that the kernels read past npad, the flag
     const int64_t nall = dia_npad + kFixThreads * kFixR;
-    uint32_t *mk = nullptr;
-    const size_t bytes = (size_t)nall * 4 + 16;
-    if (cudaMallocAsync((void **)&mk, bytes, s) != cudaSuccess) {
-        cudaGetLastError();
-        return CACG_OK;
-    }
+    uint32_t *mk = reinterpret_cast<uint32_t *>(dia64 + (size_t)dia_ndiag * dia_npad);
     int *bad = (int *)(mk + nall);
     int rc = cudaMemsetAsync(bad, 0, sizeof(int), s) == cudaSuccess ? CACG_OK : CACG_ERR_CUDA;
     int dm = -1;
@@ -382,20 +377,19 @@ int DevMatrix::build_fix(const cacg_csr *A, cudaStream_t s) {
                               cudaSuccess ||
                           cudaStreamSynchronize(s) != cudaSuccess))
         rc = CACG_ERR_CUDA;
-    if (rc != CACG_OK || hbad) {
-        cudaFreeAsync(mk, s);
-        return rc;
-    }
+    if (rc != CACG_OK || hbad) return rc;
     fix_mask = mk;
     fix_c = cv;
     fix_dmain = dm;
-    owned_bytes += bytes;
     return CACG_OK;
 }
 
 size_t dia_fix_scratch_bytes(int64_t n, int w) {
     const size_t wp = (size_t)(w + 1) / 2 * 2;
     return (size_t)n * wp * 8;
+}
+size_t dia_fix_mask_bytes(int64_t npad) {
+    return (size_t)(npad + kFixThreads * kFixR) * 4 + 16;
 }
 size_t dia_fix_small_bytes(int w) { return ((size_t)2 * kFixMaxBlocks * w + w + 1) * 4; }
 

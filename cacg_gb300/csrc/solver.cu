@@ -147,7 +147,6 @@ void DevMatrix::release() {
     if (val32) cudaFreeAsync(val32, st);
     if (dia64) cudaFreeAsync(dia64, st);
     if (dia32) cudaFreeAsync(dia32, st);
-    if (fix_mask) cudaFreeAsync(fix_mask, st);
     fix_mask = nullptr;
     rp = nullptr;
     ci = nullptr;
