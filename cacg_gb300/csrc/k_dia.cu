@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kDiaThreads, R <= 4 ? 3 : 2)
                     const T *__restrict__ Z2, int64_t ldz2, T ca, T cb, T cc) {
     constexpr int W = R + kDiaGroupMax - 1;  // register window rows
     constexpr int VN = 16 / (int)sizeof(T);
-    constexpr bool kZ2Early = R <= 4;  // registers for it
+    constexpr bool kZ2Early = CW == 1 && R <= 4;  // vectors of four rows would spill
     extern __shared__ __align__(16) unsigned char dia_smem[];
     T *vs = reinterpret_cast<T *>(dia_smem);  // [2][ndiag][BR] when R > 1
     const int lr = threadIdx.x / cpr, c = threadIdx.x % cpr;

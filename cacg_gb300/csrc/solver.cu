@@ -19,7 +19,8 @@
 // and beta (next iteration).
 //
 // Precision modes:
-//   CACG_FP64   all FP64 (parity mode with the reference).
+//   CACG_FP64   all FP64 (parity mode with the reference); over a DIA view large
+//               products run from digit planes and fixed point (planes64()).
 //   CACG_MIXED  A, S, Q, AQ in FP32 (SpMM and basis in FP32); Gram products
 //               and Q = S - Q beta on the tcgen05 tensor cores (bf16x3 slices,
 //               FP32 accumulation, Gram group sums in float-float, split-K in

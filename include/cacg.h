@@ -50,7 +50,8 @@ extern "C" {
 #define CACG_TOL_ABS_COL0 0 /* reference: ||R(:,0)|| < tol (src/bcbcgKernel.c:524) */
 #define CACG_TOL_REL_ALL 1  /* max_c ||b_c - A x_c|| / ||b_c|| <= tol (true residual) */
 
-#define CACG_FP64 0  /* plain FP64 everywhere */
+#define CACG_FP64 0  /* FP64 throughout: FMAs, or sums no less accurate (exact digit
+                        planes on the tensor cores, fixed point) over a DIA view */
 #define CACG_MIXED 1 /* FP32 basis/SpMM/updates, FP64 Gram accumulation, LU, X, R,
                         FP64 residual replacement */
 
