@@ -9,10 +9,10 @@
 //   G = V^T V,  R1 = chol(G) (upper),  Q1 = V R1^{-1},
 //   G2 = Q1^T Q1, R2 = chol(G2),       Q  = Q1 R2^{-1},   R = R2 R1,
 // which is orthogonal to working accuracy while the 2-norm condition number
-// of V stays below about u^{-1/2} (1e8); the Gram products are the split-K
-// FP64 Gram of k_gram.cu (symmetric: upper triangle computed), the small
-// Cholesky factors and triangular inverses run in one CTA, the tall x small
-// products stream V once.  A Cholesky pivot that is not positive and finite
+// of V stays below about u^{-1/2} (1e8); the Gram products and the tall x small
+// ones are the library's FP64 kernels (digit planes on the tensor cores, FMAs at
+// the sizes those do not take), the small Cholesky factors and triangular
+// inverses run in one CTA.  A Cholesky pivot that is not positive and finite
 // (V numerically rank-deficient) returns CACG_ERR_BREAKDOWN.
 #include "cacg_internal.cuh"
 
@@ -20,52 +20,67 @@ namespace cacg {
 
 constexpr int kQrMaxK = 128;
 constexpr int kQrThreads = 256;
+constexpr int kCholThreads = 512;
 
-// One CTA: R = chol(G) (upper, G = R^T R) in shared memory, Rinv = R^{-1};
-// both k x k row-major with zeros below the diagonal.  *bad set on a pivot
-// that is not positive and finite.
-__global__ void __launch_bounds__(kQrThreads)
+// One CTA: R = chol(G) (upper, G = R^T R) and Rinv = R^{-1}, both k x k
+// row-major with zeros below the diagonal.  *bad set on a pivot that is not
+// positive and finite.
+//
+// G = L D L^T by right-looking elimination with the same row operations applied
+// to the identity, whose rows (L^{-1}) take the space below the diagonal: R =
+// D^{1/2} L^T, R^{-1} = (L^{-1})^T D^{-1/2}.  On this part an FP64 division takes
+// 340 clocks and each FP64 instruction its quadrant's pipe for 64, so a step has
+// one division (in a warp a quadrant, for the multipliers), no square root (all of
+// them at the end) and one FMA an element.  The form before, a square root and a
+// division a step and then one thread a column of the inverse with a dependent FMA
+// an element, took 155 us at k = 48 and 683 at 96; this 66 and
+// 260 (the FP64 pipe of one SM, half of it lanes outside the triangles).
+__global__ void __launch_bounds__(kCholThreads)
     chol_inv_kernel(int k, const double *__restrict__ G, double *__restrict__ R,
                     double *__restrict__ Rinv, int *__restrict__ bad) {
     extern __shared__ __align__(16) double qr_sm[];
     double *A = qr_sm;  // k x k
-    const int tid = threadIdx.x, kk = k * k;
-    for (int i = tid; i < kk; i += blockDim.x) A[i] = G[i];
+    __shared__ double t[kQrMaxK], sq[kQrMaxK], rs[kQrMaxK];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kk = k * k;
+    for (int i = tid; i < kk; i += kCholThreads) A[i] = G[i];
     __syncthreads();
     for (int j = 0; j < k; ++j) {
-        // row j of R: A[j][j] = sqrt(pivot), A[j][l] /= it (l > j)
-        const double piv = A[j * k + j];
-        const bool ok = piv > 0.0 && isfinite(piv);
-        const double d = ok ? sqrt(piv) : 0.0;
-        __syncthreads();
-        if (tid == 0) {
-            A[j * k + j] = d;
-            if (!ok) *bad = 1;
+        const double *aj = A + (size_t)j * k;
+        if (tid < kQrMaxK && (warp << 5) < k - j) {
+            const double piv = aj[j];
+            // positive and finite, on the bits (an FP64 comparison is 64 clocks of the chain)
+            const uint32_t hi = (uint32_t)__double2hiint(piv);
+            const bool ok = hi < 0x7ff00000u && (hi | (uint32_t)__double2loint(piv)) != 0u;
+            const int l = j + tid;  // l = j: the pivot itself
+            if (l > j && l < k) t[l] = ok ? aj[l] / piv : 0.0;
+            if (tid == 0) {
+                sq[j] = ok ? piv : 0.0;
+                if (!ok) *bad = 1;
+            }
         }
-        for (int l = j + 1 + tid; l < k; l += blockDim.x) A[j * k + l] = ok ? A[j * k + l] / d : 0.0;
         __syncthreads();
-        // trailing upper part: A[i][l] -= R[j][i] R[j][l], j < i <= l
-        const int w = k - j - 1;
-        for (int e = tid; e < w * w; e += blockDim.x) {
-            const int i = j + 1 + e / w, l = j + 1 + e % w;
-            if (l >= i) A[i * k + l] = fma(-A[j * k + i], A[j * k + l], A[i * k + l]);
+        for (int i = j + 1 + warp; i < k; i += kCholThreads / 32) {
+            const double ti = t[i];
+            double *ai = A + (size_t)i * k;
+            for (int c = lane; c < k; c += 32) {
+                if (c < j || c >= i)
+                    ai[c] = fma(-ti, aj[c], ai[c]);
+                else if (c == j)
+                    ai[c] = -ti;
+            }
         }
         __syncthreads();
     }
-    for (int e = tid; e < kk; e += blockDim.x) {
+    for (int i = tid; i < k; i += kCholThreads) {
+        const double d = sqrt(sq[i]);
+        sq[i] = d;
+        rs[i] = 1.0 / d;
+    }
+    __syncthreads();
+    for (int e = tid; e < kk; e += kCholThreads) {
         const int i = e / k, l = e % k;
-        R[e] = l >= i ? A[e] : 0.0;
-    }
-    // R^{-1}, one column per thread: x_c = 1 / R_cc, x_i = -(sum_{l=i+1..c} R_il x_l) / R_ii
-    for (int c = tid; c < k; c += blockDim.x) {
-        for (int i = 0; i < k; ++i)
-            if (i > c) Rinv[i * k + c] = 0.0;
-        Rinv[c * k + c] = 1.0 / A[c * k + c];
-        for (int i = c - 1; i >= 0; --i) {
-            double s = 0.0;
-            for (int l = i + 1; l <= c; ++l) s = fma(A[i * k + l], Rinv[l * k + c], s);
-            Rinv[i * k + c] = -s / A[i * k + i];
-        }
+        R[e] = l > i ? A[e] * rs[i] : l == i ? sq[i] : 0.0;
+        Rinv[e] = l > i ? A[(size_t)l * k + i] * rs[l] : l == i ? rs[i] : 0.0;
     }
 }
 
@@ -89,14 +104,15 @@ __global__ void __launch_bounds__(kQrThreads)
     }
 }
 
-// R = A B for upper triangular k x k A, B (one CTA)
+// R = A B for upper triangular k x k A, B: a CTA a row, an output a thread (one
+// CTA for all rows: 26 us at k = 48, 294 at 128)
 __global__ void triu_mul_kernel(int k, const double *__restrict__ A, const double *__restrict__ B,
                                 double *__restrict__ R) {
-    for (int e = threadIdx.x; e < k * k; e += blockDim.x) {
-        const int i = e / k, c = e % k;
+    const int i = blockIdx.x;
+    for (int c = threadIdx.x; c < k; c += blockDim.x) {
         double s = 0.0;
         for (int j = i; j <= c; ++j) s = fma(A[i * k + j], B[j * k + c], s);
-        R[e] = c >= i ? s : 0.0;
+        R[i * k + c] = c >= i ? s : 0.0;
     }
 }
 
@@ -106,7 +122,7 @@ constexpr int kQrSmemMax = kQrMaxK * kQrMaxK * (int)sizeof(double);
 static int chol_inv(cudaStream_t st, int k, const double *G, double *R, double *Rinv, int *bad) {
     const int smem = (int)((size_t)k * k * sizeof(double));
     set_smem_attr(chol_inv_kernel, kQrSmemMax);
-    chol_inv_kernel<<<1, kQrThreads, smem, st>>>(k, G, R, Rinv, bad);
+    chol_inv_kernel<<<1, kCholThreads, smem, st>>>(k, G, R, Rinv, bad);
     return check_launch();
 }
 
@@ -159,7 +175,7 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R2, R2i, bad);
     if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, R2i, Q, ldq, bad);
     if (rc == CACG_OK) {
-        triu_mul_kernel<<<1, kQrThreads, 0, st>>>(k, R2, R1, R);
+        triu_mul_kernel<<<k, kQrMaxK, 0, st>>>(k, R2, R1, R);
         rc = check_launch();
     }
     int hb = 0;

@@ -216,3 +216,22 @@ def test_fixed_point_spmm_outside_range():
         assert np.array_equal(np.isfinite(info["true_relres"]), [True, False, True, True])
         # X0's other columns are zero: their residual is B, summed in another order only
         assert np.all(np.abs(info["true_relres"][[0, 2, 3]] - 1.0) <= n * 2.0 ** -53)
+
+
+@pytest.mark.parametrize("k", [1, 2, 31, 33, 64, 97, 127, 128])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -300, 2.0 ** 300])
+def test_qr_small_factor_edges(torch_cuda, k, scale):
+    """The one-CTA Cholesky factor and inverse at the edges of its 32-lane columns and 16 warps of
+    rows.  A well-conditioned block (cond < 3): each product and the factor are backward stable
+    with k u of the norms, u = 2^-53; 100 k u covers the two passes."""
+    torch = torch_cuda
+    n = 40 * k + 7
+    V = _block(torch, n, k, k, 0, "normal", 5) * scale
+    Q, R = torch.empty_like(V), torch.empty(k, k, dtype=torch.float64, device="cuda")
+    assert cg.lib().cacg_k_tsqr(n, k, ptr(V), k, ptr(Q), k, ptr(R), None) == 0
+    torch.cuda.synchronize()
+    u = 100 * k * 2.0 ** -53
+    eye = torch.eye(k, dtype=torch.float64, device="cuda")
+    assert float((Q.T @ Q - eye).norm()) <= u * k ** 0.5
+    assert float((Q @ (R / scale) - V / scale).norm()) <= u * float((V / scale).norm())
+    assert bool((torch.tril(R, -1) == 0).all()) and bool((torch.diagonal(R) > 0).all())
