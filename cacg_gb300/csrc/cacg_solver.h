@@ -45,7 +45,6 @@ struct DevMatrix {
     cudaStream_t st = nullptr;  // stream of the stream-ordered allocations
     static int create(const cacg_csr *A, bool want_f32, DevMatrix *M, cudaStream_t st);
     int build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st);
-    int build_fix(const cacg_csr *A, cudaStream_t st);
     int ensure_f32(cudaStream_t st);
     void release();
 };
@@ -108,6 +107,9 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
                    FixChain *chain = nullptr);
 size_t dia_fix_scratch_bytes(int64_t n, int w);
 size_t dia_fix_mask_bytes(int64_t npad);
+bool dia_fix_candidate(const cacg_csr *A, double *c);
+int launch_dia_fix_mask(cudaStream_t st, int64_t npad, const DiaDesc &desc, double *v64, double c,
+                        uint32_t **mask, int *dmain, int *bad);
 size_t dia_fix_small_bytes(int w);
 
 // Per-thread pinned host scratch of at least `bytes` (reused across calls).

@@ -177,21 +177,28 @@ int DevMatrix::build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st) {
         cudaFreeAsync(v64, st);
         return CACG_OK;
     }
-    CACG_CUDA_TRY(cudaMallocAsync((void **)&bad, sizeof(int), st));
+    CACG_CUDA_TRY(cudaMallocAsync((void **)&bad, 2 * sizeof(int), st));
     CACG_CUDA_TRY(cudaMemsetAsync(v64, 0, b64, st));
     if (v32) CACG_CUDA_TRY(cudaMemsetAsync(v32, 0, b32, st));
-    CACG_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int), st));
+    CACG_CUDA_TRY(cudaMemsetAsync(bad, 0, 2 * sizeof(int), st));
     const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 16);
     dia_fill_kernel<<<blocks, 256, 0, st>>>(n, npad, rp, ci, val, desc, v64, v32, bad);
     int rc = check_launch();
-    int hbad = 1;
+    // the one-value view: its flag comes back with the fill's
+    double cv = 0.0;
+    uint32_t *mask = nullptr;
+    int dmain = -1;
+    const bool one = nd > 1 && dia_fix_candidate(A, &cv);
+    if (rc == CACG_OK && one)
+        rc = launch_dia_fix_mask(st, npad, desc, v64, cv, &mask, &dmain, bad + 1);
+    int hbad[2] = {1, 1};
     if (rc == CACG_OK) {
-        if (cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        if (cudaMemcpyAsync(hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             rc = CACG_ERR_CUDA;
     }
     cudaFreeAsync(bad, st);
-    if (rc != CACG_OK || hbad) {
+    if (rc != CACG_OK || hbad[0]) {
         cudaFreeAsync(v64, st);
         if (v32) cudaFreeAsync(v32, st);
         return rc;
@@ -203,6 +210,11 @@ int DevMatrix::build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st) {
     dia32lo = v32 ? v32 + (size_t)nd * npad : nullptr;
     dia_ndiag = nd;
     owned_bytes += b64 + bfix + b32;
+    if (one && !hbad[1]) {
+        fix_mask = mask;
+        fix_c = cv;
+        fix_dmain = dmain;
+    }
     return CACG_OK;
 }
 

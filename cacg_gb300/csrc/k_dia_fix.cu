@@ -337,11 +337,9 @@ __global__ void __launch_bounds__(kFixThreads, 3)
 
 }  // namespace
 
-// one-value view of the matrix's off-diagonals (DevMatrix::build_dia): c from
-// the host arrays, presence bits on the device; leaves fix_mask NULL when the
-// off-diagonal values differ
-int DevMatrix::build_fix(const cacg_csr *A, cudaStream_t s) {
-    if (dia_ndiag <= 1 || !dia64) return CACG_OK;
+// The one-value view is worth a look: the first off-diagonal nonzero, finite and of
+// moderate size, is every other's value in 64 rows spread over the matrix.
+bool dia_fix_candidate(const cacg_csr *A, double *c) {
     double cv = 0.0;
     bool found = false;
     for (int64_t i = 0; i < A->n && !found; ++i)
@@ -352,36 +350,28 @@ int DevMatrix::build_fix(const cacg_csr *A, cudaStream_t s) {
                 break;
             }
     if (!found || !std::isfinite(cv) || std::fabs(cv) < 1e-200 || std::fabs(cv) > 1e200)
-        return CACG_OK;
-    // a few rows on the host first: most matrices of several values end here
+        return false;
     for (int t = 0; t < 64; ++t) {
         const int64_t i = A->n / 64 * t + A->n % 64 * t / 64;
         for (int32_t e = A->row_ptr[i]; e < A->row_ptr[i + 1]; ++e)
-            if (A->col_idx[e] != i && A->val[e] != 0.0 && A->val[e] != cv) return CACG_OK;
+            if (A->col_idx[e] != i && A->val[e] != 0.0 && A->val[e] != cv) return false;
     }
-    // presence words, the padding that the kernels read past npad, the flag
-    const int64_t nall = dia_npad + kFixThreads * kFixR;
-    uint32_t *mk = reinterpret_cast<uint32_t *>(dia64 + (size_t)dia_ndiag * dia_npad);
-    int *bad = (int *)(mk + nall);
-    int rc = cudaMemsetAsync(bad, 0, sizeof(int), s) == cudaSuccess ? CACG_OK : CACG_ERR_CUDA;
-    int dm = -1;
-    for (int d = 0; d < dia_ndiag; ++d)
-        if (dia.off[d] == 0) dm = d;
+    *c = cv;
+    return true;
+}
+
+// presence words behind v64's values, and the padding the kernels read past npad;
+// *bad (0 before) set when an off-diagonal value is neither 0 nor c
+int launch_dia_fix_mask(cudaStream_t st, int64_t npad, const DiaDesc &desc, double *v64, double c,
+                        uint32_t **mask, int *dmain, int *bad) {
+    const int64_t nall = npad + kFixThreads * kFixR;
+    *mask = reinterpret_cast<uint32_t *>(v64 + (size_t)desc.ndiag * npad);
+    *dmain = -1;
+    for (int d = 0; d < desc.ndiag; ++d)
+        if (desc.off[d] == 0) *dmain = d;
     const int blocks = (int)std::min<int64_t>((nall + 255) / 256, (int64_t)sm_count() * 16);
-    if (rc == CACG_OK) {
-        fix_mask_kernel<<<blocks, 256, 0, s>>>(dia_npad, nall, dia, dm, dia64, cv, mk, bad);
-        rc = check_launch();
-    }
-    int hbad = 1;
-    if (rc == CACG_OK && (cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s) !=
-                              cudaSuccess ||
-                          cudaStreamSynchronize(s) != cudaSuccess))
-        rc = CACG_ERR_CUDA;
-    if (rc != CACG_OK || hbad) return rc;
-    fix_mask = mk;
-    fix_c = cv;
-    fix_dmain = dm;
-    return CACG_OK;
+    fix_mask_kernel<<<blocks, 256, 0, st>>>(npad, nall, desc, *dmain, v64, c, *mask, bad);
+    return check_launch();
 }
 
 size_t dia_fix_scratch_bytes(int64_t n, int w) {

@@ -120,8 +120,7 @@ int DevMatrix::create(const cacg_csr *A, bool want_f32, DevMatrix *M, cudaStream
         int rc = launch_cast_f64_f32(st, A->nnz, M->val, M->val32);
         if (rc) return rc;
     }
-    const int rc = M->build_dia(A, want_f32, st);
-    return rc != CACG_OK ? rc : M->build_fix(A, st);
+    return M->build_dia(A, want_f32, st);
 }
 
 int DevMatrix::ensure_f32(cudaStream_t st) {
