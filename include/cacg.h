@@ -295,7 +295,7 @@ int cacg_k_xrupdate(int32_t vtype, int64_t n, int32_t k, int32_t m, const void *
  * with a positive diagonal; k <= 128, n >= k.  The reference's TSQR
  * (src/TSQR.c) is empty and its Householder QR (src/MatrixDecomposition.c:3-93)
  * unfinished, so this has no reference behaviour to match: CholeskyQR2 on the
- * split-K FP64 Gram, orthogonal to working accuracy for cond(V) < ~1e8;
+ * FP64 Gram, orthogonal to working accuracy for cond(V) < ~1e8;
  * CACG_ERR_BREAKDOWN when V is numerically rank-deficient. */
 int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, double *Q, int64_t ldq,
                 double *R, void *stream);
