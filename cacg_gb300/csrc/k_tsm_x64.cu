@@ -374,7 +374,9 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
                     const long long l = (long long)(D[4] * 16777216ll) +
                                         ((long long)D[5] * 65536 + (long long)D[6] * 256 + D[7]);
                     const int sc = E + (int)colK[cc + q] - (2154 - 40);
-                    v[q] = x64_scaled(x64_join(h, l), (h | l) == 0, sc);
+                    const double t = x64_join(h, l);
+                    // h 2^32 and l may cancel: the sum is what is zero (and 1 or more if not)
+                    v[q] = x64_scaled(t, __double2hiint(t) == 0, sc);
                 }
                 if (E < 0 && rv) {  // no scale for this row: FP64 FMAs
                     const double *a = (part ? g.A1 : g.A0) + row * g.lda;
