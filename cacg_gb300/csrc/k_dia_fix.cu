@@ -14,8 +14,13 @@
 // (a bit per diagonal) is exact, and the FP64 pipe is left with one conversion
 // and two FMAs per output:
 //     Y = ca c S + (ca D [+ cb]) X + cb Z1 + cc Z2      (cb folded in if Z1 is X)
-// Each x is rounded at 2^-58 of its column's largest element, once; the FMA
-// chain rounds at 2^-53 of every partial sum.
+// Each x is rounded at 2^-58 of its column's largest element M, once; the FMA chain
+// rounds at 2^-53 of every partial sum.  For spread columns that is the smaller
+// error: per row the roundings of d neighbours leave 2^-59.8 sqrt(d) M |c|, the FMAs'
+// (random signs) about 2^-54.3 sqrt(d (d + 1) / 2) rms(x) |c|, which is more while
+// M < 45 rms (5 and 7 points; 84 at 27).  So a column needs an eighth of its elements
+// at M / 16 or above (then M <= 45 rms; normal data has 62 %, a solver's basis more):
+// where one has not, a point source say, the product takes FP64 FMAs.
 //
 // Measured at 27 points, n = 262144, w = 16 (75 us a step): FP64 pipe 62 % busy,
 // the rest the latency of the window reads; four rows a thread and three CTAs an
@@ -25,10 +30,14 @@
 //
 // Three launches: column maxima (partials per block; left out in a chain of
 // basis steps, where the step that wrote X has left them), conversion (which
-// first reduces them), and the product.  A column that no scale holds (Inf, NaN, or a
-// largest magnitude beyond 2^+-400) sends the product to FP64 FMAs over the DIA values.
+// first reduces them, and counts the large elements), and the product.  A column with
+// Inf or NaN, or whose results could leave FP64's normal numbers by the exponent
+// additions, sends the product to the FMAs too: over the DIA values, with the same
+// windows, at the FP64 pipe's rate.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
+#include <type_traits>
 
 #include "cacg_internal.cuh"
 #include "cacg_solver.h"
@@ -69,9 +78,12 @@ __global__ void fix_mask_kernel(int64_t npad, int64_t nall, DiaDesc desc, int dm
 template <bool VEC>
 __global__ void __launch_bounds__(kFixThreads)
     fix_colmax_kernel(int64_t n, int w, const double *__restrict__ X, int64_t ldx,
-                      uint32_t *__restrict__ part) {
+                      uint32_t *__restrict__ part, uint32_t *__restrict__ large) {
     extern __shared__ uint32_t fix_mx[];
-    for (int i = threadIdx.x; i < w; i += blockDim.x) fix_mx[i] = 0u;
+    for (int i = threadIdx.x; i < w; i += blockDim.x) {
+        fix_mx[i] = 0u;
+        if (blockIdx.x == 0) large[i] = 0u;  // the conversion's counters
+    }
     __syncthreads();
     const int tpr = VEC ? w / 2 : w;
     const int rpb = blockDim.x / tpr;
@@ -107,15 +119,31 @@ __device__ __forceinline__ long long fix_from(double x, int E) {
     return (int32_t)xh < 0 ? -a : a;
 }
 
+// a column's scale: as x64_scale_mid's, within 2^+-range
+__device__ __forceinline__ int fix_scale(uint32_t key, int range, bool *bad) {
+    const int e = (int)(key >> 20);
+    if (key != 0u && (e < 1023 - range || e > 1023 + range)) *bad = true;
+    return key == 0u ? 1023 : e;
+}
+
+// an element of M / 16 or above (M: the power of two above its column's largest),
+// and every one of a zero column
+__device__ __forceinline__ uint32_t fix_large(double x, int E, int within) {
+    return E - (int)(((uint32_t)__double2hiint(x) >> 20) & 0x7ffu) <= within ? 1u : 0u;
+}
+
 // xi (n x wp, wp = w rounded up to even, the padding column zero); scale[0 .. w):
-// the columns' exponents, scale[w]: raised when a column has none
+// the columns' exponents, scale[w]: raised when a column has none; large[0 .. w):
+// counts of large elements, added up over the blocks
 template <bool VEC>
 __global__ void __launch_bounds__(kFixThreads)
     fix_convert_kernel(int64_t n, int w, int wp, const double *__restrict__ X, int64_t ldx,
-                       const uint32_t *__restrict__ part, int nparts, long long *__restrict__ xi,
-                       int *__restrict__ scale) {
+                       const uint32_t *__restrict__ part, int nparts, int range,
+                       long long *__restrict__ xi, int *__restrict__ scale,
+                       uint32_t *__restrict__ large) {
     extern __shared__ uint32_t fix_mx[];
-    for (int i = threadIdx.x; i < wp; i += blockDim.x) fix_mx[i] = 0u;
+    uint32_t *cnt = fix_mx + wp;
+    for (int i = threadIdx.x; i < 2 * wp; i += blockDim.x) fix_mx[i] = 0u;
     __syncthreads();
     // stripes of the partials: one atomic per thread and column group
     const int ns = max(1, (int)blockDim.x / w);
@@ -130,8 +158,10 @@ __global__ void __launch_bounds__(kFixThreads)
     __syncthreads();
     bool bad = false;
     for (int i = threadIdx.x; i < wp; i += blockDim.x) {
-        const int e = x64_scale_mid(fix_mx[i], &bad);
+        const uint32_t key = fix_mx[i];
+        const int e = fix_scale(key, range, &bad);
         fix_mx[i] = (uint32_t)e;
+        cnt[i] = key == 0u ? 0x80000000u : 0u;  // the top bit: a zero column
         if (blockIdx.x == 0 && i < w) scale[i] = e;
     }
     const int any = __syncthreads_or(bad);
@@ -140,10 +170,13 @@ __global__ void __launch_bounds__(kFixThreads)
     const int tpr = wp / 2;
     const int rpb = blockDim.x / tpr;
     const int r = threadIdx.x / tpr, c = (threadIdx.x % tpr) * 2;
-    if (r >= rpb) return;
-    const int e0 = (int)fix_mx[c], e1 = (int)fix_mx[c + 1];
+    const bool on = r < rpb;
+    const int e0 = on ? (int)fix_mx[c] : 0, e1 = on ? (int)fix_mx[c + 1] : 0;
+    const int in0 = on && cnt[c] ? INT32_MAX : 3, in1 = on && cnt[c + 1] ? INT32_MAX : 3;
+    uint32_t n0 = 0u, n1 = 0u;
 #pragma unroll 4
-    for (int64_t row = (int64_t)blockIdx.x * rpb + r; row < n; row += (int64_t)gridDim.x * rpb) {
+    for (int64_t row = (int64_t)blockIdx.x * rpb + r; on && row < n;
+         row += (int64_t)gridDim.x * rpb) {
         double2 v = make_double2(0.0, 0.0);
         if constexpr (VEC) {
             v = __ldg(reinterpret_cast<const double2 *>(X + row * ldx + c));
@@ -153,7 +186,17 @@ __global__ void __launch_bounds__(kFixThreads)
         }
         *reinterpret_cast<longlong2 *>(xi + row * wp + c) =
             make_longlong2(fix_from(v.x, e0), fix_from(v.y, e1));
+        n0 += fix_large(v.x, e0, in0);
+        n1 += fix_large(v.y, e1, in1);
     }
+    __syncthreads();  // every thread has seen the zero columns' bits
+    if (on) {
+        atomicAdd(&cnt[c], n0);
+        atomicAdd(&cnt[c + 1], n1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < w; i += blockDim.x)
+        atomicAdd(&large[i], cnt[i] & 0x7fffffffu);
 }
 
 struct FixArgs {
@@ -170,7 +213,9 @@ struct FixArgs {
     double *Y;
     const long long *xi;
     const int *scale;
-    uint32_t *ymax;  // column maxima of Y, a partial per block (NULL: not wanted)
+    const uint32_t *large;
+    uint32_t *ymax;   // column maxima of Y, a partial per block (NULL: not wanted) ...
+    uint32_t *large0;  // ... and the counters of the call that takes Y, zeroed here
 };
 
 template <bool VEC>
@@ -209,107 +254,99 @@ __global__ void __launch_bounds__(kFixThreads, 3)
         for (int i = threadIdx.x; i < a.w; i += blockDim.x)
             a.ymax[(size_t)blockIdx.x * a.w + i] = fix_mx[i];
     };
-    if (a.scale[a.w]) {
-        // a column without a scale: FP64 FMAs over the diagonals
-        for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-            for (int i = 0; i < kFixR; ++i) {
-                const int64_t row = blk * BR + (int64_t)lr * kFixR + i;
-                if (row >= a.n) break;
-                for (int q = 0; q < 2 && c + q < a.w; ++q) {
-                    double s = 0.0;
-                    for (int d = 0; d < desc.ndiag; ++d) {
-                        const int64_t xr = row + desc.off[d];
-                        if (xr < 0 || xr >= a.n) continue;
-                        s = fma(a.vals[(size_t)d * a.npad + row], a.X[xr * a.ldx + c + q], s);
-                    }
-                    double y = a.ca * s;
-                    if (a.Z1) y = fma(a.cb, a.Z1[row * a.ldz1 + c + q], y);
-                    if (a.Z2) y = fma(a.cc, a.Z2[row * a.ldz2 + c + q], y);
-                    a.Y[row * a.ldy + c + q] = y;
-                    (q ? k1 : k0) = max(q ? k1 : k0, x64_key(y));
-                }
-            }
-        }
-        put_max();
-        return;
+    bool spread = a.scale[a.w] == 0;
+    for (int i = threadIdx.x; i < a.w; i += blockDim.x) {
+        spread = spread && (int64_t)a.large[i] * 8 >= a.n;
+        if (a.ymax && blockIdx.x == 0) a.large0[i] = 0u;
     }
+    const bool fixed = __syncthreads_and(spread) != 0;
     const int e0 = c < a.w ? a.scale[c] : 1023, e1 = c + 1 < a.w ? a.scale[c + 1] : 1023;
     const double cac = a.ca * a.c;
     const int flip = cac < 0.0 ? (int)0x80000000 : 0;
     // ca c on the columns' scales
     const double c0 = scalbn(cac, e0 - 1079), c1 = scalbn(cac, e1 - 1079);
     const double fca = a.ca, fcb = a.fold ? a.cb : 0.0;
-    for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-        const int64_t r0 = blk * BR + (int64_t)lr * kFixR;
-        uint32_t m[kFixR];
-        {
-            const uint4 m0 = __ldg(reinterpret_cast<const uint4 *>(a.mask + r0));
-            m[0] = m0.x, m[1] = m0.y, m[2] = m0.z, m[3] = m0.w;
-        }
-        long long acc[kFixR][2];
+    // FIXED: sums of xi over the presence bits; else FMAs of X over the DIA values
+    auto rows = [&](auto mode) {
+        constexpr bool FIXED = decltype(mode)::value;
+        using P = typename std::conditional<FIXED, longlong2, double2>::type;
+        for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+            const int64_t r0 = blk * BR + (int64_t)lr * kFixR;
+            uint32_t m[kFixR];
+            if constexpr (FIXED) {
+                const uint4 m0 = __ldg(reinterpret_cast<const uint4 *>(a.mask + r0));
+                m[0] = m0.x, m[1] = m0.y, m[2] = m0.z, m[3] = m0.w;
+            }
+            P acc[kFixR];
 #pragma unroll
-        for (int i = 0; i < kFixR; ++i) acc[i][0] = acc[i][1] = 0;
-        for (int g = 0; g < desc.ngroups; ++g) {
-            const int d0 = desc.gstart[g], G = desc.gstart[g + 1] - d0;
-            const int64_t x0 = r0 + desc.off[d0];
-            longlong2 win[kFixW];
-            if (x0 >= 0 && x0 + kFixW <= a.n) {
-                const long long *xp = a.xi + x0 * a.wp + c;
+            for (int i = 0; i < kFixR; ++i) acc[i].x = acc[i].y = 0;
+            for (int g = 0; g < desc.ngroups; ++g) {
+                const int d0 = desc.gstart[g], G = desc.gstart[g + 1] - d0;
+                const int64_t x0 = r0 + desc.off[d0];
+                P win[kFixW];
+                if constexpr (FIXED) {
+                    if (x0 >= 0 && x0 + kFixW <= a.n) {
+                        const long long *xp = a.xi + x0 * a.wp + c;
 #pragma unroll
-                for (int t = 0; t < kFixW; ++t)
-                    if (t < kFixR + G - 1)
-                        win[t] = __ldg(reinterpret_cast<const longlong2 *>(xp + (int64_t)t * a.wp));
-            } else {
+                        for (int t = 0; t < kFixW; ++t)
+                            if (t < kFixR + G - 1)
+                                win[t] =
+                                    __ldg(reinterpret_cast<const longlong2 *>(xp + (int64_t)t * a.wp));
+                    } else {
 #pragma unroll
-                for (int t = 0; t < kFixW; ++t) {
-                    if (t < kFixR + G - 1) {
-                        int64_t xr = x0 + t;
-                        xr = xr < 0 ? 0 : (xr >= a.n ? a.n - 1 : xr);  // its bit is clear
-                        win[t] = __ldg(reinterpret_cast<const longlong2 *>(a.xi + xr * a.wp + c));
+                        for (int t = 0; t < kFixW; ++t) {
+                            if (t < kFixR + G - 1) {
+                                int64_t xr = x0 + t;
+                                xr = xr < 0 ? 0 : (xr >= a.n ? a.n - 1 : xr);  // its bit is clear
+                                win[t] = __ldg(
+                                    reinterpret_cast<const longlong2 *>(a.xi + xr * a.wp + c));
+                            }
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int t = 0; t < kFixW; ++t) {
+                        if (t < kFixR + G - 1) {
+                            const int64_t xr = x0 + t;
+                            win[t] = make_double2(0.0, 0.0);
+                            if (xr >= 0 && xr < a.n) win[t] = fix_ld<VEC>(a.X + xr * a.ldx, c, a.w);
+                        }
                     }
                 }
-            }
 #pragma unroll
-            for (int j = 0; j < kDiaGroupMax; ++j) {
-                if (j < G) {
-                    const uint32_t bit = 1u << (d0 + j);
+                for (int j = 0; j < kDiaGroupMax; ++j) {
+                    if (j < G) {
+                        if constexpr (FIXED) {
+                            const uint32_t bit = 1u << (d0 + j);
 #pragma unroll
-                    for (int i = 0; i < kFixR; ++i) {
-                        if (m[i] & bit) {
-                            acc[i][0] += win[i + j].x;
-                            acc[i][1] += win[i + j].y;
+                            for (int i = 0; i < kFixR; ++i) {
+                                if (m[i] & bit) {
+                                    acc[i].x += win[i + j].x;
+                                    acc[i].y += win[i + j].y;
+                                }
+                            }
+                        } else {
+                            // (rows past n: zeros up to npad, the presence words behind it)
+                            const double *vp = a.vals + (size_t)(d0 + j) * a.npad + r0;
+#pragma unroll
+                            for (int i = 0; i < kFixR; ++i) {
+                                const double v = r0 + i < a.n ? __ldg(vp + i) : 0.0;
+                                acc[i].x = fma(v, win[i + j].x, acc[i].x);
+                                acc[i].y = fma(v, win[i + j].y, acc[i].y);
+                            }
                         }
                     }
                 }
             }
-        }
-        const double *dv = a.dmain >= 0 ? a.vals + (size_t)a.dmain * a.npad + r0 : nullptr;
+            const double *dv = a.dmain >= 0 ? a.vals + (size_t)a.dmain * a.npad + r0 : nullptr;
 #pragma unroll
-        for (int i = 0; i < kFixR; ++i) {
-            const int64_t row = r0 + i;
-            if (row >= a.n) break;
-            const double f = fma(fca, dv ? __ldg(dv + i) : 0.0, fcb);
-            const double2 x = fix_ld<VEC>(a.X + row * a.ldx, c, a.w);
-            double t0 = x64_from_ll(acc[i][0]), t1 = x64_from_ll(acc[i][1]);
-            double2 y;
-            if constexpr (MODE == kFixPow2) {
-                // the scale, ca c and its sign go into the exponent field
-                t0 = x64_scaled(t0, acc[i][0] == 0, e0 - 1079 + a.c_pow2);
-                t1 = x64_scaled(t1, acc[i][1] == 0, e1 - 1079 + a.c_pow2);
-                t0 = __hiloint2double(__double2hiint(t0) ^ flip, __double2loint(t0));
-                t1 = __hiloint2double(__double2hiint(t1) ^ flip, __double2loint(t1));
-                y = make_double2(fma(f, x.x, t0), fma(f, x.y, t1));
-            } else {
-                if constexpr (MODE == kFixStep) {
-                    const double2 z = fix_ld<VEC>(a.Z2 + row * a.ldz2, c, a.w);
-                    y = make_double2(fma(f, x.x, -z.x), fma(f, x.y, -z.y));
-                } else {
-                    y = make_double2(f * x.x, f * x.y);
-                }
-                y.x = fma(t0, c0, y.x);
-                y.y = fma(t1, c1, y.y);
-                if constexpr (MODE == kFixAny) {
-                    if (a.Z1 && !a.fold) {
+            for (int i = 0; i < kFixR; ++i) {
+                const int64_t row = r0 + i;
+                if (row >= a.n) break;
+                double2 y;
+                if constexpr (!FIXED) {
+                    y = make_double2(a.ca * acc[i].x, a.ca * acc[i].y);
+                    if (a.Z1) {
                         const double2 z = fix_ld<VEC>(a.Z1 + row * a.ldz1, c, a.w);
                         y.x = fma(a.cb, z.x, y.x);
                         y.y = fma(a.cb, z.y, y.y);
@@ -319,19 +356,56 @@ __global__ void __launch_bounds__(kFixThreads, 3)
                         y.x = fma(a.cc, z.x, y.x);
                         y.y = fma(a.cc, z.y, y.y);
                     }
+                } else {
+                    const double f = fma(fca, dv ? __ldg(dv + i) : 0.0, fcb);
+                    const double2 x = fix_ld<VEC>(a.X + row * a.ldx, c, a.w);
+                    double t0 = x64_from_ll(acc[i].x), t1 = x64_from_ll(acc[i].y);
+                    if constexpr (MODE == kFixPow2) {
+                        // the scale, ca c and its sign go into the exponent field
+                        t0 = x64_scaled(t0, acc[i].x == 0, e0 - 1079 + a.c_pow2);
+                        t1 = x64_scaled(t1, acc[i].y == 0, e1 - 1079 + a.c_pow2);
+                        t0 = __hiloint2double(__double2hiint(t0) ^ flip, __double2loint(t0));
+                        t1 = __hiloint2double(__double2hiint(t1) ^ flip, __double2loint(t1));
+                        y = make_double2(fma(f, x.x, t0), fma(f, x.y, t1));
+                    } else {
+                        if constexpr (MODE == kFixStep) {
+                            const double2 z = fix_ld<VEC>(a.Z2 + row * a.ldz2, c, a.w);
+                            y = make_double2(fma(f, x.x, -z.x), fma(f, x.y, -z.y));
+                        } else {
+                            y = make_double2(f * x.x, f * x.y);
+                        }
+                        y.x = fma(t0, c0, y.x);
+                        y.y = fma(t1, c1, y.y);
+                        if constexpr (MODE == kFixAny) {
+                            if (a.Z1 && !a.fold) {
+                                const double2 z = fix_ld<VEC>(a.Z1 + row * a.ldz1, c, a.w);
+                                y.x = fma(a.cb, z.x, y.x);
+                                y.y = fma(a.cb, z.y, y.y);
+                            }
+                            if (a.Z2) {
+                                const double2 z = fix_ld<VEC>(a.Z2 + row * a.ldz2, c, a.w);
+                                y.x = fma(a.cc, z.x, y.x);
+                                y.y = fma(a.cc, z.y, y.y);
+                            }
+                        }
+                    }
+                }
+                k0 = max(k0, x64_key(y.x));
+                k1 = max(k1, x64_key(y.y));
+                double *yp = a.Y + row * a.ldy + c;
+                if constexpr (VEC) {
+                    *reinterpret_cast<double2 *>(yp) = y;
+                } else {
+                    yp[0] = y.x;
+                    if (c + 1 < a.w) yp[1] = y.y;
                 }
             }
-            k0 = max(k0, x64_key(y.x));
-            k1 = max(k1, x64_key(y.y));
-            double *yp = a.Y + row * a.ldy + c;
-            if constexpr (VEC) {
-                *reinterpret_cast<double2 *>(yp) = y;
-            } else {
-                yp[0] = y.x;
-                if (c + 1 < a.w) yp[1] = y.y;
-            }
         }
-    }
+    };
+    if (fixed)
+        rows(std::true_type());
+    else
+        rows(std::false_type());
     put_max();
 }
 
@@ -381,7 +455,7 @@ size_t dia_fix_scratch_bytes(int64_t n, int w) {
 size_t dia_fix_mask_bytes(int64_t npad) {
     return (size_t)(npad + kFixThreads * kFixR) * 4 + 16;
 }
-size_t dia_fix_small_bytes(int w) { return ((size_t)2 * kFixMaxBlocks * w + w + 1) * 4; }
+size_t dia_fix_small_bytes(int w) { return ((size_t)2 * kFixMaxBlocks * w + 3 * w + 1) * 4; }
 
 int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, int64_t ldx,
                    double *Y, int64_t ldy, const double *Z1, int64_t ldz1, const double *Z2,
@@ -404,7 +478,10 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
     a.ca = ca, a.cb = cb, a.cc = cc;
     int ex = 0;
     const double fr = std::frexp(std::fabs(cac), &ex);  // 0.5 for a power of two
+    // results by exponent additions or by a scaled ca c: normal numbers for columns
+    // within 2^+-range
     const bool pow2 = fr == 0.5 && ex > -300 && ex < 300;
+    const int range = ex > -100 && ex < 100 ? 800 : 400;
     a.c_pow2 = pow2 ? ex - 1 : 0;
     a.fold = Z1 && Z1 == X && ldz1 == ldx;
     a.X = X, a.Z1 = Z1, a.Z2 = Z2, a.Y = Y;
@@ -412,7 +489,10 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
     a.xi = (const long long *)xi;
     uint32_t *parts = (uint32_t *)small;  // two sets: of X, and of Y for the next step
     int *scale = (int *)(parts + (size_t)2 * kFixMaxBlocks * w);
+    uint32_t *larges = (uint32_t *)scale + w + 1;  // two sets as well
     const bool known = chain && chain->of == X && chain->w == w;
+    uint32_t *large = larges + (size_t)(known ? chain->set : 0) * w;
+    a.large = large;
     uint32_t *part = parts + (size_t)(known ? chain->set : 0) * kFixMaxBlocks * w;
     a.scale = scale;
     const bool xvec = w % 2 == 0 && ldx % 2 == 0 && aligned16(X);
@@ -425,25 +505,25 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
     int g1 = (int)std::max<int64_t>(
         1, std::min<int64_t>(std::min<int64_t>(kFixMaxBlocks, 4 * (int64_t)sm_count()),
                              (A->n + 4 * rpb - 1) / (4 * rpb)));
-    const size_t sm = (size_t)(w + 2) * 4;
+    const size_t sm = (size_t)2 * (w + 2) * 4;
     int rc = CACG_OK;
     if (known)
         g1 = chain->nparts;  // the step that wrote X left its maxima
     else if (xvec)
-        fix_colmax_kernel<true><<<g1, kFixThreads, sm, st>>>(A->n, w, X, ldx, part);
+        fix_colmax_kernel<true><<<g1, kFixThreads, sm, st>>>(A->n, w, X, ldx, part, large);
     else
-        fix_colmax_kernel<false><<<g1, kFixThreads, sm, st>>>(A->n, w, X, ldx, part);
+        fix_colmax_kernel<false><<<g1, kFixThreads, sm, st>>>(A->n, w, X, ldx, part, large);
     if (!known) rc = check_launch();
     if (rc != CACG_OK) return rc;
     const int rpc = kFixThreads / a.cpr;
     const int g2 = (int)std::max<int64_t>(
         1, std::min<int64_t>((int64_t)sm_count() * 6, (A->n + 4 * rpc - 1) / (4 * rpc)));
     if (xvec)
-        fix_convert_kernel<true><<<g2, kFixThreads, sm, st>>>(A->n, w, a.wp, X, ldx, part, g1,
-                                                              (long long *)xi, scale);
+        fix_convert_kernel<true><<<g2, kFixThreads, sm, st>>>(A->n, w, a.wp, X, ldx, part, g1, range,
+                                                              (long long *)xi, scale, large);
     else
-        fix_convert_kernel<false><<<g2, kFixThreads, sm, st>>>(A->n, w, a.wp, X, ldx, part, g1,
-                                                               (long long *)xi, scale);
+        fix_convert_kernel<false><<<g2, kFixThreads, sm, st>>>(A->n, w, a.wp, X, ldx, part, g1, range,
+                                                               (long long *)xi, scale, large);
     rc = check_launch();
     if (rc != CACG_OK) return rc;
     const int64_t nblk = (A->n + (int64_t)a.runs * kFixR - 1) / ((int64_t)a.runs * kFixR);
@@ -451,6 +531,7 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
     if (chain) {
         const int set = known ? chain->set ^ 1 : 1;
         a.ymax = parts + (size_t)set * kFixMaxBlocks * w;
+        a.large0 = larges + (size_t)set * w;
         *chain = FixChain{Y, w, set, (int)blocks};
     }
     const int mode = !Z2 && (!Z1 || a.fold) ? (pow2 ? kFixPow2 : kFixNone)

@@ -32,3 +32,32 @@ def test_products_that_cancel_exactly(torch_cuda, M, top):
     assert np.array_equal(R[:2, :2], [[32.0, 32.0 * M], [0.0, 16.0]])
     assert np.array_equal(Q[:, 1], d / 16.0)
     assert np.array_equal(Q[:, 0], np.full(1024, 2.0 ** -5))
+
+
+@pytest.mark.parametrize("kind,N,m", [("lap2d", 600, 8), ("st3d27", 40, 8), ("lap3d7", 60, 9)])
+def test_fixed_point_spmm_point_values(kind, N, m):
+    """B - A X where one element of a column is far above the others (its neighbours zero, so
+    that their rows of A X are exact): the others' rows keep the accuracy of FMAs, 35 u of
+    27 |c| max|x| of a row; the root of the sum over n rows."""
+    rp, ci, v = cg.gen_matrix(kind, N, 0.0625)
+    n = len(rp) - 1
+    assert len(v) * m >= 1e7
+    rng = np.random.default_rng(3)
+    X = np.clip(rng.standard_normal((n, m)), -5.5, 5.5)
+    mid = n // 2 + N // 2
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    near = np.zeros(n, bool)
+    near[mid] = True
+    for _ in range(2):  # two rings
+        near[ci[near[rows]]] = True
+    X[:, 2] *= 2.0 ** -50
+    X[near, 2] = 0.0
+    X[mid, 2] = 1.0
+    AX = np.stack([np.add.reduceat(v.astype(np.longdouble) * X[ci, c], rp[:-1])
+                   for c in range(m)], 1)
+    B = AX.astype(np.float64)
+    hit = ci[rp[mid]:rp[mid + 1]]
+    assert np.array_equal(AX[hit, 2], B[hit, 2])
+    _, info = cg.solve(rp, ci, v, B, X0=X, s=4, bounds=("given", 0.05, 60.0), tol=1e-8, maxit=0)
+    got = info["true_relres"][2] * np.linalg.norm(B[:, 2])
+    assert got <= 35 * 2.0 ** -53 * 2 * 27 * 5.5 * 2.0 ** -50 * n ** 0.5
