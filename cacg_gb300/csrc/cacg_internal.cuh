@@ -201,27 +201,38 @@ template <typename T>
 int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl, int ka,
                 const T *R1, int64_t ldr1, int kb1, const T *R2, int64_t ldr2, int kb2,
                 double *C1, int ldc1, double *C2, int ldc2, double *ws, size_t ws_bytes,
-                bool symmetric = false);
+                bool symmetric = false, struct ColExps *ce = nullptr);
 size_t gram_workspace_bytes(int64_t n, int ka, int kb);
 // FP64 Gram from fp16 digit planes on tcgen05 (k_gram_x64.cu); launch_gram takes
 // it for CACG_GRAM_AUTO.  CACG_ERR_UNSUPPORTED: shape or workspace not for it.
 int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
                     const double *R1, int64_t ldr1, int kb1, const double *R2, int64_t ldr2,
                     int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
-                    size_t ws_bytes);
+                    size_t ws_bytes, struct ColExps *ce = nullptr);
 size_t gram_x64_workspace_bytes(int64_t n, int ka, int kb);
+// Exponents of the columns of a Gram's L (ka) and R1 (kb1), about their norms', for
+// the tall x small products of the same blocks (device arrays; set: written).  The
+// digit-plane Gram has them from its scales; launch_col_exps takes a pass over A0
+// and, if given, A1 (n x k) for them.
+struct ColExps {
+    int *L = nullptr, *R1 = nullptr;
+    bool set = false;
+};
+int launch_col_exps(cudaStream_t st, int64_t n, int k, const double *A0, const double *A1,
+                    int64_t lda, double *ws, size_t ws_bytes, int *e0, int *e1);
 // FP64 tall x small products from digit planes (k_tsm_x64.cu), k <= 144:
 // Qout = S - Qin beta (Qout may be S); X += Q alpha, R -= AQ alpha, S0 = R,
-// norms; Y = A W.  *status gets kStatusTimeout if a bounded wait expires;
-// CACG_ERR_UNSUPPORTED for other shapes.
+// norms; Y = A W.  qexp ..: the tall operands' column exponents.  *status gets
+// kStatusTimeout if a bounded wait expires; CACG_ERR_UNSUPPORTED for other shapes.
 int launch_qupdate_x64(cudaStream_t st, int64_t n, int k, double *Qout, int64_t ldo,
-                       const double *Qin, int64_t ldq, const double *S, int64_t lds,
-                       const double *beta, int *status);
+                       const double *Qin, int64_t ldq, const int *qexp, const double *S,
+                       int64_t lds, const double *beta, int *status);
 int launch_xrupdate_x64(cudaStream_t st, int64_t n, int k, int m, const double *Q,
-                        const double *AQ, int64_t ldq, const double *alpha, double *X, double *R,
-                        double *S0, int64_t lds, double *norms, double *ws, int *status);
+                        const double *AQ, int64_t ldq, const int *qexp, const int *aqexp,
+                        const double *alpha, double *X, double *R, double *S0, int64_t lds,
+                        double *norms, double *ws, int *status);
 int launch_tallsmall_x64(cudaStream_t st, int64_t n, int K, int N, const double *A, int64_t lda,
-                         const double *W, int ldw, double *Y, int64_t ldy, int *status);
+                         const int *aexp, const double *W, int ldw, double *Y, int64_t ldy, int *status);
 
 // dst = src for an n x w FP32 block (rows of lds / ldd values)
 int launch_copy_rows_f32(cudaStream_t st, int64_t n, int w, const float *src, int64_t lds,

@@ -119,7 +119,7 @@ __device__ __forceinline__ long long fix_from(double x, int E) {
     return (int32_t)xh < 0 ? -a : a;
 }
 
-// a column's scale: as x64_scale_mid's, within 2^+-range
+// a column's scale exponent from its largest key; *bad beyond 2^+-range (Inf and NaN too)
 __device__ __forceinline__ int fix_scale(uint32_t key, int range, bool *bad) {
     const int e = (int)(key >> 20);
     if (key != 0u && (e < 1023 - range || e > 1023 + range)) *bad = true;

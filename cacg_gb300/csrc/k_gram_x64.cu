@@ -114,7 +114,7 @@ __device__ __forceinline__ void xg_cp8(void *smem, const void *g, int bytes) {
 template <int NC, bool VEC>
 __global__ void __launch_bounds__(kXgThreads, 1)
     gram_x64_kernel(int64_t n, int64_t rows_per_chunk, XgOperands o, int BA, int tilesB, int sub,
-                    int stages, const uint32_t *__restrict__ emax, double *__restrict__ part,
+                    int stages, bool scan, uint32_t *__restrict__ emax, double *__restrict__ part,
                     int *__restrict__ flags) {
     constexpr int NB = 16 * NC;
     constexpr int NQ = NB / 4;  // accumulator columns per converter thread
@@ -147,9 +147,9 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     int *flag = flags + (size_t)blockIdx.x * gridDim.y + blockIdx.y;
 
     // scales of the tile's columns: from the maxima kernel, or, where the
-    // operands stay in L2, from a pass over the chunk's rows
+    // operands stay in L2 (scan), from a pass over the chunk's rows, which leaves them
     bool bad = false;
-    if (emax) {
+    if (!scan) {
         if (tid < BA + NB) {
             const int c = tid < BA ? (a0 + tid < o.ka ? a0 + tid : -1)
                                    : (b0 + tid - BA < kb ? o.ka + b0 + tid - BA : -1);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             if (c >= 0)
                 for (int s = 0; s < sub; ++s)
                     key = max(key, emax[((size_t)blockIdx.x * sub + s) * kc + c]);
-            esc[tid] = x64_scale(key, &bad);
+            esc[tid] = x64_scale(key, &bad) << 20;
         }
     } else {
         uint32_t *keys = reinterpret_cast<uint32_t *>(esc);
@@ -198,7 +198,14 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             atomicMax(&keys[c + 1], k1);
         }
         __syncthreads();
-        if (tid < BA + NB) esc[tid] = x64_scale(keys[tid], &bad);
+        if (tid < BA + NB) {
+            const uint32_t key = keys[tid];
+            uint32_t *left = emax + (size_t)blockIdx.x * kc;
+            const int c = tid < BA ? a0 + tid : b0 + tid - BA;
+            if (tid < BA && tile_b == 0 && c < o.ka) left[c] = key;
+            if (tid >= BA && tile_a == 0 && c < kb) left[o.ka + c] = key;
+            esc[tid] = x64_scale(key, &bad) << 20;
+        }
     }
     if (__syncthreads_or(bad)) {
         if (tid == 0) *flag = 1;
@@ -348,7 +355,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
                 if (u >= upw || warp + kXgConvWarps * u >= nunits) break;
                 const double2 x = slot[(st * upw + u) * (kXgConvWarps * 32)];
                 if (more) copy_unit(st, u);  // into this thread's slot, just read
-                const int2 e = *reinterpret_cast<const int2 *>(esc + c0 + 32 * u);
+                const uint2 e = *reinterpret_cast<const uint2 *>(esc + c0 + 32 * u);
                 uint32_t w[kXPlanes];
                 x64_planes2(x.x, x.y, e.x, e.y, w);
                 if (oct0 + 4 * u < BA / 8) {
@@ -440,26 +447,35 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     if (row_t >= BA) return;
     double *out = part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * (size_t)BA * NB +
                   (size_t)row_t * NB + quarter * NQ;
-    const int ea = esc[row_t] - 2106;
+    const int ea = (esc[row_t] >> 20) - 2106;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
         const double v = fma((double)ahi[q], 16777216.0, (double)alo[q]);
-        out[q] = scalbn(v, ea + esc[BA + quarter * NQ + q]);
+        out[q] = scalbn(v, ea + (esc[BA + quarter * NQ + q] >> 20));
     }
 }
 
 // Sum of the chunks' partials: 16 threads share an output, each sums a
 // contiguous sixteenth of the chunks in order, then the sixteenths are added in
-// order.  With a raised flag the same threads form the output from L, R1, R2.
+// order.  With a raised flag the same threads form the output from L, R1, R2.  The
+// blocks from nsum on leave the exponents of L's and R1's columns (eL, eR1) instead.
 constexpr int kXrElems = 32, kXrSlices = 16;
 
 __global__ void __launch_bounds__(kXrSlices *kXrElems)
     gram_x64_reduce_kernel(const double *__restrict__ part, int nchunks, int ntiles, int BA, int NB,
                            int tilesB, int64_t n, XgOperands o, double *__restrict__ C1, int ldc1,
-                           double *__restrict__ C2, int ldc2, const int *__restrict__ flags) {
+                           double *__restrict__ C2, int ldc2, const int *__restrict__ flags,
+                           int nsum, const uint32_t *__restrict__ emax, int groups,
+                           int *__restrict__ eL, int *__restrict__ eR1) {
     __shared__ double qs[kXrSlices][kXrElems];
     const int el = threadIdx.x % kXrElems, q = threadIdx.x / kXrElems;
     const int kb = o.kb1 + o.kb2;
+    if (blockIdx.x >= nsum) {
+        const int c = (blockIdx.x - nsum) * kXrElems + el;
+        x64_col_exp(emax, groups, o.ka + kb, c, c < o.ka + (eR1 ? o.kb1 : 0), el, q,
+                    reinterpret_cast<float(*)[32]>(qs), c < o.ka ? eL + c : eR1 + (c - o.ka));
+        return;
+    }
     const int idx = blockIdx.x * kXrElems + el;
     const bool active = idx < o.ka * kb;
     const int a = active ? idx / kb : 0, b = active ? idx % kb : 0;
@@ -560,16 +576,16 @@ bool gram_x64_supported(int64_t n, int ka, int kb) {
 
 template <int NC, bool VEC>
 static void xg_launch(dim3 grid, const XgPlan &p, cudaStream_t st, int64_t n, const XgOperands &o,
-                      const uint32_t *emax, double *part, int *flags) {
+                      uint32_t *emax, double *part, int *flags) {
     set_smem_attr(gram_x64_kernel<NC, VEC>, (int)max_smem_optin());
     gram_x64_kernel<NC, VEC><<<grid, kXgThreads, p.smem, st>>>(
-        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan ? nullptr : emax, part, flags);
+        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan, emax, part, flags);
 }
 
 int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
                     const double *R1, int64_t ldr1, int kb1, const double *R2, int64_t ldr2,
                     int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
-                    size_t ws_bytes) {
+                    size_t ws_bytes, ColExps *ce) {
     const int kb = kb1 + kb2;
     if (!gram_x64_supported(n, ka, kb)) return CACG_ERR_UNSUPPORTED;
     const XgPlan p = plan_x64(n, ka, kb);
@@ -612,8 +628,41 @@ int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, in
 #undef XG_CASE
     rc = check_launch();
     if (rc != CACG_OK) return rc;
-    gram_x64_reduce_kernel<<<(ka * kb + kXrElems - 1) / kXrElems, kXrSlices * kXrElems, 0, st>>>(
-        part, p.nchunks, p.tilesA * p.tilesB, p.BA, p.NB, p.tilesB, n, o, C1, ldc1, C2, ldc2, flags);
+    const int nsum = (ka * kb + kXrElems - 1) / kXrElems;
+    const int nexp = ce ? (ka + (ce->R1 ? kb1 : 0) + kXrElems - 1) / kXrElems : 0;
+    gram_x64_reduce_kernel<<<nsum + nexp, kXrSlices * kXrElems, 0, st>>>(
+        part, p.nchunks, p.tilesA * p.tilesB, p.BA, p.NB, p.tilesB, n, o, C1, ldc1, C2, ldc2, flags,
+        nsum, emax, p.nchunks * (p.scan ? 1 : p.sub), ce ? ce->L : nullptr, ce ? ce->R1 : nullptr);
+    if (ce) ce->set = true;
+    return check_launch();
+}
+
+__global__ void __launch_bounds__(kXrSlices *kXrElems)
+    col_exps_kernel(const uint32_t *__restrict__ emax, int groups, int k, int kc,
+                    int *__restrict__ e0, int *__restrict__ e1) {
+    __shared__ float sh[kXrSlices][kXrElems];
+    const int el = threadIdx.x % kXrElems, q = threadIdx.x / kXrElems;
+    const int c = blockIdx.x * kXrElems + el;
+    x64_col_exp(emax, groups, kc, c, c < kc, el, q, sh, c < k ? e0 + c : e1 + (c - k));
+}
+
+int launch_col_exps(cudaStream_t st, int64_t n, int k, const double *A0, const double *A1,
+                    int64_t lda, double *ws, size_t ws_bytes, int *e0, int *e1) {
+    if (n <= 0 || k <= 0 || k > 256) return CACG_ERR_UNSUPPORTED;
+    const int kc = A1 ? 2 * k : k;
+    const int64_t rows = std::max<int64_t>(64, (n + 2 * sm_count() - 1) / (2 * sm_count()));
+    const int groups = (int)((n + rows - 1) / rows);
+    if (!ws || (size_t)groups * kc * 4 > ws_bytes) return CACG_ERR_UNSUPPORTED;
+    uint32_t *emax = reinterpret_cast<uint32_t *>(ws);
+    const XgOperands o{A0, A1, nullptr, lda, lda, 0, k, A1 ? k : 0, 0};
+    if (k % 2 == 0 && lda % 2 == 0 && aligned16(A0) && (!A1 || aligned16(A1)))
+        gram_x64_colmax_kernel<true><<<dim3(groups, 1), 512, 0, st>>>(n, rows, rows, o, emax);
+    else
+        gram_x64_colmax_kernel<false><<<dim3(groups, 1), 512, 0, st>>>(n, rows, rows, o, emax);
+    int rc = check_launch();
+    if (rc != CACG_OK) return rc;
+    col_exps_kernel<<<(kc + kXrElems - 1) / kXrElems, kXrSlices * kXrElems, 0, st>>>(emax, groups, k, kc,
+                                                                                   e0, e1);
     return check_launch();
 }
 

@@ -127,9 +127,9 @@ static int chol_inv(cudaStream_t st, int k, const double *G, double *R, double *
 }
 
 static int tallsmall_triu(cudaStream_t st, int64_t n, int k, const double *X, int64_t ldx,
-                          const double *W, double *Y, int64_t ldy, int *status) {
+                          const int *xexp, const double *W, double *Y, int64_t ldy, int *status) {
     if (n <= 0) return CACG_OK;
-    const int rc = launch_tallsmall_x64(st, n, k, k, X, ldx, W, k, Y, ldy, status);
+    const int rc = launch_tallsmall_x64(st, n, k, k, X, ldx, xexp, W, k, Y, ldy, status);
     if (rc != CACG_ERR_UNSUPPORTED) return rc;
     const int smem = (int)((size_t)k * k * sizeof(double));
     set_smem_attr(tallsmall_triu_kernel, kQrSmemMax);
@@ -150,7 +150,7 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
         return CACG_ERR_ARG;
     const size_t gws = (gram_workspace_bytes(n, k, k) + 255) / 256 * 256;
     const size_t q1b = ((size_t)n * k * sizeof(double) + 255) / 256 * 256;
-    const size_t small = (size_t)5 * k * k * sizeof(double);
+    const size_t small = (size_t)5 * k * k * sizeof(double) + (size_t)k * sizeof(int);
     char *buf = nullptr;
     if (cudaMallocAsync((void **)&buf, gws + q1b + small + 256, st) != cudaSuccess) {
         cudaGetLastError();
@@ -160,20 +160,26 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
     double *Q1 = (double *)(buf + gws);  // n x k, the first pass's factor
     double *G = (double *)(buf + gws + q1b), *R1 = G + (size_t)k * k, *R1i = R1 + (size_t)k * k,
            *R2 = R1i + (size_t)k * k, *R2i = R2 + (size_t)k * k;
-    int *bad = (int *)(R2i + (size_t)k * k);
+    int *bad = (int *)(R2i + (size_t)k * k), *exps = bad + 1;
     int rc = cudaMemsetAsync(bad, 0, sizeof(int), st) == cudaSuccess ? CACG_OK : CACG_ERR_CUDA;
+    // G = P^T P, and the exponents of P's columns for the product that follows
+    auto gram = [&](const double *P, int64_t ldp) {
+        ColExps ce;
+        ce.L = exps;
+        int r = launch_gram<double>(st, CACG_GRAM_AUTO, n, P, ldp, k, P, ldp, k, nullptr, 0, 0, G, k,
+                                    nullptr, 0, ws, gws, true, &ce);
+        if (r == CACG_OK && !ce.set)
+            r = launch_col_exps(st, n, k, P, nullptr, ldp, ws, gws, exps, nullptr);
+        return r;
+    };
     // pass 1: G = V^T V, R1, Q1 = V R1^{-1}
-    if (rc == CACG_OK)
-        rc = launch_gram<double>(st, CACG_GRAM_AUTO, n, V, ldv, k, V, ldv, k, nullptr, 0, 0, G, k,
-                                 nullptr, 0, ws, gws, true);
+    if (rc == CACG_OK) rc = gram(V, ldv);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R1, R1i, bad);
-    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, V, ldv, R1i, Q1, k, bad);
+    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, V, ldv, exps, R1i, Q1, k, bad);
     // pass 2: G2 = Q1^T Q1, R2, Q = Q1 R2^{-1}
-    if (rc == CACG_OK)
-        rc = launch_gram<double>(st, CACG_GRAM_AUTO, n, Q1, k, k, Q1, k, k, nullptr, 0, 0, G, k,
-                                 nullptr, 0, ws, gws, true);
+    if (rc == CACG_OK) rc = gram(Q1, k);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R2, R2i, bad);
-    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, R2i, Q, ldq, bad);
+    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, exps, R2i, Q, ldq, bad);
     if (rc == CACG_OK) {
         triu_mul_kernel<<<k, kQrMaxK, 0, st>>>(k, R2, R1, R);
         rc = check_launch();

@@ -200,8 +200,9 @@ static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slice
     L.Ssl = slices ? align256((size_t)3 * n * k * 2) : 0;
     L.R32sl = slices ? align256((size_t)3 * n * m * 2) : 0;
     // small: QtAS k*k, QtAQ k*k, QtR k*m, F 2*k*k + k, alpha k*m, beta k*k, norms m,
-    //        bnorm m, true norms m, bounds 2, scalars 16, status (int) 16
-    L.small = align256(sizeof(double) * ((size_t)5 * k * k + k + (size_t)2 * k * m +
+    //        bnorm m, true norms m, bounds 2, scalars 16, status (int), column exponents
+    //        of Q and AQ (k ints each)
+    L.small = align256(sizeof(double) * ((size_t)5 * k * k + 2 * k + (size_t)2 * k * m +
                                          3 * (size_t)m + 64));
     L.gram = align256(std::max(
         gram_workspace_bytes(n, k, k + m),
@@ -470,6 +471,7 @@ struct SolveBuffers {
     int ldr32p;
     double *QtAS, *QtAQ, *QtR, *F, *alpha, *beta, *norms, *bnorm, *tnorm, *bounds, *scal;
     int *status;
+    int *qexp, *aqexp;  // column exponents of Q and AQ (k each)
     double *gram_ws;
     size_t gram_ws_bytes;
     double *norm_ws;
@@ -504,6 +506,8 @@ static void carve(char *base, const Layout &L, int m, int k, SolveBuffers *b) {
     b->tnorm = sm; sm += m;
     b->bounds = sm; sm += 2;
     b->scal = sm; sm += 16;
+    b->qexp = (int *)sm; sm += k;
+    b->aqexp = b->qexp + k;
     b->gram_ws = (double *)(base + L.o_gram);
     b->gram_ws_bytes = L.gram;
     b->norm_ws = (double *)(base + L.o_norm);
@@ -828,9 +832,12 @@ struct Solver {
                 }
             } else {
                 rc = CACG_ERR_UNSUPPORTED;
-                if (planes64() && (double)n * k * k >= kPlanesQMin)
-                    rc = launch_qupdate_x64(st, n, k, (T *)b.S, k, (const T *)b.Q, k,
-                                            (const T *)b.S, k, b.beta, b.status);
+                if (planes64() && (double)n * k * k >= kPlanesQMin) {
+                    rc = need_exps((const double *)b.Q, nullptr);
+                    if (rc == CACG_OK)
+                        rc = launch_qupdate_x64(st, n, k, (T *)b.S, k, (const T *)b.Q, k, b.qexp,
+                                                (const T *)b.S, k, b.beta, b.status);
+                }
                 if (rc == CACG_ERR_UNSUPPORTED)
                     rc = launch_qupdate<T>(st, n, k, (T *)b.S, k, (const T *)b.Q, k,
                                            (const T *)b.S, k, b.beta);
@@ -840,6 +847,7 @@ struct Solver {
             std::swap(b.Q, b.S);
             std::swap(b.Qsl, b.Ssl);
         }
+        exps_of_q = exps_of_aq = false;  // this Q's and AQ's are not known yet
         const T *Q = (const T *)b.Q;
         T *AQ = (T *)b.AQ;
         prof.begin(CACG_PHASE_AQ, spmm_bytes(k, 0), 2.0 * (double)A->nnz * k);
@@ -877,7 +885,7 @@ struct Solver {
             rc = launch_gram_tcs(st, n, b.Qsl, k, k, b.AQsl, k, k, b.R32sl, m, m, b.QtAQ, k,
                                  b.QtR, m, b.gram_ws, b.gram_ws_bytes);
         else
-            rc = gram<T>(Q, k, AQ, k, k, Rp, ldrp, m, b.QtAQ, k, b.QtR, m, true);
+            rc = gram<T>(Q, k, AQ, k, k, Rp, ldrp, m, b.QtAQ, k, b.QtR, m, true, true);
         prof.end();
         if (rc) return rc;
         prof.begin(CACG_PHASE_LU, 16.0 * k * k, (2.0 / 3.0) * k * k * k + 2.0 * k * k * m);
@@ -918,7 +926,8 @@ struct Solver {
     // symmetric: L^T R1 with R1 = A L (Q^T A Q), only its upper triangle is
     // computed and mirrored (FP64 CUDA-core Gram)
     int gram(const T *Lm, int ka, const T *R1, int64_t ldr1, int kb1, const T *R2, int64_t ldr2,
-             int kb2, double *C1, int ldc1, double *C2, int ldc2, bool symmetric = false) {
+             int kb2, double *C1, int ldc1, double *C2, int ldc2, bool symmetric = false,
+             bool want_exps = false) {
         const int64_t n = A->n;
         if constexpr (std::is_same<T, float>::value) {
             if ((p.gram_variant == CACG_GRAM_AUTO || p.gram_variant == CACG_GRAM_TC5) &&
@@ -932,9 +941,26 @@ struct Solver {
         }
         int v = p.gram_variant == CACG_GRAM_TC ? CACG_GRAM_FMA : p.gram_variant;
         if (v == CACG_GRAM_AUTO && std::is_same<T, double>::value && !planes64()) v = CACG_GRAM_FMA;
-        return launch_gram<T>(st, v, n, Lm, k, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1, ldc1, C2,
-                              ldc2, b.gram_ws, b.gram_ws_bytes,
-                              symmetric && std::is_same<T, double>::value);
+        ColExps ce;
+        ce.L = b.qexp;
+        ce.R1 = b.aqexp;
+        const int rc = launch_gram<T>(st, v, n, Lm, k, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1, ldc1,
+                                      C2, ldc2, b.gram_ws, b.gram_ws_bytes,
+                                      symmetric && std::is_same<T, double>::value,
+                                      want_exps ? &ce : nullptr);
+        if (ce.set) exps_of_q = exps_of_aq = true;
+        return rc;
+    }
+
+    // column exponents of Q (and of AQ, if given) for the digit-plane updates: the
+    // Gram's Q^T [AQ | R] leaves them where it is made from digit planes itself
+    bool exps_of_q = false, exps_of_aq = false;
+    int need_exps(const double *Q, const double *AQ) {
+        if (exps_of_q && (!AQ || exps_of_aq)) return CACG_OK;
+        const int rc = launch_col_exps(st, A->n, k, Q, AQ, k, b.gram_ws, b.gram_ws_bytes, b.qexp,
+                                       b.aqexp);
+        if (rc == CACG_OK) exps_of_q = true, exps_of_aq = AQ != nullptr;
+        return rc;
     }
 
     template <typename T>
@@ -963,8 +989,10 @@ struct Solver {
         }
         if constexpr (std::is_same<T, double>::value) {
             if (planes64() && (double)A->n * k * m >= kPlanesXrMin) {
-                const int rc = launch_xrupdate_x64(st, A->n, k, m, Q, AQ, k, b.alpha, X, b.R, (T *)b.S,
-                                                   k, b.norms, b.norm_ws, b.status);
+                int rc = need_exps(Q, AQ);
+                if (rc == CACG_OK)
+                    rc = launch_xrupdate_x64(st, A->n, k, m, Q, AQ, k, b.qexp, b.aqexp, b.alpha, X,
+                                             b.R, (T *)b.S, k, b.norms, b.norm_ws, b.status);
                 if (rc != CACG_ERR_UNSUPPORTED) return rc;
             }
         }

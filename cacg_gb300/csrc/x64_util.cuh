@@ -41,19 +41,47 @@ __device__ __forceinline__ int x64_scale(uint32_t key, bool *bad) {
     return e < kXMinExp ? kXMinExp : e;
 }
 
-// the same where results are scaled by exponent-field additions alone: scales
-// within 2^+-400 (x64_scaled's range for a product of two)
-__device__ __forceinline__ int x64_scale_mid(uint32_t key, bool *bad) {
-    const int e = (int)(key >> 20);
-    if (key != 0u && (e < 1023 - 400 || e > 1023 + 400)) *bad = true;
-    return key == 0u ? 1023 : e;
+// A column's exponent for the tall x small products: of about its 2-norm, from the
+// maxima of its row groups (emax: ngroups x kc keys, column c), at least that of its
+// largest element; 1023 for a zero column and one with Inf or NaN.  Called by 16
+// threads a column (q) of a block, sh their shared scratch.
+__device__ __forceinline__ void x64_col_exp(const uint32_t *__restrict__ emax, int ngroups, int kc,
+                                            int c, bool on, int el, int q, float (*sh)[32],
+                                            int *__restrict__ out) {
+    uint32_t *shk = reinterpret_cast<uint32_t *>(&sh[0][0]);
+    uint32_t k = 0u;
+    if (on)
+        for (int g = q; g < ngroups; g += 16) k = max(k, emax[(size_t)g * kc + c]);
+    shk[q * 32 + el] = k;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) k = max(k, shk[i * 32 + el]);
+    __syncthreads();
+    const int E = (int)(k >> 20);
+    float s = 0.f;
+    if (on && k != 0u && E < 0x7ff)
+        for (int g = q; g < ngroups; g += 16) {
+            const int d = 2 * (E - (int)(emax[(size_t)g * kc + c] >> 20));
+            if (d < 127) s += __uint_as_float((uint32_t)(127 - d) << 23);  // 2^-d
+        }
+    sh[q][el] = s;
+    __syncthreads();
+    if (q == 0 && on) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) t += sh[i][el];
+        // t >= 1: half its binary logarithm
+        const int h = ((int)(__float_as_uint(t) >> 23) - 126) >> 1;
+        *out = k == 0u || E >= 0x7ff ? 1023 : min(E + max(h, 0), 2046);
+    }
 }
 
-// the seven balanced digits of x at scale E, biased by 128: bytes 0 .. 5 of
-// (hi, lo) are d_0 + 128 .. d_5 + 128, the top 16 bits d_6 + 128 (0 .. 256)
-__device__ __forceinline__ void x64_digits(double x, int E, uint32_t &lo, uint32_t &hi) {
+// the seven balanced digits of x at scale E (E20: in units of 2^-20, E at least x's
+// exponent, and 64 for a zero), biased by 128: bytes 0 .. 5 of (hi, lo) are d_0 + 128
+// .. d_5 + 128, the top 16 bits d_6 + 128 (0 .. 256)
+__device__ __forceinline__ void x64_digits(double x, uint32_t E20, uint32_t &lo, uint32_t &hi) {
     const uint32_t xh = (uint32_t)__double2hiint(x), xl = (uint32_t)__double2loint(x);
-    const int s = E - (int)((xh >> 20) & 0x7ffu);
+    const uint32_t s = (E20 - (xh & 0x7ff00000u)) >> 20;
     const uint32_t mh = (xh & 0xfffffu) | 0x100000u;
     uint64_t m;  // 8 x the 53-bit significand, shifted right (by 64 or more: 0): 2 |X|, a bit to round on
     const uint64_t m8 = ((uint64_t)__funnelshift_l(xl, mh, 3) << 32) | (uint64_t)(xl << 3);
@@ -67,8 +95,8 @@ __device__ __forceinline__ void x64_digits(double x, int E, uint32_t &lo, uint32
     hi = (uint32_t)(v >> 32);
 }
 
-// plane words of two values: w[p] = {digit 6-p of x0 (low half), of x1 (high half)} as fp16
-__device__ __forceinline__ void x64_planes2(double x0, double x1, int E0, int E1,
+// plane words of two values at scales E0, E1 (units of 2^-20): w[p] = {digit 6-p of x0 (low half), of x1 (high half)} as fp16
+__device__ __forceinline__ void x64_planes2(double x0, double x1, uint32_t E0, uint32_t E1,
                                             uint32_t (&w)[kXPlanes]) {
     uint32_t l0, h0, l1, h1;
     x64_digits(x0, E0, l0, h0);

@@ -34,6 +34,91 @@ def test_products_that_cancel_exactly(torch_cuda, M, top):
     assert np.array_equal(Q[:, 0], np.full(1024, 2.0 ** -5))
 
 
+def _stencil(kind, N, shift, m, seed=7):
+    rp, ci, v = cg.gen_matrix(kind, N, shift)
+    return rp, ci, v, cg.gen_rhs("normal", len(rp) - 1, m, seed)
+
+
+def _relres(rp, ci, v, B, X):
+    AX = np.stack([np.add.reduceat(v.astype(np.longdouble) * X[ci, c], rp[:-1])
+                   for c in range(X.shape[1])], 1)
+    return (np.sqrt(((B - AX) ** 2).sum(0)) / np.linalg.norm(B, axis=0)).astype(np.float64)
+
+
+# exponents of the right-hand sides' scales, column 0 the smallest
+SPREADS = [(0, 46, 10, 30), (0, 27, 33, 40), (-300, 100, 0, 200)]
+
+
+@pytest.mark.parametrize("kind,N,m,s", [("lap2d", 256, 4, 4), ("lap3d7", 40, 8, 4)])
+@pytest.mark.parametrize("spread", SPREADS)
+def test_solve_columns_of_different_magnitude(kind, N, m, s, spread):
+    """The block iteration is equivariant under a scale per right-hand side, exactly so for
+    powers of two: X is the unscaled call's X scaled, bit for bit, in as many iterations."""
+    rp, ci, v, B = _stencil(kind, N, 0.05, m)
+    n = len(rp) - 1
+    assert n * (s * m) ** 2 >= 2e6 and n * s * m * m >= 4e6  # the digit-plane updates' range
+    d = 2.0 ** np.resize(spread, m).astype(np.float64)
+    kw = dict(s=s, bounds="gerschgorin", tol=1e-9, maxit=300)
+    X1, i1 = cg.solve(rp, ci, v, B, **kw)
+    X2, i2 = cg.solve(rp, ci, v, B * d, **kw)
+    assert i1["status"] == 0 and i2["status"] == 0
+    assert i1["iterations"] == i2["iterations"]
+    assert np.array_equal(X2, X1 * d)
+
+
+@pytest.mark.parametrize("kind,N,m,s", [("lap2d", 256, 4, 4), ("lap3d7", 40, 8, 4)])
+@pytest.mark.parametrize("spread", SPREADS)
+def test_drop_in_columns_of_different_magnitude(kind, N, m, s, spread):
+    """The reference's stop rule looks at column 0's recurrence alone: the true residual of
+    every column has to agree with it (here: of column 0, the one the rule promises)."""
+    rp, ci, v, B = _stencil(kind, N, 0.05, m)
+    d = 2.0 ** np.resize(spread, m).astype(np.float64)
+    eps = 1e-8 * float(np.linalg.norm(B[:, 0]))
+    out = []
+    for scale in (np.ones(m), d / d[0]):
+        X = np.zeros_like(B)
+        Bs = B * scale
+        cg.bcbcg_v1(rp.astype(np.int64), ci.astype(np.int64), v, Bs, X, s, eps)
+        assert cg.last_status() == 0
+        out.append((X / scale, cg.last_iterations()))
+        assert _relres(rp, ci, v, Bs, X)[0] <= 1.01e-8
+    assert out[0][1] == out[1][1]
+    assert np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("n,k", [(20000, 16), (20000, 2), (6000, 96), (3000, 128), (257, 5)])
+@pytest.mark.parametrize("lo,hi", [(0, -7), (-7, 0), (-30, 30), (40, -40)])
+def test_qr_columns_of_different_magnitude(torch_cuda, n, k, lo, hi):
+    """QR of a block whose columns have magnitudes 10^lo .. 10^hi: CholeskyQR is equivariant
+    under a scale per column, and so each *column* of Q R - V stays at rounding: a chain of k
+    FMAs and the two passes, 100 k u of the column, u = 2^-53."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(3)
+    V = torch.randn(n, k, dtype=torch.float64, device="cuda", generator=g)
+    V *= 10.0 ** torch.linspace(lo, hi, k, device="cuda", dtype=torch.float64)
+    Q, R = _qr(torch, V)
+    v, u = V.cpu().numpy(), 100 * k * 2.0 ** -53
+    E = (Q.astype(np.longdouble) @ R.astype(np.longdouble) - v).astype(np.float64)
+    norm = np.linalg.norm(v, axis=0)
+    assert np.all(np.linalg.norm(E / norm, axis=0) <= u)
+    assert np.linalg.norm(Q.T @ Q - np.eye(k)) <= u * k ** 0.5
+
+
+@pytest.mark.parametrize("n", [1000, 20000])
+def test_qr_one_column_in_one_row(torch_cuda, n):
+    """A column whose weight lies in one row beside spread ones: magnitudes by norm, not by the
+    largest element."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(4)
+    V = torch.randn(n, 24, dtype=torch.float64, device="cuda", generator=g)
+    V[:, 7] *= 1e-9
+    V[n // 3, 7] = 1.0
+    Q, R = _qr(torch, V)
+    v, u = V.cpu().numpy(), 100 * 24 * 2.0 ** -53
+    E = (Q.astype(np.longdouble) @ R.astype(np.longdouble) - v).astype(np.float64)
+    assert np.all(np.linalg.norm(E, axis=0) <= u * np.linalg.norm(v, axis=0))
+
+
 @pytest.mark.parametrize("kind,N,m", [("lap2d", 600, 8), ("st3d27", 40, 8), ("lap3d7", 60, 9)])
 def test_fixed_point_spmm_point_values(kind, N, m):
     """B - A X where one element of a column is far above the others (its neighbours zero, so
