@@ -68,7 +68,7 @@ struct BcgState {
         const int v = p.gram_variant == CACG_GRAM_AUTO && A->dia_ndiag == 0 ? CACG_GRAM_FMA
                                                                             : p.gram_variant;
         return launch_gram<double>(st, v, n, L, m, m, Rm, m, m, nullptr, 0, 0, C,
-                                   m, nullptr, 0, gram_ws, gram_ws_bytes);
+                                   m, nullptr, 0, gram_ws, gram_ws_bytes, false, nullptr, true);
     }
     // Y = M^{-1} RHS (m x m), M factored into F
     int solve(const double *M, const double *RHS, double *Y) {

@@ -201,14 +201,16 @@ template <typename T>
 int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl, int ka,
                 const T *R1, int64_t ldr1, int kb1, const T *R2, int64_t ldr2, int kb2,
                 double *C1, int ldc1, double *C2, int ldc2, double *ws, size_t ws_bytes,
-                bool symmetric = false, struct ColExps *ce = nullptr);
+                bool symmetric = false, struct ColExps *ce = nullptr, bool normwise = false);
 size_t gram_workspace_bytes(int64_t n, int ka, int kb);
 // FP64 Gram from fp16 digit planes on tcgen05 (k_gram_x64.cu); launch_gram takes
-// it for CACG_GRAM_AUTO.  CACG_ERR_UNSUPPORTED: shape or workspace not for it.
+// it for CACG_GRAM_AUTO.  symmetric: L^T R1 is (its upper triangle counts); normwise:
+// accurate to the columns' norms, not to |L|^T |R|.  CACG_ERR_UNSUPPORTED: shape or
+// workspace not for it.
 int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
                     const double *R1, int64_t ldr1, int kb1, const double *R2, int64_t ldr2,
                     int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
-                    size_t ws_bytes, struct ColExps *ce = nullptr);
+                    size_t ws_bytes, bool symmetric, bool normwise, struct ColExps *ce);
 size_t gram_x64_workspace_bytes(int64_t n, int ka, int kb);
 // Exponents of the columns of a Gram's L (ka) and R1 (kb1), about their norms', for
 // the tall x small products of the same blocks (device arrays; set: written).  The

@@ -615,7 +615,7 @@ template <typename T>
 int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl, int ka,
                 const T *R1, int64_t ldr1, int kb1, const T *R2, int64_t ldr2, int kb2,
                 double *C1, int ldc1, double *C2, int ldc2, double *ws, size_t ws_bytes,
-                bool symmetric, ColExps *ce) {
+                bool symmetric, ColExps *ce, bool normwise) {
     const int kb = kb1 + kb2;
     if (ka <= 0 || kb <= 0 || n < 0 || !C1 || (kb2 > 0 && !C2)) return CACG_ERR_ARG;
     if (variant != CACG_GRAM_AUTO && variant != CACG_GRAM_FMA && variant != CACG_GRAM_DMMA)
@@ -626,7 +626,7 @@ int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl
                                       ldc2, ws, ws_bytes);
             if (rc != CACG_ERR_UNSUPPORTED) return rc;
             rc = launch_gram_x64(st, n, L, ldl, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1, ldc1, C2,
-                                 ldc2, ws, ws_bytes, ce);
+                                 ldc2, ws, ws_bytes, symmetric, normwise, ce);
             if (rc != CACG_ERR_UNSUPPORTED) return rc;
         }
     }
@@ -711,10 +711,10 @@ int launch_gram_reduce(cudaStream_t st, const double *part, int nchunks, int nti
 
 template int launch_gram<double>(cudaStream_t, int, int64_t, const double *, int64_t, int,
                                  const double *, int64_t, int, const double *, int64_t, int,
-                                 double *, int, double *, int, double *, size_t, bool, ColExps *);
+                                 double *, int, double *, int, double *, size_t, bool, ColExps *, bool);
 template int launch_gram<float>(cudaStream_t, int, int64_t, const float *, int64_t, int,
                                 const float *, int64_t, int, const float *, int64_t, int,
-                                double *, int, double *, int, double *, size_t, bool, ColExps *);
+                                double *, int, double *, int, double *, size_t, bool, ColExps *, bool);
 
 }  // namespace cacg
 

@@ -7,27 +7,52 @@
 //
 // Why: this part's FP64 pipe gives 1.2 TFLOP/s, 1/1600 of its fp16 tensor
 // rate, and an FP64 FMA Gram keeps it 96 % busy; 28 fp16 digit-plane products
-// (x64_util.cuh) do the same sum 20 times faster, with less rounding.
+// (x64_util.cuh) do the same sum 20 times faster.
 //
-// Four launches:
-//   colmax   the largest magnitude of every column over each row chunk (a
-//            column's digits share one scale per chunk);
+// Accuracy.  A digit holds an element to 2^-56 of the power of two M above its
+// column's largest in the row chunk, so a row's product is within 2^-53 M_a M_b
+// (the roundings and the dropped planes; 2^-58 is usual), whatever the product's
+// own size.  An FMA chain's error goes with sum |L||R|, and that can be far
+// smaller: rows graded against each other, one large element a column.  So the
+// planes are for chunks where it is not.  With D_a the sum over the rows of
+// log2(M_a / |L_ra|), the arithmetic-geometric mean inequality gives
+//     sum_r |L_ra||R_rb| >= rows M_a M_b 2^-(D_a + D_b)/rows
+// and a chunk with (max D_a + max D_b) / rows above kXgSpread is summed by FP64
+// FMAs.  (A zero has no error in its row; counting kXgSpread bits for it keeps the
+// bound true for the rows left.)  The planes' error is then below 2^(kXgSpread - 53) of
+// sum |L||R|, and about 2^(kXgSpread - 58) / sqrt(rows) of it in practice: 2^-49 at 64
+// rows, 2^-52 at 6000, at the line.  Normal data stays at 8 to 10 bits.
+//
+// The solvers ask for less (normwise): their Gram matrices have to be accurate to
+// ||L_a|| ||R_b||, since that is what the factorisation and the updates keep, and their
+// blocks have columns of up to 17 bits (varying coefficients, 32 right-hand sides) and
+// far more (point sources).  M_a <= 2 ||L_a||, so the planes give that without the line:
+// about 2^-57 for spread columns, 2^-51 where one element of 6000 rows carries both.
+// Point sources, alone and beside spread right-hand sides, tolerances to 1e-12: the
+// iterations and residuals of the FMA Gram, in 13 to 29 % of the time.
+//
+// Two or three launches:
+//   colmax   the largest magnitude and the sum of the logarithms of every column
+//            over each row chunk (a column's digits share one scale per chunk);
+//            small operands are scanned by the product kernel itself;
 //   gram     split-K over row chunks, one CTA of 17 warps per SM: 16 converter
 //            warps copy 32-row steps to shared memory (cp.async into slots
 //            that only the copying thread reads: no barrier), split them into
 //            digit planes (MN-major core matrices, double-buffered) and one
-//            thread issues the MMAs.  The B planes are stacked side by side in
+//            warp issues the MMAs.  The B planes are stacked side by side in
 //            the MMA's N dimension and the accumulators of p + q = 0 .. 6 lie
 //            side by side in tensor memory, so plane p of A is multiplied with
 //            planes 0 .. 6-p of B by one or two wide MMAs: A is read from
 //            shared memory 10 times a step instead of 28.  After 128 rows the
 //            integer sums (below 2^24, exact) are folded into integer
 //            registers (64 + 24 bits per output, exact), and scaled to FP64
-//            once per chunk;
-//   reduce   sums the chunks' FP64 partials in a fixed order.  Where a chunk
-//            raised its flag (Inf or NaN in a column, a column below 2^-959,
-//            a wait that ran out) it recomputes its outputs by FP64 FMAs.
+//            once per chunk.  A chunk over the line above, or with Inf, NaN or a
+//            column below 2^-959, is summed by the same CTA's FP64 FMAs instead;
+//   reduce   sums the chunks' FP64 partials in a fixed order (and recomputes the
+//            outputs should a wait of the product kernel have run out).
 #include <algorithm>
+#include <cstdint>
+#include <type_traits>
 
 #include "cacg_internal.cuh"
 #include "tc5_util.cuh"
@@ -40,6 +65,8 @@ constexpr int kXgM = 128;                          // MMA M (L columns, zero-pad
 constexpr int kXgGroup = 4;                        // steps per accumulation group (128 rows)
 constexpr int kXgConvWarps = 16;
 constexpr int kXgThreads = 32 * kXgConvWarps + 32;  // + the MMA issuer's warp
+constexpr int kXgSpread = 12;  // bits: see above
+constexpr int kXgNoLine = INT32_MAX;
 constexpr int kXgMaxUnits = 6;  // (8 columns, 8 rows) units per warp and step
 constexpr int kXgMaxStages = 4;  // steps of raw rows in flight
 constexpr unsigned kXgABytes = kXPlanes * kXgM * kXgKT * 2;  // A planes of one step
@@ -51,15 +78,40 @@ struct XgOperands {
 };
 
 // ------------------------------------------------------------ column maxima
-// emax[(chunk * sub + s) * (ka + kb) + column]: block (chunk, s) covers the
-// s-th part of the chunk's rows
-template <bool VEC>
+// Sums of a column's logarithms, in units of 2^-8 (the key's exponent and first
+// mantissa bits: at most log2 |x| + 1023), and its zeros beside them
+constexpr int kXgZeroBit = 42;
+__device__ __forceinline__ uint64_t xg_log(uint32_t key) {
+    return key == 0u ? 1ull << kXgZeroBit : (uint64_t)(key >> 12);
+}
+// such sums added up in shared memory by 32-bit parts (a 64-bit shared addition is a
+// loop: 64 threads of a column take it for 30 us a launch)
+struct XgLogSum {
+    uint32_t lo, hi, zeros;
+};
+__device__ __forceinline__ void xg_add(XgLogSum &t, uint64_t s) {
+    const uint64_t l = s & ((1ull << kXgZeroBit) - 1);
+    atomicAdd(&t.lo, (uint32_t)l & 0xfffffu);
+    atomicAdd(&t.hi, (uint32_t)(l >> 20));
+    if (s >> kXgZeroBit) atomicAdd(&t.zeros, (uint32_t)(s >> kXgZeroBit));
+}
+__device__ __forceinline__ uint64_t xg_logs(const XgLogSum &t) {
+    return ((uint64_t)t.hi << 20) + t.lo;
+}
+
+// emax, elog[(chunk * sub + s) * (ka + kb) + column]: block (chunk, s) covers the
+// s-th part of the chunk's rows (LOG: the logarithms too)
+template <bool VEC, bool LOG>
 __global__ void __launch_bounds__(512)
     gram_x64_colmax_kernel(int64_t n, int64_t rows_per_chunk, int64_t rows_per_sub, XgOperands o,
-                           uint32_t *__restrict__ emax) {
+                           uint32_t *__restrict__ emax, unsigned long long *__restrict__ elog) {
     __shared__ uint32_t mx[3 * 256];
+    __shared__ XgLogSum lg[LOG ? 3 * 256 : 1];
     const int kc = o.ka + o.kb1 + o.kb2;
-    for (int i = threadIdx.x; i < kc; i += blockDim.x) mx[i] = 0u;
+    for (int i = threadIdx.x; i < kc; i += blockDim.x) {
+        mx[i] = 0u;
+        if constexpr (LOG) lg[i] = XgLogSum{0u, 0u, 0u};
+    }
     __syncthreads();
     const int64_t c0 = (int64_t)blockIdx.x * rows_per_chunk;
     const int64_t rb = c0 + (int64_t)blockIdx.y * rows_per_sub;
@@ -75,25 +127,37 @@ __global__ void __launch_bounds__(512)
             const int r = threadIdx.x / tpr, c = (threadIdx.x % tpr) * (VEC ? 2 : 1);
             if (r < rpb) {
                 uint32_t k0 = 0u, k1 = 0u;
+                uint64_t s0 = 0, s1 = 0;
 #pragma unroll 8
                 for (int64_t row = rb + r; row < re; row += rpb) {
                     if constexpr (VEC) {
                         const double2 v = __ldg(reinterpret_cast<const double2 *>(p + row * ld + c));
-                        k0 = max(k0, x64_key(v.x));
-                        k1 = max(k1, x64_key(v.y));
+                        const uint32_t e0 = x64_key(v.x), e1 = x64_key(v.y);
+                        k0 = max(k0, e0);
+                        k1 = max(k1, e1);
+                        if constexpr (LOG) s0 += xg_log(e0), s1 += xg_log(e1);
                     } else {
-                        k0 = max(k0, x64_key(__ldg(p + row * ld + c)));
+                        const uint32_t e0 = x64_key(__ldg(p + row * ld + c));
+                        k0 = max(k0, e0);
+                        if constexpr (LOG) s0 += xg_log(e0);
                     }
                 }
                 atomicMax(&mx[base + c], k0);
                 if constexpr (VEC) atomicMax(&mx[base + c + 1], k1);
+                if constexpr (LOG) {
+                    xg_add(lg[base + c], s0);
+                    if constexpr (VEC) xg_add(lg[base + c + 1], s1);
+                }
             }
         }
         base += w;
     }
     __syncthreads();
-    uint32_t *out = emax + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * kc;
-    for (int i = threadIdx.x; i < kc; i += blockDim.x) out[i] = mx[i];
+    const size_t out = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * kc;
+    for (int i = threadIdx.x; i < kc; i += blockDim.x) {
+        emax[out + i] = mx[i];
+        if constexpr (LOG) elog[out + i] = xg_logs(lg[i]) | (uint64_t)lg[i].zeros << kXgZeroBit;
+    }
 }
 
 // -------------------------------------------------------------- the products
@@ -108,13 +172,96 @@ __device__ __forceinline__ void xg_cp8(void *smem, const void *g, int bytes) {
                  : "memory");
 }
 
+// The chunk's products by FP64 FMAs, rows in order: an FMA holds its quadrant's pipe for
+// 64 clocks, so what counts is full warps, the same number on every quadrant (the tile's
+// outputs in a row over 512 threads); the two shared loads beside it do not matter.
+// sym: outputs below the diagonal of L^T R1 are left out (their mirror images are read).
+// n = 884736, 96 x 112: 21.0 ms (15.8 with the FMA kernel of k_gram.cu, whose tiles are
+// alike: here one CTA of two has 64 columns and one 48); Q^T A Q does half.
+template <int NB>
+__device__ __noinline__ void xg_fma_chunk(unsigned char *smem, int64_t rbeg, int64_t rend,
+                                          const XgOperands &o, int a0, int b0, int BA, int sym,
+                                          double *__restrict__ out) {
+    constexpr int KT = 32, T = 512, kE = kXgM * NB / T;
+    const int kb = o.kb1 + o.kb2, tid = threadIdx.x, W = BA + NB;
+    double *t = reinterpret_cast<double *>(smem);            // KT x W
+    int *first = reinterpret_cast<int *>(t + KT * (kXgM + NB));  // outputs before row a; their count
+    const int na = min(BA, o.ka - a0), nb = min(NB, kb - b0);
+    // row a of the tile has the columns from left(a) on
+    auto left = [&](int a) { return sym ? max(0, min(min(a0 + a, o.kb1) - b0, nb)) : 0; };
+    __syncthreads();
+    if (tid == 0) {
+        int c = 0;
+        for (int a = 0; a < na; ++a) {
+            first[a] = c;
+            c += nb - left(a);
+        }
+        first[na] = c;
+    }
+    __syncthreads();
+    const int total = first[na], E = (total + T - 1) / T;
+    double acc[kE];
+    int at[kE];  // columns of the output's operands in t
+#pragma unroll
+    for (int e = 0; e < kE; ++e) {
+        const int i = tid + e * T;
+        acc[e] = 0.0;
+        at[e] = BA << 16;
+        if (tid < T && i < total) {
+            int lo = 0, hi = na;  // first[lo] <= i < first[hi]
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (first[mid] <= i)
+                    lo = mid;
+                else
+                    hi = mid;
+            }
+            at[e] = lo | (BA + left(lo) + i - first[lo]) << 16;
+        }
+    }
+    for (int64_t r0 = rbeg; r0 < rend; r0 += KT) {
+        __syncthreads();
+        for (int i = tid; i < KT * W; i += kXgThreads) {
+            const int r = i / W, c = i % W, b = b0 + c - BA;
+            const int64_t row = r0 + r;
+            double v = 0.0;
+            if (row >= rend) {
+            } else if (c < BA) {
+                if (a0 + c < o.ka) v = __ldg(o.L + row * o.ldl + a0 + c);
+            } else if (b < o.kb1) {
+                v = __ldg(o.R1 + row * o.ldr1 + b);
+            } else if (b < kb) {
+                v = __ldg(o.R2 + row * o.ldr2 + (b - o.kb1));
+            }
+            t[i] = v;
+        }
+        __syncthreads();
+        if (tid >= T) continue;
+        for (int r = 0; r < KT; r += 4) {
+            const double *p = t + r * W;
+#pragma unroll
+            for (int e = 0; e < kE; ++e) {
+                if (e >= E) break;
+                const double *x = p + (at[e] & 0xffff), *y = p + (at[e] >> 16);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[e] = fma(x[u * W], y[u * W], acc[e]);
+            }
+        }
+    }
+    if (tid >= T) return;
+#pragma unroll
+    for (int e = 0; e < kE; ++e)
+        if (tid + e * T < total) out[(at[e] & 0xffff) * NB + (at[e] >> 16) - BA] = acc[e];
+}
+
 // NB = 16 * NC columns of [R1 | R2] per output tile (7 NB <= 512 columns of
 // tensor memory); VEC: widths and row strides even and bases 16-byte aligned,
 // so a pair of columns is one 16-byte copy.
 template <int NC, bool VEC>
 __global__ void __launch_bounds__(kXgThreads, 1)
     gram_x64_kernel(int64_t n, int64_t rows_per_chunk, XgOperands o, int BA, int tilesB, int sub,
-                    int stages, bool scan, uint32_t *__restrict__ emax, double *__restrict__ part,
+                    int stages, bool scan, int sym, int line, uint32_t *__restrict__ emax,
+                    const unsigned long long *__restrict__ elog, double *__restrict__ part,
                     int *__restrict__ flags) {
     constexpr int NB = 16 * NC;
     constexpr int NQ = NB / 4;  // accumulator columns per converter thread
@@ -123,7 +270,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     constexpr unsigned buf_bytes = kXgABytes + b_bytes;
     constexpr int tmem_cols = NC == 1 ? 128 : NC == 2 ? 256 : 512;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // [plane buffers x2][raw slots][scales][mbarriers][tmem slot][abort]
+    // [plane buffers x2][raw slots][scales][mbarriers][tmem slot][abort][spread x2]
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, and known to be
     const int nunits = (BA / 8 + NB / 8) * (kXgKT / 8);
@@ -147,21 +294,44 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     int *flag = flags + (size_t)blockIdx.x * gridDim.y + blockIdx.y;
 
     // scales of the tile's columns: from the maxima kernel, or, where the
-    // operands stay in L2 (scan), from a pass over the chunk's rows, which leaves them
+    // operands stay in L2 (scan), from a pass over the chunk's rows, which leaves them;
+    // and the bits by which its elements fall short of them, on average
+    int *spread = reinterpret_cast<int *>(tmem_slot + 2);
+    if (tid < 2) spread[tid] = 0;
     bool bad = false;
+    const bool lined = line != kXgNoLine;
+    auto short_bits = [&](uint32_t key, uint64_t logs, uint64_t zeros) {
+        if (key == 0u) return 0;  // no element, no error
+        const double rows = (double)(rend - rbeg);
+        const double d = (rows - (double)zeros) * (double)(((key >> 20) + 1) << 8) - (double)logs +
+                         (double)zeros * (kXgSpread << 8);
+        return (int)fmin(d / rows + 1.0, 1e6);
+    };
+    int lacks = 0;
     if (!scan) {
         if (tid < BA + NB) {
             const int c = tid < BA ? (a0 + tid < o.ka ? a0 + tid : -1)
                                    : (b0 + tid - BA < kb ? o.ka + b0 + tid - BA : -1);
             uint32_t key = 0u;
+            uint64_t logs = 0, zeros = 0;
             if (c >= 0)
-                for (int s = 0; s < sub; ++s)
-                    key = max(key, emax[((size_t)blockIdx.x * sub + s) * kc + c]);
+                for (int s = 0; s < sub; ++s) {
+                    const size_t at = ((size_t)blockIdx.x * sub + s) * kc + c;
+                    key = max(key, emax[at]);
+                    const uint64_t l = lined ? elog[at] : 0;
+                    logs += l & ((1ull << kXgZeroBit) - 1);
+                    zeros += l >> kXgZeroBit;
+                }
             esc[tid] = x64_scale(key, &bad) << 20;
+            if (lined) lacks = short_bits(key, logs, zeros);
         }
     } else {
         uint32_t *keys = reinterpret_cast<uint32_t *>(esc);
-        if (tid < BA + NB) keys[tid] = 0u;
+        XgLogSum *logs = reinterpret_cast<XgLogSum *>(smem_raw);
+        if (tid < BA + NB) {
+            keys[tid] = 0u;
+            logs[tid] = XgLogSum{0u, 0u, 0u};
+        }
         __syncthreads();
         const int tpr = (BA + NB) / 2, rpb = kXgThreads / tpr;
         const int r = tid / tpr, c = 2 * (tid % tpr);
@@ -177,25 +347,42 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             };
             int64_t l0, l1;
             const double *q0 = col_ptr(c, l0), *q1 = col_ptr(c + 1, l1);
-            uint32_t k0 = 0u, k1 = 0u;
-            if constexpr (VEC) {
-                if (q0) {
+            auto scan_rows = [&](auto with_logs) {
+                constexpr bool LOG = decltype(with_logs)::value;
+                uint32_t k0 = 0u, k1 = 0u;
+                uint64_t s0 = 0, s1 = 0;
+                auto take = [&](double x, uint32_t &k, uint64_t &l) {
+                    const uint32_t e = x64_key(x);
+                    k = max(k, e);
+                    if constexpr (LOG) l += xg_log(e);
+                };
+                if constexpr (VEC) {
+                    if (q0) {
 #pragma unroll 8
+                        for (int64_t row = rbeg + r; row < rend; row += rpb) {
+                            const double2 v = __ldg(reinterpret_cast<const double2 *>(q0 + row * l0));
+                            take(v.x, k0, s0);
+                            take(v.y, k1, s1);
+                        }
+                    }
+                } else {
+#pragma unroll 4
                     for (int64_t row = rbeg + r; row < rend; row += rpb) {
-                        const double2 v = __ldg(reinterpret_cast<const double2 *>(q0 + row * l0));
-                        k0 = max(k0, x64_key(v.x));
-                        k1 = max(k1, x64_key(v.y));
+                        if (q0) take(__ldg(q0 + row * l0), k0, s0);
+                        if (q1) take(__ldg(q1 + row * l1), k1, s1);
                     }
                 }
-            } else {
-#pragma unroll 4
-                for (int64_t row = rbeg + r; row < rend; row += rpb) {
-                    if (q0) k0 = max(k0, x64_key(__ldg(q0 + row * l0)));
-                    if (q1) k1 = max(k1, x64_key(__ldg(q1 + row * l1)));
+                atomicMax(&keys[c], k0);
+                atomicMax(&keys[c + 1], k1);
+                if constexpr (LOG) {
+                    xg_add(logs[c], s0);
+                    xg_add(logs[c + 1], s1);
                 }
-            }
-            atomicMax(&keys[c], k0);
-            atomicMax(&keys[c + 1], k1);
+            };
+            if (lined)
+                scan_rows(std::true_type());
+            else
+                scan_rows(std::false_type());
         }
         __syncthreads();
         if (tid < BA + NB) {
@@ -204,11 +391,15 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             const int c = tid < BA ? a0 + tid : b0 + tid - BA;
             if (tid < BA && tile_b == 0 && c < o.ka) left[c] = key;
             if (tid >= BA && tile_a == 0 && c < kb) left[o.ka + c] = key;
+            if (lined) lacks = short_bits(key, xg_logs(logs[tid]), logs[tid].zeros);
             esc[tid] = x64_scale(key, &bad) << 20;
         }
     }
-    if (__syncthreads_or(bad)) {
-        if (tid == 0) *flag = 1;
+    if (lacks > 0) atomicMax(&spread[tid >= BA], lacks);
+    if (__syncthreads_or(bad) || spread[0] + spread[1] > line) {
+        xg_fma_chunk<NB>(smem_raw, rbeg, rend, o, a0, b0, BA, sym,
+                         part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * (size_t)BA * NB);
+        if (tid == 0) *flag = 0;
         return;
     }
 
@@ -465,7 +656,7 @@ __global__ void __launch_bounds__(kXrSlices *kXrElems)
     gram_x64_reduce_kernel(const double *__restrict__ part, int nchunks, int ntiles, int BA, int NB,
                            int tilesB, int64_t n, XgOperands o, double *__restrict__ C1, int ldc1,
                            double *__restrict__ C2, int ldc2, const int *__restrict__ flags,
-                           int nsum, const uint32_t *__restrict__ emax, int groups,
+                           int sym, int nsum, const uint32_t *__restrict__ emax, int groups,
                            int *__restrict__ eL, int *__restrict__ eR1) {
     __shared__ double qs[kXrSlices][kXrElems];
     const int el = threadIdx.x % kXrElems, q = threadIdx.x / kXrElems;
@@ -481,8 +672,11 @@ __global__ void __launch_bounds__(kXrSlices *kXrElems)
     const int a = active ? idx / kb : 0, b = active ? idx % kb : 0;
     double s = 0.0;
     {
-        const int tile = (a / BA) * tilesB + (b / NB);
-        const size_t off = (size_t)tile * BA * NB + (size_t)(a % BA) * NB + (b % NB);
+        // (sym: below the diagonal of L^T R1, the mirror image)
+        const bool lower = sym && b < a && b < o.kb1;
+        const int pa = lower ? b : a, pb = lower ? a : b;
+        const int tile = (pa / BA) * tilesB + (pb / NB);
+        const size_t off = (size_t)tile * BA * NB + (size_t)(pa % BA) * NB + (pb % NB);
         const size_t stride = (size_t)ntiles * BA * NB;
         const int per = (nchunks + kXrSlices - 1) / kXrSlices;
         const int p1 = min(nchunks, q * per + per);
@@ -521,7 +715,7 @@ struct XgPlan {
     int BA, NB, tilesA, tilesB, nchunks, sub, stages;
     bool scan;  // column maxima inside the product kernel
     int64_t rows_per_chunk, rows_per_sub;
-    size_t smem, part_bytes, emax_bytes, total;
+    size_t smem, part_bytes, emax_bytes, elog_bytes, total;
 };
 
 static XgPlan plan_x64(int64_t n, int ka, int kb) {
@@ -555,8 +749,9 @@ static XgPlan plan_x64(int64_t n, int ka, int kb) {
     // k = 20 (+5): 41.7 either way); larger ones by a maxima kernel on more blocks
     p.scan = (double)n * (ka * p.tilesB + (double)kb * p.tilesA) * 8.0 <= 4e6;
     p.part_bytes = (size_t)p.nchunks * tiles * p.BA * p.NB * sizeof(double);
-    p.emax_bytes = (size_t)p.nchunks * p.sub * (ka + kb) * 4;
-    p.total = p.part_bytes + p.emax_bytes + (size_t)p.nchunks * tiles * sizeof(int) + 64;
+    p.elog_bytes = (size_t)p.nchunks * p.sub * (ka + kb) * 8;
+    p.emax_bytes = p.elog_bytes / 2;
+    p.total = p.part_bytes + p.elog_bytes + p.emax_bytes + (size_t)p.nchunks * tiles * sizeof(int) + 64;
     return p;
 }
 
@@ -576,24 +771,29 @@ bool gram_x64_supported(int64_t n, int ka, int kb) {
 
 template <int NC, bool VEC>
 static void xg_launch(dim3 grid, const XgPlan &p, cudaStream_t st, int64_t n, const XgOperands &o,
-                      uint32_t *emax, double *part, int *flags) {
+                      int sym, int line, uint32_t *emax, const unsigned long long *elog, double *part,
+                      int *flags) {
     set_smem_attr(gram_x64_kernel<NC, VEC>, (int)max_smem_optin());
     gram_x64_kernel<NC, VEC><<<grid, kXgThreads, p.smem, st>>>(
-        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan, emax, part, flags);
+        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan, sym, line, emax, elog, part, flags);
 }
 
 int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
                     const double *R1, int64_t ldr1, int kb1, const double *R2, int64_t ldr2,
                     int kb2, double *C1, int ldc1, double *C2, int ldc2, double *ws,
-                    size_t ws_bytes, ColExps *ce) {
+                    size_t ws_bytes, bool symmetric, bool normwise, ColExps *ce) {
     const int kb = kb1 + kb2;
     if (!gram_x64_supported(n, ka, kb)) return CACG_ERR_UNSUPPORTED;
     const XgPlan p = plan_x64(n, ka, kb);
     if (p.total > ws_bytes || !ws || p.smem > max_smem_optin()) return CACG_ERR_UNSUPPORTED;
     double *part = ws;
-    uint32_t *emax = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(ws) + p.part_bytes);
+    unsigned long long *elog =
+        reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(ws) + p.part_bytes);
+    uint32_t *emax = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(elog) + p.elog_bytes);
     int *flags = reinterpret_cast<int *>(reinterpret_cast<char *>(emax) + (p.emax_bytes + 15) / 16 * 16);
     const XgOperands o{L, R1, R2, ldl, ldr1, ldr2, ka, kb1, kb2};
+    const int sym = symmetric && ka == kb1;
+    const int line = normwise ? kXgNoLine : kXgSpread << 8;
     // 16-byte pairs: even widths, even strides, aligned bases
     const bool vec = ka % 2 == 0 && kb1 % 2 == 0 && kb2 % 2 == 0 && ldl % 2 == 0 &&
                      ldr1 % 2 == 0 && aligned16(L) && aligned16(R1) &&
@@ -601,21 +801,22 @@ int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, in
     const dim3 mgrid(p.nchunks, p.sub);
     int rc = CACG_OK;
     if (p.scan) {
-    } else if (vec)
-        gram_x64_colmax_kernel<true><<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o,
-                                                            emax);
-    else
-        gram_x64_colmax_kernel<false><<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o,
-                                                             emax);
+    } else {
+        auto kernel = vec ? (normwise ? gram_x64_colmax_kernel<true, false>
+                                      : gram_x64_colmax_kernel<true, true>)
+                          : (normwise ? gram_x64_colmax_kernel<false, false>
+                                      : gram_x64_colmax_kernel<false, true>);
+        kernel<<<mgrid, 512, 0, st>>>(n, p.rows_per_chunk, p.rows_per_sub, o, emax, elog);
+    }
     if (!p.scan) rc = check_launch();
     if (rc != CACG_OK) return rc;
     const dim3 grid(p.nchunks, p.tilesA * p.tilesB);
 #define XG_CASE(NC)                                                       \
     case NC:                                                              \
         if (vec)                                                          \
-            xg_launch<NC, true>(grid, p, st, n, o, emax, part, flags);    \
+            xg_launch<NC, true>(grid, p, st, n, o, sym, line, emax, elog, part, flags);    \
         else                                                              \
-            xg_launch<NC, false>(grid, p, st, n, o, emax, part, flags);   \
+            xg_launch<NC, false>(grid, p, st, n, o, sym, line, emax, elog, part, flags);   \
         break;
     switch (p.NB / 16) {
         XG_CASE(1)
@@ -631,7 +832,7 @@ int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, in
     const int nsum = (ka * kb + kXrElems - 1) / kXrElems;
     const int nexp = ce ? (ka + (ce->R1 ? kb1 : 0) + kXrElems - 1) / kXrElems : 0;
     gram_x64_reduce_kernel<<<nsum + nexp, kXrSlices * kXrElems, 0, st>>>(
-        part, p.nchunks, p.tilesA * p.tilesB, p.BA, p.NB, p.tilesB, n, o, C1, ldc1, C2, ldc2, flags,
+        part, p.nchunks, p.tilesA * p.tilesB, p.BA, p.NB, p.tilesB, n, o, C1, ldc1, C2, ldc2, flags, sym,
         nsum, emax, p.nchunks * (p.scan ? 1 : p.sub), ce ? ce->L : nullptr, ce ? ce->R1 : nullptr);
     if (ce) ce->set = true;
     return check_launch();
@@ -656,9 +857,9 @@ int launch_col_exps(cudaStream_t st, int64_t n, int k, const double *A0, const d
     uint32_t *emax = reinterpret_cast<uint32_t *>(ws);
     const XgOperands o{A0, A1, nullptr, lda, lda, 0, k, A1 ? k : 0, 0};
     if (k % 2 == 0 && lda % 2 == 0 && aligned16(A0) && (!A1 || aligned16(A1)))
-        gram_x64_colmax_kernel<true><<<dim3(groups, 1), 512, 0, st>>>(n, rows, rows, o, emax);
+        gram_x64_colmax_kernel<true, false><<<dim3(groups, 1), 512, 0, st>>>(n, rows, rows, o, emax, nullptr);
     else
-        gram_x64_colmax_kernel<false><<<dim3(groups, 1), 512, 0, st>>>(n, rows, rows, o, emax);
+        gram_x64_colmax_kernel<false, false><<<dim3(groups, 1), 512, 0, st>>>(n, rows, rows, o, emax, nullptr);
     int rc = check_launch();
     if (rc != CACG_OK) return rc;
     col_exps_kernel<<<(kc + kXrElems - 1) / kXrElems, kXrSlices * kXrElems, 0, st>>>(emax, groups, k, kc,

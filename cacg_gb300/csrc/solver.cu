@@ -947,7 +947,7 @@ struct Solver {
         const int rc = launch_gram<T>(st, v, n, Lm, k, ka, R1, ldr1, kb1, R2, ldr2, kb2, C1, ldc1,
                                       C2, ldc2, b.gram_ws, b.gram_ws_bytes,
                                       symmetric && std::is_same<T, double>::value,
-                                      want_exps ? &ce : nullptr);
+                                      want_exps ? &ce : nullptr, true);
         if (ce.set) exps_of_q = exps_of_aq = true;
         return rc;
     }

@@ -86,6 +86,26 @@ def test_drop_in_columns_of_different_magnitude(kind, N, m, s, spread):
     assert np.array_equal(out[0][0], out[1][0])
 
 
+@pytest.mark.parametrize("kind,N,m,s", [("lap2d", 400, 8, 4), ("lap3d7", 64, 8, 8)])
+def test_solve_point_sources(kind, N, m, s):
+    """Right-hand sides with one nonzero, alone and beside normal ones: columns whose elements
+    fall off over hundreds of orders of magnitude.  The FMA variant's iterations and residual."""
+    rp, ci, v, B = _stencil(kind, N, 0.5, m)
+    n = len(rp) - 1
+    assert n * (s * m) ** 2 >= 2e6 and n * s * m * m >= 4e6
+    for point in (range(m), range(0, m, 2)):
+        Bp = B.copy()
+        for c in point:
+            Bp[:, c] = 0.0
+            Bp[(n // 2 + 977 * c) % n, c] = 1.0
+        kw = dict(s=s, bounds="gerschgorin", tol=1e-11, maxit=200)
+        X1, i1 = cg.solve(rp, ci, v, Bp, **kw)
+        X2, i2 = cg.solve(rp, ci, v, Bp, gram="fma", **kw)
+        assert i1["status"] == 0 and i2["status"] == 0
+        assert abs(i1["iterations"] - i2["iterations"]) <= 1
+        assert _relres(rp, ci, v, Bp, X1).max() <= 1.01e-11
+
+
 @pytest.mark.parametrize("n,k", [(20000, 16), (20000, 2), (6000, 96), (3000, 128), (257, 5)])
 @pytest.mark.parametrize("lo,hi", [(0, -7), (-7, 0), (-30, 30), (40, -40)])
 def test_qr_columns_of_different_magnitude(torch_cuda, n, k, lo, hi):
@@ -117,6 +137,61 @@ def test_qr_one_column_in_one_row(torch_cuda, n):
     v, u = V.cpu().numpy(), 100 * 24 * 2.0 ** -53
     E = (Q.astype(np.longdouble) @ R.astype(np.longdouble) - v).astype(np.float64)
     assert np.all(np.linalg.norm(E, axis=0) <= u * np.linalg.norm(v, axis=0))
+
+
+def _gram(torch, L, R, variant=0):
+    C = torch.empty(L.shape[1], R.shape[1], dtype=torch.float64, device="cuda")
+    assert cg.lib().cacg_k_gram(0, variant, L.shape[0], ptr(L), L.shape[1], L.shape[1], ptr(R),
+                                R.shape[1], R.shape[1], None, 0, 0, ptr(C), R.shape[1],
+                                None) == 0
+    return C.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,ka,kb", [(300, 20, 24), (2000, 24, 24), (5000, 96, 112),
+                                     (40000, 17, 33), (3000, 130, 70)])
+@pytest.mark.parametrize("kind", ["rows", "spikes", "tails", "zeros", "huge"])
+def test_gram_rows_of_different_magnitude(torch_cuda, n, ka, kb, kind):
+    """L^T R with rows of L and R graded against each other, with single large elements in
+    different rows, with decaying columns: within n u of |L|^T |R| (n FMAs), u = 2^-53."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(8)
+    L = torch.randn(n, ka, dtype=torch.float64, device="cuda", generator=g)
+    R = torch.randn(n, kb, dtype=torch.float64, device="cuda", generator=g)
+    if kind == "rows":
+        d = 10.0 ** (torch.rand(n, 1, dtype=torch.float64, device="cuda", generator=g) * 12 - 6)
+        L, R = L * d, R / d
+    elif kind == "spikes":  # one large element a column, never in a row that both have
+        L, R = L.sign(), R.sign()
+        i = torch.arange(ka, device="cuda")
+        L[2 * i % n, i] = 2.0 ** 60
+        R[2 * i % n, :] = 0.0
+        j = torch.arange(kb, device="cuda")
+        R[(2 * j + 1) % n, j] = 2.0 ** 60
+        L[(2 * j + 1) % n, :] = 0.0
+    elif kind == "tails":  # a column's weight near its own row
+        r = torch.arange(n, device="cuda", dtype=torch.float64)[:, None]
+        at = torch.linspace(0, n - 1, ka, device="cuda", dtype=torch.float64)
+        L = L * torch.exp(-40.0 * (r - at).abs() / n)
+        at = torch.linspace(n - 1, 0, kb, device="cuda", dtype=torch.float64)
+        R = R * torch.exp(-40.0 * (r - at).abs() / n)
+    elif kind == "zeros":  # three rows in four are zero in one or the other
+        r = torch.arange(n, device="cuda")
+        L = L * 10.0 ** (-9.0 * (r % 4 == 0))[:, None]
+        L[r % 4 == 1] = 0.0
+        R[r % 4 >= 2] = 0.0
+        R = R * 10.0 ** (-9.0 * (r % 4 == 1))[:, None]
+    else:
+        L = L * 1e300
+        L[::7] = L[::7] * 1e-290
+        R = R * 1e-300
+        R[::7] = R[::7] * 1e290
+    C = _gram(torch, L, R)
+    l, r = L.cpu().numpy().astype(np.longdouble), R.cpu().numpy().astype(np.longdouble)
+    ref, mag = np.zeros((ka, kb), np.longdouble), np.zeros((ka, kb), np.longdouble)
+    for a in range(ka):
+        ref[a] = l[:, a] @ r
+        mag[a] = np.abs(l[:, a]) @ np.abs(r)
+    assert np.all(np.abs(C - ref) <= n * 2.0 ** -53 * mag)
 
 
 @pytest.mark.parametrize("kind,N,m", [("lap2d", 600, 8), ("st3d27", 40, 8), ("lap3d7", 60, 9)])
