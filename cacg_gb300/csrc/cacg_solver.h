@@ -123,7 +123,10 @@ int solve_bcg_on_device(const DevMatrix *A, const double *B, double *X, int m,
 
 // Device bytes of one solve's state (S, Q, AQ, R, small matrices, reduction
 // workspaces), the admission cost of a request.
-size_t solve_workspace_bytes(int64_t n, int m, int s, int prec, bool lanczos);
+size_t solve_workspace_bytes(int64_t n, int m, int s, int prec, bool lanczos, int fix);
+// Scratch of the fixed-point SpMM that a solve can use if its matrix has the one-value
+// view: 0 none, 1 for A Q, 2 for the basis steps too (n x m more)
+int dia_fix_level(const cacg_params &p, int64_t nnz, int m);
 
 // Solve with device B, X.  ws_external (>= solve_workspace_bytes) may be
 // given; otherwise a cached workspace is used.

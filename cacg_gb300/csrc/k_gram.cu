@@ -471,8 +471,15 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-static size_t tiny_bytes(int ka, int kb) {
-    return ka <= kTinyMax && kb <= kTinyMax ? (size_t)kTinyBlocks * ka * kb * sizeof(double) : 0;
+static int tiny_blocks(int64_t n, int ka) {
+    const int rows = (kTinyThreads / 32) * (32 / ka);  // rows a block takes at a time
+    return (int)std::max<int64_t>(
+        1, std::min<int64_t>((n + 4 * rows - 1) / (4 * rows), std::min(4 * sm_count(), kTinyBlocks)));
+}
+
+static size_t tiny_bytes(int64_t n, int ka, int kb) {
+    if (ka > kTinyMax || kb > kTinyMax) return 0;
+    return (size_t)tiny_blocks(n, ka) * ka * kb * sizeof(double);
 }
 
 static int launch_gram_tiny(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,
@@ -480,16 +487,14 @@ static int launch_gram_tiny(cudaStream_t st, int64_t n, const double *L, int64_t
                             int64_t ldr2, int kb2, double *C1, int ldc1, double *C2, int ldc2,
                             double *ws, size_t ws_bytes) {
     const int kb = kb1 + kb2;
-    if (n <= 0 || ka > kTinyMax || kb > kTinyMax || !ws || tiny_bytes(ka, kb) > ws_bytes)
+    if (n <= 0 || ka > kTinyMax || kb > kTinyMax || !ws || tiny_bytes(n, ka, kb) > ws_bytes)
         return CACG_ERR_UNSUPPORTED;
     // the digit planes' time hardly grows with the columns here, the FMAs' does.
     // Through cacg_k_gram (about 38 us of it the call), planes and this: n = 884736,
     // 8 x 10 222 and 162 us, 12 x 15 273 and 417; n = 50653, 12 x 15 52 and 60;
     // n = 16384, 12 x 15 44 and 42
     if (ka * kb > 80 && (double)n * ka * kb > 3e6) return CACG_ERR_UNSUPPORTED;
-    const int rows = (kTinyThreads / 32) * (32 / ka);  // rows a block takes at a time
-    const int blocks = (int)std::max<int64_t>(
-        1, std::min<int64_t>((n + 4 * rows - 1) / (4 * rows), std::min(4 * sm_count(), kTinyBlocks)));
+    const int blocks = tiny_blocks(n, ka);
 #define TINY_CASE(KB)                                                                             \
     if (kb <= KB) {                                                                               \
         gram_tiny_kernel<KB><<<blocks, kTinyThreads, 0, st>>>(n, L, ldl, ka, R1, ldr1, kb1, R2,   \
@@ -608,7 +613,7 @@ size_t gram_workspace_bytes(int64_t n, int ka, int kb) {
         size_t b2 = (size_t)q.nchunks * q.tilesA * q.tilesB * q.BA * q.BB * sizeof(double);
         best = std::max(best, std::max(b1, b2));
     }
-    return std::max(std::max(best, gram_x64_workspace_bytes(n, ka, kb)), tiny_bytes(ka, kb));
+    return std::max(std::max(best, gram_x64_workspace_bytes(n, ka, kb)), tiny_bytes(n, ka, kb));
 }
 
 template <typename T>

@@ -69,6 +69,7 @@ struct Request {
     double *X_out;
     size_t cost;
     bool batched = false;
+    int fix = 0;    // scratch of the fixed-point SpMM (dia_fix_level)
     int skips = 0;  // admissions that passed this request over
     int state = 0;  // 0 queued, 1 running, 2 done
     int status = CACG_PENDING;
@@ -244,7 +245,7 @@ struct Server {
         int rc = DevMatrix::create(&A, r->p.precision == CACG_MIXED, &M, st);
         size_t bx = (size_t)r->n * r->m * sizeof(double);
         size_t wsb = solve_workspace_bytes(r->n, r->m, r->p.s, r->p.precision,
-                                           r->p.bounds_mode == CACG_BOUNDS_LANCZOS);
+                                           r->p.bounds_mode == CACG_BOUNDS_LANCZOS, r->fix);
         double *dB = nullptr, *dX = nullptr;
         void *ws = nullptr;
         if (rc == CACG_OK && cudaMallocAsync((void **)&dB, bx, st) != cudaSuccess) rc = CACG_ERR_OOM;
@@ -1073,7 +1074,7 @@ int cacg_server_submit(cacg_server *srv, const cacg_csr *A, const double *B, int
                      (size_t)A->nnz * 18 + (size_t)(A->n + 64) * 12 * 2;
         return mat + 2 * (size_t)A->n * m * 8 +
                solve_workspace_bytes(A->n, m, p->s, p->precision,
-                                     p->bounds_mode == CACG_BOUNDS_LANCZOS);
+                                     p->bounds_mode == CACG_BOUNDS_LANCZOS, r->fix);
     };
     if (r->batched && s->cfg.batch_max_rows == 0 && p->precision == CACG_FP64 &&
         p->gram_variant == CACG_GRAM_AUTO && p->spmm_format != CACG_SPMM_CSR &&
@@ -1084,6 +1085,16 @@ int cacg_server_submit(cacg_server *srv, const cacg_csr *A, const double *B, int
                   ? blayout(A->n, A->nnz, m, p->s, p->precision == CACG_MIXED).total
                   : stream_cost();
     if ((int64_t)r->cost > s->cfg.mem_budget_bytes) return CACG_ERR_BUSY;
+    // the fixed-point SpMM's scratch, where the budget has room for it
+    double c;
+    if (!r->batched && looks_diagonal(A) && dia_fix_candidate(A, &c)) {
+        r->fix = dia_fix_level(*p, A->nnz, m);
+        const size_t with = stream_cost();
+        if ((int64_t)with > s->cfg.mem_budget_bytes)
+            r->fix = 0;
+        else
+            r->cost = with;
+    }
     {
         std::lock_guard<std::mutex> lk(s->mu);
         r->ticket = s->next_ticket++;

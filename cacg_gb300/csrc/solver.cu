@@ -179,14 +179,16 @@ static bool use_slice_planes(int m, int s, int prec, int gram_variant, int exact
            m % 8 == 0 && (size_t)k * k * sizeof(float) <= 160 * 1024;
 }
 
-static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slices = false) {
+// fix: scratch of the fixed-point SpMM (FP64, a matrix with the one-value view), for
+// the A Q product (1) or for the basis steps too (2)
+static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slices = false,
+                     int fix = 0) {
     Layout L{};
     const int k = s * m;
     const size_t es = prec == CACG_MIXED ? 4 : 8;
     L.slices = slices;
-    // FP64: the S buffer also holds the fixed-point copy of Q, an even number of
-    // columns wide
-    const int ks = prec == CACG_FP64 ? (k + 1) / 2 * 2 : k;
+    // (the S buffer also holds the fixed-point copy of Q, an even number of columns wide)
+    const int ks = fix > 0 ? (k + 1) / 2 * 2 : k;
     L.S = L.Q = L.AQ = align256((size_t)n * ks * es + 64);
     L.R = align256((size_t)n * m * 8);
     L.R32 = prec == CACG_MIXED ? align256((size_t)n * m * 4) : 0;
@@ -212,8 +214,8 @@ static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slice
                            : (size_t)0));
     L.norm = align256(norm_workspace_doubles(n, std::max(m, 2)) * sizeof(double) + 4096);
     L.lanczos = lanczos ? align256((size_t)3 * n * 8) : 0;
-    L.xi = prec == CACG_FP64 ? align256(dia_fix_scratch_bytes(n, m)) : 0;
-    L.fixs = prec == CACG_FP64 ? align256(dia_fix_small_bytes(k)) : 0;
+    L.xi = fix > 1 ? align256(dia_fix_scratch_bytes(n, m)) : 0;
+    L.fixs = fix > 0 ? align256(dia_fix_small_bytes(k)) : 0;
     size_t o = 0;
     L.o_S = o; o += L.S;
     L.o_Q = o; o += L.Q;
@@ -237,9 +239,17 @@ static Layout layout(int64_t n, int m, int s, int prec, bool lanczos, bool slice
     return L;
 }
 
-size_t solve_workspace_bytes(int64_t n, int m, int s, int prec, bool lanczos) {
-    return layout(n, m, s, prec, lanczos, use_slice_planes(m, s, prec, CACG_GRAM_TC_SLICES, 0))
+size_t solve_workspace_bytes(int64_t n, int m, int s, int prec, bool lanczos, int fix) {
+    return layout(n, m, s, prec, lanczos, use_slice_planes(m, s, prec, CACG_GRAM_TC_SLICES, 0),
+                  fix)
         .total;
+}
+
+int dia_fix_level(const cacg_params &p, int64_t nnz, int m) {
+    if (p.precision != CACG_FP64 || p.gram_variant != CACG_GRAM_AUTO ||
+        p.spmm_format != CACG_SPMM_AUTO || (double)nnz * p.s * m < kDiaFixMin)
+        return 0;
+    return (double)nnz * m < kDiaFixMin ? 1 : 2;
 }
 
 // A growable cache of one device workspace per thread-less use (the bench
@@ -1201,14 +1211,21 @@ int solve_on_device(const DevMatrix *A, const double *B, double *X, int m,
     if (S.prec == CACG_MIXED && !A->val32) return CACG_ERR_ARG;
     bool lz = p.bounds_mode == CACG_BOUNDS_LANCZOS;
     const bool sl = use_slice_planes(m, p.s, p.precision, p.gram_variant, p.exact_updates);
-    Layout L = layout(A->n, m, p.s, p.precision, lz, sl);
+    // the fixed-point SpMM's scratch where there is room for it, else without
+    const int fix = A->fix_mask ? dia_fix_level(p, A->nnz, m) : 0;
+    Layout L = layout(A->n, m, p.s, p.precision, lz, sl, fix);
     S.slices = sl;
     void *ws = ws_external;
     bool from_cache = false;
     if (ws) {
+        if (fix && ws_external_bytes < L.total) L = layout(A->n, m, p.s, p.precision, lz, sl);
         if (ws_external_bytes < L.total) return CACG_ERR_ARG;
     } else {
         int rc = ws_acquire(L.total, &ws, &from_cache);
+        if (rc && fix) {
+            L = layout(A->n, m, p.s, p.precision, lz, sl);
+            rc = ws_acquire(L.total, &ws, &from_cache);
+        }
         if (rc) return rc;
     }
     carve((char *)ws, L, m, S.k, &S.b);
@@ -1354,7 +1371,7 @@ int32_t cacg_matrix_diagonals(const cacg_matrix *A) {
 }
 
 int64_t cacg_workspace_bytes(int64_t n, int32_t m, int32_t s, int32_t precision) {
-    return (int64_t)solve_workspace_bytes(n, m, s, precision, true);
+    return (int64_t)solve_workspace_bytes(n, m, s, precision, true, 0);
 }
 
 int cacg_solve_device(cacg_matrix *A, const double *B_dev, double *X_dev, int32_t m,

@@ -202,3 +202,30 @@ def test_requests_beyond_batched_limits_run_on_stream_worker(lib):
     for X, info in outs:
         assert info["status"] == 0 and info["true_relres_max"] <= 1e-8
     assert O.port_true_relres(rp, ci, v, B, outs[0][0]).max() <= 1e-8
+
+
+@pytest.mark.parametrize("n,m,s,before", [
+    (1000, 1, 4, 175360), (2500, 4, 4, 1305600), (20000, 8, 4, 19862016),
+    (40000, 16, 4, 79355648), (65536, 32, 4, 260774912), (262144, 8, 8, 437237760),
+    (1000000, 16, 6, 2482810880)])
+def test_fp64_workspace_is_the_states(lib, n, m, s, before):
+    """The admission cost without the fixed-point SpMM's copy of a block (n m doubles, 5 % of
+    the whole at s = 6), which is taken where there is room: the sizes from before that kernel,
+    and 11 KB (5 % below 10000 rows) for the scales and column exponents."""
+    assert lib.cacg_workspace_bytes(n, m, s, 0) <= before + max(11 * 1024, 0.05 * before * (n < 10000))
+
+
+@pytest.mark.parametrize("slack", [0, 1 << 30])
+def test_server_at_the_budget_of_the_state(lib, slack):
+    """A request whose cost fills the budget is admitted, and solves without that scratch."""
+    rp, ci, v = cg.gen_matrix("lap3d7", 64, 0.3)
+    n, nnz, m, s = len(rp) - 1, len(v), 8, 8
+    B = cg.gen_rhs("normal", n, m, 5)
+    matrix = (n + 1) * 4 + nnz * 28 + nnz * 18 + (n + 64) * 24
+    budget = matrix + 16 * n * m + lib.cacg_workspace_bytes(n, m, s, 0)
+    p = cg.Params(s=s, bounds=("lanczos", 30), tol=1e-9, maxit=100)
+    srv = cg.Server(mem_budget_bytes=budget + slack, max_active=1)
+    X, info = srv.wait(srv.submit(rp, ci, v, B, p))
+    srv.close()
+    assert info["status"] == 0
+    assert O.port_true_relres(rp, ci, v, B, X).max() <= 1.01e-9
