@@ -107,6 +107,9 @@ int launch_dia_fix(cudaStream_t st, const DevMatrix *A, int w, const double *X, 
                    FixChain *chain = nullptr);
 size_t dia_fix_scratch_bytes(int64_t n, int w);
 size_t dia_fix_mask_bytes(int64_t npad);
+// Whether DevMatrix::create will build the DIA view of this host matrix (memory
+// permitting): few diagonals with modest padding, rows sorted and in range
+bool dia_view_of(const cacg_csr *A);
 bool dia_fix_candidate(const cacg_csr *A, double *c);
 int launch_dia_fix_mask(cudaStream_t st, int64_t npad, const DiaDesc &desc, double *v64, double c,
                         uint32_t **mask, int *dmain, int *bad);

@@ -117,12 +117,52 @@ __global__ void dia_offsets_kernel(int64_t n, const int32_t *__restrict__ rp,
     }
 }
 
+// a view needs at most kDiaMax diagonals with modest padding
+static bool dia_padding_ok(int64_t nd, int64_t n, int64_t nnz) {
+    return (double)nd * (double)n <= 1.5 * (double)nnz + 64.0;
+}
+
+bool dia_view_of(const cacg_csr *A) {
+    const int64_t n = A->n, nnz = A->nnz;
+    if (n < 1 || nnz < 1 || A->row_ptr[0] != 0 || !dia_padding_ok(1, n, nnz)) return false;
+    int64_t offs[kDiaMax];
+    int cnt = 0, plen = -1;
+    for (int64_t i = 0; i < n; ++i) {
+        const int64_t b = A->row_ptr[i], e = A->row_ptr[i + 1];
+        if (b > e || e > nnz) return false;
+        const int32_t *c = A->col_idx + b;
+        const int len = (int)std::min<int64_t>(e - b, kDiaMax + 1);
+        if (len > kDiaMax) return false;
+        if (len == 0) {
+            plen = -1;
+            continue;
+        }
+        if (c[len - 1] >= n) return false;
+        // most rows have the offsets of the row before: its columns and one
+        bool same = len == plen;
+        for (int j = 0; same && j < len; ++j) same = c[j] == c[j - len] + 1;
+        plen = len;
+        if (same) continue;
+        int64_t prev = -1;
+        for (int j = 0; j < len; ++j) {
+            if (c[j] <= prev) return false;
+            prev = c[j];
+            const int64_t o = (int64_t)c[j] - i;
+            int t = 0;
+            while (t < cnt && offs[t] != o) ++t;
+            if (t < cnt) continue;
+            if (cnt == kDiaMax) return false;
+            offs[cnt++] = o;
+        }
+    }
+    return dia_padding_ok(cnt, n, nnz);
+}
+
 int DevMatrix::build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st) {
     dia_ndiag = 0;
     const int64_t n = A->n;
     if (n < 1 || A->nnz < 1) return CACG_OK;
-    // a view needs at most kDiaMax diagonals with modest padding: n * nd <= 1.5 nnz
-    if ((double)n > 1.5 * (double)A->nnz + 64.0) return CACG_OK;
+    if (!dia_padding_ok(1, n, A->nnz)) return CACG_OK;
     std::set<int64_t> offs;
     {
         unsigned long long *gtab = nullptr;
@@ -148,7 +188,7 @@ int DevMatrix::build_dia(const cacg_csr *A, bool want_f32, cudaStream_t st) {
     const int nd = (int)offs.size();
     if (nd == 0) return CACG_OK;
     // keep the view only when padding is modest
-    if ((double)nd * (double)n > 1.5 * (double)A->nnz + 64.0) return CACG_OK;
+    if (!dia_padding_ok(nd, n, A->nnz)) return CACG_OK;
     DiaDesc desc{};
     desc.ndiag = nd;
     int i = 0;

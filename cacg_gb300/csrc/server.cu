@@ -127,25 +127,6 @@ static bool batch_eligible(const cacg_params &p, int m) {
            (p.precision == CACG_FP64 || p.precision == CACG_MIXED) && p.maxit >= 0;
 }
 
-// Whether the nonzeros seem to lie on few diagonals (a DIA view): up to 256 rows
-// spread over the matrix hold at most kDiaMax distinct offsets.
-static bool looks_diagonal(const cacg_csr *A) {
-    int64_t offs[kDiaMax];
-    int cnt = 0;
-    const int64_t step = std::max<int64_t>(1, A->n / 256);
-    for (int64_t i = 0; i < A->n; i += step) {
-        for (int32_t e = A->row_ptr[i]; e < A->row_ptr[i + 1]; ++e) {
-            const int64_t o = (int64_t)A->col_idx[e] - i;
-            int j = 0;
-            while (j < cnt && offs[j] != o) ++j;
-            if (j < cnt) continue;
-            if (cnt == kDiaMax) return false;
-            offs[cnt++] = o;
-        }
-    }
-    return cnt > 0;
-}
-
 // FP64 requests of more rows than this leave the batched kernels (which do their
 // products on the FP64 pipe) for a stream worker, whose solver does them on the
 // tensor cores, if the caller has set no row limit and the matrix has diagonals
@@ -1076,9 +1057,11 @@ int cacg_server_submit(cacg_server *srv, const cacg_csr *A, const double *B, int
                solve_workspace_bytes(A->n, m, p->s, p->precision,
                                      p->bounds_mode == CACG_BOUNDS_LANCZOS, r->fix);
     };
+    int known = -1;  // the matrix will have a DIA view
+    auto view = [&]() { return (known < 0 ? known = dia_view_of(A) : known) != 0; };
     if (r->batched && s->cfg.batch_max_rows == 0 && p->precision == CACG_FP64 &&
         p->gram_variant == CACG_GRAM_AUTO && p->spmm_format != CACG_SPMM_CSR &&
-        A->n > kFp64BatchRows && looks_diagonal(A) &&
+        A->n > kFp64BatchRows && view() &&
         (int64_t)stream_cost() <= s->cfg.mem_budget_bytes)
         r->batched = false;
     r->cost = r->batched
@@ -1086,9 +1069,10 @@ int cacg_server_submit(cacg_server *srv, const cacg_csr *A, const double *B, int
                   : stream_cost();
     if ((int64_t)r->cost > s->cfg.mem_budget_bytes) return CACG_ERR_BUSY;
     // the fixed-point SpMM's scratch, where the budget has room for it
+    const int level = r->batched ? 0 : dia_fix_level(*p, A->nnz, m);
     double c;
-    if (!r->batched && looks_diagonal(A) && dia_fix_candidate(A, &c)) {
-        r->fix = dia_fix_level(*p, A->nnz, m);
+    if (level > 0 && view() && dia_fix_candidate(A, &c)) {
+        r->fix = level;
         const size_t with = stream_cost();
         if ((int64_t)with > s->cfg.mem_budget_bytes)
             r->fix = 0;

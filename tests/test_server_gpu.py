@@ -229,3 +229,33 @@ def test_server_at_the_budget_of_the_state(lib, slack):
     srv.close()
     assert info["status"] == 0
     assert O.port_true_relres(rp, ci, v, B, X).max() <= 1.01e-9
+
+
+@pytest.mark.parametrize("links,batched", [(0, False), (3, False), (40, True)])
+def test_fp64_requests_without_a_view_stay_batched(lib, links, batched):
+    """A grid with a few extra couplings: with a DIA view (five diagonals, or a few more) an
+    FP64 request takes the single-request solver, else it stays with the batched kernels."""
+    rp, ci, v = cg.gen_matrix("lap2d", 100, 0.5)
+    n = len(rp) - 1
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    D = {(int(r), int(c)): float(x) for r, c, x in zip(rows, ci, v)}
+    for k in range(links):  # between rows 1 .. 38, which few samples of the rows would meet
+        i, j = 1 + k % 30, 5000 + 41 * k
+        if links == 3:
+            j = i + 200  # one offset
+        D[(i, j)] = D[(j, i)] = -0.01
+        D[(i, i)] += 0.01
+        D[(j, j)] += 0.01
+    keys = sorted(D)
+    rp = np.searchsorted([r for r, _ in keys], np.arange(n + 1)).astype(np.int32)
+    ci = np.array([c for _, c in keys], np.int32)
+    v = np.array([D[k] for k in keys])
+    view = cg.Matrix(rp, ci, v).diagonals() > 0
+    assert view == (not batched)
+    B = cg.gen_rhs("normal", n, 3, 5)
+    srv = cg.Server(mem_budget_bytes=1 << 30, max_active=1)
+    X, info = srv.wait(srv.submit(rp, ci, v, B, cg.Params(s=4, tol=1e-8, maxit=300)))
+    steps = srv.engine_stats()["steps"]
+    srv.close()
+    assert info["status"] == 0 and (steps > 0) == batched
+    assert O.port_true_relres(rp, ci, v, B, X).max() <= 1.01e-8
