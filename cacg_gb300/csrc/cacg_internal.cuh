@@ -203,6 +203,8 @@ int launch_gram(cudaStream_t st, int variant, int64_t n, const T *L, int64_t ldl
                 double *C1, int ldc1, double *C2, int ldc2, double *ws, size_t ws_bytes,
                 bool symmetric = false, struct ColExps *ce = nullptr, bool normwise = false);
 size_t gram_workspace_bytes(int64_t n, int ka, int kb);
+// poll limit of the tensor-core kernels' pipeline waits (cacg_set_pipeline_wait_limit)
+long long pipeline_wait_limit();
 // FP64 Gram from fp16 digit planes on tcgen05 (k_gram_x64.cu); launch_gram takes
 // it for CACG_GRAM_AUTO.  symmetric: L^T R1 is (its upper triangle counts); normwise:
 // accurate to the columns' norms, not to |L|^T |R|.  CACG_ERR_UNSUPPORTED: shape or

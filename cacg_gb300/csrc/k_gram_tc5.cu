@@ -704,10 +704,12 @@ __global__ void __launch_bounds__(t5w_threads(NC8), 1)
     }
 }
 
-// Poll limit of the warp-specialised Gram's pipeline waits (the drain waits
+// Poll limit of the pipeline waits of the warp-specialised Gram, the digit-plane
+// Gram and the tall x small products from digit planes (the drain waits
 // keep kT5SpinLimit): cacg_set_pipeline_wait_limit shortens it so a test can
 // make those waits run out.
 static std::atomic<long long> g_pipe_polls{kT5SpinLimit};
+long long pipeline_wait_limit() { return g_pipe_polls.load(); }
 
 struct T5Plan {
     int BA, BB, tilesA, tilesB, nchunks, tmem_half;

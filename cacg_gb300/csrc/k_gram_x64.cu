@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     gram_x64_kernel(int64_t n, int64_t rows_per_chunk, XgOperands o, int BA, int tilesB, int sub,
                     int stages, bool scan, int sym, int line, uint32_t *__restrict__ emax,
                     const unsigned long long *__restrict__ elog, double *__restrict__ part,
-                    int *__restrict__ flags) {
+                    int *__restrict__ flags, long long polls) {
     constexpr int NB = 16 * NC;
     constexpr int NQ = NB / 4;  // accumulator columns per converter thread
     constexpr unsigned lbo_a = (kXgM / 8) * 128, lbo_b = (kXPlanes * NB / 8) * 128;
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
         };
         auto fold = [&](int64_t g) {
             const bool okg = __all_sync(
-                0xffffffffu, t5_mbar_wait_or_abort(gdone, (unsigned)(g & 1), abort_flag));
+                0xffffffffu, t5_mbar_wait_or_abort(gdone, (unsigned)(g & 1), abort_flag, polls));
             if (!okg) return false;
             t5_fence_after();
             const unsigned ta = tmem + ((unsigned)(32 * quad) << 16) + (unsigned)(quarter * NQ);
@@ -526,7 +526,8 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             const int b = (int)(j & 1);
             if (j >= 2) {
                 const bool w =
-                    t5_mbar_wait_or_abort(&sfree[b], (unsigned)(((j >> 1) - 1) & 1), abort_flag);
+                    t5_mbar_wait_or_abort(&sfree[b], (unsigned)(((j >> 1) - 1) & 1), abort_flag,
+                                          polls);
                 if (!__all_sync(0xffffffffu, w)) {
                     ok = false;
                     break;
@@ -579,9 +580,9 @@ __global__ void __launch_bounds__(kXgThreads, 1)
             const int b = (int)(j & 1);
             const int64_t g = j / kXgGroup;
             const bool w =
-                t5_mbar_wait_or_abort(&sfull[b], (unsigned)((j >> 1) & 1), abort_flag) &&
+                t5_mbar_wait_or_abort(&sfull[b], (unsigned)((j >> 1) & 1), abort_flag, polls) &&
                 (j % kXgGroup != 0 || g < 1 ||
-                 t5_mbar_wait_or_abort(gfree, (unsigned)((g - 1) & 1), abort_flag));
+                 t5_mbar_wait_or_abort(gfree, (unsigned)((g - 1) & 1), abort_flag, polls));
             if (!__all_sync(0xffffffffu, w)) {
                 if (lane == 0) *abort_flag = 1;
                 break;
@@ -775,7 +776,8 @@ static void xg_launch(dim3 grid, const XgPlan &p, cudaStream_t st, int64_t n, co
                       int *flags) {
     set_smem_attr(gram_x64_kernel<NC, VEC>, (int)max_smem_optin());
     gram_x64_kernel<NC, VEC><<<grid, kXgThreads, p.smem, st>>>(
-        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan, sym, line, emax, elog, part, flags);
+        n, p.rows_per_chunk, o, p.BA, p.tilesB, p.sub, p.stages, p.scan, sym, line, emax, elog, part, flags,
+        pipeline_wait_limit());
 }
 
 int launch_gram_x64(cudaStream_t st, int64_t n, const double *L, int64_t ldl, int ka,

@@ -82,6 +82,7 @@ struct XtArgs {
     int64_t ldo;
     double *X, *R, *S0;  // kXtXR (S0 may be NULL)
     int64_t lds;
+    long long polls;  // limit of the pipeline's waits
     double *part;  // kXtXR: gridDim.x x N sums of squares of the new R (may be NULL)
     int *status;
 };
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
             if (job >= 2) {
                 ok = __all_sync(0xffffffffu, t5_mbar_wait_or_abort(
                                                  &tfree[x], (unsigned)(((job >> 1) - 1) & 1),
-                                                 abort_flag));
+                                                 abort_flag, g.polls));
                 if (!ok) break;
             }
             const bool more = job + 1 < njobs;
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
                 if (step >= 2) {
                     ok = __all_sync(0xffffffffu, t5_mbar_wait_or_abort(
                                                      &sfree[b], (unsigned)(((step >> 1) - 1) & 1),
-                                                     abort_flag));
+                                                     abort_flag, g.polls));
                     if (!ok) break;
                 }
                 int fc[8];
@@ -432,8 +433,8 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
                     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(
                         reinterpret_cast<const char *>(src) + b));
             ok = __all_sync(0xffffffffu,
-                            t5_mbar_wait_or_abort(&rfull[x], ph, abort_flag) &&
-                                t5_mbar_wait_or_abort(&tdone[x], ph, abort_flag));
+                            t5_mbar_wait_or_abort(&rfull[x], ph, abort_flag, g.polls) &&
+                                t5_mbar_wait_or_abort(&tdone[x], ph, abort_flag, g.polls));
             if (!ok) break;
             t5_fence_after();
             const int re = rowE[x * kXtM + rt], E = re & (kXtFar - 1);
@@ -556,16 +557,18 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
             const int x = (int)(job & 1);
             // the accumulator set's previous tile has been read
             if (kBufs == 2 && job >= 2)
-                ok = t5_mbar_wait_or_abort(&tfree[x], (unsigned)(((job >> 1) - 1) & 1), abort_flag);
+                ok = t5_mbar_wait_or_abort(&tfree[x], (unsigned)(((job >> 1) - 1) & 1), abort_flag,
+                                           g.polls);
             if (kBufs == 1 && job >= 1)
                 ok = t5_mbar_wait_or_abort(&tfree[x ^ 1], (unsigned)(((job - 1) >> 1) & 1),
-                                           abort_flag);
+                                           abort_flag, g.polls);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             for (int ch = 0; ch < nchunk; ++ch, ++step) {
                 const int b = (int)(step & 1);
                 ok = __all_sync(0xffffffffu, t5_mbar_wait_or_abort(
-                                                 &sfull[b], (unsigned)((step >> 1) & 1), abort_flag));
+                                                 &sfull[b], (unsigned)((step >> 1) & 1), abort_flag,
+                                                 g.polls));
                 if (!ok) break;
                 t5_fence_after();
                 const unsigned abase = t5_smem_u32(smem_raw + b * kXtABytes);
@@ -602,8 +605,11 @@ __global__ void __launch_bounds__(xt_threads(kXtConvWarps), 1) tsm_x64_kernel(Xt
             }
         }
         if (!ok && lane == 0) *abort_flag = 1;
-        // every committed MMA finishes before tensor memory goes (bounded)
+        // every committed MMA finishes before tensor memory goes, and every commit's
+        // arrival lands before the barriers do (bounded)
         if (last >= 0) t5_mbar_wait(&sfree[last & 1], (unsigned)((last >> 1) & 1));
+        const int done = (last + 1) / nchunk - 1;  // the last job whose last chunk was issued
+        if (done >= 0) t5_mbar_wait(&tdone[done & 1], (unsigned)((done >> 1) & 1));
     }
     t5_fence_before();
     const int gave_up = __syncthreads_or(*abort_flag);
@@ -640,6 +646,7 @@ template <int MODE>
 static int xt_launch(cudaStream_t st, XtArgs g, int *blocks = nullptr) {
     if (g.n <= 0) return CACG_OK;
     if (g.K <= 0 || g.K > kXtMaxK || g.N <= 0 || !g.e0) return CACG_ERR_UNSUPPORTED;
+    g.polls = pipeline_wait_limit();
     const int maxsm = (int)max_smem_optin();
     int tn = (g.N + 63) / 64, NB;
     for (;; ++tn) {

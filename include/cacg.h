@@ -271,8 +271,9 @@ int cacg_k_gram_noalloc(int32_t vtype, int32_t variant, int64_t n, const void *L
 /* No counterpart in the reference.  Every wait of the tcgen05 kernels on an
  * mbarrier is bounded; on expiry the kernel drains its own copies and MMAs in
  * flight, frees its tensor memory, sets a status word and returns, and the
- * solver reports CACG_ERR_TIMEOUT.  This sets the poll limit of the tcgen05
- * Gram's pipeline waits (process-wide; polls < 0 restores the default of
+ * solver reports CACG_ERR_TIMEOUT.  This sets the poll limit of the tensor-core
+ * kernels' pipeline waits (Gram of both precisions, FP64 updates and QR
+ * products; process-wide; polls < 0 restores the default of
  * 2^22) so that a test can make them run out; the drain waits keep the full
  * bound. */
 int cacg_set_pipeline_wait_limit(int64_t polls);

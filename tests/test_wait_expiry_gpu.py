@@ -63,3 +63,47 @@ def test_solve_reports_timeout_and_next_solve_is_unchanged(lib, torch_cuda):
     X1, i1 = cg.solve(rp, ci, v, B, **kw)
     assert i1["status"] == 0 and i1["iterations"] == i0["iterations"]
     assert np.array_equal(X0, X1)
+
+
+@pytest.mark.parametrize("n,k", [(5000, 48), (400, 20), (300, 128)])
+def test_qr_wait_expiry_then_recovery(lib, torch_cuda, n, k):
+    """The digit-plane products' waits run out: CACG_ERR_TIMEOUT, not the breakdown that the
+    second pass meets in the first one's incomplete result.  (The digit-plane Gram recovers by
+    itself: its reduction recomputes the outputs.)"""
+    torch = torch_cuda
+    V = dev(torch, O.gen_rhs("normal", n, k, 1))
+
+    def qr():
+        Q, R = torch.full_like(V, 7.0), torch.zeros(k, k, dtype=torch.float64, device="cuda")
+        rc = lib.cacg_k_tsqr(n, k, ptr(V), k, ptr(Q), k, ptr(R), None)
+        return rc, host(Q), host(R)
+
+    rc0, Q0, R0 = qr()
+    assert rc0 == 0
+    lib.cacg_set_pipeline_wait_limit(0)
+    try:
+        rc1, _, _ = qr()
+    finally:
+        lib.cacg_set_pipeline_wait_limit(-1)
+    assert rc1 == -5  # CACG_ERR_TIMEOUT
+    rc2, Q2, R2 = qr()
+    assert rc2 == 0 and np.array_equal(Q0, Q2) and np.array_equal(R0, R2)
+
+
+@pytest.mark.parametrize("n,ka,kb", [(5000, 48, 64), (300, 20, 24), (2000, 130, 70)])
+def test_fp64_gram_wait_expiry_is_recomputed(lib, torch_cuda, n, ka, kb):
+    """A chain of FP64 FMAs and sixteen partial sums: (n + 16) u of |L|^T |R|, u = 2^-53."""
+    torch = torch_cuda
+    L, R = O.gen_rhs("normal", n, ka, 1), O.gen_rhs("normal", n, kb, 2)
+    dL, dR = dev(torch, L), dev(torch, R)
+    Cm = torch.zeros((ka, kb), dtype=torch.float64, device="cuda")
+    lib.cacg_set_pipeline_wait_limit(0)
+    try:
+        rc = lib.cacg_k_gram(0, 0, n, ptr(dL), ka, ka, ptr(dR), kb, kb, None, 0, 0, ptr(Cm), kb,
+                             None)
+        C = host(Cm)
+    finally:
+        lib.cacg_set_pipeline_wait_limit(-1)
+    assert rc == 0
+    ref = L.astype(np.longdouble).T @ R.astype(np.longdouble)
+    assert np.all(np.abs(C - ref) <= (n + 16) * 2.0 ** -53 * (np.abs(L).T @ np.abs(R)))
