@@ -23,8 +23,8 @@ constexpr int kQrThreads = 256;
 constexpr int kCholThreads = 512;
 
 // One CTA: R = chol(G) (upper, G = R^T R) and Rinv = R^{-1}, both k x k
-// row-major with zeros below the diagonal.  *bad set on a pivot that is not
-// positive and finite.
+// row-major with zeros below the diagonal.  *bad gets kStatusBreakdown on a pivot that
+// is not positive and finite (beside a kStatusTimeout of the product before).
 //
 // G = L D L^T by right-looking elimination with the same row operations applied
 // to the identity, whose rows (L^{-1}) take the space below the diagonal: R =
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kCholThreads)
             if (l > j && l < k) t[l] = ok ? aj[l] / piv : 0.0;
             if (tid == 0) {
                 sq[j] = ok ? piv : 0.0;
-                if (!ok) *bad = 1;
+                if (!ok) atomicOr(bad, kStatusBreakdown);
             }
         }
         __syncthreads();
