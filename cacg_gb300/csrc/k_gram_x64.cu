@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(kXgThreads, 1)
     };
     int lacks = 0;
     if (!scan) {
+        __syncthreads();  // spread is 0 before anyone's bits go in
         if (tid < BA + NB) {
             const int c = tid < BA ? (a0 + tid < o.ka ? a0 + tid : -1)
                                    : (b0 + tid - BA < kb ? o.ka + b0 + tid - BA : -1);
