@@ -9,17 +9,17 @@
 //   G = V^T V,  R1 = chol(G) (upper),  Q1 = V R1^{-1},
 //   G2 = Q1^T Q1, R2 = chol(G2),       Q  = Q1 R2^{-1},   R = R2 R1,
 // which is orthogonal to working accuracy while the 2-norm condition number
-// of V stays below about u^{-1/2} (1e8); the Gram products and the tall x small
-// ones are the library's FP64 kernels (digit planes on the tensor cores, FMAs at
-// the sizes those do not take), the small Cholesky factors and triangular
-// inverses run in one CTA.  A Cholesky pivot that is not positive and finite
-// (V numerically rank-deficient) returns CACG_ERR_BREAKDOWN.
+// of V, its columns scaled to one norm, stays below about u^{-1/2} (1e8; the
+// columns' own magnitudes do not count).  The Gram products are the library's
+// (FP64 FMAs for few columns or rows, else digit planes on the tensor cores), the
+// tall x small ones go by digit planes at every size, and the small Cholesky
+// factors and triangular inverses run in one CTA.  A Cholesky pivot that is not
+// positive and finite (V numerically rank-deficient) returns CACG_ERR_BREAKDOWN.
 #include "cacg_internal.cuh"
 
 namespace cacg {
 
 constexpr int kQrMaxK = 128;
-constexpr int kQrThreads = 256;
 constexpr int kCholThreads = 512;
 
 // One CTA: R = chol(G) (upper, G = R^T R) and Rinv = R^{-1}, both k x k
@@ -84,26 +84,6 @@ __global__ void __launch_bounds__(kCholThreads)
     }
 }
 
-// Y = X W with W k x k upper triangular (row-major, in shared memory):
-// Y[r][c] = sum_{j <= c} X[r][j] W[j][c], one thread per output.
-__global__ void __launch_bounds__(kQrThreads)
-    tallsmall_triu_kernel(int64_t n, int k, const double *__restrict__ X, int64_t ldx,
-                          const double *__restrict__ W, double *__restrict__ Y, int64_t ldy) {
-    extern __shared__ __align__(16) double ts_sm[];
-    for (int i = threadIdx.x; i < k * k; i += blockDim.x) ts_sm[i] = W[i];
-    __syncthreads();
-    const int64_t total = n * (int64_t)k;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = e / k;
-        const int c = (int)(e - r * k);
-        const double *x = X + r * ldx;
-        double s = 0.0;
-        for (int j = 0; j <= c; ++j) s = fma(x[j], ts_sm[j * k + c], s);
-        Y[r * ldy + c] = s;
-    }
-}
-
 // R = A B for upper triangular k x k A, B: a CTA a row, an output a thread (one
 // CTA for all rows: 26 us at k = 48, 294 at 128)
 __global__ void triu_mul_kernel(int k, const double *__restrict__ A, const double *__restrict__ B,
@@ -123,19 +103,6 @@ static int chol_inv(cudaStream_t st, int k, const double *G, double *R, double *
     const int smem = (int)((size_t)k * k * sizeof(double));
     set_smem_attr(chol_inv_kernel, kQrSmemMax);
     chol_inv_kernel<<<1, kCholThreads, smem, st>>>(k, G, R, Rinv, bad);
-    return check_launch();
-}
-
-static int tallsmall_triu(cudaStream_t st, int64_t n, int k, const double *X, int64_t ldx,
-                          const int *xexp, const double *W, double *Y, int64_t ldy, int *status) {
-    if (n <= 0) return CACG_OK;
-    const int rc = launch_tallsmall_x64(st, n, k, k, X, ldx, xexp, W, k, Y, ldy, status);
-    if (rc != CACG_ERR_UNSUPPORTED) return rc;
-    const int smem = (int)((size_t)k * k * sizeof(double));
-    set_smem_attr(tallsmall_triu_kernel, kQrSmemMax);
-    const int64_t blocks = std::min<int64_t>((n * k + kQrThreads - 1) / kQrThreads,
-                                             (int64_t)sm_count() * 4);
-    tallsmall_triu_kernel<<<(unsigned)blocks, kQrThreads, smem, st>>>(n, k, X, ldx, W, Y, ldy);
     return check_launch();
 }
 
@@ -175,11 +142,11 @@ extern "C" int cacg_k_tsqr(int64_t n, int32_t k, const double *V, int64_t ldv, d
     // pass 1: G = V^T V, R1, Q1 = V R1^{-1}
     if (rc == CACG_OK) rc = gram(V, ldv);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R1, R1i, bad);
-    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, V, ldv, exps, R1i, Q1, k, bad);
+    if (rc == CACG_OK) rc = launch_tallsmall_x64(st, n, k, k, V, ldv, exps, R1i, k, Q1, k, bad);
     // pass 2: G2 = Q1^T Q1, R2, Q = Q1 R2^{-1}
     if (rc == CACG_OK) rc = gram(Q1, k);
     if (rc == CACG_OK) rc = chol_inv(st, k, G, R2, R2i, bad);
-    if (rc == CACG_OK) rc = tallsmall_triu(st, n, k, Q1, k, exps, R2i, Q, ldq, bad);
+    if (rc == CACG_OK) rc = launch_tallsmall_x64(st, n, k, k, Q1, k, exps, R2i, k, Q, ldq, bad);
     if (rc == CACG_OK) {
         triu_mul_kernel<<<k, kQrMaxK, 0, st>>>(k, R2, R1, R);
         rc = check_launch();
