@@ -543,9 +543,8 @@ def run_serving(args):
 # DRAM bytes (read + write) per call of each phase (one Gram product = the
 # tcgen05 split-K kernel and its reduction; one X/R update = the update and
 # its norm sum), from one ncu capture of the 27-point 96^3 mixed solve
-# (n = 884,736; per-kernel table with the command in
-# profiles/ncu_traffic_st27_96_m16.md); every figure is linear in n at fixed
-# m and s.
+# (n = 884,736; the per-kernel table is among the profiles); every figure is
+# linear in n at fixed m and s.
 TRAFFIC_96 = {"basis_spmm": 297.8e6, "aq_spmm": 732.9e6, "qupdate": 963.5e6,
               "xrupdate": 1210.7e6, "gram": (679.7e6 + 739.7e6) / 2 + 12.2e6}
 TRAFFIC_96_N = 884736

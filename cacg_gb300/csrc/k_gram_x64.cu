@@ -763,10 +763,11 @@ size_t gram_x64_workspace_bytes(int64_t n, int ka, int kb) {
     return std::max(b, plan_x64(n, ka, kb).total);
 }
 
-// n < 256: an FMA chain of so few rows rounds less than the planes drop.  Above,
-// this kernel is the faster one for every width: measured through cacg_k_gram at
-// n = 1369 / 16384 / 884736, k = 4 (+1): 45 / 51 / 217 us against 100 / 102 /
-// 1843 us of the FMA kernel; k = 96 (+16): 60 / 80 / 1207 against 240 / 428 / 15862.
+// n < 256: an FMA chain of so few rows rounds less than the planes drop.  Above, for
+// the columns that gram_tiny_kernel leaves, this kernel is the faster one but for a
+// tie at the fewest: through cacg_k_gram (some 15 us of it the call), planes and FMAs,
+// n = 1369 / 16384 / 884736: 20 x 25 26 / 38 / 383 us against 24 / 39 / 870; 32 x 40
+// 30 / 40 / 414 against 37 / 63 / 1975; 96 x 112 42 / 69 / 1088 against 194 / 382 / 15816.
 bool gram_x64_supported(int64_t n, int ka, int kb) {
     return n >= 256 && ka > 0 && kb > 0 && ka <= 256 && kb <= 512;
 }

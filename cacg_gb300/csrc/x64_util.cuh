@@ -13,8 +13,11 @@
 // 6 - p; the 28 plane products with p + q <= 6 are kept (the dropped ones are
 // below 2^-56 of the largest product), accumulated per p + q.  So each sum is
 // exact up to the rounding of X at 2^-55 of its vector's largest element and
-// the dropped products: tighter than an FP64 FMA chain, which rounds every
-// partial sum.
+// the dropped products.  That error goes with the largest elements of the two
+// vectors, an FMA chain's with the elements that are multiplied: for vectors of even
+// magnitude it is the smaller one, for graded ones it need not be.  Each kernel
+// says what keeps it there: k_gram_x64.cu a line beyond which a chunk takes FMAs,
+// k_tsm_x64.cu an exponent per column of the tall operand.
 #pragma once
 
 #include <cuda_fp16.h>

@@ -50,12 +50,21 @@ extern "C" {
 #define CACG_TOL_ABS_COL0 0 /* reference: ||R(:,0)|| < tol (src/bcbcgKernel.c:524) */
 #define CACG_TOL_REL_ALL 1  /* max_c ||b_c - A x_c|| / ||b_c|| <= tol (true residual) */
 
-#define CACG_FP64 0  /* FP64 throughout: FMAs, or sums no less accurate (exact digit
-                        planes on the tensor cores, fixed point) over a DIA view */
+#define CACG_FP64 0  /* FP64 in and out.  Products by FP64 FMAs; over a DIA view also
+                        as exact integer sums (digit planes on the tensor cores, fixed
+                        point) of operands held to 55 bits and more of a largest
+                        element: of a column (Gram chunk, SpMM) or a row whose columns
+                        are scaled by their norms (updates).  Errors are normwise
+                        those of FMAs; columns' magnitudes do not count */
 #define CACG_MIXED 1 /* FP32 basis/SpMM/updates, FP64 Gram accumulation, LU, X, R,
                         FP64 residual replacement */
 
-#define CACG_GRAM_AUTO 0
+#define CACG_GRAM_AUTO 0 /* FP64: digit planes on the tensor cores where they are
+                            accurate to |L|^T |R| as FMAs are (row chunks whose elements
+                            spread further take FMAs), FMAs for few columns or rows.
+                            In a solve the planes' error is to ||L_a|| ||R_b||.
+                            FP32: in a solve CACG_GRAM_TC5, or CACG_GRAM_TC for shapes
+                            it does not take; in cacg_k_gram the CUDA cores */
 #define CACG_GRAM_FMA 1  /* FP64 FMA pipe */
 #define CACG_GRAM_DMMA 2 /* FP64 tensor core (mma.sync m8n8k4 f64) */
 #define CACG_GRAM_TC 3   /* FP32 inputs on the bf16 tensor cores: three bf16 slices
