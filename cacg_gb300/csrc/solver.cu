@@ -572,11 +572,26 @@ static void tridiag_extremes(const std::vector<double> &a, const std::vector<dou
     *hi = kth(k - 1);
 }
 
-// FP64 multiply-adds (n k k, n k m) from which the digit-plane updates are the
-// faster ones: below, the FMA kernels' work is less than the planes' set-up.
-// Q: n = 16384, k = 4 14.1 us FMA, 14.5 planes; n = 32768, k = 16 24 and 14.
-// X / R: n = 32768, k = 16, m = 4 31 and 33; n = 50653, k = 20, m = 5 51 and 49.
+// Where the digit-plane updates are the faster ones.  Their time goes with the columns
+// that are split and put out, the FMAs' with the products: below some columns they
+// do not pay for any n (us an outer iteration, FMAs / planes, the column exponents
+// included; n = 262144 and 1e6):
+//   Q    k = 4 220 / 256, 432 / 527; k = 8 319 / 332, 807 / 831; k = 9 509 / 404,
+//        1612 / 1139; k = 12 456 / 421, 1340 / 1214
+//   X/R  m = 1, k = 48 1819 / 1899, 5761 / 6052; m = 2, k = 40 1156 / 1202, 3498 / 3646;
+//        m = 4, k = 16 482 / 505, 1434 / 1496; m = 4, k = 32 829 / 802, 2523 / 2408;
+//        m = 5, k = 20 639 / 639, 1957 / 1954; m = 8, k = 16 522 / 479, 1550 / 1399
+// and above, some products have to be there for their set-up (n k k, n k m).
+// Q: n = 8000, k = 12 129 / 133, k = 16 155 / 150; n = 27000, k = 9 167 / 164.
+// X/R: n = 27000, k = 20, m = 5 and k = 16, m = 8 no difference.
 constexpr double kPlanesQMin = 2e6, kPlanesXrMin = 4e6;
+constexpr int kPlanesQMinK = 9, kPlanesXrMinM = 4, kPlanesXrMinKM = 100;
+static bool planes_q(int64_t n, int k) {
+    return k >= kPlanesQMinK && (double)n * k * k >= kPlanesQMin;
+}
+static bool planes_xr(int64_t n, int k, int m) {
+    return m >= kPlanesXrMinM && k * m >= kPlanesXrMinKM && (double)n * k * m >= kPlanesXrMin;
+}
 
 struct Solver {
     const DevMatrix *A;
@@ -842,7 +857,7 @@ struct Solver {
                 }
             } else {
                 rc = CACG_ERR_UNSUPPORTED;
-                if (planes64() && (double)n * k * k >= kPlanesQMin) {
+                if (planes64() && planes_q(n, k)) {
                     rc = need_exps((const double *)b.Q, nullptr);
                     if (rc == CACG_OK)
                         rc = launch_qupdate_x64(st, n, k, (T *)b.S, k, (const T *)b.Q, k, b.qexp,
@@ -998,7 +1013,7 @@ struct Solver {
             }
         }
         if constexpr (std::is_same<T, double>::value) {
-            if (planes64() && (double)A->n * k * m >= kPlanesXrMin) {
+            if (planes64() && planes_xr(A->n, k, m)) {
                 int rc = need_exps(Q, AQ);
                 if (rc == CACG_OK)
                     rc = launch_xrupdate_x64(st, A->n, k, m, Q, AQ, k, b.qexp, b.aqexp, b.alpha, X,

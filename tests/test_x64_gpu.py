@@ -235,3 +235,19 @@ def test_qr_small_factor_edges(torch_cuda, k, scale):
     assert float((Q.T @ Q - eye).norm()) <= u * k ** 0.5
     assert float((Q @ (R / scale) - V / scale).norm()) <= u * float((V / scale).norm())
     assert bool((torch.tril(R, -1) == 0).all()) and bool((torch.diagonal(R) > 0).all())
+
+
+@pytest.mark.parametrize("kind,N,m,s", [("lap2d", 400, 2, 4), ("lap2d", 400, 3, 3), ("lap2d", 400, 4, 4),
+                                        ("lap2d", 400, 4, 7), ("lap2d", 400, 3, 9), ("lap3d7", 37, 5, 4),
+                                        ("lap3d7", 37, 1, 8), ("lap3d7", 37, 1, 10)])
+def test_solves_around_the_updates_columns(kind, N, m, s):
+    """Either side of the columns from which the updates take digit planes (k = 8 and 9; m = 3
+    and 4, k m = 64, 100 and 112): the FMA kernels' iterations, and X to what two solutions of
+    residual 1e-10 may differ by (a condition number of at most hi / lo)."""
+    rp, ci, v = cg.gen_matrix(kind, N, 0.1)
+    B = cg.gen_rhs("normal", len(rp) - 1, m, 11)
+    lo, hi = 0.1, 8.1 if kind == "lap2d" else 12.1
+    p = dict(s=s, bounds=("given", lo, hi), tol=1e-10, maxit=500)
+    (X1, i1), (X2, i2) = (cg.solve(rp, ci, v, B, gram=g, **p) for g in ("auto", "fma"))
+    assert i1["status"] == 0 and i2["status"] == 0 and abs(i1["iterations"] - i2["iterations"]) <= 1
+    assert np.all(np.linalg.norm(X1 - X2, axis=0) <= 2e-10 * (hi / lo) * np.linalg.norm(X2, axis=0))
