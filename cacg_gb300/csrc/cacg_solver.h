@@ -92,7 +92,7 @@ int launch_dia_wide(cudaStream_t st, const DevMatrix *A, int w, const float *X, 
 // and below kDiaFixMin products (nnz w): three launches then cost more than the
 // FMAs.  7-point n = 50653, w = 20 (7.0e6): 31.6 us against 28.4 us of the FMA
 // kernel; n = 262144, w = 8 (14.5e6): 42.8 against 46.4, w = 64: 210 against 316;
-// 27-point n = 884736, w = 16: 230 against 747, w = 96: 1471 against 4630.
+// 27-point n = 884736, w = 16: 235 against 747, w = 96: 1497 against 4630.
 constexpr double kDiaFixMin = 1e7;
 // chain: calls of which each takes the Y of the one before as its X, with the
 // same scratch and nothing between that writes either: the column maxima of X
